@@ -43,14 +43,27 @@ constexpr int kCxrThreads = 256;  // two resident blocks per SM (128 registers e
 // Reflection rows per pass: 120 on the float path (a pass's prefilter
 // survivors then fill the block's threads about twice, with a smaller idle
 // tail than at 64 rows, measured 10 % faster on the control variate's
-// sub-sample), 64 on the FP64 path, whose staged tables need the room.
+// sub-sample), 48 on the FP64 path, whose staged tables need the room.
 template <class Real>
-constexpr int row_chunk() { return sizeof(Real) == 4 ? 120 : 64; }
+constexpr int row_chunk() { return sizeof(Real) == 4 ? 120 : 48; }
 template <class Real>
 constexpr int pair_queue() { return kSegTile * row_chunk<Real>(); }  // every pair of a pass may keep a line
-constexpr int kXQueue = 2048;   // queued exact-window bins per class and pass
+// Kept lines wait here until a whole round of kCxrThreads is there.
+template <class Real>
+constexpr int line_queue() { return pair_queue<Real>() + kCxrThreads; }
+constexpr int kStripBins = 31;  // bins a warp owns in the whole-axis phase (32 edges)
+// Window lines collected before the window phase runs; one more round of
+// kCxrThreads lines always fits.
+constexpr int kWideCap = 2 * kCxrThreads;
+constexpr int kWideRun = kWideCap - kCxrThreads;
+// Classes of window lines: 4, 8, 16 or 32 lanes a line (two edges a lane), or
+// the block's warps together over strips of the axis (kWinStrip: windows of more
+// than kStripSpan bins a side; kWinAxis: no moments, every bin).
+enum WinClass { kWin4 = 0, kWin8, kWin16, kWin32, kWinStrip, kWinAxis, kWinClasses };
+constexpr int kStripSpan = 124;
+// Strip lines wait for one another over several window phases.
+constexpr int kStripRun = kCxrThreads / 2;
 constexpr int kMaxTab = 4096;   // E_tab / delta staged in shared memory up to this size
-constexpr int kMaxMu = 4;
 
 // Math of the line chain. FP64 uses IEEE operations throughout (parity with
 // the reference's FP64 chain); the float path uses the SFU approximations
@@ -179,6 +192,28 @@ __device__ __forceinline__ void bracket(const Real *grid, int n, Real x, int &id
     frac = rdiv(x - grid[i - 1], grid[i] - grid[i - 1]);
     below = x <= grid[0];
     above = x >= grid[n - 1];
+}
+
+// A bracket kept with its cell's bounds: the passes of one pair move the
+// energy by parts in 1e5, so most land in the cell already found and cost a
+// comparison instead of a search (the same index and fraction either way).
+template <class Real>
+struct Cell {
+    Real x0, x1, frac;
+    int idx;
+    bool below, above;
+};
+
+template <class Real>
+__device__ __forceinline__ void locate(Cell<Real> &c, const Real *grid, int n, Real x, const TabIndex &ti) {
+    if (x > c.x0 && x < c.x1) {
+        c.frac = rdiv(x - c.x0, c.x1 - c.x0);
+        c.below = c.above = false;
+    } else {
+        bracket<Real>(grid, n, x, c.idx, c.frac, c.below, c.above, ti);
+        c.x0 = grid[c.idx - 1];
+        c.x1 = grid[c.idx];
+    }
 }
 
 template <class Real, class T>
@@ -355,6 +390,7 @@ struct PairAmps {
 template <class Real>
 struct Resonance {
     Real delta, denom;
+    Cell<Real> cell;
     bool keep;
 };
 
@@ -373,13 +409,12 @@ __device__ __forceinline__ Resonance<Real> pair_resonance(const SegPre<Real> &sp
     const Real denom_vac = sp.denom_row + r_den;
     // cxr/_kernels.py:702-765
     Real denom = denom_vac, previous = denom, delta = (Real)NAN;
+    Cell<Real> cell;
+    cell.x0 = cell.x1 = (Real)0;
     for (int pass = 0; pass < 3; ++pass) {
         const Real Er = hbarc * rdiv(v_dot_g_exact, denom);
-        int ix;
-        Real fr;
-        bool bl, ab;
-        bracket<Real>(E_tab, n_tab, Er, ix, fr, bl, ab, ti);
-        delta = gather<Real>(delta_tab, n_tab, ix, fr, bl, ab);
+        locate<Real>(cell, E_tab, n_tab, Er, ti);
+        delta = gather<Real>(delta_tab, n_tab, cell.idx, cell.frac, cell.below, cell.above);
         previous = denom;
         denom = denom_vac - delta * sp.v_dot_grad;
     }
@@ -390,18 +425,18 @@ __device__ __forceinline__ Resonance<Real> pair_resonance(const SegPre<Real> &sp
     const Real E_res = hbarc * omega;
     bool keep = sp.radiates && (E_res > (Real)t.lo_keep) && (E_res > (Real)10) && (E_res < (Real)t.hi_keep);
     keep = keep && (denom > (Real)0) && (omega * sp.inv_E <= (Real)1 - rdiv((Real)1, sp.gamma));
-    return Resonance<Real>{delta, denom, keep};
+    return Resonance<Real>{delta, denom, cell, keep};
 }
 
 // The rest of the chain from the resonance: the line's slope, the attenuation
-// at the line energy and the complex amplitudes. The float path stops after
-// the resonance for dropped pairs; FP64 completes every pair so its per-pair
-// output matches the reference's arrays.
+// at the line energy and the complex amplitudes. The chain stops after the
+// resonance for dropped pairs, unless ``all_pairs`` asks for the values of every
+// pair (FP64 with per-pair output, which matches the reference's arrays).
 template <class Real, bool kLayered>
 __device__ __forceinline__ PairAmps<Real> pair_amps_from(const SegPre<Real> &sp, const RowPre<Real> &rw,
                                                          const Resonance<Real> &res, const Real *E_tab,
                                                          const Real *log_mu, int n_tab, int n_mu,
-                                                         const pb_cxr_tables &t, const TabIndex &ti) {
+                                                         const pb_cxr_tables &t, const TabIndex &ti, bool all_pairs) {
     const Real Gx = rw.G[0], Gy = rw.G[1], Gz = rw.G[2];
     const Real g2 = rw.g2, n_dot_g = rw.n_dot_g;
     const Real hbarc = (Real)kHbarcEvAng;
@@ -429,16 +464,15 @@ __device__ __forceinline__ PairAmps<Real> pair_amps_from(const SegPre<Real> &sp,
     // cxr/_block_prologue.py:53-62, cxr/_recoil.py:100-118
     o.slope = denom * rdiv((Real)1, (Real)1 - omega * sp.inv_E);
     o.keep = res.keep;
-    if constexpr (sizeof(Real) == 4) {
-        if (!res.keep) return o;
-    }
-    int ix;
-    Real fr;
-    bool bl, ab;
-    bracket<Real>(E_tab, n_tab, E_res, ix, fr, bl, ab, ti);
+    if (!res.keep && !(sizeof(Real) == 8 && all_pairs)) return o;
+    Cell<Real> cell = res.cell;
+    locate<Real>(cell, E_tab, n_tab, E_res, ti);
+    const int ix = cell.idx;
+    const Real fr = cell.frac;
+    const bool bl = cell.below, ab = cell.above;
     Real lfr;
     {
-        const Real x0 = E_tab[ix - 1], x1 = E_tab[ix];
+        const Real x0 = cell.x0, x1 = cell.x1;
         Real bx = fmin(fmax(E_res, x0), x1);
         if (isnan(E_res)) bx = E_res;
         if constexpr (sizeof(Real) == 8) {
@@ -490,7 +524,7 @@ __device__ __forceinline__ PairAmps<Real> pair_amps(const SegPre<Real> &sp, cons
                                                     int n_tab, int n_mu, const pb_cxr_tables &t,
                                                     const TabIndex &ti) {
     const Resonance<Real> res = pair_resonance<Real>(sp, rw, E_tab, delta_tab, n_tab, t, ti);
-    return pair_amps_from<Real, kLayered>(sp, rw, res, E_tab, log_mu, n_tab, n_mu, t, ti);
+    return pair_amps_from<Real, kLayered>(sp, rw, res, E_tab, log_mu, n_tab, n_mu, t, ti, false);
 }
 
 // The incoherent line of a pair: resonance, width and weight
@@ -500,15 +534,14 @@ __device__ Line<Real> pair_line_from(const SegPre<Real> &sp, const RowPre<Real> 
                                      const Real *E_tab, const Real *log_mu, int n_tab, int n_mu,
                                      const pb_cxr_tables &t, const TabIndex &ti, const EscSeg<Real> *es,
                                      const pb_cxr_args &a, const Real *lay_t) {
-    const PairAmps<Real> p = pair_amps_from<Real, kLayered>(sp, rw, res, E_tab, log_mu, n_tab, n_mu, t, ti);
+    const bool all_pairs = a.pair_E != nullptr;
+    const PairAmps<Real> p = pair_amps_from<Real, kLayered>(sp, rw, res, E_tab, log_mu, n_tab, n_mu, t, ti, all_pairs);
     Line<Real> out;
     out.good = false;
     out.E_res = p.E_res;
     out.a_width = (Real)NAN;
     out.weight = (Real)NAN;
-    if constexpr (sizeof(Real) == 4) {
-        if (!p.keep) return out;
-    }
+    if (!p.keep && !(sizeof(Real) == 8 && all_pairs)) return out;
     const Real A2 = (p.A_re[0] * p.A_re[0] + p.A_im[0] * p.A_im[0]) + (p.A_re[1] * p.A_re[1] + p.A_im[1] * p.A_im[1]);
     Real T_abs;
     if constexpr (kLayered) T_abs = esc_transmission<Real>(*es, a, lay_t, (double)p.E_res);
@@ -610,7 +643,7 @@ __device__ double sincsq_tail(double x) {
     if (u == 0.0) {
         su = 1.0;
     } else {
-        su = sin(kPi * u) / (kPi * u);
+        su = sinpi(u) / (kPi * u);
     }
     const double r = si_minus_half_pi(t) / kPi - u * su * su;
     return x >= 0.0 ? r : -r;
@@ -644,27 +677,6 @@ __device__ __forceinline__ double centre_of(const BinAxis &ax, int c) {
     return 0.5 * (ax.edges[c] + ax.edges[c + 1]);
 }
 
-// Far-field envelope expansion about centre c: 1/((A-d)(B-d)) ~
-// f0 + f1 d + f2 d^2 with A = E_lo - E_c, B = E_hi - E_c, d = E_r - E_c
-// (any common unit: the form scales as 1/unit^2). Float on the mixed path.
-template <bool kMixed>
-__device__ __forceinline__ double far_envelope(double A, double B, double d) {
-    if constexpr (kMixed) {
-        const float Af = (float)A, Bf = (float)B, df = (float)d;
-        const float AB = Af * Bf;
-        const float r = __frcp_rn(AB);
-        const float f1 = (Af + Bf) * r * r;
-        const float f2 = (Af * Af + AB + Bf * Bf) * r * r * r;
-        return (double)(r + df * (f1 + df * f2));
-    } else {
-        const double AB = A * B;
-        const double r = 1.0 / AB;
-        const double f1 = (A + B) * r * r;
-        const double f2 = (A * A + AB + B * B) * r * r * r;
-        return r + d * (f1 + d * f2);
-    }
-}
-
 // Oscillatory part of the sinc^2 antiderivative beyond the asymptotic
 // threshold (Abramowitz & Stegun 5.2.8, 5.2.34-35): with u = 2 pi |x|,
 //   int sinc^2 = (1/(2 pi^2)) (1/x_a - 1/x_b) + (1/pi) [Q(u)]_a^b,
@@ -672,83 +684,57 @@ __device__ __forceinline__ double far_envelope(double A, double B, double d) {
 // where 1/u - f(u) ~ (1/u) sum_{k>=1} (-1)^(k+1) (2k)!/u^2k and
 // g(u) ~ (1/u^2) sum_{k>=0} (-1)^k (2k+1)!/u^2k. The envelope term carries
 // the mass without the cancellation of a difference of antiderivatives.
-__device__ __forceinline__ double q_osc_f64(double u) {
-    const double inv_u = 1.0 / u;
-    const double y = inv_u * inv_u;
-    double p1 = 0.0, p2 = 0.0;
-    // 13 terms: the first omitted one at u = 48 is below 1e-17 of the leading.
-    double t1 = 2.0 * y, t2 = 1.0;
-    for (int k = 1; k <= 13; ++k) {
-        p1 += t1;
-        p2 += t2;
-        t1 *= -(2.0 * k + 1.0) * (2.0 * k + 2.0) * y;
-        t2 *= -(2.0 * k) * (2.0 * k + 1.0) * y;
+constexpr int kOscTerms = 13;  // the first omitted one at u = 48 is below 1e-17 of the leading
+struct OscSeries {
+    double c1[kOscTerms], c2[kOscTerms];  // (-1)^k (2k+2)!, (-1)^k (2k+1)!
+};
+__host__ __device__ constexpr OscSeries make_osc_series() {
+    OscSeries s{};
+    double f = 1.0;
+    for (int k = 0; k < kOscTerms; ++k) {
+        f *= 2.0 * k + 1.0;
+        s.c2[k] = (k & 1) ? -f : f;
+        f *= 2.0 * k + 2.0;
+        s.c1[k] = (k & 1) ? -f : f;
+    }
+    return s;
+}
+
+// Far limit of an edge: |x| past u = 2 pi |x| = 24 (float) or 48 (FP64).
+template <class R>
+__device__ __forceinline__ constexpr R far_limit() { return (R)((sizeof(R) == 4 ? 24.0 : 48.0) / (2.0 * kPi)); }
+
+// sign(x) Q(2 pi |x|) with iu = 1 / (2 pi x) given (Q is odd in x and iu).
+__device__ __forceinline__ double q_osc(double x, double iu) {
+    constexpr OscSeries c = make_osc_series();
+    const double y = iu * iu;
+    double p1, p2;
+    if (fabs(iu) < 1.0 / 200.0) {
+        // u > 200: six terms reach 14!/200^12 < 3e-17 of the leading one.
+        p1 = c.c1[5];
+        p2 = c.c2[5];
+#pragma unroll
+        for (int k = 4; k >= 0; --k) { p1 = fma(p1, y, c.c1[k]); p2 = fma(p2, y, c.c2[k]); }
+    } else {
+        p1 = c.c1[kOscTerms - 1];
+        p2 = c.c2[kOscTerms - 1];
+#pragma unroll
+        for (int k = kOscTerms - 2; k >= 0; --k) { p1 = fma(p1, y, c.c1[k]); p2 = fma(p2, y, c.c2[k]); }
     }
     double sn, cs;
-    sincos(u, &sn, &cs);
-    return cs * p1 * inv_u - sn * p2 * y;
+    sincospi(2.0 * x, &sn, &cs);
+    return y * (cs * p1 * iu - sn * p2);
 }
-
-// Float form for the mixed path; the phase u is reduced in double first.
-__device__ __forceinline__ double q_osc_f32(double u) {
-    const float inv_u = __frcp_rn((float)u);
-    const float yf = inv_u * inv_u;
-    const float p1 = yf * (2.0f + yf * (-24.0f + yf * (720.0f + yf * (-40320.0f + yf * 3628800.0f))));
-    const float p2 = 1.0f + yf * (-6.0f + yf * (120.0f + yf * (-5040.0f + yf * 362880.0f)));
-    const double r = u - 2.0 * kPi * rint(u * (0.5 / kPi));
+__device__ __forceinline__ float q_osc(float x, float iu) {
+    const float y = iu * iu;
+    const float p1 = 2.0f + y * (-24.0f + y * (720.0f + y * (-40320.0f + y * 3628800.0f)));
+    const float p2 = 1.0f + y * (-6.0f + y * (120.0f + y * (-5040.0f + y * 362880.0f)));
+    // x to [-1/2, 1/2] turns by adding and taking off 1.5 2^23 (an FADD each
+    // where the rounding instruction runs at the SFU's rate).
+    constexpr float kRound = 12582912.0f;
     float sn, cs;
-    __sincosf((float)r, &sn, &cs);
-    return (double)(cs * p1 * inv_u - sn * p2 * yf);
-}
-
-// One bin edge of a line, in both antiderivative forms it may be needed in.
-struct EdgeCache {
-    bool valid;
-    double x;       // line-centred first-zero units
-    bool has_r, has_q;
-    double r;       // R(x), the sinc^2 antiderivative minus sign(x)/2
-    double q;       // Q(2 pi |x|), the oscillatory part of the far form
-};
-
-template <bool kMixed>
-__device__ __forceinline__ double edge_r(EdgeCache &e) {
-    if (!e.has_r) { e.r = sincsq_tail(e.x); e.has_r = true; }
-    return e.r;
-}
-
-template <bool kMixed>
-__device__ __forceinline__ double edge_q(EdgeCache &e) {
-    if (!e.has_q) {
-        const double u = 2.0 * kPi * fabs(e.x);
-        e.q = kMixed ? q_osc_f32(u) : q_osc_f64(u);
-        e.has_q = true;
-    }
-    return e.q;
-}
-
-// Exact mass of sinc^2 over [lo.x, hi.x]: the far closed form when both
-// edges are beyond the asymptotic threshold on one side, else the
-// difference of antiderivatives.
-template <bool kMixed>
-__device__ __forceinline__ double bin_mass(EdgeCache &lo, EdgeCache &hi) {
-    const double u_lim = kMixed ? 24.0 : 48.0;
-    const double x_lo = lo.x, x_hi = hi.x;
-    const double u_lo = 2.0 * kPi * fabs(x_lo), u_hi = 2.0 * kPi * fabs(x_hi);
-    if ((x_lo > 0.0 || x_hi < 0.0) && fmin(u_lo, u_hi) >= u_lim) {
-        const bool pos = x_lo > 0.0;
-        const double a = pos ? x_lo : -x_hi;
-        const double b = pos ? x_hi : -x_lo;
-        double env;
-        if constexpr (kMixed) {
-            env = (double)__fdividef((float)((b - a) * kInv2Pi2), (float)a * (float)b);
-        } else {
-            env = (b - a) * kInv2Pi2 / (a * b);
-        }
-        const double osc = pos ? (edge_q<kMixed>(hi) - edge_q<kMixed>(lo))
-                               : (edge_q<kMixed>(lo) - edge_q<kMixed>(hi));
-        return env + osc / kPi;
-    }
-    return edge_r<kMixed>(hi) - edge_r<kMixed>(lo) + ((x_lo < 0.0 && x_hi >= 0.0) ? 1.0 : 0.0);
+    __sincosf(6.28318530717958648f * (x - __fsub_rn(__fadd_rn(x, kRound), kRound)), &sn, &cs);
+    return y * (cs * p1 * iu - sn * p2);
 }
 
 // Bin-mean deposit of a line: exact bin integrals within the line's window
@@ -762,10 +748,11 @@ __device__ __forceinline__ double bin_mass(EdgeCache &lo, EdgeCache &hi) {
 struct LineWindow {
     int c;        // centre bin (may lie off the axis)
     int b0, nb;   // first exact bin and count
+    int K;        // half width of the window [bins]
     bool mom;     // far field through the moments
 };
 
-__device__ __forceinline__ LineWindow line_window(double E_r, double a, const BinAxis &ax,
+__device__ __forceinline__ LineWindow line_window(double E_r, double inv_a, const BinAxis &ax,
                                                   double exact_widths, int K_far, bool moments) {
     const int n = ax.n;
     LineWindow lw;
@@ -775,13 +762,14 @@ __device__ __forceinline__ LineWindow line_window(double E_r, double a, const Bi
     if (!lw.mom) {
         K = n + (lw.c < 0 ? -lw.c : (lw.c >= n ? lw.c - n + 1 : 0));
     } else {
-        const double kk = ceil(exact_widths * kPi / (a * ax.w));
+        const double kk = ceil(exact_widths * kPi * (inv_a * ax.inv_w));
         K = kk > (double)(2 * n) ? 2 * n : (kk < (double)K_far ? K_far : (int)kk);
     }
     int b0 = lw.c - K, b1 = lw.c + K;
     if (b0 < 0) b0 = 0;
     if (b1 > n - 1) b1 = n - 1;
     lw.b0 = b0;
+    lw.K = K;
     lw.nb = b1 >= b0 ? b1 - b0 + 1 : 0;
     return lw;
 }
@@ -832,100 +820,6 @@ __device__ __forceinline__ double sincsq_midpoint_mean(double xc, double dx) {
     return (double)series * kInv2Pi2;
 }
 
-// Per-line constants of the deposit: s = a / pi converts energy to
-// first-zero units and scale = w pi / a turns a bin's mass into its weighted
-// mean; both are formed once per line, so a bin on a uniform axis costs no
-// FP64 division beyond the far-envelope reciprocal.
-struct LineDep {
-    double E_r, s, scale;
-};
-
-// The far envelope this line's moments already spread onto bin b (more than
-// K_far bins from the centre), which the exact window takes back out:
-// w / (2 a^2) / ((E_lo - E_r)(E_hi - E_r)) = (w / (2 pi^2)) / (x_lo x_hi).
-template <bool kMixed>
-__device__ __forceinline__ double far_correction(const LineDep &L, int b, const LineWindow &lw, const BinAxis &ax,
-                                                 int K_far, double e0, double e1) {
-    if (!(lw.mom && (b - lw.c > K_far || lw.c - b > K_far))) return 0.0;
-    const double E_c = centre_of(ax, lw.c);
-    return (L.scale * L.s) * kInv2Pi2 *
-           far_envelope<kMixed>(L.s * (e0 - E_c), L.s * (e1 - E_c), L.s * (L.E_r - E_c));
-}
-
-// Exact-window classes of a bin. The cheap ones are evaluated where they are
-// found; the others are queued so that a warp evaluates one kind at a time.
-enum BinClass { kBinDone = 0, kBinExact = 1, kBinExactCf = 2 };
-
-// Evaluates bin b of a line when it is cheap: the midpoint series for a bin
-// much narrower than the line, the far closed form when both edges lie past
-// the asymptotic threshold on one side (ec carries the shared edge between
-// consecutive such bins). Otherwise returns the class of exact work it needs:
-// kBinExactCf when an edge falls in the continued-fraction range of Si.
-template <bool kMixed>
-__device__ __forceinline__ int bin_fast(const LineDep &L, int b, const LineWindow &lw, const BinAxis &ax,
-                                        int K_far, EdgeCache &ec, double &v) {
-    const double e0 = ax.edges[b], e1 = ax.edges[b + 1];
-    const double x_lo = L.s * (e0 - L.E_r), x_hi = L.s * (e1 - L.E_r);
-    const double dxw = L.s * (e1 - e0);
-    const double xc = 0.5 * (x_lo + x_hi);
-    if (dxw <= 0.1 && fabs(xc) >= 2.0) {
-        ec.valid = false;
-        v = (L.scale * L.s) * sincsq_midpoint_mean<kMixed>(xc, dxw);
-    } else {
-        constexpr double u_lim = kMixed ? 24.0 : 48.0;
-        const double u_min = 2.0 * kPi * fmin(fabs(x_lo), fabs(x_hi));
-        if (!((x_lo > 0.0 || x_hi < 0.0) && u_min >= u_lim)) {
-            ec.valid = false;
-            const double t_lo = 2.0 * kPi * fabs(x_lo), t_hi = 2.0 * kPi * fabs(x_hi);
-            const bool cf = (t_lo > 13.0 && t_lo < 40.0) || (t_hi > 13.0 && t_hi < 40.0);
-            return cf ? kBinExactCf : kBinExact;
-        }
-        EdgeCache lo_e;
-        if (ec.valid && ec.x == x_lo) {
-            lo_e = ec;
-        } else {
-            lo_e.valid = true;
-            lo_e.x = x_lo;
-            lo_e.has_r = lo_e.has_q = false;
-        }
-        EdgeCache hi_e;
-        hi_e.valid = true;
-        hi_e.x = x_hi;
-        hi_e.has_r = hi_e.has_q = false;
-        const double mass = bin_mass<kMixed>(lo_e, hi_e);
-        ec = hi_e;
-        const double inv_width = ax.uniform ? ax.inv_w : 1.0 / (e1 - e0);
-        v = mass * L.scale * inv_width;
-    }
-    v -= far_correction<kMixed>(L, b, lw, ax, K_far, e0, e1);
-    return kBinDone;
-}
-
-// Bin b of a line by the difference of sinc^2 antiderivatives at its edges.
-template <bool kMixed>
-__device__ __forceinline__ double bin_exact(const LineDep &L, int b, const LineWindow &lw, const BinAxis &ax,
-                                            int K_far) {
-    const double e0 = ax.edges[b], e1 = ax.edges[b + 1];
-    EdgeCache lo_e, hi_e;
-    lo_e.valid = hi_e.valid = true;
-    lo_e.x = L.s * (e0 - L.E_r);
-    hi_e.x = L.s * (e1 - L.E_r);
-    lo_e.has_r = lo_e.has_q = hi_e.has_r = hi_e.has_q = false;
-    const double mass = bin_mass<kMixed>(lo_e, hi_e);
-    const double inv_width = ax.uniform ? ax.inv_w : 1.0 / (e1 - e0);
-    return mass * L.scale * inv_width - far_correction<kMixed>(L, b, lw, ax, K_far, e0, e1);
-}
-
-// ---- mixed path: the cheap classes entirely in float ----------------------
-// The line's E_r is float on this path already, so first-zero coordinates in
-// float lose nothing further: |x| < ~2^8 in any window keeps ~1e-5 absolute.
-struct EdgeCacheF {
-    bool valid, has_r;
-    float x, q, r;  // q = Q(2 pi |x|) of the far form, r = R(x)
-    float iu;       // far form: 1 / (2 pi |x|) of the cached edge
-    float ia;       // far correction: 1 / (s (edge - E_c)) of the cached edge (0: unset)
-};
-
 // Reciprocal on the SFU alone (rcp.approx, about 1 ulp): the mixed path's
 // bin forms carry float rounding far below their tolerance.
 __device__ __forceinline__ float rcp_fast(float x) {
@@ -933,19 +827,7 @@ __device__ __forceinline__ float rcp_fast(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-
-// Q(2 pi |x|) of q_osc_x_f32 with its reciprocal 1 / (2 pi |x|) returned in iu.
-__device__ __forceinline__ float q_osc_iu_f32(float x, float &iu) {
-    const float ax = fabsf(x);
-    const float inv_u = rcp_fast(6.28318530717958648f * ax);
-    iu = inv_u;
-    const float yf = inv_u * inv_u;
-    const float p1 = yf * (2.0f + yf * (-24.0f + yf * (720.0f + yf * (-40320.0f + yf * 3628800.0f))));
-    const float p2 = 1.0f + yf * (-6.0f + yf * (120.0f + yf * (-5040.0f + yf * 362880.0f)));
-    float sn, cs;
-    __sincosf(6.28318530717958648f * (ax - rintf(ax)), &sn, &cs);
-    return cs * p1 * inv_u - sn * p2 * yf;
-}
+__device__ __forceinline__ double rcp_fast(double x) { return 1.0 / x; }
 
 // R(x) = F(x) - sign(x)/2 of sincsq_tail in float:
 // Si(t) - pi/2 = -f(t) cos t - g(t) sin t with t = 2 pi |x| and the rational
@@ -973,21 +855,6 @@ __device__ __forceinline__ float sincsq_tail_f32(float x) {
     const float lobe = u > 0.0f ? __fdividef(sp * sp, 9.86960440108935862f * u) : 0.0f;
     const float r = si_m * (float)kInvPi - lobe;
     return x >= 0.0f ? r : -r;
-}
-
-// Q(2 pi |x|) of q_osc_f32 with the phase reduced in float.
-__device__ __forceinline__ float q_osc_x_f32(float x) {
-    const float u = 6.28318530717958648f * fabsf(x);
-    const float inv_u = __frcp_rn(u);
-    const float yf = inv_u * inv_u;
-    const float p1 = yf * (2.0f + yf * (-24.0f + yf * (720.0f + yf * (-40320.0f + yf * 3628800.0f))));
-    const float p2 = 1.0f + yf * (-6.0f + yf * (120.0f + yf * (-5040.0f + yf * 362880.0f)));
-    // sin u, cos u with u = 2 pi |x|: reduce |x| to [-1/2, 1/2] turns.
-    const float ax = fabsf(x);
-    const float red = ax - rintf(ax);
-    float sn, cs;
-    __sincosf(6.28318530717958648f * red, &sn, &cs);
-    return cs * p1 * inv_u - sn * p2 * yf;
 }
 
 // Mean of sinc^2 over a bin of width dx in first-zero units centred on xc
@@ -1022,74 +889,79 @@ __device__ __forceinline__ float sincsq_midpoint_mean_f32(float xc, float dx) {
     return series * (float)kInv2Pi2;
 }
 
-// Bin b of a line on the mixed path, every class in float (always returns
-// kBinDone): edges_f is the float copy of the bin edges, c the line's centre
-// bin when its far field goes through the moments (else INT_MIN), E_c that
-// bin's centre.
-__device__ __forceinline__ int bin_fast_f32(float E_r, float s, float scale, int b, int c, float E_c,
-                                            const float *edges_f, bool uniform, float inv_w, int K_far,
-                                            EdgeCacheF &ec, float &v) {
-    const float e0 = edges_f[b], e1 = edges_f[b + 1];
-    const float x_lo = s * (e0 - E_r), x_hi = s * (e1 - E_r);
-    const float dxw = s * (e1 - e0);
-    const float xc = 0.5f * (x_lo + x_hi);
-    const float w = scale * s;
-    const bool consec = ec.valid && ec.x == x_lo;  // the previous bin of this line, cached
-    if (dxw <= 0.1f && fabsf(xc) >= 2.0f) {
-        ec.valid = false;
-        v = w * sincsq_midpoint_mean_f32(xc, dxw);
-    } else {
-        // Far closed form (u_lim = 24): both edges past 24 / (2 pi) on one side.
-        constexpr float x_lim = (float)(24.0 / (2.0 * kPi));
-        const bool cached = ec.valid && ec.x == x_lo;
-        float mass;
-        if (!((x_lo > 0.0f && x_lo >= x_lim) || (x_hi < 0.0f && -x_hi >= x_lim))) {
-            // Difference of antiderivatives.
-            const float r_lo = (cached && ec.has_r) ? ec.r : sincsq_tail_f32(x_lo);
-            const float r_hi = sincsq_tail_f32(x_hi);
-            ec.valid = true;
-            ec.has_r = true;
-            ec.x = x_hi;
-            ec.r = r_hi;
-            mass = r_hi - r_lo + ((x_lo < 0.0f && x_hi >= 0.0f) ? 1.0f : 0.0f);
-        } else {
-            // Far closed form: the envelope (1/lo - 1/hi) / (2 pi^2) from the
-            // edges' reciprocals 1/(2 pi |x|), which the phase terms need
-            // anyway, plus the oscillation (Q(hi) - Q(lo)) / pi.
-            const bool reuse = cached && !ec.has_r;
-            float iu_lo, iu_hi;
-            const float q_lo = reuse ? ec.q : q_osc_iu_f32(x_lo, iu_lo);
-            if (reuse) iu_lo = ec.iu;
-            const float q_hi = q_osc_iu_f32(x_hi, iu_hi);
-            ec.valid = true;
-            ec.has_r = false;
-            ec.x = x_hi;
-            ec.q = q_hi;
-            ec.iu = iu_hi;
-            const bool pos = x_lo > 0.0f;
-            const float env = (pos ? (iu_lo - iu_hi) : (iu_hi - iu_lo)) * (float)kInvPi;
-            const float osc = pos ? (q_hi - q_lo) : (q_lo - q_hi);
-            mass = env + osc * (float)kInvPi;
-        }
-        v = mass * scale * (uniform ? inv_w : __frcp_rn(e1 - e0));
+__device__ __forceinline__ float tail_of(float x) { return sincsq_tail_f32(x); }
+__device__ __forceinline__ double tail_of(double x) { return sincsq_tail(x); }
+__device__ __forceinline__ float midpoint_mean(float xc, float dx) { return sincsq_midpoint_mean_f32(xc, dx); }
+__device__ __forceinline__ double midpoint_mean(double xc, double dx) { return sincsq_midpoint_mean<false>(xc, dx); }
+
+// ---- the deposit as a function of bin edges --------------------------------
+// pi times the mass of sinc^2 in a bin is a difference of one function of its
+// edges, pi R(x) = pi (F(x) - sign(x)/2) (plus pi in the bin that holds x = 0).
+// Past the far limit pi R(x) = Q(x) - 1/(2 pi x), both odd in x, which float
+// keeps without cancellation for bins wider than 0.1 first-zero widths; narrower
+// ones take the midpoint series away from the centre.
+//
+// Where the moments spread the far envelope of the line (bins more than K_far
+// from its centre bin c), the exact window takes that envelope back out. Its
+// expansion about the centre is itself a difference over the bin's edges: with
+// Dm the edge's distance from the centre of bin c in bins, d = (E_r - E_c) / w
+// and A = s w Dm (first-zero units), the spread f0 + f1 d + f2 d^2 is
+// [T(A) - T(B)] / (B - A) with T(A) = (1 + t + t^2) / A, t = d / Dm. So
+//   pi R(x) + T(A) / (2 pi)
+// is the edge function there, and past the far limit, since x = A (1 - t),
+// 1/x - T(A) = t^3 / x makes it Q(x) - t^3 / (2 pi x): the envelope and its
+// expansion never meet as two large numbers.
+template <class R>
+__device__ __forceinline__ R edge_near_bins(R x) {
+    if (fabs(x) >= far_limit<R>()) {
+        const R iu = rcp_fast((R)(2.0 * kPi) * x);
+        return q_osc(x, iu) - iu;
     }
-    if (c != INT_MIN && (b - c > K_far || c - b > K_far)) {
-        // The envelope the moments spread here: with ra = 1/A, rb = 1/B,
-        // A = s (e0 - E_c), B = s (e1 - E_c), r = ra rb:
-        // r + d (r (ra + rb) + d r (ra^2 + ra rb + rb^2)), d = s (E_r - E_c).
-        const float ra = (consec && ec.ia != 0.0f) ? ec.ia : rcp_fast(s * (e0 - E_c));
-        const float rb = rcp_fast(s * (e1 - E_c));
-        ec.ia = rb;
-        const float d = s * (E_r - E_c);
-        const float r = ra * rb;
-        const float f1 = r * (ra + rb);
-        const float f2 = r * fmaf(ra, ra + rb, rb * rb);
-        v -= w * (float)kInv2Pi2 * (r + d * (f1 + d * f2));
-    } else {
-        ec.ia = 0.0f;
-    }
-    return kBinDone;
+    return (R)kPi * tail_of(x);
 }
+
+// x and Dm of one sign (an edge outside the centre bin).
+template <class R>
+__device__ __forceinline__ R edge_window_far(R x, R Dm, R d) {
+    const R ux = (R)(2.0 * kPi) * x;
+    const R r = rcp_fast(ux * Dm);  // one reciprocal for 1/(2 pi x) and 1/Dm
+    const R iu = r * Dm;
+    const R t = d * (r * ux);
+    return q_osc(x, iu) - (iu * t) * (t * t);
+}
+
+// sw: the bin width in first-zero units.
+template <class R>
+__device__ __forceinline__ R edge_window_near(R x, R Dm, R d, R sw) {
+    const R iD = rcp_fast(Dm);
+    const R t = d * iD;
+    return (R)kPi * tail_of(x) + (R)(0.5 / kPi) * (iD * rcp_fast(sw)) * fma(t, t, (R)1 + t);
+}
+
+// The edge function of a window edge.
+template <class R>
+__device__ __forceinline__ R edge_window_bins(R x, R Dm, R d, R sw) {
+    if (fabs(x) >= far_limit<R>()) return edge_window_far<R>(x, Dm, d);
+    return edge_window_near<R>(x, Dm, d, sw);
+}
+
+// pi times the mass (less the spread envelope) of a bin of at most 0.1 first-zero
+// widths, |xc| >= 2, by the midpoint series: Dm its left edge, xc its centre.
+template <class R>
+__device__ __forceinline__ R window_midpoint(R xc, R Dm, R d, R sw) {
+    const R ra = rcp_fast(sw * Dm), rb = rcp_fast(sw * (Dm + (R)1));
+    const R r = ra * rb, dx = sw * d;
+    const R far = r + dx * (r * (ra + rb) + dx * r * fma(ra, ra + rb, rb * rb));
+    return sw * ((R)kPi * midpoint_mean(xc, sw) - (R)(0.5 / kPi) * far);
+}
+
+// One line of the window list, read back as broadcasts.
+template <class R>
+struct alignas(16) WinLine {
+    R sw, scale, d, E_r;  // bin width in first-zero units, w / a, (E_r - E_c) / bin width
+    int c, D0, D1;        // centre bin, window bins D0 <= |b - c| <= D1 on the axis
+    int pad;
+};
 
 __device__ __forceinline__ void smem_add(float *p, float v) {
     asm volatile("red.shared.add.f32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "f"(v) : "memory");
@@ -1101,10 +973,10 @@ __device__ __forceinline__ void smem_add(double *p, double v) {
 // A kept line's three far-field moments about its centre bin, added to the
 // direction's moments in global memory (L2 reductions: a few per kept line,
 // so the block keeps no on-chip copy of the moment array).
-__device__ __forceinline__ void line_moments(double E_r, double a, double w, const LineWindow &lw,
+__device__ __forceinline__ void line_moments(double E_r, double inv_a, double w, const LineWindow &lw,
                                              const BinAxis &ax, double *mom) {
     const int slot = lw.c + ax.pad;
-    const double m = w / (2.0 * a * a);
+    const double m = 0.5 * w * (inv_a * inv_a);
     const double dd = E_r - centre_of(ax, lw.c);
     atomicAdd(&mom[3 * slot + 0], m);
     atomicAdd(&mom[3 * slot + 1], m * dd);
@@ -1119,8 +991,16 @@ __device__ __forceinline__ void line_moments(double E_r, double a, double w, con
 //       window and compacts the survivors into a shared queue (warp ballot);
 //   A1  the full chain runs densely over the survivors and pushes kept lines
 //       onto a second shared queue;
-//   B   the queued lines' (line, bin) work is cut into 4-item chunks spread
-//       over the block; edges shared by consecutive bins are evaluated once.
+//   B1  lines leave the queue in whole rounds of one per thread (the rest
+//       waits for the next pass): the owner thread adds the line's far-field
+//       moments and the bins within K_far of its centre, and passes lines
+//       whose exact window is wider on to a window list;
+//   B2  when the window list is full, groups of 4 to 32 lanes (by the window's
+//       width) take a line each: a lane holds two bin edges, evaluates the edge
+//       function once each and gets the third from the next lane. The widest
+//       windows wait for more of their kind and are summed strip by strip.
+// B is bound by FP32/FP64 issue and the SFU (one reciprocal, one sine, one
+// cosine per edge).
 template <class Real, bool kLayered>
 __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a, int K_far, int far_pad) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1143,32 +1023,30 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     SegPre<Real> *segs = reinterpret_cast<SegPre<Real> *>(cur);
     cur += sizeof(SegPre<Real>) * kSegTile;
     cur = (unsigned char *)(((uintptr_t)cur + 15) & ~(uintptr_t)15);
+    constexpr int kLineQueue = line_queue<Real>();
     Real *qE = reinterpret_cast<Real *>(cur);
-    Real *qA = qE + kQueue;
-    Real *qW = qA + kQueue;
-    int *qStart = reinterpret_cast<int *>(qW + kQueue);   // kQueue + 1 prefix entries
-    int *qB0 = qStart + kQueue + 1;
-    int *qC = qB0 + kQueue;
-    int *pq = qC + kQueue;                                  // surviving pair ids
-    int *scratch = pq + kQueue;                             // warp sums + counters
-    int *xq = scratch + 64;                                 // exact bins: [plain | continued fraction]
-    // (the float path evaluates every bin class in place: no exact-bin queue)
-    cur = reinterpret_cast<unsigned char *>(xq + ((binmean && !kMixed) ? 2 * kXQueue : 0));
+    Real *qA = qE + kLineQueue;
+    Real *qW = qA + kLineQueue;
+    cur = (unsigned char *)(((uintptr_t)(qW + kLineQueue) + 15) & ~(uintptr_t)15);
+    WinLine<Real> *wLine = reinterpret_cast<WinLine<Real> *>(cur);  // window list
+    uint16_t *wIdx = reinterpret_cast<uint16_t *>(wLine + kWideCap);  // its lines by class
+    int *scratch = reinterpret_cast<int *>(wIdx + kWinClasses * kWideCap);  // counters
+    uint16_t *pq = reinterpret_cast<uint16_t *>(scratch + 64);  // surviving pair ids
+    cur = reinterpret_cast<unsigned char *>(pq + kQueue);
     cur = (unsigned char *)(((uintptr_t)cur + 15) & ~(uintptr_t)15);
     const bool tab_smem = n_tab <= kMaxTab;
     Real *E_tab_s = reinterpret_cast<Real *>(cur);
     Real *delta_s = E_tab_s + (tab_smem ? n_tab : 0);
     Real *logmu_s = delta_s + (tab_smem ? n_tab : 0);
     Real *dtail_s = logmu_s + (tab_smem ? n_tab * n_mu : 0);
-    const bool has_dtail = kMixed && tab_smem && a.tables.delta_tail_absmax != nullptr && a.pair_E == nullptr;
+    const bool has_dtail = tab_smem && a.tables.delta_tail_absmax != nullptr && a.pair_E == nullptr;
     cur = reinterpret_cast<unsigned char *>(dtail_s + (tab_smem ? n_tab : 0));
     cur = (unsigned char *)(((uintptr_t)cur + 15) & ~(uintptr_t)15);
     double *spec_s = reinterpret_cast<double *>(cur);
     const int n_mom = n_E + 2 * far_pad;
-    float *spec_f = reinterpret_cast<float *>(spec_s + (binmean ? n_E : 0));
-    float *edges_f = spec_f + (binmean ? n_E : 0);  // mixed path: float bin edges
+    float *spec_f = reinterpret_cast<float *>(spec_s + (binmean ? n_E : 0));  // mixed path: float partials
     // Layered absorber: per-segment escape pieces, layer thicknesses and bounds.
-    unsigned char *esc_raw = reinterpret_cast<unsigned char *>(edges_f + (binmean && kMixed ? n_E + 1 : 0));
+    unsigned char *esc_raw = reinterpret_cast<unsigned char *>(spec_f + (binmean && kMixed ? n_E : 0));
     esc_raw = (unsigned char *)(((uintptr_t)esc_raw + 15) & ~(uintptr_t)15);
     EscSeg<Real> *esc = reinterpret_cast<EscSeg<Real> *>(esc_raw);
     double *lay_zt = reinterpret_cast<double *>(esc + (kLayered ? kSegTile : 0));
@@ -1176,12 +1054,13 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     Real *lay_t = reinterpret_cast<Real *>(lay_zb + (kLayered ? kMaxEscLayers : 0));
     int &q_count = scratch[40];
     int &p_count = scratch[42];
-    int *xq_count = scratch + 44;  // two counters
-    // A queued bin packs (line, bin) as line << 21 | bin.
-    const bool use_xq = n_E < (1 << 21);
+    int &w_count = scratch[43];
+    int *w_class = scratch + 48;  // lines per class
+    int &strip_next = scratch[44];
 
     const int tid = threadIdx.x;
     const unsigned lane = tid & 31u;
+    const int warp = tid >> 5, n_warps = kCxrThreads / 32;
     if (tab_smem) {
         for (int j = tid; j < n_tab; j += blockDim.x) {
             E_tab_s[j] = (Real)a.tables.E_tab[j];
@@ -1192,11 +1071,12 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     }
     const Real *dtail = has_dtail ? dtail_s : nullptr;
     if (binmean) {
-        for (int j = tid; j < n_E; j += blockDim.x) { spec_s[j] = 0.0; spec_f[j] = 0.0f; }
+        for (int j = tid; j < n_E; j += blockDim.x) spec_s[j] = 0.0;
         if (kMixed)
-            for (int j = tid; j <= n_E; j += blockDim.x) edges_f[j] = (float)a.edges[j];
+            for (int j = tid; j < n_E; j += blockDim.x) spec_f[j] = 0.0f;
     }
-    if (tid == 0) { q_count = 0; p_count = 0; xq_count[0] = 0; xq_count[1] = 0; }
+    if (tid == 0) { q_count = 0; p_count = 0; w_count = 0; strip_next = 0; }
+    if (tid < kWinClasses) w_class[tid] = 0;
     if constexpr (kLayered) {
         if (tid < a.n_layer) {
             lay_zt[tid] = a.z_top[tid];
@@ -1237,54 +1117,322 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     __syncthreads();
     if (kLayered && scratch[46]) return;
 
-    const int64_t n_tiles = (n_seg + kSegTile - 1) / kSegTile;
-    const int64_t n_work = n_tiles * a.n_dir;
+    const int n_chunks = (n_g + kRowChunk - 1) / kRowChunk;
+    int seg_tile = kSegTile;
+    while (seg_tile > 4 && (n_seg + seg_tile - 1) / seg_tile * a.n_dir * n_chunks < 4 * (int64_t)gridDim.x)
+        seg_tile >>= 1;
+    const int64_t n_tiles = (n_seg + seg_tile - 1) / seg_tile;
+    const int64_t n_work = n_tiles * a.n_dir * n_chunks;
     const int64_t w_begin = n_work * blockIdx.x / gridDim.x;
     const int64_t w_end = n_work * (blockIdx.x + 1) / gridDim.x;
     const bool pairs_out = a.pair_E != nullptr;
     const bool lines_out = a.line_E != nullptr;
     const double exact_widths = K_far > 0 ? a.exact_widths : 0.0;
-    const int n_warps = blockDim.x >> 5;
+    const Real inv_w_r = (Real)ax.inv_w;
+    // B adds into float partials on the mixed path, else into the spectrum.
+    auto *const spec_part = [&] {
+        if constexpr (kMixed) return spec_f;
+        else return spec_s;
+    }();
     int d_cur = -1;
+    int rounds = 0;  // rounds since the float partials were last folded
 
-    auto flush = [&](int d) {
+    // B1: the line in queue slot j, if any, by this thread.
+    auto near_round = [&](int j, int d) {
+        int cls = kWinClasses;
+        WinLine<Real> wl{};
+        if (j >= 0) {
+            const double Ed = (double)qE[j], wd = (double)qW[j], inv_a = 1.0 / (double)qA[j];
+            const LineWindow lw = line_window(Ed, inv_a, ax, exact_widths, K_far, K_far > 0);
+            const Real sx = (Real)(kMixed ? (float)qA[j] * (float)kInvPi : (double)qA[j] * kInvPi);
+            wl.E_r = qE[j];
+            wl.scale = (Real)(wd * inv_a);
+            if (a.counters) {
+                atomicAdd(&a.counters[0], 1ULL);
+                atomicAdd(&a.counters[1], (unsigned long long)lw.nb);
+            }
+            if (lw.mom) {
+                line_moments(Ed, inv_a, wd, lw, ax, a.far_moments + (int64_t)d * n_mom * 3);
+                wl.sw = sx * (Real)ax.w;
+                wl.d = (Real)((Ed - centre_of(ax, lw.c)) * ax.inv_w);
+                wl.c = lw.c;
+                if (lw.nb > 0) {
+                    // window bins on the axis, by distance from the centre bin
+                    const int left = lw.c - lw.b0, right = lw.b0 + lw.nb - 1 - lw.c;
+                    wl.D0 = max(K_far + 1, max(-left, -right));
+                    wl.D1 = max(left, right);
+                    const int span = wl.D1 - wl.D0 + 1;
+                    if (span > 0)
+                        cls = span <= 3 ? kWin4 : span <= 7 ? kWin8 : span <= 15 ? kWin16 : span <= kStripSpan ? kWin32 : kWinStrip;
+                    // bins narrower than 0.1 first-zero widths take the midpoint series
+                    if (span > 0 && wl.sw <= (Real)0.1) cls = kWinStrip;
+                }
+                // the bins c - K_far .. c + K_far, left to right
+                const Real out = wl.scale * (Real)ax.inv_w;
+                const int eb = lw.c - K_far;
+                auto edge_x = [&](int k) {
+                    if constexpr (kMixed) return wl.sw * ((Real)(k - K_far) - (Real)0.5 - wl.d);
+                    else return sx * (ax.edges[min(max(eb + k, 0), n_E)] - wl.E_r);
+                };
+                Real x_lo = edge_x(0);
+                Real f_lo = edge_near_bins<Real>(x_lo);
+                for (int k = 0; k <= 2 * K_far; ++k) {
+                    const int bin = eb + k;
+                    const Real x_hi = edge_x(k + 1);
+                    const Real f_hi = edge_near_bins<Real>(x_hi);
+                    Real mass = f_hi - f_lo + ((x_lo < (Real)0 && x_hi >= (Real)0) ? (Real)kPi : (Real)0);
+                    const Real xc = (Real)0.5 * (x_lo + x_hi);
+                    if (wl.sw <= (Real)0.1 && fabs(xc) >= (Real)2) mass = (Real)kPi * wl.sw * midpoint_mean(xc, wl.sw);
+                    if (bin >= 0 && bin < n_E) smem_add(&spec_part[bin], out * mass);
+                    x_lo = x_hi;
+                    f_lo = f_hi;
+                }
+            } else {
+                wl.sw = sx;  // the whole axis: first-zero units per eV
+                if (lw.nb > 0) cls = kWinAxis;
+            }
+        }
+        const unsigned mask = __ballot_sync(0xffffffffu, cls < kWinClasses);
+        int base = 0;
+        if (lane == 0 && mask) base = atomicAdd(&w_count, __popc(mask));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (cls < kWinClasses) {
+            const int k = base + __popc(mask & ((1u << lane) - 1u));
+            wLine[k] = wl;
+            wIdx[cls * kWideCap + atomicAdd(&w_class[cls], 1)] = (uint16_t)k;
+        }
+    };
+
+    // B2: window bins outside the near bins. A group of G lanes takes one line:
+    // its lower half the bins right of the centre, its upper half those left of
+    // it. A lane holds two neighbouring edges from bin distance D on outwards and
+    // the bins outside of each (G - 1 edges, G - 1 bins a side and visit), the
+    // outer edge of its second bin from the next lane.
+    auto visit = [&](const WinLine<Real> &l, int D, int G, bool live) {
+        const int h = (int)lane & (G / 2 - 1);
+        const bool left = (lane & (unsigned)(G / 2)) != 0;
+        const Real sgn = left ? (Real)-1 : (Real)1;
+        const int Dh = D + 2 * h;                      // distance of this lane's first bin
+        const Real Dm = sgn * ((Real)Dh - (Real)0.5);  // its inner edge
+        const int bin = left ? l.c - Dh : l.c + Dh;
+        Real x0, x1;
+        if constexpr (kMixed) {
+            x0 = l.sw * (Dm - l.d);
+            x1 = fma(sgn, l.sw, x0);
+        } else {
+            const int edge = left ? bin + 1 : bin;
+            const Real s = l.sw * inv_w_r;
+            x0 = s * (ax.edges[min(max(edge, 0), n_E)] - l.E_r);
+            x1 = s * (ax.edges[min(max(left ? edge - 1 : edge + 1, 0), n_E)] - l.E_r);
+        }
+        const Real f0 = edge_window_bins<Real>(x0, Dm, l.d, l.sw);
+        const Real f1 = edge_window_bins<Real>(x1, Dm + sgn, l.d, l.sw);
+        const Real f2 = __shfl_down_sync(0xffffffffu, f0, 1);
+        const Real out = sgn * l.scale * inv_w_r;
+        const int next = left ? bin - 1 : bin + 1;
+        if (live && Dh <= l.D1 && bin >= 0 && bin < n_E) smem_add(&spec_part[bin], out * (f1 - f0));
+        if (live && h < G / 2 - 1 && Dh < l.D1 && next >= 0 && next < n_E) smem_add(&spec_part[next], out * (f2 - f1));
+    };
+
+    auto window_phase = [&]() {
+        for (int cls = kWin4; cls <= kWin16; ++cls) {  // one visit a line
+            const int G = 4 << cls, per = 32 / G, n = w_class[cls];
+            for (int i = warp * per; i < n; i += n_warps * per) {
+                const int k = i + (int)lane / G;
+                const WinLine<Real> &l = wLine[wIdx[cls * kWideCap + min(k, n - 1)]];
+                visit(l, l.D0, G, k < n);
+            }
+        }
+        for (int i = warp; i < w_class[kWin32]; i += n_warps) {
+            const WinLine<Real> &l = wLine[wIdx[kWin32 * kWideCap + i]];
+            for (int D = l.D0; D <= l.D1; D += 31) visit(l, D, 32, true);
+        }
+    };
+
+    // Wide windows: a warp takes strips of 31 bins in turn, a lane holds one edge
+    // of the strip and sums its bin over the lines in a register (no atomics).
+    auto strip_phase = [&]() {
+        const int nw = w_class[kWinStrip];
+        for (int first = warp * kStripBins; first < n_E; first += n_warps * kStripBins) {
+            const int last = min(first + kStripBins, n_E) - 1;
+            const int bin = first + (int)lane;
+            const double e = kMixed ? 0.0 : ax.edges[min(bin, n_E)];
+            Real acc = 0;
+            for (int k = 0; k < nw; ++k) {
+                const WinLine<Real> &l = wLine[wIdx[kWinStrip * kWideCap + k]];
+                if (first > l.c + l.D1 || last < l.c - l.D1) continue;
+                const Real sw = l.sw, D = (Real)(bin - l.c), Dm = D - (Real)0.5;
+                const bool on = fabs(D) >= (Real)l.D0 && fabs(D) <= (Real)l.D1;
+                Real x;
+                if constexpr (kMixed) x = sw * (Dm - l.d);
+                else x = (sw * inv_w_r) * (e - l.E_r);
+                Real mass;
+                if (sw > (Real)0.1) {
+                    const Real f = edge_window_bins<Real>(x, Dm, l.d, sw);
+                    mass = __shfl_down_sync(0xffffffffu, f, 1) - f;
+                } else {
+                    const Real f = fabs(x) < (Real)2.2 ? edge_window_near<Real>(x, Dm, l.d, sw) : (Real)0;
+                    mass = __shfl_down_sync(0xffffffffu, f, 1) - f;
+                    const Real xc = fma((Real)0.5, sw, x);
+                    if (fabs(xc) >= (Real)2) mass = window_midpoint<Real>(xc, Dm, l.d, sw);
+                }
+                if (on) acc = fma(l.scale, mass, acc);
+            }
+            if (lane < kStripBins && bin < n_E) spec_s[bin] += (double)acc * ax.inv_w;
+        }
+    };
+
+    // Lines integrated over the whole axis (no moments): every line reaches
+    // every bin, so a warp takes strips of 31 bins in turn, a lane holds one
+    // edge of the strip and sums its bin over the lines in a register.
+    auto axis_phase = [&]() {
+        const int n_strips = (n_E + kStripBins - 1) / kStripBins, nw = w_class[kWinAxis];
+        while (true) {
+            int strip = 0;
+            if (lane == 0) strip = atomicAdd(&strip_next, 1);
+            strip = __shfl_sync(0xffffffffu, strip, 0);
+            if (strip >= n_strips) break;
+            const int bin = strip * kStripBins + (int)lane;
+            const double e_lo = a.edges[min(bin, n_E)];
+            const Real e = (Real)e_lo;
+            Real acc = 0;
+            for (int k = 0; k < nw; ++k) {
+                const WinLine<Real> &l = wLine[wIdx[kWinAxis * kWideCap + k]];
+                const Real x = l.sw * (e - l.E_r);
+                const Real x_hi = __shfl_down_sync(0xffffffffu, x, 1);
+                const Real sw = x_hi - x, xc = (Real)0.5 * (x + x_hi);
+                const bool narrow = sw <= (Real)0.1 && fabs(xc) >= (Real)2;
+                const unsigned wide_bins = __ballot_sync(0xffffffffu, !narrow && lane < kStripBins);
+                const bool need = ((wide_bins | (wide_bins << 1)) >> lane) & 1u;
+                const Real f = need ? edge_near_bins<Real>(x) : (Real)0;
+                Real mass = __shfl_down_sync(0xffffffffu, f, 1) - f +
+                            ((x < (Real)0 && x_hi >= (Real)0) ? (Real)kPi : (Real)0);
+                if (narrow) mass = (Real)kPi * sw * midpoint_mean(xc, sw);
+                acc = fma(l.scale, mass, acc);
+            }
+            if (lane < kStripBins && bin < n_E) {
+                // this warp owns the strip's bins until the phase ends
+                const double inv_w = ax.uniform ? ax.inv_w : 1.0 / (a.edges[bin + 1] - e_lo);
+                spec_s[bin] += (double)acc * inv_w;
+            }
+        }
+    };
+
+    // Lines leave the queue in whole rounds; ``flush`` takes what is left too
+    // (before the direction changes). Every condition is uniform over the block.
+    auto deposit = [&](bool flush) {
+        int nq = q_count;
+        bool more = flush ? nq > 0 || w_count > 0 : nq >= kCxrThreads;
+        if (flush) __syncthreads();  // every thread has read w_count
+        while (more) {
+            const int take = min(nq, kCxrThreads);
+            near_round(tid < take ? nq - take + tid : -1, d_cur);
+            nq -= take;
+            __syncthreads();
+            const int nw = w_count;
+            const bool leave = flush && nq == 0;
+            if (nw > kWideRun || (leave && nw > 0)) {
+                window_phase();
+                const int n_strip = w_class[kWinStrip], n_axis = w_class[kWinAxis];
+                const bool strips = n_strip > kStripRun || (leave && n_strip > 0);
+                // FP64: the window's adds and the strips' sums share spec_s
+                __syncthreads();
+                if (strips) strip_phase();
+                if (n_axis > 0) {
+                    if (strips) __syncthreads();
+                    axis_phase();
+                }
+                // strip lines that wait move to the front of the list
+                WinLine<Real> wl;
+                const bool keep = !strips && tid < n_strip;
+                if (keep) wl = wLine[wIdx[kWinStrip * kWideCap + tid]];
+                __syncthreads();
+                if (keep) {
+                    wLine[tid] = wl;
+                    wIdx[kWinStrip * kWideCap + tid] = (uint16_t)tid;
+                }
+                if (tid < kWinClasses) w_class[tid] = tid == kWinStrip && !strips ? n_strip : 0;
+                if (tid == 0) { w_count = strips ? 0 : n_strip; strip_next = 0; }
+            }
+            if constexpr (kMixed) {
+                // Fold the float partials into the FP64 spectrum every four
+                // rounds: about a thousand lines' adds keep float well inside
+                // the path's tolerance.
+                if (K_far > 0 && ++rounds == 4) {
+                    for (int j = tid; j < n_E; j += blockDim.x) {
+                        const float v = spec_f[j];
+                        if (v != 0.0f) { spec_s[j] += (double)v; spec_f[j] = 0.0f; }
+                    }
+                    rounds = 0;
+                }
+            }
+            more = flush ? nq > 0 : nq >= kCxrThreads;
+            __syncthreads();
+        }
+        if (tid == 0) q_count = nq;
+    };
+
+    auto publish = [&](int d) {
         // Publish (and clear) the block's spectrum of direction d.
         __syncthreads();
-        if (binmean && d >= 0) {
-            double *gspec = a.spec + (int64_t)d * n_E;
-            for (int j = tid; j < n_E; j += blockDim.x) {
-                if (spec_s[j] != 0.0) atomicAdd(&gspec[j], spec_s[j]);
-                spec_s[j] = 0.0;
-            }
+        if constexpr (kMixed) {
+            for (int j = tid; j < n_E; j += blockDim.x) { spec_s[j] += (double)spec_f[j]; spec_f[j] = 0.0f; }
+        }
+        rounds = 0;
+        double *gspec = a.spec + (int64_t)d * n_E;
+        for (int j = tid; j < n_E; j += blockDim.x) {
+            if (spec_s[j] != 0.0) atomicAdd(&gspec[j], spec_s[j]);
+            spec_s[j] = 0.0;
         }
         __syncthreads();
     };
 
-    for (int64_t wk = w_begin; wk < w_end; ++wk) {
-        const int d = (int)(wk / n_tiles);
-        const int64_t tile = wk - (int64_t)d * n_tiles;
-        if (d != d_cur) {
-            flush(d_cur);
-            d_cur = d;
-        }
-        const double *nh = a.n_hat + 3 * d;
-        const int64_t s0 = tile * kSegTile;
-        const int nst = (int)((n_seg - s0) < kSegTile ? (n_seg - s0) : kSegTile);
+    // Work units: (direction, row chunk, segment tile), tiles innermost, so a
+    // block stages its rows once per run of tiles. Chunk k holds rows k,
+    // k + n_chunks, ...: neighbouring rows of a reflection list radiate alike, so
+    // the chunks carry equal work. Fewer than four units a block: halve the tile, so that a short
+    // segment list still reaches every SM (a tile below four segments leaves
+    // most threads of a pass idle).
+    int64_t d_ch = -1;
+    for (int64_t wk = w_begin;; ++wk) {
+        const bool end = wk >= w_end;
+        const int64_t dc = end ? 0 : wk / n_tiles;
+        const int64_t tile = wk - dc * n_tiles;
+        const int d = (int)(dc / n_chunks);
+        // The lines the last unit queued: whole rounds, or all of them before
+        // the direction changes or the block ends.
+        const bool leave = end || d != d_cur;
         __syncthreads();
+        if (tid == 0) p_count = 0;
+        if (binmean && d_cur >= 0) {
+            deposit(leave);
+            if (leave) publish(d_cur);
+        }
+        if (end) break;
+        d_cur = d;
+        const double *nh = a.n_hat + 3 * d;
+        const int64_t s0 = tile * seg_tile;
+        const int nst = (int)((n_seg - s0) < seg_tile ? (n_seg - s0) : seg_tile);
+        const bool rad = tid < nst && a.elec_id[s0 + tid] < a.Ne &&
+                         (a.seg_layer == nullptr || a.seg_layer[s0 + tid] == a.emit_layer);
+        // (also the barrier before the staged rows and segments are replaced)
+        if (!__syncthreads_or(rad) && !pairs_out) continue;
         if (tid < nst) seg_precompute<Real>(segs[tid], a, s0 + tid, nh);
         if constexpr (kLayered) {
             if (tid < nst) esc_precompute<Real>(esc[tid], a, s0 + tid, nh, lay_zt, lay_zb);
         }
-        for (int g0 = 0; g0 < n_g; g0 += kRowChunk) {
-            const int ng = (n_g - g0) < kRowChunk ? (n_g - g0) : kRowChunk;
+        {
+            const int g0 = (int)(dc - (int64_t)d * n_chunks);
+            const int ng = (n_g - g0 + n_chunks - 1) / n_chunks;
             // q / ng for the pass's pair ids q < kSegTile * ng by a multiply-high:
             // magic = floor((2^32 - 1) / ng) + 1 is at least 2^32 / ng and
             // exceeds it by under one, so q magic / 2^32 lies in
-            // [q / ng, q / ng + q / 2^32) and its floor is exact for q < 2^32 / ng.
+            // [q / ng, q / ng + q / 2^32) and its floor is exact for q < 2^32 / ng
+            // (one row: magic does not fit 32 bits, and the quotient is q).
             const unsigned ng_magic = (unsigned)(0xFFFFFFFFull / (unsigned)ng) + 1u;
-            __syncthreads();
-            for (int j = tid; j < ng; j += blockDim.x) {
-                const int g = g0 + j;
+            const auto seg_of = [&](int q) { return ng == 1 ? q : (int)__umulhi((unsigned)q, ng_magic); };
+            for (int j = tid; j < (dc != d_ch ? ng : 0); j += blockDim.x) {
+                const int g = g0 + j * n_chunks;
                 RowPre<Real> &r = rows[j];
                 const double *G = a.tables.G + 3 * g;
                 const double *ES = a.tables.ES + 3 * ((int64_t)d * n_g + g);
@@ -1301,24 +1449,40 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
                 r.wm = (Real)a.tables.WM[g];
                 r.row = a.tables.row_table[g];
             }
+            d_ch = dc;
             __syncthreads();
             // ---- A0: prefilter and compact the surviving pairs ----
             const int n_pairs = nst * ng;
             int n_surv;
             if (dtail != nullptr) {
+                // Lane ``it`` keeps the survivors' mask of the warp's iteration
+                // ``it`` (at most pair_queue / kCxrThreads = 8 of them): one
+                // shared counter update a warp and pass.
                 const int n_it0 = (n_pairs + (int)blockDim.x - 1) / (int)blockDim.x;
+                unsigned mine = 0;
                 for (int it = 0; it < n_it0; ++it) {
                     const int q = it * blockDim.x + tid;
                     bool ok = false;
                     if (q < n_pairs) {
-                        const int si = (int)__umulhi((unsigned)q, ng_magic);
+                        const int si = seg_of(q);
                         ok = pair_may_keep<Real>(segs[si], rows[q - si * ng], E_tab, dtail, n_tab, a.tables, ti);
                     }
                     const unsigned mask = __ballot_sync(0xffffffffu, ok);
-                    int base = 0;
-                    if (lane == 0 && mask) base = atomicAdd(&p_count, __popc(mask));
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    if (ok) pq[base + __popc(mask & ((1u << lane) - 1u))] = q;
+                    if ((int)lane == it) mine = mask;
+                }
+                int incl = __popc(mine);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if ((int)lane >= o) incl += v;
+                }
+                int base = 0;
+                if (lane == 31 && incl) base = atomicAdd(&p_count, incl);
+                base = __shfl_sync(0xffffffffu, base, 31) + incl - __popc(mine);  // of iteration ``lane``
+                for (int it = 0; it < n_it0; ++it) {
+                    const unsigned mask = __shfl_sync(0xffffffffu, mine, it);
+                    const int at = __shfl_sync(0xffffffffu, base, it);
+                    if ((mask >> lane) & 1u)
+                        pq[at + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)(it * blockDim.x + tid);
                 }
                 __syncthreads();
                 n_surv = p_count;
@@ -1332,13 +1496,13 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
                 Line<Real> ln;
                 ln.good = false;
                 if (k < n_surv) {
-                    const int q = dtail != nullptr ? pq[k] : k;
-                    const int si = (int)__umulhi((unsigned)q, ng_magic);
+                    const int q = dtail != nullptr ? (int)pq[k] : k;
+                    const int si = seg_of(q);
                     const int gi = q - si * ng;
                     ln = pair_line<Real, kLayered>(segs[si], rows[gi], E_tab, delta_tab, log_mu, n_tab, n_mu,
                                                    a.tables, ti, esc + si, a, lay_t);
                     if (pairs_out) {
-                        const int64_t o = ((int64_t)d * n_seg + s0 + si) * n_g + g0 + gi;
+                        const int64_t o = ((int64_t)d * n_seg + s0 + si) * n_g + g0 + gi * n_chunks;
                         a.pair_E[o] = (double)ln.E_res;
                         a.pair_a[o] = (double)ln.a_width;
                         a.pair_w[o] = (double)ln.weight;
@@ -1370,157 +1534,8 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
                     }
                 }
             }
-            if (!binmean) {
-                __syncthreads();
-                if (tid == 0) p_count = 0;
-                continue;
-            }
-            __syncthreads();
-            // ---- B: windows, scan, spread (line, bin) chunks ----
-            const int nq = q_count;
-            for (int j = tid; j < nq; j += blockDim.x) {
-                const LineWindow lw = line_window((double)qE[j], (double)qA[j], ax, exact_widths, K_far,
-                                                  K_far > 0);
-                qStart[j] = lw.nb;
-                qB0[j] = lw.b0;
-                qC[j] = lw.mom ? lw.c : INT_MIN;
-                if (lw.mom)
-                    line_moments((double)qE[j], (double)qA[j], (double)qW[j], lw, ax,
-                                 a.far_moments + (int64_t)d * n_mom * 3);
-                // From here on qW holds the line's mass-to-mean scale w pi / a.
-                qW[j] = (Real)((double)qW[j] * kPi / (double)qA[j]);
-            }
-            __syncthreads();
-            {
-                const int per = (nq + (int)blockDim.x - 1) / (int)blockDim.x;
-                const int j0 = tid * per;
-                int local = 0;
-                for (int j = j0; j < j0 + per && j < nq; ++j) local += qStart[j];
-                int incl = local;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if ((int)lane >= o) incl += v;
-                }
-                if (lane == 31) scratch[tid >> 5] = incl;
-                __syncthreads();
-                if (tid == 0) {
-                    int run = 0;
-                    for (int w = 0; w < n_warps; ++w) { const int v = scratch[w]; scratch[w] = run; run += v; }
-                    scratch[41] = run;
-                }
-                __syncthreads();
-                int run = scratch[tid >> 5] + incl - local;
-                for (int j = j0; j < j0 + per && j < nq; ++j) { const int v = qStart[j]; qStart[j] = run; run += v; }
-                __syncthreads();
-                if (tid == 0) qStart[nq] = scratch[41];
-                __syncthreads();
-            }
-            const int n_items = qStart[nq];
-            if (a.counters && tid == 0) {
-                atomicAdd(&a.counters[0], (unsigned long long)nq);
-                atomicAdd(&a.counters[1], (unsigned long long)n_items);
-            }
-            // Each thread walks one contiguous run of (line, bin) items: one
-            // line search per pass, line constants held in registers, and
-            // consecutive bins of a line share their edge evaluations.
-            {
-                const int per = (n_items + (int)blockDim.x - 1) / (int)blockDim.x;
-                const int i_begin = min(tid * per, n_items);
-                const int i_end = min(i_begin + per, n_items);
-                int line = 0;
-                if (i_begin < i_end) {
-                    int lo = 0, hi = nq;  // last line with qStart[line] <= i_begin
-                    while (hi - lo > 1) {
-                        const int mid = (lo + hi) >> 1;
-                        if (qStart[mid] <= i_begin) lo = mid; else hi = mid;
-                    }
-                    line = lo - 1;
-                }
-                int next = i_begin, start = 0;
-                LineWindow lw{};
-                LineDep L{};
-                float Er_f = 0.0f, s_f = 0.0f, scale_f = 0.0f, Ec_f = 0.0f;
-                EdgeCache ec;
-                ec.valid = false;
-                EdgeCacheF ecf;
-                ecf.valid = false;
-                for (int item = i_begin; item < i_end; ++item) {
-                    if (item >= next) {
-                        do {
-                            ++line;
-                            next = qStart[line + 1];
-                        } while (item >= next);
-                        start = qStart[line];
-                        lw.c = qC[line];
-                        lw.mom = lw.c != INT_MIN;
-                        lw.b0 = qB0[line];
-                        L = LineDep{(double)qE[line], (double)qA[line] * kInvPi, (double)qW[line]};
-                        if constexpr (kMixed) {
-                            Er_f = (float)qE[line];
-                            s_f = (float)qA[line] * (float)kInvPi;
-                            scale_f = (float)qW[line];
-                            Ec_f = lw.mom ? (float)centre_of(ax, lw.c) : 0.0f;
-                        }
-                        ec.valid = false;
-                        ecf.valid = false;
-                    }
-                    const int b = lw.b0 + (item - start);
-                    if constexpr (kMixed) {
-                        float vf;
-                        bin_fast_f32(Er_f, s_f, scale_f, b, lw.c, Ec_f, edges_f, ax.uniform, (float)ax.inv_w, K_far,
-                                     ecf, vf);
-                        smem_add(&spec_f[b], vf);
-                    } else {
-                        double v;
-                        const int cls = bin_fast<kMixed>(L, b, lw, ax, K_far, ec, v);
-                        if (cls != kBinDone) {
-                            const int slot = use_xq ? atomicAdd(&xq_count[cls - 1], 1) : kXQueue;
-                            if (slot < kXQueue) {
-                                xq[(cls - 1) * kXQueue + slot] = (line << 21) | b;
-                                continue;
-                            }
-                            v = bin_exact<kMixed>(L, b, lw, ax, K_far);  // queue full
-                        }
-                        smem_add(&spec_s[b], v);
-                    }
-                }
-            }
-            // Queued exact bins, one class at a time.
-            __syncthreads();
-            for (int cls = 0; cls < 2; ++cls) {
-                const int nx = min(xq_count[cls], kXQueue);
-                for (int k = tid; k < nx; k += blockDim.x) {
-                    const int packed = xq[cls * kXQueue + k];
-                    const int line = packed >> 21;
-                    const int b = packed & ((1 << 21) - 1);
-                    LineWindow lw;
-                    lw.c = qC[line];
-                    lw.mom = lw.c != INT_MIN;
-                    lw.b0 = qB0[line];
-                    const LineDep L{(double)qE[line], (double)qA[line] * kInvPi, (double)qW[line]};
-                    const double v = bin_exact<kMixed>(L, b, lw, ax, K_far);
-                    if constexpr (kMixed) smem_add(&spec_f[b], (float)v);
-                    else smem_add(&spec_s[b], v);
-                }
-            }
-            if constexpr (kMixed) {
-                // Fold the float partials into the FP64 spectrum once per
-                // segment tile (after its last row chunk, uniform over the
-                // block): a tile's few hundred (line, bin) adds per bin keep
-                // float well inside the path's tolerance.
-                if (g0 + kRowChunk >= n_g) {
-                    __syncthreads();
-                    for (int j = tid; j < n_E; j += blockDim.x) {
-                        const float v = spec_f[j];
-                        if (v != 0.0f) { spec_s[j] += (double)v; spec_f[j] = 0.0f; }
-                    }
-                }
-            }
-            __syncthreads();
-            if (tid == 0) { q_count = 0; p_count = 0; xq_count[0] = 0; xq_count[1] = 0; }
         }
     }
-    flush(d_cur);
 }
 
 // Far-field finalize: spec[d][b] += sum_c M[d][c] . envelope(b, c) over the
@@ -1683,13 +1698,12 @@ static size_t cxr_smem_bytes(const pb_cxr_args &a, int far_pad, bool with_moment
     constexpr int kRowChunk = row_chunk<Real>();
     constexpr int kQueue = pair_queue<Real>();
     size_t b = sizeof(RowPre<Real>) * kRowChunk + sizeof(SegPre<Real>) * kSegTile + 16;
-    b += sizeof(Real) * 3 * kQueue + sizeof(int) * (4 * kQueue + 1 + 64) + 16;
+    b += sizeof(Real) * 3 * line_queue<Real>() + 16 +
+         (sizeof(WinLine<Real>) + sizeof(uint16_t) * kWinClasses) * kWideCap + sizeof(int) * 64 +
+         sizeof(uint16_t) * kQueue + 16;
     if (a.tables.n_tab <= kMaxTab) b += sizeof(Real) * (size_t)a.tables.n_tab * (3 + a.tables.n_mu);
     b += 16;
-    if (a.quadrature == PB_QUAD_BINMEAN) {
-        b += (sizeof(double) + sizeof(float)) * (size_t)a.n_E + (sizeof(Real) == 8 ? sizeof(int) * 2 * kXQueue : 0);
-        if (sizeof(Real) == 4) b += sizeof(float) * ((size_t)a.n_E + 1) + 16;
-    }
+    if (a.quadrature == PB_QUAD_BINMEAN) b += (sizeof(double) + (sizeof(Real) == 4 ? sizeof(float) : 0)) * (size_t)a.n_E;
     if (a.n_layer > 0)
         b += 16 + sizeof(EscSeg<Real>) * kSegTile + sizeof(double) * 2 * kMaxEscLayers + sizeof(Real) * kMaxEscLayers;
     return b;
@@ -1706,7 +1720,7 @@ static cudaError_t launch_cxr_t(const pb_cxr_args &a, cudaStream_t s, int sms, i
     if (a.n_layer > 0 && (!a.z_top || !a.z_bot || !a.mu_off || !a.mu_knot || !a.mu_value || !a.mu_slope))
         return cudaErrorInvalidValue;
     size_t smem = cxr_smem_bytes<Real>(a, far_pad, K_far > 0);
-    if (smem > 220 * 1024) return cudaErrorInvalidValue;
+    if (smem > 220 * 1024 || (binmean && a.n_E > 65535)) return cudaErrorInvalidValue;
     // The float path reads its tables from the shared-memory staging only.
     if (sizeof(Real) == 4 && a.tables.n_tab > kMaxTab) return cudaErrorInvalidValue;
     auto kern = a.n_layer > 0 ? cxr_kernel<Real, true> : cxr_kernel<Real, false>;
@@ -1725,7 +1739,8 @@ static cudaError_t launch_cxr_t(const pb_cxr_args &a, cudaStream_t s, int sms, i
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCxrThreads, smem);
     if (err != cudaSuccess) return err;
     if (per_sm < 1) per_sm = 1;
-    const int64_t work = (a.n_seg + kSegTile - 1) / kSegTile * (int64_t)a.n_dir;
+    constexpr int kRowChunk = row_chunk<Real>();
+    const int64_t work = (a.n_seg + 3) / 4 * (int64_t)a.n_dir * ((a.tables.n_g + kRowChunk - 1) / kRowChunk);
     int64_t gx = (int64_t)sms * per_sm;
     if (gx > work) gx = work;
     if (gx < 1) gx = 1;
@@ -1814,6 +1829,7 @@ __device__ bool coh_record(const pb_cxr_args &a, const double *t_start, int64_t 
     const int n_tab = a.tables.n_tab;
     const PairAmps<double> p = pair_amps<double, false>(sp, rw, a.tables.E_tab, a.tables.delta, a.tables.log_mu,
                                                         n_tab, a.tables.n_mu, a.tables, ti);
+    if (!p.keep) return false;
     double apb, bma, qq;
     formation_coefficients(sp.path0 * p.mu, sp.path1 * p.mu, apb, bma, qq);
     // exact vacuum centre / width and recoil phase over the age, with the

@@ -28,9 +28,10 @@ constexpr int kBremChunk = 256;
 constexpr int kBremMaxEl = 4;
 constexpr int kBremMaxDir = 16;
 
-// A staged segment. FP64 keeps the reference's factors; the float path
-// folds the per-segment ones of its cross-section form (brem_nsig):
-// beta_i holds beta_i / p_i^2 and nL[el] holds n_el L Z_el^2 den_i[el].
+// A staged segment with the per-segment factors of the cross section folded in
+// (brem_nsig), den_i = 1 - exp(-2 pi Z alpha / beta_i): the float path's beta_i
+// holds beta_i / p_i^2 and its nL[el] holds n_el L Z_el^2 den_i[el]; FP64 keeps
+// them all in nL[el] = n_el L Z_el^2 den_i[el] beta_i / p_i^2.
 template <class Real>
 struct alignas(sizeof(Real) == 4 ? 16 : 8) BremSeg {
     Real T;       // keV
@@ -42,8 +43,6 @@ struct alignas(sizeof(Real) == 4 ? 16 : 8) BremSeg {
     // reciprocal (inv_e2, infinite for a segment parallel to the faces).
     Real e0, e1, e2, inv_e2;
     Real nL[kBremMaxEl];     // n_el * 1e24 * L * 1e-8  [1/cm^2]
-    // 1 - exp(-2 pi Z alpha / beta_i); the float path folds it into nL.
-    Real den_i[sizeof(Real) == 8 ? kBremMaxEl : 1];
 };
 
 __device__ __forceinline__ double b_sqrt(double x) { return sqrt(x); }
@@ -159,12 +158,9 @@ __device__ __forceinline__ void brem_stage(BremSeg<Real> &b, const pb_brem_args 
     for (int el = 0; el < a.n_el; ++el) {
         b.nL[el] = rad ? (Real)(a.n_ang3[el] * 1e24) * (Real)1 * path_cm : (Real)0;
         const Real den_i = (Real)1 - b_exp(-za * (Real)a.Z[el] / b.beta_i);
-        if constexpr (sizeof(Real) == 4) {
-            const Real Z = (Real)a.Z[el];
-            b.nL[el] *= Z * Z * den_i;
-        } else {
-            b.den_i[el] = den_i;
-        }
+        const Real Z = (Real)a.Z[el];
+        b.nL[el] *= Z * Z * den_i;
+        if constexpr (sizeof(Real) == 8) b.nL[el] *= b.beta_i / (p_i * p_i);
     }
     if constexpr (sizeof(Real) == 4) b.beta_i = b.beta_i / (p_i * p_i);
 }
@@ -174,6 +170,7 @@ struct BremKConst {
     float kc;     // k / (m c^2)^2  [1/keV]
     float c2mk;   // 2 m c^2 - k    [keV]
     float c0k;    // c0 ln 2 / k_ev
+    double c0k64; // c0 / k_ev (FP64 path)
 };
 
 // sum_el n_el L dsigma/dk(Z_el, T, k) of one staged segment (brem.py:396-479).
@@ -192,15 +189,13 @@ __device__ __forceinline__ Real brem_nsig(const BremSeg<Real> &b, Real k, Real T
     const int n_el = NEL > 0 ? NEL : n_el_rt;
     Real nsig = 0;
     if constexpr (sizeof(Real) == 8) {
+        // p_f with the reference's own rounding: p_i - p_f cancels (k << T)
         const Real p_f = b_sqrt(T_f * (T_f + (Real)2 * mc2)) / mc2;
-        const Real beta_f = p_f / ((Real)1 + T_f / mc2);
+        const Real inv_beta_f = fma(T_f, (Real)(1.0 / 510.99895), (Real)1) / p_f;
         const Real born_log = b_log((b.p_i + p_f) / fmax(b.p_i - p_f, (Real)1e-30));
-        for (int el = 0; el < n_el; ++el) {
-            const Real Z = Zs[el];
-            const Real elwert = b.beta_i / beta_f * b.den_i[el] / ((Real)1 - b_exp(-za * Z / beta_f));
-            const Real dsig = c0 * (Z * Z) / k_ev / (b.p_i * b.p_i) * born_log * elwert;
-            nsig += b.nL[el] * dsig;
-        }
+        const Real common = kk.c0k64 * born_log * inv_beta_f;
+        for (int el = 0; el < n_el; ++el)  // nL holds n L Z^2 den_i beta_i / p_i^2
+            nsig += b.nL[el] * common / ((Real)1 - b_exp(-za * Zs[el] * inv_beta_f));
     } else {
         const float inv_mc2 = 1.0f / 510.99895f;
         const float q = T_f * (T_f + 2.0f * mc2);
@@ -389,11 +384,12 @@ __device__ __forceinline__ void brem_J2(F2 Tf, float T, float p_i, float bp, F2 
     }
 }
 
-
-// Whether the launch's directions take the packed moment kernel: one exit
-// face and relative spread rho = Delta / f_min <= 0.01 (the same test both
-// brem kernels make, so exactly one of them scores the launch).
-__device__ __forceinline__ bool brem_packed_applies(const pb_brem_args &a, int d0, int nd, double &f_c, double &dl) {
+// Whether the directions d0 .. d0 + nd - 1 leave through one face with path
+// factors in f_c +- dl, dl <= limit f_min. The kernels that share a launch make
+// the same test, so exactly one of them scores it: limit 0.01 for the packed
+// moment kernel.
+__device__ __forceinline__ bool brem_one_face(const pb_brem_args &a, int d0, int nd, double limit, double &f_c,
+                                              double &dl) {
     int n_up = 0;
     double f_lo = 1e300, f_hi = 0.0;
     for (int dd = 0; dd < nd; ++dd) {
@@ -405,13 +401,81 @@ __device__ __forceinline__ bool brem_packed_applies(const pb_brem_args &a, int d
     }
     f_c = 0.5 * (f_lo + f_hi);
     dl = 0.5 * (f_hi - f_lo);
-    return (n_up == nd || n_up == 0) && dl <= 0.01 * f_lo;
+    return (n_up == nd || n_up == 0) && dl <= limit * f_lo;
 }
 
 template <int N>
 struct MomentOrder {
     static constexpr int value = N;
 };
+
+// Direction moments of the FP64 path and of the layered absorber: the same
+// recurrence as the packed kernel's. The truncation after order N is below
+// rho^(N+1) / sqrt(2 pi (N+1)) of the unattenuated term: FP64 takes N = 5 for
+// rho <= 0.002 and N = 9 for rho <= 0.02 (both below 2e-17), the mixed layered
+// path N = 3 for rho <= 0.01 (2e-9).
+template <class Real>
+constexpr double moment_limit() { return sizeof(Real) == 8 ? 0.02 : 0.01; }
+
+// Q_n += w P_n of one affine piece: a = optical depth of its shallower end along
+// the face normal, b = the depth difference of its ends, both per unit path
+// factor. Two exponentials serve every direction of the group, where each
+// direction took two of its own.
+template <int N>
+__device__ __forceinline__ void add_moments(double w, double a, double b, double f_c, double dl, double (&Q)[N + 1]) {
+    const double x = b * f_c;
+    const double Ea = exp(-a * f_c), em = -expm1(-x);
+    double P = w * Ea * f_c * (x > 1.0e-5 ? em / x : 1.0 - 0.5 * x + x * x / 6.0);
+    Q[0] += P;
+    if constexpr (N > 0) {
+        const double ah = -dl * a, ch = -dl * (a + b);
+        double R = w * dl * (Ea - Ea * em);
+#pragma unroll
+        for (int n = 1; n <= N; ++n) {
+            P = fma(ah, P, R);
+            R *= ch;
+            Q[n] += P;
+        }
+    }
+}
+template <int N>
+__device__ __forceinline__ void add_moments(float w, float a, float b, float f_c, float dl, float (&Q)[N + 1]) {
+    constexpr float kLog2e = 1.44269504f;
+    const float x = b * f_c;
+    const float Ea = ex2_approx(-kLog2e * a * f_c);
+    float P, Ec;
+    if (x > 0.35f) {
+        Ec = ex2_approx(-kLog2e * (a + b) * f_c);
+        P = w * (Ea - Ec) * (f_c * rcp_approx(x));
+    } else {
+        // phi(x) = (1 - e^-x) / x to x^7: truncation below 1e-9
+        const float phi = fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, -1.0f / 40320.0f, 1.0f / 5040.0f),
+                                                                              -1.0f / 720.0f), 1.0f / 120.0f),
+                                                       -1.0f / 24.0f), 1.0f / 6.0f), -0.5f), 1.0f);
+        P = w * Ea * f_c * phi;
+        Ec = Ea - Ea * (x * phi);
+    }
+    Q[0] += P;
+    if constexpr (N > 0) {
+        const float ah = -dl * a, ch = -dl * (a + b);
+        float R = w * dl * Ec;
+#pragma unroll
+        for (int n = 1; n <= N; ++n) {
+            P = fmaf(ah, P, R);
+            R *= ch;
+            Q[n] += P;
+        }
+    }
+}
+
+// (1 / f) sum_n ((f - f_c) / dl)^n Q_n / n! from the summed moments Q(n).
+template <class F>
+__device__ __forceinline__ double moments_at(int N, double f, double f_c, double dl, F Q) {
+    const double h = dl > 0.0 ? (f - f_c) / dl : 0.0;
+    double v = Q(N);
+    for (int n = N; n > 0; --n) v = fma(v, h / (double)n, Q(n - 1));
+    return v / f;
+}
 
 template <int NEL>
 __global__ void __launch_bounds__(kBremPackedThreads, 3)
@@ -428,7 +492,7 @@ __global__ void __launch_bounds__(kBremPackedThreads, 3)
     __shared__ Pk pk[kBremChunk];
     const int nd = (a.n_dir - d0) < kBremMaxDir ? (a.n_dir - d0) : kBremMaxDir;
     double f_c_d, dl_d;
-    if (a.precision != PB_MIXED || !brem_packed_applies(a, d0, nd, f_c_d, dl_d)) return;
+    if (a.precision != PB_MIXED || !brem_one_face(a, d0, nd, 0.01, f_c_d, dl_d)) return;
     const bool up_all = a.n_hat[3 * d0 + 2] < 0.0;
     // Moment order: 2 where rho = Delta / f_min <= 0.002 (truncation below
     // rho^3 / sqrt(6 pi) < 2e-9 of the unattenuated term), else 3.
@@ -729,7 +793,7 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
     // (brem_moment_packed_kernel) scores this launch.
     if constexpr (sizeof(Real) == 4) {
         double fc_p, dl_p;
-        if (brem_packed_applies(a, d0, nd, fc_p, dl_p)) return;
+        if (brem_one_face(a, d0, nd, 0.01, fc_p, dl_p)) return;
     }
     // Moment form (see brem_moment_chunk): float, one exit face, and the
     // path factors within rho = Delta / f_min <= 0.05 of their centre.
@@ -754,6 +818,12 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
             mom_invf[threadIdx.x] = (float)(1.0 / f);
         }
     }
+    if constexpr (sizeof(Real) == 8) {
+        if (brem_one_face(a, d0, nd, moment_limit<double>(), f_c, dl)) {
+            const double rho = dl / (f_c - dl);
+            order = dl == 0.0 ? 0 : (rho <= 0.002 ? 5 : 9);
+        }
+    }
     const double k_kev_d = on ? a.E_grid[e] / 1e3 : 1.0;
     const Real k = (Real)k_kev_d;
     const Real mu = on ? (Real)a.mu[e] : (Real)0;
@@ -762,6 +832,7 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
     BremKConst kk;
     kk.kc = (float)(k_kev_d / (510.99895 * 510.99895));
     kk.c2mk = (float)(2.0 * 510.99895 - k_kev_d);
+    kk.c0k64 = 16.0 / 3.0 * kAlphaFs * kReCm2 / fmax(k_kev_d * 1e3, 1e-30);
     kk.c0k = (float)(16.0 / 3.0 * kAlphaFs * kReCm2 * 0.6931471805599453 / fmax(k_kev_d * 1e3, 1e-30));
 #pragma unroll
     for (int j = 0; j < kBremMaxDir; ++j) acc[j][threadIdx.x] = 0.0;
@@ -815,6 +886,30 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
                     for (int dd = 0; dd < nd; ++dd)
                         acc[dd][threadIdx.x] += (double)brem_moment_eval<5>(Q, mom_h[dd]) * (double)mom_invf[dd];
                 }
+                continue;
+            }
+        }
+        if constexpr (sizeof(Real) == 8) {
+            // acc[n] holds the thread's summed moment n until the end
+            const bool up_all = side_all > 0;
+            const auto moments = [&](auto tag) {
+                constexpr int N = decltype(tag)::value;
+                double Q[N + 1] = {};
+                for (int j = 0; j < nc; ++j) {
+                    const BremSeg<double> &b = segs[j];
+                    const double T_f = b.T - k;
+                    if (!(T_f > 1e-6 && k > 0.0)) continue;
+                    const double nsig = brem_nsig<double, NEL>(b, k, T_f, Zs, n_el, k_ev, c0, za, mc2, kk, zl);
+                    const double lo = up_all ? fmin(b.e0, b.e1) : T_slab - fmax(b.e0, b.e1);
+                    add_moments<N>(nsig, mu * lo, mu * fabs(b.e1 - b.e0), f_c, dl, Q);
+                }
+#pragma unroll
+                for (int n = 0; n <= N; ++n) acc[n][threadIdx.x] += Q[n];
+            };
+            if (order >= 0) {
+                if (order == 0) moments(MomentOrder<0>{});
+                else if (order == 5) moments(MomentOrder<5>{});
+                else moments(MomentOrder<9>{});
                 continue;
             }
         }
@@ -879,6 +974,17 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
             for (int dd = 0; dd < kBremMaxDir; ++dd) acc[dd][threadIdx.x] += (double)part[dd];
         }
     }
+    if constexpr (sizeof(Real) == 8) {
+        if (order >= 0) {
+            if (on)
+                for (int dd = 0; dd < nd; ++dd) {
+                    const double f = 1.0 / fmax(fabs(a.n_hat[3 * (d0 + dd) + 2]), 1.0e-12);
+                    const double v = moments_at(order, f, f_c, dl, [&](int n) { return acc[n][threadIdx.x]; });
+                    if (v != 0.0) atomicAdd(&a.spec[(int64_t)(d0 + dd) * a.n_E + e], v);
+                }
+            return;
+        }
+    }
     if (on) {
 #pragma unroll
         for (int dd = 0; dd < kBremMaxDir; ++dd)
@@ -901,12 +1007,21 @@ struct BremPieces {
 
 constexpr int kBremChunkLayered = 64;
 
-template <class Real>
+// Blocks gather the emitting layer's segments of their slice into a list and
+// stage whole chunks of it: a layer's set of a stack radiates from its own
+// segments alone, most of which sit in other layers' sets. Directions of one
+// detector (one face, narrow spread) go through the moments (kMoments); the
+// others are scored one by one, two exponentials each. Measured on the three
+// layers of the 10 MeV stack (160,000 segments, 4096 energies, 64 directions).
+template <class Real, bool kMoments>
 __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_brem_args a, int64_t n_seg, int d0) {
     constexpr int kChunk = kBremChunkLayered;
     __shared__ BremSeg<Real> segs[kChunk];
     __shared__ BremPieces<Real> pcs[kChunk];
-    __shared__ double acc[kBremMaxDir][kBremThreads];
+    __shared__ int list[kChunk + kBremThreads];  // emitting segments of the slice, offsets from s_begin
+    __shared__ int n_list;
+    constexpr int kOrder = sizeof(Real) == 8 ? 9 : 3;  // highest moment
+    __shared__ double acc[kMoments ? kOrder + 1 : kBremMaxDir][kBremThreads];
     __shared__ Real Zs[kBremMaxEl];
     __shared__ float zl[kBremMaxEl];  // 2 pi alpha Z log2(e)
     __shared__ Real inv_nz[kBremMaxDir];
@@ -914,6 +1029,9 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     __shared__ double zt_s[kMaxEscLayers], zb_s[kMaxEscLayers];
     __shared__ int bad;
     const int nd = (a.n_dir - d0) < kBremMaxDir ? (a.n_dir - d0) : kBremMaxDir;
+    double f_c, dl;
+    // both instances make the same test: one of them scores the launch
+    if (brem_one_face(a, d0, nd, moment_limit<Real>(), f_c, dl) != kMoments) return;
     const int n_el = a.n_el;
     const int nl = a.n_layer;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -973,9 +1091,10 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     BremKConst kk;
     kk.kc = (float)(k_kev_d / (510.99895 * 510.99895));
     kk.c2mk = (float)(2.0 * 510.99895 - k_kev_d);
+    kk.c0k64 = 16.0 / 3.0 * kAlphaFs * kReCm2 / fmax(k_kev_d * 1e3, 1e-30);
     kk.c0k = (float)(16.0 / 3.0 * kAlphaFs * kReCm2 * 0.6931471805599453 / fmax(k_kev_d * 1e3, 1e-30));
 #pragma unroll
-    for (int j = 0; j < kBremMaxDir; ++j) acc[j][threadIdx.x] = 0.0;
+    for (int j = 0; j < (kMoments ? kOrder + 1 : kBremMaxDir); ++j) acc[j][threadIdx.x] = 0.0;
     if (a.n_seg_device) {
         const int64_t live = (int64_t)*a.n_seg_device;
         if (live < n_seg) n_seg = live;
@@ -987,11 +1106,30 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     int64_t s_end = s_begin + per < n_seg ? s_begin + per : n_seg;
     if (s_end < s_begin) s_end = s_begin;
     const Real T_stack = (Real)zb_s[nl - 1];
-    for (int64_t c0s = s_begin; c0s < s_end; c0s += kChunk) {
-        const int nc = (int)((s_end - c0s) < kChunk ? (s_end - c0s) : kChunk);
+    const bool up_all = a.n_hat[3 * d0 + 2] < 0.0;
+    if (threadIdx.x == 0) n_list = 0;
+    int64_t next = s_begin;  // first segment not looked at yet
+    while (true) {
         __syncthreads();
+        int have = n_list;
+        while (have < kChunk && next < s_end) {
+            __syncthreads();  // every thread has read n_list
+            const int64_t s = next + threadIdx.x;
+            const bool rad = s < s_end && a.elec_id[s] < a.Ne && (a.seg_layer == nullptr || a.seg_layer[s] == a.emit_layer);
+            const unsigned mask = __ballot_sync(0xffffffffu, rad);
+            const int lane = threadIdx.x & 31;
+            int base = 0;
+            if (lane == 0 && mask) base = atomicAdd(&n_list, __popc(mask));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (rad) list[base + __popc(mask & ((1u << lane) - 1u))] = (int)(s - s_begin);
+            next += kBremThreads;
+            __syncthreads();
+            have = n_list;
+        }
+        const int nc = have < kChunk ? have : kChunk;
+        if (nc == 0) break;
         for (int j = threadIdx.x; j < nc; j += blockDim.x) {
-            const int64_t s = c0s + j;
+            const int64_t s = s_begin + list[have - nc + j];
             brem_stage<Real>(segs[j], a, s, T_stack, mc2, za);
             const double half = 0.5 * a.L[s];
             const double z = a.r_mid[3 * s + 2], vz = a.v_hat[3 * s + 2];
@@ -1007,17 +1145,28 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
             }
         }
         __syncthreads();
+        if (threadIdx.x == 0) n_list = have - nc;
         if (!on) continue;
-        Real part[kBremMaxDir];
+        constexpr int kPart = kMoments ? kOrder + 1 : kBremMaxDir;
+        Real part[kPart];
 #pragma unroll
-        for (int dd = 0; dd < kBremMaxDir; ++dd) part[dd] = 0;
+        for (int dd = 0; dd < kPart; ++dd) part[dd] = 0;
         for (int j = 0; j < nc; ++j) {
             const BremSeg<Real> &b = segs[j];
             const Real T_f = b.T - k;
             if (!(T_f > (Real)1e-6 && k > (Real)0)) continue;
             const Real nsig = brem_nsig<Real>(b, k, T_f, Zs, n_el, k_ev, c0, za, mc2, kk, zl);
             const BremPieces<Real> &P = pcs[j];
-            for (int p = 0; p < P.np; ++p) {
+            if constexpr (kMoments) {
+                for (int p = 0; p < P.np; ++p) {
+                    const int m = P.m[p];
+                    const Real mum = esc_pick<Real>(mu_l, m);
+                    // the piece end nearer the exit face
+                    const Real lo = up_all ? esc_pick<Real>(c_up, m) + mum * fmin(P.u0[p], P.u1[p])
+                                           : esc_pick<Real>(c_dn, m) + mum * (esc_pick<Real>(t_l, m) - fmax(P.u0[p], P.u1[p]));
+                    add_moments<kOrder>(nsig * P.f[p], lo, mum * fabs(P.u1[p] - P.u0[p]), (Real)f_c, (Real)dl, part);
+                }
+            } else for (int p = 0; p < P.np; ++p) {
                 const int m = P.m[p];
                 const Real mum = esc_pick<Real>(mu_l, m), tm = esc_pick<Real>(t_l, m);
                 const Real cu = esc_pick<Real>(c_up, m), cd = esc_pick<Real>(c_dn, m);
@@ -1025,7 +1174,7 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
                 const Real dn0 = cd + mum * (tm - P.u0[p]), dn1 = cd + mum * (tm - P.u1[p]);
                 const Real w = nsig * P.f[p];
 #pragma unroll
-                for (int dd = 0; dd < kBremMaxDir; ++dd) {
+                for (int dd = 0; dd < kPart; ++dd) {
                     if (dd < nd) {
                         const Real f = inv_nz[dd];
                         const Real t0 = (up[dd] ? up0 : dn0) * f;
@@ -1036,9 +1185,16 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
             }
         }
 #pragma unroll
-        for (int dd = 0; dd < kBremMaxDir; ++dd) acc[dd][threadIdx.x] += (double)part[dd];
+        for (int dd = 0; dd < kPart; ++dd) acc[dd][threadIdx.x] += (double)part[dd];
     }
-    if (on) {
+    if constexpr (kMoments) {
+        if (on)
+            for (int dd = 0; dd < nd; ++dd) {
+                const double f = 1.0 / fmax(fabs(a.n_hat[3 * (d0 + dd) + 2]), 1.0e-12);
+                const double v = moments_at(kOrder, f, f_c, dl, [&](int n) { return acc[n][threadIdx.x]; });
+                if (v != 0.0) atomicAdd(&a.spec[(int64_t)(d0 + dd) * a.n_E + e], v);
+            }
+    } else if (on) {
 #pragma unroll
         for (int dd = 0; dd < kBremMaxDir; ++dd)
             if (dd < nd && acc[dd][threadIdx.x] != 0.0)
@@ -1051,24 +1207,26 @@ cudaError_t launch_brem(const pb_brem_args &a, cudaStream_t s, int sms) {
     if (a.n_layer > 0) {
         if (a.n_layer > kMaxEscLayers) return cudaErrorInvalidValue;
         const unsigned gx = (unsigned)((a.n_E + kBremThreads - 1) / kBremThreads);
-        int per_sm = 0;
-        cudaError_t oe = a.precision == PB_MIXED
-                             ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, brem_layered_kernel<float>,
-                                                                             kBremThreads, 0)
-                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, brem_layered_kernel<double>,
-                                                                             kBremThreads, 0);
-        if (oe != cudaSuccess) return oe;
-        if (per_sm < 1) per_sm = 1;
-        int64_t gy = (int64_t)sms * per_sm / (int64_t)gx;
-        const int64_t max_y = (a.n_seg + kBremChunkLayered - 1) / kBremChunkLayered;
-        if (gy > max_y) gy = max_y;
-        if (gy < 1) gy = 1;
-        dim3 grid(gx, (unsigned)gy, 1);
-        for (int d0 = 0; d0 < a.n_dir; d0 += kBremMaxDir) {
-            if (a.precision == PB_MIXED) brem_layered_kernel<float><<<grid, kBremThreads, 0, s>>>(a, a.n_seg, d0);
-            else brem_layered_kernel<double><<<grid, kBremThreads, 0, s>>>(a, a.n_seg, d0);
-            cudaError_t err = cudaGetLastError();
-            if (err != cudaSuccess) return err;
+        using LKern = void (*)(const pb_brem_args, int64_t, int);
+        const LKern kerns[2] = {a.precision == PB_MIXED ? (LKern)brem_layered_kernel<float, true>
+                                                        : (LKern)brem_layered_kernel<double, true>,
+                                a.precision == PB_MIXED ? (LKern)brem_layered_kernel<float, false>
+                                                        : (LKern)brem_layered_kernel<double, false>};
+        for (int k = 0; k < 2; ++k) {
+            int per_sm = 0;
+            const cudaError_t oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[k], kBremThreads, 0);
+            if (oe != cudaSuccess) return oe;
+            if (per_sm < 1) per_sm = 1;
+            int64_t gy = (int64_t)sms * per_sm / (int64_t)gx;
+            const int64_t max_y = (a.n_seg + kBremChunkLayered - 1) / kBremChunkLayered;
+            if (gy > max_y) gy = max_y;
+            if (gy < 1) gy = 1;
+            const dim3 grid(gx, (unsigned)gy, 1);
+            for (int d0 = 0; d0 < a.n_dir; d0 += kBremMaxDir) {
+                kerns[k]<<<grid, kBremThreads, 0, s>>>(a, a.n_seg, d0);
+                const cudaError_t err = cudaGetLastError();
+                if (err != cudaSuccess) return err;
+            }
         }
         return cudaSuccess;
     }

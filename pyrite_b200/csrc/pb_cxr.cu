@@ -958,7 +958,7 @@ __device__ __forceinline__ R window_midpoint(R xc, R Dm, R d, R sw) {
 // One line of the window list, read back as broadcasts.
 template <class R>
 struct alignas(16) WinLine {
-    R sw, scale, d, E_r;  // bin width in first-zero units, w / a, (E_r - E_c) / bin width
+    R s, scale, d, E_r;   // a / pi, w / a, (E_r - E_c) / bin width
     int c, D0, D1;        // centre bin, window bins D0 <= |b - c| <= D1 on the axis
     int pad;
 };
@@ -1045,8 +1045,9 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     double *spec_s = reinterpret_cast<double *>(cur);
     const int n_mom = n_E + 2 * far_pad;
     float *spec_f = reinterpret_cast<float *>(spec_s + (binmean ? n_E : 0));  // mixed path: float partials
+    float *edges_f = spec_f + (binmean && kMixed ? n_E : 0);                    // and float bin edges
     // Layered absorber: per-segment escape pieces, layer thicknesses and bounds.
-    unsigned char *esc_raw = reinterpret_cast<unsigned char *>(spec_f + (binmean && kMixed ? n_E : 0));
+    unsigned char *esc_raw = reinterpret_cast<unsigned char *>(edges_f + (binmean && kMixed ? n_E + 1 : 0));
     esc_raw = (unsigned char *)(((uintptr_t)esc_raw + 15) & ~(uintptr_t)15);
     EscSeg<Real> *esc = reinterpret_cast<EscSeg<Real> *>(esc_raw);
     double *lay_zt = reinterpret_cast<double *>(esc + (kLayered ? kSegTile : 0));
@@ -1073,7 +1074,10 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     if (binmean) {
         for (int j = tid; j < n_E; j += blockDim.x) spec_s[j] = 0.0;
         if (kMixed)
-            for (int j = tid; j < n_E; j += blockDim.x) spec_f[j] = 0.0f;
+            for (int j = tid; j <= n_E; j += blockDim.x) {
+                if (j < n_E) spec_f[j] = 0.0f;
+                edges_f[j] = (float)a.edges[j];
+            }
     }
     if (tid == 0) { q_count = 0; p_count = 0; w_count = 0; strip_next = 0; }
     if (tid < kWinClasses) w_class[tid] = 0;
@@ -1128,7 +1132,14 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     const bool pairs_out = a.pair_E != nullptr;
     const bool lines_out = a.line_E != nullptr;
     const double exact_widths = K_far > 0 ? a.exact_widths : 0.0;
-    const Real inv_w_r = (Real)ax.inv_w;
+    const Real w_r = (Real)ax.w, inv_w_r = (Real)ax.inv_w;
+    const Real s_narrow = (Real)(0.1 * ax.inv_w);  // uniform axis: bins of 0.1 first-zero widths
+    // Bin edge j, clamped to the axis (a clamped edge bounds no bin).
+    const auto edge_at = [&](int j) {
+        j = min(max(j, 0), n_E);
+        if constexpr (kMixed) return edges_f[j];
+        else return ax.edges[j];
+    };
     // B adds into float partials on the mixed path, else into the spectrum.
     auto *const spec_part = [&] {
         if constexpr (kMixed) return spec_f;
@@ -1146,6 +1157,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
             const LineWindow lw = line_window(Ed, inv_a, ax, exact_widths, K_far, K_far > 0);
             const Real sx = (Real)(kMixed ? (float)qA[j] * (float)kInvPi : (double)qA[j] * kInvPi);
             wl.E_r = qE[j];
+            wl.s = sx;
             wl.scale = (Real)(wd * inv_a);
             if (a.counters) {
                 atomicAdd(&a.counters[0], 1ULL);
@@ -1153,7 +1165,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
             }
             if (lw.mom) {
                 line_moments(Ed, inv_a, wd, lw, ax, a.far_moments + (int64_t)d * n_mom * 3);
-                wl.sw = sx * (Real)ax.w;
+                const Real sw = sx * w_r;
                 wl.d = (Real)((Ed - centre_of(ax, lw.c)) * ax.inv_w);
                 wl.c = lw.c;
                 if (lw.nb > 0) {
@@ -1165,30 +1177,25 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
                     if (span > 0)
                         cls = span <= 3 ? kWin4 : span <= 7 ? kWin8 : span <= 15 ? kWin16 : span <= kStripSpan ? kWin32 : kWinStrip;
                     // bins narrower than 0.1 first-zero widths take the midpoint series
-                    if (span > 0 && wl.sw <= (Real)0.1) cls = kWinStrip;
+                    if (span > 0 && sx <= s_narrow) cls = kWinStrip;
                 }
                 // the bins c - K_far .. c + K_far, left to right
                 const Real out = wl.scale * (Real)ax.inv_w;
                 const int eb = lw.c - K_far;
-                auto edge_x = [&](int k) {
-                    if constexpr (kMixed) return wl.sw * ((Real)(k - K_far) - (Real)0.5 - wl.d);
-                    else return sx * (ax.edges[min(max(eb + k, 0), n_E)] - wl.E_r);
-                };
-                Real x_lo = edge_x(0);
+                Real x_lo = sx * (edge_at(eb) - wl.E_r);
                 Real f_lo = edge_near_bins<Real>(x_lo);
                 for (int k = 0; k <= 2 * K_far; ++k) {
                     const int bin = eb + k;
-                    const Real x_hi = edge_x(k + 1);
+                    const Real x_hi = sx * (edge_at(bin + 1) - wl.E_r);
                     const Real f_hi = edge_near_bins<Real>(x_hi);
                     Real mass = f_hi - f_lo + ((x_lo < (Real)0 && x_hi >= (Real)0) ? (Real)kPi : (Real)0);
                     const Real xc = (Real)0.5 * (x_lo + x_hi);
-                    if (wl.sw <= (Real)0.1 && fabs(xc) >= (Real)2) mass = (Real)kPi * wl.sw * midpoint_mean(xc, wl.sw);
+                    if (sx <= s_narrow && fabs(xc) >= (Real)2) mass = (Real)kPi * sw * midpoint_mean(xc, sw);
                     if (bin >= 0 && bin < n_E) smem_add(&spec_part[bin], out * mass);
                     x_lo = x_hi;
                     f_lo = f_hi;
                 }
             } else {
-                wl.sw = sx;  // the whole axis: first-zero units per eV
                 if (lw.nb > 0) cls = kWinAxis;
             }
         }
@@ -1215,18 +1222,12 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
         const int Dh = D + 2 * h;                      // distance of this lane's first bin
         const Real Dm = sgn * ((Real)Dh - (Real)0.5);  // its inner edge
         const int bin = left ? l.c - Dh : l.c + Dh;
-        Real x0, x1;
-        if constexpr (kMixed) {
-            x0 = l.sw * (Dm - l.d);
-            x1 = fma(sgn, l.sw, x0);
-        } else {
-            const int edge = left ? bin + 1 : bin;
-            const Real s = l.sw * inv_w_r;
-            x0 = s * (ax.edges[min(max(edge, 0), n_E)] - l.E_r);
-            x1 = s * (ax.edges[min(max(left ? edge - 1 : edge + 1, 0), n_E)] - l.E_r);
-        }
-        const Real f0 = edge_window_bins<Real>(x0, Dm, l.d, l.sw);
-        const Real f1 = edge_window_bins<Real>(x1, Dm + sgn, l.d, l.sw);
+        const int edge = left ? bin + 1 : bin;
+        const Real x0 = l.s * (edge_at(edge) - l.E_r);
+        const Real x1 = l.s * (edge_at(left ? edge - 1 : edge + 1) - l.E_r);
+        const Real sw = l.s * w_r;
+        const Real f0 = edge_window_bins<Real>(x0, Dm, l.d, sw);
+        const Real f1 = edge_window_bins<Real>(x1, Dm + sgn, l.d, sw);
         const Real f2 = __shfl_down_sync(0xffffffffu, f0, 1);
         const Real out = sgn * l.scale * inv_w_r;
         const int next = left ? bin - 1 : bin + 1;
@@ -1256,18 +1257,16 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
         for (int first = warp * kStripBins; first < n_E; first += n_warps * kStripBins) {
             const int last = min(first + kStripBins, n_E) - 1;
             const int bin = first + (int)lane;
-            const double e = kMixed ? 0.0 : ax.edges[min(bin, n_E)];
+            const Real e = edge_at(bin);
             Real acc = 0;
             for (int k = 0; k < nw; ++k) {
                 const WinLine<Real> &l = wLine[wIdx[kWinStrip * kWideCap + k]];
                 if (first > l.c + l.D1 || last < l.c - l.D1) continue;
-                const Real sw = l.sw, D = (Real)(bin - l.c), Dm = D - (Real)0.5;
+                const Real sw = l.s * w_r, D = (Real)(bin - l.c), Dm = D - (Real)0.5;
                 const bool on = fabs(D) >= (Real)l.D0 && fabs(D) <= (Real)l.D1;
-                Real x;
-                if constexpr (kMixed) x = sw * (Dm - l.d);
-                else x = (sw * inv_w_r) * (e - l.E_r);
+                const Real x = l.s * (e - l.E_r);
                 Real mass;
-                if (sw > (Real)0.1) {
+                if (l.s > s_narrow) {
                     const Real f = edge_window_bins<Real>(x, Dm, l.d, sw);
                     mass = __shfl_down_sync(0xffffffffu, f, 1) - f;
                 } else {
@@ -1298,7 +1297,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
             Real acc = 0;
             for (int k = 0; k < nw; ++k) {
                 const WinLine<Real> &l = wLine[wIdx[kWinAxis * kWideCap + k]];
-                const Real x = l.sw * (e - l.E_r);
+                const Real x = l.s * (e - l.E_r);
                 const Real x_hi = __shfl_down_sync(0xffffffffu, x, 1);
                 const Real sw = x_hi - x, xc = (Real)0.5 * (x + x_hi);
                 const bool narrow = sw <= (Real)0.1 && fabs(xc) >= (Real)2;
@@ -1703,7 +1702,8 @@ static size_t cxr_smem_bytes(const pb_cxr_args &a, int far_pad, bool with_moment
          sizeof(uint16_t) * kQueue + 16;
     if (a.tables.n_tab <= kMaxTab) b += sizeof(Real) * (size_t)a.tables.n_tab * (3 + a.tables.n_mu);
     b += 16;
-    if (a.quadrature == PB_QUAD_BINMEAN) b += (sizeof(double) + (sizeof(Real) == 4 ? sizeof(float) : 0)) * (size_t)a.n_E;
+    if (a.quadrature == PB_QUAD_BINMEAN)
+        b += sizeof(double) * (size_t)a.n_E + (sizeof(Real) == 4 ? sizeof(float) * (2 * (size_t)a.n_E + 1) : 0);
     if (a.n_layer > 0)
         b += 16 + sizeof(EscSeg<Real>) * kSegTile + sizeof(double) * 2 * kMaxEscLayers + sizeof(Real) * kMaxEscLayers;
     return b;

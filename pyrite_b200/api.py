@@ -50,23 +50,66 @@ def _device(device=None) -> torch.device:
 
 
 class _Holder:
-    """Keeps device tensors alive while the C structures point at them."""
+    """Keeps device tensors alive while the C structures point at them.
 
-    def __init__(self, device):
+    ``pack=True`` (one call's inputs): small host arrays are laid out in one
+    host block and go to the device in one copy at ``commit()``, which the call
+    makes before its first launch; a scoring call otherwise spends most of a
+    short run on some twenty separate copies."""
+
+    _PACK_BYTES = 1 << 17   # the block
+    _PACK_MAX = 1 << 14     # the largest array that goes into it
+
+    def __init__(self, device, pack=False):
         self.device = device
         self.keep = []
         self.inputs = []  # device tensors filled from host data (the call's inputs)
+        self._used = self._sent = 0
+        if pack:
+            self._host = np.empty(self._PACK_BYTES, dtype=np.uint8)
+            self._block = torch.empty(self._PACK_BYTES, dtype=torch.uint8, device=device)
+            self.keep.append(self._block)
+        else:
+            self._host = None
+
+    def _packed(self, a: np.ndarray, dtype):
+        """A view of the packed block holding ``a``, or None if it does not go there."""
+        off = (self._used + 255) & ~255
+        if self._host is None or not 0 < a.nbytes <= self._PACK_MAX or off + a.nbytes > self._PACK_BYTES:
+            return None
+        self._host[off:off + a.nbytes] = a.reshape(-1).view(np.uint8)
+        self._used = off + a.nbytes
+        return self._block[off:off + a.nbytes].view(dtype).view(a.shape)
+
+    def commit(self):
+        """Send what the packed block has gained (before a launch that reads it)."""
+        if self._used > self._sent:
+            self._block[self._sent:self._used].copy_(torch.from_numpy(self._host[self._sent:self._used]))
+            self._sent = self._used
 
     def f64(self, a) -> torch.Tensor:
-        t = torch.as_tensor(np.ascontiguousarray(a, dtype=np.float64) if not torch.is_tensor(a) else a)
-        t = t.to(self.device, torch.float64).contiguous()
+        if not torch.is_tensor(a):
+            a = np.ascontiguousarray(a, dtype=np.float64)
+            t = self._packed(a, torch.float64)
+            if t is not None:
+                return t
+            a = torch.as_tensor(a)
+        t = a.to(self.device, torch.float64).contiguous()
         self.keep.append(t)
         self.inputs.append(t)
         return t
 
+    _NP = {torch.int32: np.int32, torch.int64: np.int64}
+
     def typed(self, a, dtype) -> torch.Tensor:
-        t = a if torch.is_tensor(a) else torch.as_tensor(np.ascontiguousarray(a))
-        t = t.to(self.device, dtype).contiguous()
+        if not torch.is_tensor(a):
+            a = np.ascontiguousarray(a)
+            if a.dtype == self._NP.get(dtype):
+                t = self._packed(a, dtype)
+                if t is not None:
+                    return t
+            a = torch.as_tensor(a)
+        t = a.to(self.device, dtype).contiguous()
         self.keep.append(t)
         self.inputs.append(t)
         return t
@@ -75,6 +118,11 @@ class _Holder:
         t = torch.zeros(shape, dtype=dtype, device=self.device)
         self.keep.append(t)
         return t
+
+    def flag(self, dtype) -> torch.Tensor:
+        """One zeroed counter or status word; packed with the inputs."""
+        t = self._packed(np.zeros(1, dtype=self._NP[dtype]), dtype)
+        return self.zeros(1, dtype) if t is None else t
 
     def empty(self, shape, dtype) -> torch.Tensor:
         t = torch.empty(shape, dtype=dtype, device=self.device)
@@ -418,6 +466,7 @@ def _segments_on_device(h: _Holder, segments: dict):
 
 
 MAX_ESCAPE_LAYERS = 4
+_LINE_BYTES = 1 << 28  # line buffer of one node-sampling launch
 
 
 def _escape_layers(layers):
@@ -481,7 +530,7 @@ def mc_cxr_spectrum(segments, E_grid_eV, crystal, hkl_list, *, tables: LineTable
     """
     dev = _device(device)
     lib = L.load()
-    h = _Holder(dev)
+    h = _Holder(dev, pack=True)
     cr = CRYSTALS[crystal] if isinstance(crystal, str) else crystal
     n_hats = np.atleast_2d(np.asarray(n_hat, dtype=float))
     n_hats = n_hats / np.linalg.norm(n_hats, axis=1, keepdims=True)
@@ -496,79 +545,85 @@ def mc_cxr_spectrum(segments, E_grid_eV, crystal, hkl_list, *, tables: LineTable
     n_dir = n_hats.shape[0]
     n_E = int(E_grid.size)
     quad = L.PB_QUAD_BINMEAN if line_quadrature == "bin-mean" else L.PB_QUAD_NODE
-    spec = h.zeros((n_dir, n_E), torch.float64)
-    status = h.zeros(1, torch.int32)
     n_g = int(rows.G.shape[0])
-    pairs = None
-    out = np.zeros((n_dir, n_E))
-    pair_out = []
-    for d in range(n_dir):
-        a = L.PbCxrArgs()
-        a.precision = _PREC[precision]
-        a.quadrature = quad
-        a.n_dir = 1
-        a.n_hat = _ptr(h.f64(n_hats[d]))
-        a.thickness = float(segments["thickness_ang"])
-        a.Ne = int(segments["Ne"])
-        a.n_seg = seg["n"]
-        a.r_mid, a.v_hat, a.L = _ptr(seg["r_mid"]), _ptr(seg["v_hat"]), _ptr(seg["L"])
-        a.E_keV, a.elec_id = _ptr(seg["E"]), _ptr(seg["elec_id"])
-        t = _fill_tables(h, rows, tables, lo_keep, hi_keep)
-        t.ES = _ptr(h.f64(rows.ES[d]))
-        t.EP = _ptr(h.f64(rows.EP[d]))
-        a.tables = t
-        if layers is not None:
-            z_top, z_bot = _escape_layers(layers)
-            if mu_tables is None or len(mu_tables) != z_top.size:
-                raise ValueError("a layered absorber needs one mu table per layer")
-            a.n_layer = int(z_top.size)
-            a.z_top, a.z_bot = _ptr(h.f64(z_top)), _ptr(h.f64(z_bot))
-            a.mu_off = _ptr(h.typed(np.cumsum([0] + [len(k) for k, _v, _s in mu_tables]).astype(np.int32), torch.int32))
-            a.mu_knot = _ptr(h.f64(np.concatenate([np.asarray(k, float) for k, _v, _s in mu_tables])))
-            a.mu_value = _ptr(h.f64(np.concatenate([np.asarray(v, float) for _k, v, _s in mu_tables])))
-            a.mu_slope = _ptr(h.f64(np.concatenate([np.asarray(sl, float) for _k, _v, sl in mu_tables])))
-        sl_t = _seg_layer(h, segments, emit_layer)
-        if sl_t is not None:
-            a.seg_layer, a.emit_layer = _ptr(sl_t), int(emit_layer)
-        a.n_E = n_E
-        a.E_grid = _ptr(h.f64(E_grid))
-        spec_d = h.zeros(n_E, torch.float64)
-        a.spec = _ptr(spec_d)
-        a.status = _ptr(status)
-        if quad == L.PB_QUAD_BINMEAN:
-            edges = energy_bin_edges(E_grid)
-            a.edges = _ptr(h.f64(edges))
-            w = np.diff(edges)
-            uniform = np.allclose(w, w[0], rtol=1e-9, atol=0.0)
-            if exact_widths is not None and exact_widths > 0 and uniform:
-                a.exact_widths = float(exact_widths)
-                pad = int(np.ceil(max(edges[0] - lo_keep, hi_keep - edges[-1]) / w[0])) + 2
-                a.far_pad = pad
-                a.far_moments = _ptr(h.zeros((n_E + 2 * pad) * 3, torch.float64))
-            else:
-                a.exact_widths = 0.0
-                a.far_pad = -1
+    n_pair = max(1, seg["n"] * n_g)
+    spec = h.zeros((n_dir, n_E), torch.float64)
+    pair_out = None
+    if return_pairs:
+        pair_out = [h.empty(n_dir * n_pair, torch.float64) for _ in range(3)] + [h.zeros(n_dir * n_pair, torch.uint8)]
+    # ---- one argument set; the directions of a launch differ in its pointers
+    a = L.PbCxrArgs()
+    a.precision = _PREC[precision]
+    a.quadrature = quad
+    a.thickness = float(segments["thickness_ang"])
+    a.Ne = int(segments["Ne"])
+    a.n_seg = seg["n"]
+    a.r_mid, a.v_hat, a.L = _ptr(seg["r_mid"]), _ptr(seg["v_hat"]), _ptr(seg["L"])
+    a.E_keV, a.elec_id = _ptr(seg["E"]), _ptr(seg["elec_id"])
+    if len(rows.ES) < n_dir or len(rows.EP) < n_dir:
+        raise IndexError(f"the reflection rows hold fewer directions than the {n_dir} asked for")
+    n_hat_d, ES, EP = h.f64(n_hats), h.f64(rows.ES[:n_dir]), h.f64(rows.EP[:n_dir])
+    a.tables = _fill_tables(h, rows, tables, lo_keep, hi_keep)
+    if layers is not None:
+        z_top, z_bot = _escape_layers(layers)
+        if mu_tables is None or len(mu_tables) != z_top.size:
+            raise ValueError("a layered absorber needs one mu table per layer")
+        a.n_layer = int(z_top.size)
+        a.z_top, a.z_bot = _ptr(h.f64(z_top)), _ptr(h.f64(z_bot))
+        a.mu_off = _ptr(h.typed(np.cumsum([0] + [len(k) for k, _v, _s in mu_tables]).astype(np.int32), torch.int32))
+        a.mu_knot = _ptr(h.f64(np.concatenate([np.asarray(k, float) for k, _v, _s in mu_tables])))
+        a.mu_value = _ptr(h.f64(np.concatenate([np.asarray(v, float) for _k, v, _s in mu_tables])))
+        a.mu_slope = _ptr(h.f64(np.concatenate([np.asarray(sl, float) for _k, _v, sl in mu_tables])))
+    sl_t = _seg_layer(h, segments, emit_layer)
+    if sl_t is not None:
+        a.seg_layer, a.emit_layer = _ptr(sl_t), int(emit_layer)
+    a.n_E = n_E
+    a.E_grid = _ptr(h.f64(E_grid))
+    a.status = _ptr(h.flag(torch.int32))
+    # Bin means never leave the chip: every direction in one launch. Node
+    # sampling buffers a direction's lines, so a launch takes as many
+    # directions as their lines fit _LINE_BYTES.
+    group = n_dir
+    if quad == L.PB_QUAD_BINMEAN:
+        edges = energy_bin_edges(E_grid)
+        a.edges = _ptr(h.f64(edges))
+        w = np.diff(edges)
+        uniform = np.allclose(w, w[0], rtol=1e-9, atol=0.0)
+        if exact_widths is not None and exact_widths > 0 and uniform:
+            a.exact_widths = float(exact_widths)
+            pad = int(np.ceil(max(edges[0] - lo_keep, hi_keep - edges[-1]) / w[0])) + 2
+            a.far_pad = pad
+            a.far_moments = _ptr(h.empty(n_dir * (n_E + 2 * pad) * 3, torch.float64))  # cleared by the call
         else:
-            cap = max(1, seg["n"] * n_g)
-            a.line_capacity = cap
-            a.line_count = _ptr(h.zeros(1, torch.int64))
-            a.line_E, a.line_a = _ptr(h.empty(cap, torch.float64)), _ptr(h.empty(cap, torch.float64))
-            a.line_w = _ptr(h.empty(cap, torch.float64))
-            a.line_dir = _ptr(h.zeros(cap, torch.int32))
+            a.exact_widths = 0.0
+            a.far_pad = -1
+    else:
+        group = max(1, min(n_dir, _LINE_BYTES // (28 * n_pair)))
+        cap = group * n_pair
+        a.line_capacity = cap
+        a.line_count = _ptr(h.flag(torch.int64))
+        a.line_E, a.line_a = _ptr(h.empty(cap, torch.float64)), _ptr(h.empty(cap, torch.float64))
+        a.line_w = _ptr(h.empty(cap, torch.float64))
+        a.line_dir = _ptr(h.empty(cap, torch.int32))
+    h.commit()
+    for d in range(0, n_dir, group):
+        a.n_dir = min(group, n_dir - d)
+        a.n_hat = n_hat_d.data_ptr() + 24 * d
+        a.tables.ES, a.tables.EP = (t.data_ptr() + 24 * n_g * d for t in (ES, EP))
+        a.spec = spec.data_ptr() + 8 * n_E * d
         if return_pairs:
-            m = seg["n"] * n_g
-            pe, pa, pw = (h.empty(m, torch.float64) for _ in range(3))
-            pg = h.zeros(m, torch.uint8)
-            a.pair_E, a.pair_a, a.pair_w, a.pair_good = _ptr(pe), _ptr(pa), _ptr(pw), _ptr(pg)
-            pair_out.append((pe, pa, pw, pg))
+            off = d * seg["n"] * n_g
+            a.pair_E, a.pair_a, a.pair_w = (t.data_ptr() + 8 * off for t in pair_out[:3])
+            a.pair_good = pair_out[3].data_ptr() + off
         L.check(lib.pb_cxr_score(C.byref(a), _stream_ptr(stream)), "pb_cxr_score")
-        torch.cuda.synchronize(dev)
-        out[d] = spec_d.cpu().numpy()
+    torch.cuda.synchronize(dev)
+    out = spec.cpu().numpy()
     out /= int(segments["Ne"])
     result = out[0] if single else out
     if return_pairs:
-        pairs = [tuple(x.cpu().numpy() for x in p) for p in pair_out]
-        return result, pairs
+        m = seg["n"] * n_g
+        host = [x.cpu().numpy() for x in pair_out]
+        return result, [tuple(x[d * m:(d + 1) * m] for x in host) for d in range(n_dir)]
     return result
 
 
@@ -593,7 +648,7 @@ def mc_brem_spectrum(segments, E_grid_eV, *, composition, n_hat, mu=None, precis
 
     dev = _device(device)
     lib = L.load()
-    h = _Holder(dev)
+    h = _Holder(dev, pack=True)
     seg = _segments_on_device(h, segments)
     n_hats = np.atleast_2d(np.asarray(n_hat, dtype=float))
     n_hats = n_hats / np.linalg.norm(n_hats, axis=1, keepdims=True)
@@ -631,12 +686,13 @@ def mc_brem_spectrum(segments, E_grid_eV, *, composition, n_hat, mu=None, precis
         a.seg_layer, a.emit_layer = _ptr(sl_t), int(emit_layer)
     spec = h.zeros((n_dir, n_E), torch.float64)
     a.spec = _ptr(spec)
-    a.status = _ptr(h.zeros(1, torch.int32))
+    a.status = _ptr(h.flag(torch.int32))
     if depth_nodes:
         nb = C.c_int64(0)
         L.check(lib.pb_brem_work_size(C.byref(a), C.byref(nb)), "pb_brem_work_size")
         if nb.value > 0:
             a.work, a.work_bytes = _ptr(h.empty(int(nb.value), torch.uint8)), int(nb.value)
+    h.commit()
     L.check(lib.pb_brem_score(C.byref(a), _stream_ptr(stream)), "pb_brem_score")
     torch.cuda.synchronize(dev)
     out = spec.cpu().numpy() / (4.0 * np.pi) / int(segments["Ne"])
@@ -744,7 +800,7 @@ def mc_characteristic_spectrum(segments, E_grid_eV, *, lines: CharacteristicLine
         return out[0] if single else out
     dev = _device(device)
     lib = L.load()
-    h = _Holder(dev)
+    h = _Holder(dev, pack=True)
     seg = _segments_on_device(h, segments)
     mu = np.atleast_2d(np.asarray(mu_by_line, dtype=float))[:, kept]
     n_layer = 0 if layers is None else len(layers)
@@ -774,14 +830,15 @@ def mc_characteristic_spectrum(segments, E_grid_eV, *, lines: CharacteristicLine
     a.mu = _ptr(h.f64(mu))
     yields = h.zeros((n_dir, int(kept.size)), torch.float64)
     a.line_yield = _ptr(yields)
-    a.status = _ptr(h.zeros(1, torch.int32))
+    a.status = _ptr(h.flag(torch.int32))
     sl_t = _seg_layer(h, segments, emit_layer)
     if sl_t is not None:
         a.seg_layer, a.emit_layer = _ptr(sl_t), int(emit_layer)
     s = _stream_ptr(stream)
+    spec, prof = h.zeros((n_dir, n_E), torch.float64), h.f64(profiles)
+    h.commit()
     L.check(lib.pb_char_yields(C.byref(a), s), "pb_char_yields")
-    spec = h.zeros((n_dir, n_E), torch.float64)
-    L.check(lib.pb_char_spectrum(n_dir, int(kept.size), n_E, _ptr(yields), _ptr(h.f64(profiles)), _ptr(spec), s),
+    L.check(lib.pb_char_spectrum(n_dir, int(kept.size), n_E, _ptr(yields), _ptr(prof), _ptr(spec), s),
             "pb_char_spectrum")
     torch.cuda.synchronize(dev)
     out = spec.cpu().numpy() / (4.0 * np.pi) / Ne

@@ -65,7 +65,7 @@ def coherent_reduce(records, row_count, row_weight, E_grid_eV, delta_omega, *, s
     field and its per-electron squared fields (``pb_coherent_blend``).
     """
     dev = _device(device)
-    h = _Holder(dev)
+    h = _Holder(dev, pack=True)
     row_count = np.asarray(row_count, dtype=np.int64)
     if row_count.ndim != 1 or row_count.size < 1 or np.any(row_count < 0):
         raise ValueError("row_count must be a nonempty 1-D array of nonnegative counts")
@@ -112,6 +112,7 @@ def coherent_reduce(records, row_count, row_weight, E_grid_eV, delta_omega, *, s
     a.spec = spec.data_ptr()
     a.work, a.work_bytes = work.data_ptr(), nbytes
     a.status = None if status is None else status.data_ptr()
+    h.commit()
     if blend:
         b = L.PbCoherentBlendArgs()
         b.base = a
@@ -141,7 +142,7 @@ def coherent_records(segments, E_grid_eV, *, tables, rows, n_hat, device=None, s
 
     dev = _device(device)
     lib = L.load()
-    h = _Holder(dev)
+    h = _Holder(dev, pack=True)
     seg = _segments_on_device(h, segments)
     n_g = int(rows.G.shape[0])
     E_grid = np.asarray(E_grid_eV, dtype=np.float64)
@@ -178,8 +179,9 @@ def coherent_records(segments, E_grid_eV, *, tables, rows, n_hat, device=None, s
     L.check(lib.pb_coherent_records_work_size(seg["n"], n_g, C.byref(nbytes)), "pb_coherent_records_work_size")
     work = h.empty((max(int(nbytes.value), 1),), torch.uint8)
     a.work, a.work_bytes = work.data_ptr(), int(nbytes.value)
-    status = h.zeros(1, torch.int32)
+    status = h.flag(torch.int32)
     a.status = status.data_ptr()
+    h.commit()
     L.check(lib.pb_coherent_records(C.byref(a), _stream_ptr(stream)), "pb_coherent_records")
     off = row_off.cpu().numpy()
     if int(status.item()) != 0:

@@ -563,90 +563,95 @@ __device__ __forceinline__ Line<Real> pair_line(const SegPre<Real> &sp, const Ro
     return pair_line_from<Real, kLayered>(sp, rw, res, E_tab, log_mu, n_tab, n_mu, t, ti, es, a, lay_t);
 }
 
-// ---- sine integral and the sinc^2 antiderivative --------------------------
-// Si(t) - pi/2 for t >= 0: power series for t <= 13; the continued fraction of
-// E1(i t) by the modified Lentz method (Numerical Recipes "cisi") for
-// 13 < t < 40; the asymptotic auxiliary-function series beyond
-// (Abramowitz & Stegun 5.2.34-5.2.35): Si - pi/2 = -f cos t - g sin t.
-constexpr int kSiTerms = 31;  // k = 30 term at t = 13 is ~3e-18
-struct SiSeries {
-    double c[kSiTerms];  // (-1)^k / ((2k+1) (2k+1)!)
+// ---- the sinc^2 antiderivative ---------------------------------------------
+// R(x) = F(x) - sign(x)/2, F the integral of sinc^2 from 0, for |x| < 8 in FP64:
+// a Taylor polynomial of degree 23 about the middle c_k = 1/4 + k/2 of each half
+// unit. With h = x - c_k, 1 - cos 2 pi x = 1 + (-1)^k sin 2 pi h exactly, so
+// sinc^2(x) = (1 - cos 2 pi x) / (2 pi^2 (c_k + h)^2) has its coefficients from
+// the recurrence of a division by (c_k + h)^2; integrated term by term and
+// matched at the interval ends from R(0) = -1/2. Truncation: the n-th term is
+// below (pi/2)^n / n! at |h| = 1/4, 1e-19 for n = 24; the recurrence's rounding
+// stays below 1e-14 (it grows as n (h / c_k)^n). 23 multiply-adds replace a
+// 31-term series of the sine integral below |x| = 2.1 and a continued fraction
+// with two divisions a step above.
+constexpr int kSincParts = 16, kSincDeg = 23;
+struct SincTable {
+    double c[kSincParts][kSincDeg + 1];
 };
-__host__ __device__ constexpr SiSeries make_si_series() {
-    SiSeries s{};
-    double fact = 1.0;
-    for (int k = 0; k < kSiTerms; ++k) {
-        if (k > 0) fact *= (2.0 * k) * (2.0 * k + 1.0);
-        s.c[k] = ((k & 1) ? -1.0 : 1.0) / ((2.0 * k + 1.0) * fact);
-    }
-    return s;
-}
-
-__device__ double si_minus_half_pi(double t) {
-    if (t <= 13.0) {
-        // Power series in Horner form with compile-time coefficients; the
-        // sum of |terms| at t = 13 is ~2e4, so ~5e-12 absolute accuracy.
-        constexpr SiSeries kSi = make_si_series();
-        const double t2 = t * t;
-        double p = kSi.c[kSiTerms - 1];
-#pragma unroll
-        for (int k = kSiTerms - 2; k >= 0; --k) p = fma(p, t2, kSi.c[k]);
-        return p * t - 0.5 * kPi;
-    }
-    double s, c;
-    sincos(t, &s, &c);
-    if (t >= 40.0) {
-        const double inv_t = 1.0 / t;
-        const double y = inv_t * inv_t;
-        // f t = 1 - 2!/t^2 + 4!/t^4 - ..., g t^2 = 1 - 3!/t^2 + 5!/t^4 - ...
-        double f = 1.0, g = 1.0, tf = 1.0, tg = 1.0;
-        for (int k = 1; k < 12; ++k) {
-            tf *= -(2.0 * k - 1.0) * (2.0 * k) * y;
-            tg *= -(2.0 * k) * (2.0 * k + 1.0) * y;
-            f += tf;
-            g += tg;
-            if (fabs(tf) < 1e-17 && fabs(tg) < 1e-17) break;
+__host__ __device__ constexpr SincTable make_sinc_table() {
+    SincTable t{};
+    double left = -0.5;  // R at the left end of the interval
+    for (int k = 0; k < kSincParts; ++k) {
+        const double c = 0.25 + 0.5 * k, sg = (k & 1) ? -1.0 : 1.0;
+        double s[kSincDeg + 1] = {}, f = 1.0;  // f = (2 pi)^n / n!
+        for (int n = 0; n <= kSincDeg; ++n) {
+            double num = n == 0 ? 1.0 : 0.0;
+            if (n > 0) {
+                f *= 2.0 * kPi / n;
+                if (n & 1) num = ((n >> 1) & 1) ? -sg * f : sg * f;
+            }
+            num /= 2.0 * kPi * kPi;
+            s[n] = (num - (n > 0 ? 2.0 * c * s[n - 1] : 0.0) - (n > 1 ? s[n - 2] : 0.0)) / (c * c);
         }
-        f *= inv_t;
-        g *= y;
-        return -f * c - g * s;
+        double lo = 0.0, hi = 0.0;  // the polynomial without its constant at h = -1/4, 1/4
+        for (int n = kSincDeg; n > 0; --n) {
+            t.c[k][n] = s[n - 1] / n;
+            lo = (lo + t.c[k][n]) * -0.25;
+            hi = (hi + t.c[k][n]) * 0.25;
+        }
+        t.c[k][0] = left - lo;
+        left = t.c[k][0] + hi;
     }
-    double br = 1.0, bi = t;
-    double inv = 1.0 / (br * br + bi * bi);
-    double dr = br * inv, di = -bi * inv;
-    double hr = dr, hi = di;
-    double cr = 1e300, ci = 0.0;
-    for (int i = 2; i < 200; ++i) {
-        const double a = -(double)(i - 1) * (double)(i - 1);
-        br += 2.0;
-        const double xr = a * dr + br, xi = a * di + bi;
-        inv = 1.0 / (xr * xr + xi * xi);
-        dr = xr * inv;
-        di = -xi * inv;
-        inv = a / (cr * cr + ci * ci);
-        cr = br + cr * inv;
-        ci = bi - ci * inv;
-        const double delr = cr * dr - ci * di, deli = cr * di + ci * dr;
-        const double nhr = hr * delr - hi * deli, nhi = hr * deli + hi * delr;
-        hr = nhr;
-        hi = nhi;
-        if (fabs(delr - 1.0) + fabs(deli) < 1e-16) break;
-    }
-    return c * hi - s * hr;
+    return t;
+}
+__device__ const SincTable kSincTable = make_sinc_table();
+
+__device__ __forceinline__ double sincsq_tail(double x) {
+    const double u = fabs(x);
+    const int k = min((int)(2.0 * u), kSincParts - 1);
+    const double h = u - (0.25 + 0.5 * k);
+    const double *c = kSincTable.c[k];
+    double r = c[kSincDeg];
+#pragma unroll
+    for (int n = kSincDeg - 1; n >= 0; --n) r = fma(r, h, c[n]);
+    return x >= 0.0 ? r : -r;
 }
 
-// R(x) = F(x) - sign(x)/2, F the integral of sinc^2 from 0.
-__device__ double sincsq_tail(double x) {
-    const double u = fabs(x);
-    const double t = 2.0 * kPi * u;
-    double su;
-    if (u == 0.0) {
-        su = 1.0;
-    } else {
-        su = sinpi(u) / (kPi * u);
+// sin and cos of 2 pi x: the quarter turn nearest to x is taken off (adding and
+// subtracting 1.5 2^52 rounds 4 x, |x| < 2^48), the rest, within an eighth of a
+// turn, goes to the Taylor series (terms to g^15 and g^16: truncation 5e-17),
+// about half the issue slots of the library's sincospi, whose argument is not
+// limited to a few thousand turns.
+struct TurnSeries {
+    double s[8], c[9];
+};
+__host__ __device__ constexpr TurnSeries make_turn_series() {
+    TurnSeries t{};
+    double f = 1.0;  // (2 pi)^n / n!
+    for (int n = 0; n <= 16; ++n) {
+        if (n > 0) f *= 2.0 * kPi / n;
+        const double v = ((n >> 1) & 1) ? -f : f;
+        if (n & 1) t.s[n >> 1] = v;
+        else t.c[n >> 1] = v;
     }
-    const double r = si_minus_half_pi(t) / kPi - u * su * su;
-    return x >= 0.0 ? r : -r;
+    return t;
+}
+__device__ __forceinline__ void sincos_turns(double x, double &sn, double &cs) {
+    constexpr TurnSeries t = make_turn_series();
+    constexpr double kRound = 6755399441055744.0;  // 1.5 2^52
+    const double m = __dadd_rn(4.0 * x, kRound);
+    const int q = __double2loint(m);
+    const double g = fma(__dsub_rn(m, kRound), -0.25, x);
+    const double y = g * g;
+    double s = t.s[7], c = t.c[8];
+#pragma unroll
+    for (int k = 6; k >= 0; --k) s = fma(s, y, t.s[k]);
+#pragma unroll
+    for (int k = 7; k >= 0; --k) c = fma(c, y, t.c[k]);
+    s *= g;
+    const double a = (q & 1) ? c : s, b = (q & 1) ? s : c;
+    sn = (q & 2) ? -a : a;
+    cs = ((q + 1) & 2) ? -b : b;
 }
 
 constexpr double kInvPi = 1.0 / kPi;
@@ -710,11 +715,18 @@ __device__ __forceinline__ double q_osc(double x, double iu) {
     const double y = iu * iu;
     double p1, p2;
     if (fabs(iu) < 1.0 / 200.0) {
-        // u > 200: six terms reach 14!/200^12 < 3e-17 of the leading one.
-        p1 = c.c1[5];
-        p2 = c.c2[5];
+        // u > 200: six terms reach 14!/200^12 < 3e-17 of the leading one,
+        // three of them 8!/3000^6 < 6e-17 past u = 3000.
+        p1 = c.c1[2];
+        p2 = c.c2[2];
+        if (fabs(iu) > 1.0 / 3000.0) {
+            p1 = c.c1[5];
+            p2 = c.c2[5];
 #pragma unroll
-        for (int k = 4; k >= 0; --k) { p1 = fma(p1, y, c.c1[k]); p2 = fma(p2, y, c.c2[k]); }
+            for (int k = 4; k >= 2; --k) { p1 = fma(p1, y, c.c1[k]); p2 = fma(p2, y, c.c2[k]); }
+        }
+#pragma unroll
+        for (int k = 1; k >= 0; --k) { p1 = fma(p1, y, c.c1[k]); p2 = fma(p2, y, c.c2[k]); }
     } else {
         p1 = c.c1[kOscTerms - 1];
         p2 = c.c2[kOscTerms - 1];
@@ -722,7 +734,7 @@ __device__ __forceinline__ double q_osc(double x, double iu) {
         for (int k = kOscTerms - 2; k >= 0; --k) { p1 = fma(p1, y, c.c1[k]); p2 = fma(p2, y, c.c2[k]); }
     }
     double sn, cs;
-    sincospi(2.0 * x, &sn, &cs);
+    sincos_turns(x, sn, cs);
     return y * (cs * p1 * iu - sn * p2);
 }
 __device__ __forceinline__ float q_osc(float x, float iu) {
@@ -780,44 +792,33 @@ __device__ __forceinline__ LineWindow line_window(double E_r, double inv_a, cons
 // (montecarlo/spectrum/cxr/_bin_quadrature.py:179-221, the reference's
 // device bin mean, on by default there). Valid for dx <= 0.1 and |xc| >= 2, where the omitted term is below
 // 2.5e-9 of the envelope 1/(2 pi^2 xc^2).
-template <bool kMixed>
 __device__ __forceinline__ double sincsq_midpoint_mean(double xc, double dx) {
-    using R = typename std::conditional<kMixed, float, double>::type;
-    // sin(pi xc), cos(pi xc) from the argument reduced to [-1, 1] in double.
-    R sp, cp;
-    if constexpr (kMixed) {
-        // Reduce to [-1, 1] exactly in double before the float argument.
-        const double red = xc - 2.0 * rint(0.5 * xc);
-        __sincosf((float)(kPi * red), &sp, &cp);
-    } else {
-        sincospi(xc, &sp, &cp);
-    }
-    const R om = (R)(2.0 * kPi);
-    const R a0 = (R)2 * sp * sp;
-    const R s2 = (R)2 * sp * cp;
-    const R c2 = (cp - sp) * (cp + sp);
-    const R a1 = om * s2, a2 = om * om * c2;
-    const R om3 = om * om * om;
-    const R a3 = -om3 * s2, a4 = -om3 * om * c2;
-    const R a5 = om3 * om * om * s2, a6 = om3 * om3 * c2;
-    R q;
-    if constexpr (kMixed) q = __frcp_rn((float)xc);
-    else q = 1.0 / xc;
-    const R h0 = q * q;
-    const R h1 = (R)-2 * h0 * q;
-    const R h2 = (R)-3 * h1 * q;
-    const R h3 = (R)-4 * h2 * q;
-    const R h4 = (R)-5 * h3 * q;
-    const R h5 = (R)-6 * h4 * q;
-    const R h6 = (R)-7 * h5 * q;
-    const R f0 = a0 * h0;
-    const R f2 = a2 * h0 + (R)2 * a1 * h1 + a0 * h2;
-    const R f4 = a4 * h0 + (R)4 * a3 * h1 + (R)6 * a2 * h2 + (R)4 * a1 * h3 + a0 * h4;
-    const R f6 = a6 * h0 + (R)6 * a5 * h1 + (R)15 * a4 * h2 + (R)20 * a3 * h3 + (R)15 * a2 * h4 +
-                 (R)6 * a1 * h5 + a0 * h6;
-    const R d2 = (R)(dx * dx);
-    const R series = f0 + d2 * (f2 * (R)(1.0 / 24.0) + d2 * (f4 * (R)(1.0 / 1920.0) + d2 * (f6 * (R)(1.0 / 322560.0))));
-    return (double)series * kInv2Pi2;
+    double sp, cp;  // of pi xc
+    sincos_turns(0.5 * xc, sp, cp);
+    const double om = 2.0 * kPi;
+    const double a0 = 2.0 * sp * sp;
+    const double s2 = 2.0 * sp * cp;
+    const double c2 = (cp - sp) * (cp + sp);
+    const double a1 = om * s2, a2 = om * om * c2;
+    const double om3 = om * om * om;
+    const double a3 = -om3 * s2, a4 = -om3 * om * c2;
+    const double a5 = om3 * om * om * s2, a6 = om3 * om3 * c2;
+    const double q = 1.0 / xc;
+    const double h0 = q * q;
+    const double h1 = -2.0 * h0 * q;
+    const double h2 = -3.0 * h1 * q;
+    const double h3 = -4.0 * h2 * q;
+    const double h4 = -5.0 * h3 * q;
+    const double h5 = -6.0 * h4 * q;
+    const double h6 = -7.0 * h5 * q;
+    const double f0 = a0 * h0;
+    const double f2 = a2 * h0 + 2.0 * a1 * h1 + a0 * h2;
+    const double f4 = a4 * h0 + 4.0 * a3 * h1 + 6.0 * a2 * h2 + 4.0 * a1 * h3 + a0 * h4;
+    const double f6 = a6 * h0 + 6.0 * a5 * h1 + 15.0 * a4 * h2 + 20.0 * a3 * h3 + 15.0 * a2 * h4 + 6.0 * a1 * h5 +
+                      a0 * h6;
+    const double d2 = dx * dx;
+    const double series = f0 + d2 * (f2 * (1.0 / 24.0) + d2 * (f4 * (1.0 / 1920.0) + d2 * (f6 * (1.0 / 322560.0))));
+    return series * kInv2Pi2;
 }
 
 // Reciprocal on the SFU alone (rcp.approx, about 1 ulp): the mixed path's
@@ -829,7 +830,7 @@ __device__ __forceinline__ float rcp_fast(float x) {
 }
 __device__ __forceinline__ double rcp_fast(double x) { return 1.0 / x; }
 
-// R(x) = F(x) - sign(x)/2 of sincsq_tail in float:
+// R(x) of sincsq_tail in float:
 // Si(t) - pi/2 = -f(t) cos t - g(t) sin t with t = 2 pi |x| and the rational
 // auxiliary functions of Abramowitz & Stegun 5.2.38-5.2.39 (|error| < 5e-7 for
 // t >= 1); its Maclaurin series below t = 1.
@@ -892,7 +893,7 @@ __device__ __forceinline__ float sincsq_midpoint_mean_f32(float xc, float dx) {
 __device__ __forceinline__ float tail_of(float x) { return sincsq_tail_f32(x); }
 __device__ __forceinline__ double tail_of(double x) { return sincsq_tail(x); }
 __device__ __forceinline__ float midpoint_mean(float xc, float dx) { return sincsq_midpoint_mean_f32(xc, dx); }
-__device__ __forceinline__ double midpoint_mean(double xc, double dx) { return sincsq_midpoint_mean<false>(xc, dx); }
+__device__ __forceinline__ double midpoint_mean(double xc, double dx) { return sincsq_midpoint_mean(xc, dx); }
 
 // ---- the deposit as a function of bin edges --------------------------------
 // pi times the mass of sinc^2 in a bin is a difference of one function of its
@@ -1637,15 +1638,43 @@ __global__ void __launch_bounds__(kFarBins * kFarSlices) far_field_conv_kernel(c
 }
 
 // Node reduction of buffered lines: spec[d][e] += sum_j w_j sinc^2(x_je),
-// x = a (E_e - E_j) / pi, with the phase a (E_e - E_j) formed in double.
+// x = a (E_e - E_j) / pi, formed in FP64. sinc^2 needs sin^2 alone, so the phase
+// is reduced to half a turn about the nearest integer x (no quadrants) and the
+// sine is one Taylor series to (pi f)^21 (FP64, truncation 1e-18) or the SFU's
+// (mixed). Lines are staged in shared memory with a / pi and w / pi^2 ready, and
+// four lines are in flight per thread: the loop is bound by the latency of its
+// division otherwise (300 segments x 144 rows x 781 nodes: 130 -> 65 us).
+constexpr int kNodeTile = 128;
+
+__device__ __forceinline__ double sin_pi_series(double f) {
+    constexpr int kTerms = 11;
+    struct C {
+        double c[kTerms];
+    };
+    constexpr C t = [] {
+        C r{};
+        double v = 1.0;  // pi^n / n!
+        for (int n = 1; n <= 2 * kTerms - 1; ++n) {
+            v *= kPi / n;
+            if (n & 1) r.c[n >> 1] = ((n >> 1) & 1) ? -v : v;
+        }
+        return r;
+    }();
+    const double y = f * f;
+    double s = t.c[kTerms - 1];
+#pragma unroll
+    for (int k = kTerms - 2; k >= 0; --k) s = fma(s, y, t.c[k]);
+    return s * f;
+}
+
 template <class Real>
-__global__ void node_reduce_kernel(const double *E_grid, int n_E, const double *line_E,
-                                   const double *line_a, const double *line_w, const int32_t *line_dir,
-                                   const unsigned long long *line_count, int64_t capacity,
-                                   double *spec) {
-    constexpr int kTile = 256;
-    __shared__ double sE[kTile], sA[kTile], sW[kTile];
-    __shared__ int sD[kTile];
+__global__ void __launch_bounds__(kNodeTile) node_reduce_kernel(const double *E_grid, int n_E, const double *line_E,
+                                                                const double *line_a, const double *line_w,
+                                                                const int32_t *line_dir,
+                                                                const unsigned long long *line_count,
+                                                                int64_t capacity, double *spec) {
+    __shared__ double sE[kNodeTile], sA[kNodeTile], sW[kNodeTile];
+    __shared__ int sD[kNodeTile];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     int64_t n_lines = (int64_t)*line_count;
     if (n_lines > capacity) n_lines = capacity;
@@ -1653,39 +1682,45 @@ __global__ void node_reduce_kernel(const double *E_grid, int n_E, const double *
     const int64_t j0 = per * blockIdx.y;
     const int64_t j1 = j0 + per < n_lines ? j0 + per : n_lines;
     const double E = e < n_E ? E_grid[e] : 0.0;
+    const auto term = [&](int k) {
+        constexpr double kRound = 6755399441055744.0;  // 1.5 2^52
+        const double x = sA[k] * (E - sE[k]);
+        const double f = x - __dsub_rn(__dadd_rn(x, kRound), kRound);
+        double s;
+        if constexpr (sizeof(Real) == 8) s = sin_pi_series(f);
+        else s = (double)__sinf((float)(kPi * f));
+        const double v = sW[k] * (s * s) / (x * x);
+        return fabs(x) > 1.0e-20 ? v : sW[k] * (kPi * kPi);  // sinc^2(0) = 1
+    };
     // Accumulate per direction seen in this chunk (directions are few).
     double acc = 0.0;
     int cur_dir = -1;
-    for (int64_t t0 = j0; t0 < j1; t0 += kTile) {
-        const int nt = (int)((j1 - t0) < kTile ? (j1 - t0) : kTile);
+    for (int64_t t0 = j0; t0 < j1; t0 += kNodeTile) {
+        const int nt = (int)((j1 - t0) < kNodeTile ? (j1 - t0) : kNodeTile);
         __syncthreads();
         for (int j = threadIdx.x; j < nt; j += blockDim.x) {
             sE[j] = line_E[t0 + j];
-            sA[j] = line_a[t0 + j];
-            sW[j] = line_w[t0 + j];
+            sA[j] = line_a[t0 + j] / kPi;
+            sW[j] = line_w[t0 + j] / (kPi * kPi);
             sD[j] = line_dir[t0 + j];
         }
         __syncthreads();
         if (e < n_E) {
-            for (int k = 0; k < nt; ++k) {
+            int k = 0;
+            while (k < nt) {
                 if (sD[k] != cur_dir) {
                     if (cur_dir >= 0 && acc != 0.0) atomicAdd(&spec[(int64_t)cur_dir * n_E + e], acc);
                     acc = 0.0;
                     cur_dir = sD[k];
                 }
-                double x = sA[k] * (E - sE[k]) / kPi;
-                if (x == 0.0) x = 1.0e-20;
-                double s;
-                if constexpr (sizeof(Real) == 8) {
-                    const double y = kPi * x;
-                    s = sin(y) / y;
+                if (k + 4 <= nt && sD[k + 1] == cur_dir && sD[k + 2] == cur_dir && sD[k + 3] == cur_dir) {
+                    const double t0v = term(k), t1v = term(k + 1), t2v = term(k + 2), t3v = term(k + 3);
+                    acc += (t0v + t1v) + (t2v + t3v);
+                    k += 4;
                 } else {
-                    // y = pi x reduced to [-pi, pi] in double, sine in float.
-                    const double y = kPi * x;
-                    const double r = y - 2.0 * kPi * rint(y / (2.0 * kPi));
-                    s = (double)__sinf((float)r) / y;
+                    acc += term(k);
+                    k += 1;
                 }
-                acc += sW[k] * (s * s);
             }
         }
     }
@@ -1764,8 +1799,11 @@ static cudaError_t launch_cxr_t(const pb_cxr_args &a, cudaStream_t s, int sms, i
         if (err != cudaSuccess) return err;
     }
     if (a.quadrature == PB_QUAD_NODE && a.line_E != nullptr && a.spec != nullptr) {
-        dim3 ng((unsigned)((a.n_E + 127) / 128), 64);
-        node_reduce_kernel<Real><<<ng, 128, 0, s>>>(a.E_grid, a.n_E, a.line_E, a.line_a, a.line_w,
+        // about eight blocks an SM over the node tiles
+        const unsigned gx = (unsigned)((a.n_E + kNodeTile - 1) / kNodeTile);
+        const unsigned gy = std::max(1u, (unsigned)(sms * 8) / gx);
+        dim3 ng(gx, gy);
+        node_reduce_kernel<Real><<<ng, kNodeTile, 0, s>>>(a.E_grid, a.n_E, a.line_E, a.line_a, a.line_w,
                                                     a.line_dir, a.line_count, a.line_capacity, a.spec);
         err = cudaGetLastError();
     }

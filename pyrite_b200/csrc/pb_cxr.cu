@@ -1301,7 +1301,8 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
                 const Real x = l.s * (e - l.E_r);
                 const Real x_hi = __shfl_down_sync(0xffffffffu, x, 1);
                 const Real sw = x_hi - x, xc = (Real)0.5 * (x + x_hi);
-                const bool narrow = sw <= (Real)0.1 && fabs(xc) >= (Real)2;
+                // (lane 31 holds the strip's last edge and no bin)
+                const bool narrow = sw <= (Real)0.1 && fabs(xc) >= (Real)2 && lane < kStripBins;
                 const unsigned wide_bins = __ballot_sync(0xffffffffu, !narrow && lane < kStripBins);
                 const bool need = ((wide_bins | (wide_bins << 1)) >> lane) & 1u;
                 const Real f = need ? edge_near_bins<Real>(x) : (Real)0;

@@ -1967,15 +1967,19 @@ __global__ void __launch_bounds__(1024) coh_rec_scan_kernel(int64_t n_seg, const
     if (tid == 0) count[g] = carry;
 }
 
-// Row offsets from the counts (one thread: rows are few).
+// Row offsets from the counts: one warp, 32 rows at a time.
 __global__ void coh_rec_offsets_kernel(int n_g, const int64_t *count, int64_t *row_off) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        int64_t run = 0;
-        row_off[0] = 0;
-        for (int g = 0; g < n_g; ++g) {
-            run += count[g];
-            row_off[g + 1] = run;
+    const int lane = threadIdx.x;
+    int64_t run = 0;
+    if (lane == 0) row_off[0] = 0;
+    for (int g0 = 0; g0 < n_g; g0 += 32) {
+        int64_t v = g0 + lane < n_g ? count[g0 + lane] : 0;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int64_t u = __shfl_up_sync(0xffffffffu, v, d);
+            if (lane >= d) v += u;
         }
+        if (g0 + lane < n_g) row_off[g0 + lane + 1] = run + v;
+        run += __shfl_sync(0xffffffffu, v, 31);
     }
 }
 

@@ -20,6 +20,7 @@
 #include "pb_common.cuh"
 #include "pb_internal.h"
 #include "pb_layers.cuh"
+#include "pb_moments.cuh"
 
 namespace pb {
 
@@ -54,13 +55,6 @@ __device__ __forceinline__ float b_log(float x) { return logf(x); }
 __device__ __forceinline__ double b_expm1(double x) { return expm1(x); }
 __device__ __forceinline__ float b_expm1(float x) { return expm1f(x); }
 
-// Base-2 exponential on the SFU (about 2 ulp), for the float path.
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Two floats in one 64-bit register pair, and the packed FP32 arithmetic of
 // sm_100 (one instruction for both halves).
 __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
@@ -93,13 +87,6 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 __device__ __forceinline__ float lg2_approx(float x) {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// Reciprocal on the SFU (about 1 ulp), for the float path.
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -384,98 +371,10 @@ __device__ __forceinline__ void brem_J2(F2 Tf, float T, float p_i, float bp, F2 
     }
 }
 
-// Whether the directions d0 .. d0 + nd - 1 leave through one face with path
-// factors in f_c +- dl, dl <= limit f_min. The kernels that share a launch make
-// the same test, so exactly one of them scores it: limit 0.01 for the packed
-// moment kernel.
-__device__ __forceinline__ bool brem_one_face(const pb_brem_args &a, int d0, int nd, double limit, double &f_c,
-                                              double &dl) {
-    int n_up = 0;
-    double f_lo = 1e300, f_hi = 0.0;
-    for (int dd = 0; dd < nd; ++dd) {
-        const double nz = a.n_hat[3 * (d0 + dd) + 2];
-        n_up += nz < 0.0 ? 1 : 0;
-        const double f = 1.0 / fmax(fabs(nz), 1.0e-12);
-        f_lo = fmin(f_lo, f);
-        f_hi = fmax(f_hi, f);
-    }
-    f_c = 0.5 * (f_lo + f_hi);
-    dl = 0.5 * (f_hi - f_lo);
-    return (n_up == nd || n_up == 0) && dl <= limit * f_lo;
-}
-
 template <int N>
 struct MomentOrder {
     static constexpr int value = N;
 };
-
-// Direction moments of the FP64 path and of the layered absorber: the same
-// recurrence as the packed kernel's. The truncation after order N is below
-// rho^(N+1) / sqrt(2 pi (N+1)) of the unattenuated term: FP64 takes N = 5 for
-// rho <= 0.002 and N = 9 for rho <= 0.02 (both below 2e-17), the mixed layered
-// path N = 3 for rho <= 0.01 (2e-9).
-template <class Real>
-constexpr double moment_limit() { return sizeof(Real) == 8 ? 0.02 : 0.01; }
-
-// Q_n += w P_n of one affine piece: a = optical depth of its shallower end along
-// the face normal, b = the depth difference of its ends, both per unit path
-// factor. Two exponentials serve every direction of the group, where each
-// direction took two of its own.
-template <int N>
-__device__ __forceinline__ void add_moments(double w, double a, double b, double f_c, double dl, double (&Q)[N + 1]) {
-    const double x = b * f_c;
-    const double Ea = exp(-a * f_c), em = -expm1(-x);
-    double P = w * Ea * f_c * (x > 1.0e-5 ? em / x : 1.0 - 0.5 * x + x * x / 6.0);
-    Q[0] += P;
-    if constexpr (N > 0) {
-        const double ah = -dl * a, ch = -dl * (a + b);
-        double R = w * dl * (Ea - Ea * em);
-#pragma unroll
-        for (int n = 1; n <= N; ++n) {
-            P = fma(ah, P, R);
-            R *= ch;
-            Q[n] += P;
-        }
-    }
-}
-template <int N>
-__device__ __forceinline__ void add_moments(float w, float a, float b, float f_c, float dl, float (&Q)[N + 1]) {
-    constexpr float kLog2e = 1.44269504f;
-    const float x = b * f_c;
-    const float Ea = ex2_approx(-kLog2e * a * f_c);
-    float P, Ec;
-    if (x > 0.35f) {
-        Ec = ex2_approx(-kLog2e * (a + b) * f_c);
-        P = w * (Ea - Ec) * (f_c * rcp_approx(x));
-    } else {
-        // phi(x) = (1 - e^-x) / x to x^7: truncation below 1e-9
-        const float phi = fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, -1.0f / 40320.0f, 1.0f / 5040.0f),
-                                                                              -1.0f / 720.0f), 1.0f / 120.0f),
-                                                       -1.0f / 24.0f), 1.0f / 6.0f), -0.5f), 1.0f);
-        P = w * Ea * f_c * phi;
-        Ec = Ea - Ea * (x * phi);
-    }
-    Q[0] += P;
-    if constexpr (N > 0) {
-        const float ah = -dl * a, ch = -dl * (a + b);
-        float R = w * dl * Ec;
-#pragma unroll
-        for (int n = 1; n <= N; ++n) {
-            P = fmaf(ah, P, R);
-            R *= ch;
-            Q[n] += P;
-        }
-    }
-}
-
-// (1 / f) sum_n ((f - f_c) / dl)^n Q_n / n! from the summed moments Q(n).
-template <class F>
-__device__ __forceinline__ double moments_at(int N, double f, double f_c, double dl, F Q) {
-    const double h = dl > 0.0 ? (f - f_c) / dl : 0.0;
-    double v = Q(N);
-    for (int n = N; n > 0; --n) v = fma(v, h / (double)n, Q(n - 1));
-    return v / f;
-}
 
 template <int NEL>
 __global__ void __launch_bounds__(kBremPackedThreads, 3)
@@ -492,7 +391,7 @@ __global__ void __launch_bounds__(kBremPackedThreads, 3)
     __shared__ Pk pk[kBremChunk];
     const int nd = (a.n_dir - d0) < kBremMaxDir ? (a.n_dir - d0) : kBremMaxDir;
     double f_c_d, dl_d;
-    if (a.precision != PB_MIXED || !brem_one_face(a, d0, nd, 0.01, f_c_d, dl_d)) return;
+    if (a.precision != PB_MIXED || !one_face(a.n_hat, d0, nd, 0.01, f_c_d, dl_d)) return;
     const bool up_all = a.n_hat[3 * d0 + 2] < 0.0;
     // Moment order: 2 where rho = Delta / f_min <= 0.002 (truncation below
     // rho^3 / sqrt(6 pi) < 2e-9 of the unattenuated term), else 3.
@@ -793,7 +692,7 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
     // (brem_moment_packed_kernel) scores this launch.
     if constexpr (sizeof(Real) == 4) {
         double fc_p, dl_p;
-        if (brem_one_face(a, d0, nd, 0.01, fc_p, dl_p)) return;
+        if (one_face(a.n_hat, d0, nd, 0.01, fc_p, dl_p)) return;
     }
     // Moment form (see brem_moment_chunk): float, one exit face, and the
     // path factors within rho = Delta / f_min <= 0.05 of their centre.
@@ -819,7 +718,7 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
         }
     }
     if constexpr (sizeof(Real) == 8) {
-        if (brem_one_face(a, d0, nd, moment_limit<double>(), f_c, dl)) {
+        if (one_face(a.n_hat, d0, nd, moment_limit<double>(), f_c, dl)) {
             const double rho = dl / (f_c - dl);
             order = dl == 0.0 ? 0 : (rho <= 0.002 ? 5 : 9);
         }
@@ -1031,7 +930,7 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     const int nd = (a.n_dir - d0) < kBremMaxDir ? (a.n_dir - d0) : kBremMaxDir;
     double f_c, dl;
     // both instances make the same test: one of them scores the launch
-    if (brem_one_face(a, d0, nd, moment_limit<Real>(), f_c, dl) != kMoments) return;
+    if (one_face(a.n_hat, d0, nd, moment_limit<Real>(), f_c, dl) != kMoments) return;
     const int n_el = a.n_el;
     const int nl = a.n_layer;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;

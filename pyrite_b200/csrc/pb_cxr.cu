@@ -70,6 +70,9 @@ constexpr int kMaxTab = 4096;   // E_tab / delta staged in shared memory up to t
 // (division by reciprocal, sqrt by reciprocal square root, base-2 exp/log),
 // each within a few ulp, which the 1 % spectrum tolerance of the mixed path
 // absorbs many times over.
+// A rounded product the compiler does not contract into the following addition.
+__device__ __forceinline__ float r_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double r_mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double r_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float r_sqrt(float x) { return x > 0.0f ? x * rsqrtf(x) : sqrtf(x); }
 __device__ __forceinline__ double r_exp(double x) { return exp(x); }
@@ -406,7 +409,9 @@ __device__ __forceinline__ Resonance<Real> pair_resonance(const SegPre<Real> &sp
     const Real r_den = n_dot_g * sp.inv_E;
     const Real v_dot_g = sp.vx * Gx + sp.vy * Gy + sp.vz * Gz;
     const Real v_dot_g_exact = v_dot_g - r_num;
-    const Real denom_vac = sp.denom_row + r_den;
+    // (rounded as written, so that a float line lies at the same energy in the slab
+    // and the layered instance: one ulp is 4e-3 eV at 40 keV)
+    const Real denom_vac = sp.denom_row + r_mul(n_dot_g, sp.inv_E);
     // cxr/_kernels.py:702-765
     Real denom = denom_vac, previous = denom, delta = (Real)NAN;
     Cell<Real> cell;

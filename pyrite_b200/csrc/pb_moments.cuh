@@ -1,0 +1,116 @@
+// Direction moments of the segment-mean escape.
+//
+// A piece of a segment escapes towards a direction with path factor f = 1/|n_z|
+// with the mean of exp(-(a + b u) f) over u in [0, 1]: a the optical depth of the
+// end nearer the exit face, b the depth difference of the ends, both along the
+// face normal. g(f) = (exp(-a f) - exp(-(a + b) f)) / b, its Taylor coefficients
+// about a centre f_c follow without cancellation and do not depend on the
+// direction, so the directions of one detector share two exponentials.
+#pragma once
+
+#include "pb_common.cuh"
+
+namespace pb {
+
+// Base-2 exponential on the SFU (about 2 ulp), for the float path.
+__device__ __forceinline__ float ex2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Reciprocal on the SFU (about 1 ulp), for the float path.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Whether the directions d0 .. d0 + nd - 1 leave through one face with path
+// factors 1 / |n_z| in f_c +- dl, dl <= limit f_min. Kernels that share a launch
+// make the same test, so exactly one of them scores it.
+__device__ __forceinline__ bool one_face(const double *n_hat, int d0, int nd, double limit, double &f_c, double &dl) {
+    int n_up = 0;
+    double f_lo = 1e300, f_hi = 0.0;
+    for (int dd = 0; dd < nd; ++dd) {
+        const double nz = n_hat[3 * (d0 + dd) + 2];
+        n_up += nz < 0.0 ? 1 : 0;
+        const double f = 1.0 / fmax(fabs(nz), 1.0e-12);
+        f_lo = fmin(f_lo, f);
+        f_hi = fmax(f_hi, f);
+    }
+    f_c = 0.5 * (f_lo + f_hi);
+    dl = 0.5 * (f_hi - f_lo);
+    return (n_up == nd || n_up == 0) && dl <= limit * f_lo;
+}
+
+// Direction moments of the segment-mean escape, for the FP64 bremsstrahlung, the
+// layered absorber and the characteristic lines (the mixed single-slab kernels
+// carry packed forms of the same recurrence). The truncation after order N is below
+// rho^(N+1) / sqrt(2 pi (N+1)) of the unattenuated term: FP64 takes N = 5 for
+// rho <= 0.002 and N = 9 for rho <= 0.02 (both below 2e-17), the mixed layered
+// path N = 3 for rho <= 0.01 (2e-9).
+template <class Real>
+constexpr double moment_limit() { return sizeof(Real) == 8 ? 0.02 : 0.01; }
+
+// Q_n += w P_n of one affine piece: a = optical depth of its shallower end along
+// the face normal, b = the depth difference of its ends, both per unit path
+// factor. Two exponentials serve every direction of the group, where each
+// direction took two of its own.
+template <int N>
+__device__ __forceinline__ void add_moments(double w, double a, double b, double f_c, double dl, double (&Q)[N + 1]) {
+    const double x = b * f_c;
+    const double Ea = exp(-a * f_c), em = -expm1(-x);
+    double P = w * Ea * f_c * (x > 1.0e-5 ? em / x : 1.0 - 0.5 * x + x * x / 6.0);
+    Q[0] += P;
+    if constexpr (N > 0) {
+        const double ah = -dl * a, ch = -dl * (a + b);
+        double R = w * dl * (Ea - Ea * em);
+#pragma unroll
+        for (int n = 1; n <= N; ++n) {
+            P = fma(ah, P, R);
+            R *= ch;
+            Q[n] += P;
+        }
+    }
+}
+template <int N>
+__device__ __forceinline__ void add_moments(float w, float a, float b, float f_c, float dl, float (&Q)[N + 1]) {
+    constexpr float kLog2e = 1.44269504f;
+    const float x = b * f_c;
+    const float Ea = ex2_approx(-kLog2e * a * f_c);
+    float P, Ec;
+    if (x > 0.35f) {
+        Ec = ex2_approx(-kLog2e * (a + b) * f_c);
+        P = w * (Ea - Ec) * (f_c * rcp_approx(x));
+    } else {
+        // phi(x) = (1 - e^-x) / x to x^7: truncation below 1e-9
+        const float phi = fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, -1.0f / 40320.0f, 1.0f / 5040.0f),
+                                                                              -1.0f / 720.0f), 1.0f / 120.0f),
+                                                       -1.0f / 24.0f), 1.0f / 6.0f), -0.5f), 1.0f);
+        P = w * Ea * f_c * phi;
+        Ec = Ea - Ea * (x * phi);
+    }
+    Q[0] += P;
+    if constexpr (N > 0) {
+        const float ah = -dl * a, ch = -dl * (a + b);
+        float R = w * dl * Ec;
+#pragma unroll
+        for (int n = 1; n <= N; ++n) {
+            P = fmaf(ah, P, R);
+            R *= ch;
+            Q[n] += P;
+        }
+    }
+}
+
+// (1 / f) sum_n ((f - f_c) / dl)^n Q_n / n! from the summed moments Q(n).
+template <class F>
+__device__ __forceinline__ double moments_at(int N, double f, double f_c, double dl, F Q) {
+    const double h = dl > 0.0 ? (f - f_c) / dl : 0.0;
+    double v = Q(N);
+    for (int n = N; n > 0; --n) v = fma(v, h / (double)n, Q(n - 1));
+    return v / f;
+}
+
+}  // namespace pb

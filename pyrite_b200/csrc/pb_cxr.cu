@@ -1399,12 +1399,33 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     // the chunks carry equal work. Fewer than four units a block: halve the tile, so that a short
     // segment list still reaches every SM (a tile below four segments leaves
     // most threads of a pass idle).
-    int64_t d_ch = -1;
-    for (int64_t wk = w_begin;; ++wk) {
+    int64_t d_ch = -1, win = -1;
+    // Tiles without a radiating segment are passed over a window of kCxrThreads
+    // segments at a time: one flag word per warp, a tile is 4, 8 or 16 of its bits.
+    unsigned *const rad_words = reinterpret_cast<unsigned *>(scratch);
+    const int per_win = kCxrThreads / seg_tile;
+    int64_t wk = w_begin, dc = n_work > 0 ? w_begin / n_tiles : 0, tile = w_begin - dc * n_tiles;
+    const auto next_unit = [&]() {
+        ++wk;
+        if (++tile == n_tiles) { tile = 0; ++dc; }
+    };
+    for (;; next_unit()) {
+        for (; wk < w_end && !pairs_out; next_unit()) {
+            if (tile / per_win != win) {
+                win = tile / per_win;
+                const int64_t sg = win * kCxrThreads + tid;
+                const bool rad = sg < n_seg && a.elec_id[sg] < a.Ne &&
+                                 (a.seg_layer == nullptr || a.seg_layer[sg] == a.emit_layer);
+                const unsigned mask = __ballot_sync(0xffffffffu, rad);
+                __syncthreads();  // the last window's flags have been read
+                if (lane == 0) rad_words[warp] = mask;
+                __syncthreads();
+            }
+            const int bit = (int)(tile % per_win) * seg_tile;
+            if ((rad_words[bit >> 5] >> (bit & 31)) & ((1u << seg_tile) - 1u)) break;
+        }
         const bool end = wk >= w_end;
-        const int64_t dc = end ? 0 : wk / n_tiles;
-        const int64_t tile = wk - dc * n_tiles;
-        const int d = (int)(dc / n_chunks);
+        const int d = (int)dc / n_chunks;
         // The lines the last unit queued: whole rounds, or all of them before
         // the direction changes or the block ends.
         const bool leave = end || d != d_cur;
@@ -1419,16 +1440,13 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
         const double *nh = a.n_hat + 3 * d;
         const int64_t s0 = tile * seg_tile;
         const int nst = (int)((n_seg - s0) < seg_tile ? (n_seg - s0) : seg_tile);
-        const bool rad = tid < nst && a.elec_id[s0 + tid] < a.Ne &&
-                         (a.seg_layer == nullptr || a.seg_layer[s0 + tid] == a.emit_layer);
-        // (also the barrier before the staged rows and segments are replaced)
-        if (!__syncthreads_or(rad) && !pairs_out) continue;
+        __syncthreads();  // before the staged rows and segments are replaced
         if (tid < nst) seg_precompute<Real>(segs[tid], a, s0 + tid, nh);
         if constexpr (kLayered) {
             if (tid < nst) esc_precompute<Real>(esc[tid], a, s0 + tid, nh, lay_zt, lay_zb);
         }
         {
-            const int g0 = (int)(dc - (int64_t)d * n_chunks);
+            const int g0 = (int)dc - d * n_chunks;
             const int ng = (n_g - g0 + n_chunks - 1) / n_chunks;
             // q / ng for the pass's pair ids q < kSegTile * ng by a multiply-high:
             // magic = floor((2^32 - 1) / ng) + 1 is at least 2^32 / ng and

@@ -320,23 +320,63 @@ __device__ __forceinline__ Real beta_from_keV(Real E) {
 }
 
 // core_geometry.py:16-35
+// The part of the rotation that does not need the polar angle: the transverse
+// axes of the direction and the azimuth, ready before the energy of the event is.
 template <class Real>
-__device__ __forceinline__ void rotate(Real &dx, Real &dy, Real &dz, Real cos_t, Real phi) {
-    const Real st2 = (Real)1 - cos_t * cos_t;
-    const Real sin_t = m_sqrt(st2 > (Real)0 ? st2 : (Real)0);
-    const Real cp = m_cos(phi), sp = m_sin(phi);
-    Real refx, refy;
-    if (fabs(dx) < (Real)0.9) { refx = 1; refy = 0; } else { refx = 0; refy = 1; }
+struct Azimuth {
+    Real ux, uy, uz, wx, wy, wz, cp, sp;
+};
+
+template <class Real>
+__device__ __forceinline__ Azimuth<Real> azimuth(Real dx, Real dy, Real dz, Real phi) {
+    Azimuth<Real> z;
+    z.cp = m_cos(phi);
+    z.sp = m_sin(phi);
+    const bool x_ref = fabs(dx) < (Real)0.9;
+    const Real refx = x_ref ? (Real)1 : (Real)0, refy = x_ref ? (Real)0 : (Real)1;
     Real ux = -dz * refy, uy = dz * refx, uz = dx * refy - dy * refx;
     const Real um = m_sqrt(ux * ux + uy * uy + uz * uz);
-    ux /= um; uy /= um; uz /= um;
-    const Real wx = dy * uz - dz * uy, wy = dz * ux - dx * uz, wz = dx * uy - dy * ux;
-    const Real a = sin_t * cp, b = sin_t * sp;
-    const Real ox = cos_t * dx + a * ux + b * wx;
-    const Real oy = cos_t * dy + a * uy + b * wy;
-    const Real oz = cos_t * dz + a * uz + b * wz;
+    z.ux = ux / um; z.uy = uy / um; z.uz = uz / um;
+    z.wx = dy * z.uz - dz * z.uy;
+    z.wy = dz * z.ux - dx * z.uz;
+    z.wz = dx * z.uy - dy * z.ux;
+    return z;
+}
+
+template <class Real>
+__device__ __forceinline__ void rotate(Real &dx, Real &dy, Real &dz, Real cos_t, const Azimuth<Real> &z) {
+    const Real st2 = (Real)1 - cos_t * cos_t;
+    const Real sin_t = m_sqrt(st2 > (Real)0 ? st2 : (Real)0);
+    const Real a = sin_t * z.cp, b = sin_t * z.sp;
+    const Real ox = cos_t * dx + a * z.ux + b * z.wx;
+    const Real oy = cos_t * dy + a * z.uy + b * z.wy;
+    const Real oz = cos_t * dz + a * z.uz + b * z.wz;
     const Real m = m_sqrt(ox * ox + oy * oy + oz * oz);
     dx = ox / m; dy = oy / m; dz = oz / m;
+}
+
+// Draws d, d + 1 and d + 2 of a stream. Two Philox blocks hold them (three
+// single draws would run three).
+template <int kRng>
+__device__ __forceinline__ void uniform3(uint64_t key, uint64_t d, double &u0, double &u1, double &u2) {
+    if constexpr (kRng == PB_RNG_PHILOX) {
+        const uint64_t block = d >> 1;
+        uint32_t a[4] = {(uint32_t)block, (uint32_t)(block >> 32), 0u, 0u};
+        uint32_t b[4] = {(uint32_t)(block + 1), (uint32_t)((block + 1) >> 32), 0u, 0u};
+        philox4x32_10(a[0], a[1], a[2], a[3], (uint32_t)key, (uint32_t)(key >> 32));
+        philox4x32_10(b[0], b[1], b[2], b[3], (uint32_t)key, (uint32_t)(key >> 32));
+        const bool odd = d & 1ULL;
+        const auto to_unit = [](uint32_t x, uint32_t y) {
+            return ((double)(x >> 5) * 67108864.0 + (double)(y >> 6)) * (1.0 / 9007199254740992.0);
+        };
+        u0 = odd ? to_unit(a[2], a[3]) : to_unit(a[0], a[1]);
+        u1 = odd ? to_unit(b[0], b[1]) : to_unit(a[2], a[3]);
+        u2 = odd ? to_unit(b[2], b[3]) : to_unit(b[0], b[1]);
+    } else {
+        u0 = splitmix_uniform(key, d);
+        u1 = splitmix_uniform(key, d + 1);
+        u2 = splitmix_uniform(key, d + 2);
+    }
 }
 
 // LUT view (shared or global memory) in the flight precision.
@@ -359,10 +399,10 @@ __device__ __forceinline__ void lut_index(const LutView<Real> &t, double E, int 
     if constexpr (sizeof(Real) == 8) x = (log(E) - t.log_E_min) * t.inv_dlogE;
     else x = (logf((float)E) - (float)t.log_E_min) * (float)t.inv_dlogE;
     const int last = t.ne - 1;
-    if (x >= (Real)last) { i = last - 1; f = 1; return; }
-    if (x > (Real)0) { const int ii = (int)x; i = ii; f = x - (Real)ii; return; }
-    i = 0;
-    f = 0;
+    const bool top = x >= (Real)last, in = x > (Real)0;
+    const int ii = in && !top ? (int)x : 0;
+    i = top ? last - 1 : ii;
+    f = top ? (Real)1 : in ? x - (Real)ii : (Real)0;
 }
 
 template <class Real>
@@ -568,7 +608,6 @@ __global__ void __launch_bounds__(256) transport_kernel(const pb_transport_args 
     Real dx = 0, dy = 0, dz = 1;
     double E = 0.0, clk = 0.0;
     int64_t nseg = 0, steps = 0;
-    Real tau_left = -1;
     // LUT index of the current energy, where the last event looked it up.
     bool have_idx = false;
     int idx_E = 0;
@@ -632,7 +671,6 @@ __global__ void __launch_bounds__(256) transport_kernel(const pb_transport_args 
                     draws = 0;
                     nseg = 0;
                     steps = 0;
-                    tau_left = -1;
                     have_idx = false;
                 } else {
                     i = -2;
@@ -657,6 +695,17 @@ __global__ void __launch_bounds__(256) transport_kernel(const pb_transport_args 
             const int n_el = ly.n_el[L];
             const double E_j = E;
             const Real Er = (Real)E_j;
+            // The event's draws and what follows from them and the direction
+            // alone, ahead of the chain step -> energy -> angle: tau, (with
+            // several elements, the element,) polar and azimuthal draw.
+            double u_tau, u_b, u_c;
+            uniform3<kRng>(key, draws, u_tau, u_b, u_c);
+            const bool several = n_el > 1;
+            const double u_phi = several ? uniform<kRng>(key, draws + 3) : u_c;
+            const double u_cos = several ? u_c : u_b;
+            const Azimuth<Real> azi = azimuth<Real>(dx, dy, dz, (Real)(2.0 * kPi) * (Real)u_phi);
+            const Real tau = (Real)(-log(u_tau));
+            draws += 1;
             int li = 0;
             Real lf = 0;
             Real total_rate = 0;
@@ -677,19 +726,12 @@ __global__ void __launch_bounds__(256) transport_kernel(const pb_transport_args 
                 }
             }
             const Real lam = (Real)1e8 / total_rate;
-            if (tau_left < (Real)0) {
-                tau_left = (Real)(-log(uniform<kRng>(key, draws)));
-                draws += 1;
-            }
-            Real step = tau_left * lam;
-            bool cross_up = false, cross_dn = false;
-            if (dz < (Real)0) {
-                const Real sb = (Real)((pz - z_top) / (double)(-dz));
-                if (step > sb) { step = sb; cross_up = true; }
-            } else if (dz > (Real)0) {
-                const Real sb = (Real)((z_bot - pz) / (double)dz);
-                if (step > sb) { step = sb; cross_dn = true; }
-            }
+            Real step = tau * lam;
+            // distance to the face ahead (none for dz = 0: the quotient is unused)
+            const bool down = dz > (Real)0, ups = dz < (Real)0;
+            const Real sb = (Real)((ups ? pz - z_top : z_bot - pz) / (double)(ups ? -dz : dz));
+            bool cross_up = ups && step > sb, cross_dn = down && step > sb;
+            if (cross_up || cross_dn) step = sb;
             bool exit_top = cross_up && z_top <= 0.0;
             bool exit_bot = cross_dn && z_bot >= z_total;
             const bool geometry_event = cross_up || cross_dn;
@@ -854,7 +896,6 @@ __global__ void __launch_bounds__(256) transport_kernel(const pb_transport_args 
             pz = pz + (double)(step * dz);
             E = E_end;
             clk = t_end;
-            tau_left = (Real)-1;
             have_idx = false;
             if (exit_top || exit_bot || cutoff) {
                 code = exit_top ? EXIT_BACK : exit_bot ? EXIT_TRANS : EXIT_CUTOFF;
@@ -864,7 +905,7 @@ __global__ void __launch_bounds__(256) transport_kernel(const pb_transport_args 
             } else {
                 int i_el = 0;
                 if (n_el > 1) {
-                    const double u = uniform<kRng>(key, draws);
+                    const double u = u_b;
                     draws += 1;
                     i_el = n_el - 1;
                     if constexpr (kLut) {
@@ -895,17 +936,15 @@ __global__ void __launch_bounds__(256) transport_kernel(const pb_transport_args 
                 } else {
                     alpha = (Real)ly.sjn[L * max_el + i_el] / (Real)E;
                 }
-                const double cos_ud = uniform<kRng>(key, draws);
+                const double cos_ud = u_cos;
                 const Real cos_u = (Real)cos_ud;
-                draws += 1;
-                const Real phi_u = (Real)uniform<kRng>(key, draws);
-                draws += 1;
+                draws += 2;
                 Real cos_t;
                 if (kTab && p.elastic_model == PB_ELASTIC_ELSEPA)
                     cos_t = (Real)elsepa_cos_theta(p.elsepa, L * max_el + i_el, E, cos_ud);
                 else
                     cos_t = (Real)1 - (Real)2 * alpha * cos_u / ((Real)1 + alpha - cos_u);
-                rotate<Real>(dx, dy, dz, cos_t, (Real)(2.0 * kPi) * phi_u);
+                rotate<Real>(dx, dy, dz, cos_t, azi);
                 steps += 1;
             }
         }

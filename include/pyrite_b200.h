@@ -539,6 +539,13 @@ int pb_mlp_pack(int32_t rows, int32_t cols, const float *W, void *Wb, int32_t ld
 int pb_segments_sample(const pb_segments *src, int64_t stride, const pb_segments *dst, unsigned int *status,
                        void *stream);
 
+/* Pack the rows of n histories, laid out src[i * cap + s] with seg_count[i] <= cap
+ * rows each (pb_transport_args.rows), one history after another: row s of
+ * history i goes to dst[offset[i] + s], every field of src (all must be set in
+ * both). seg_count and offset are device arrays. */
+int pb_rows_compact(const pb_rows *src, int64_t n, int64_t cap, const int64_t *seg_count, const int64_t *offset,
+                    const pb_rows *dst, void *stream);
+
 /* Copy n device byte ranges in one launch: desc (device memory) holds n
  * triples (source address, destination address, bytes) as int64. Ranges must
  * not overlap. The host API moves a step's scattered inputs and outputs

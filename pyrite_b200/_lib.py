@@ -205,6 +205,7 @@ class PbCoherentBlendArgs(C.Structure):
 # Exported symbols declared by include/pyrite_b200.h, checked by the tests.
 EXPORTS = (
     "pb_abi_version",
+    "pb_rows_compact",
     "pb_last_error",
     "pb_device_count",
     "pb_transport",
@@ -271,6 +272,7 @@ def load(path: Path | None = None):
     lib.pb_cxr_score.argtypes = [C.POINTER(PbCxrArgs), _vp]
     lib.pb_brem_score.argtypes = [C.POINTER(PbBremArgs), _vp]
     lib.pb_brem_work_size.argtypes = [C.POINTER(PbBremArgs), C.POINTER(_i64)]
+    lib.pb_rows_compact.argtypes = [C.POINTER(PbRows), _i64, _i64, _vp, _vp, C.POINTER(PbRows), _vp]
     lib.pb_copy_segments.argtypes = [_i32, _vp, _vp]
     lib.pb_cxr_score_noalloc.argtypes = [C.POINTER(PbCxrArgs), _vp]
     lib.pb_char_yields.argtypes = [C.POINTER(PbCharArgs), _vp]

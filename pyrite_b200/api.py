@@ -37,6 +37,13 @@ from .tables import (
     reflection_rows,
 )
 
+# Fields of a segment row: result key, pb_rows member, type, values per row.
+_ROW_FIELDS = (("r_mid", "r_mid", torch.float64, 3), ("v_hat", "v_hat", torch.float64, 3), ("L_ang", "L", torch.float64, 1),
+               ("E_keV", "E_start", torch.float64, 1), ("E_end_keV", "E_end", torch.float64, 1),
+               ("t_ang", "t_start", torch.float64, 1), ("t_end_ang", "t_end", torch.float64, 1),
+               ("elec_id", "elec_id", torch.int64, 1), ("flight_id", "flight", torch.int64, 1),
+               ("layer", "layer", torch.int16, 1), ("event_kind", "event", torch.int8, 1))
+
 EXIT_NAMES = ("n_cutoff_stopped", "n_backscattered", "n_transmitted", "n_side_exited",
               "n_step_limited", "n_missed")
 
@@ -231,6 +238,20 @@ _RNG = {"splitmix": L.PB_RNG_SPLITMIX, "philox": L.PB_RNG_PHILOX}
 _PREC = {"fp64": L.PB_FP64, "mixed": L.PB_MIXED}
 
 
+def _row_block(h: "_Holder", m: int):
+    """Storage of ``m`` segment rows in one device block, field after field:
+    (pb_rows, block, [(key, offset, bytes, type, shape)])."""
+    r, parts, off = L.PbRows(), [], 0
+    for key, member, dtype, k in _ROW_FIELDS:
+        nb = m * k * dtype.itemsize
+        parts.append((key, member, off, nb, dtype, (m, 3) if k == 3 else (m,)))
+        off = (off + nb + 255) & ~255
+    block = h.empty(max(off, 1), torch.uint8)
+    for _key, member, o, _nb, _dtype, _shape in parts:
+        setattr(r, member, block.data_ptr() + o)
+    return r, block, [(key, o, nb, dtype, shape) for key, _m, o, nb, dtype, shape in parts]
+
+
 def _fill_elsepa(h: "_Holder", g: ElsepaGroup) -> "L.PbElsepa":
     t = L.PbElsepa()
     t.n_mu, t.cells = int(g.mu.size), int(g.guide.shape[1] - 1)
@@ -304,7 +325,7 @@ def simulate_trajectories(E0_keV, Ne, thickness_ang=None, element=None, n_atoms_
         check_stopping_range(stop, float(E_cut_keV), E_hi)
         lut = False  # table stopping runs on the exact core
     dev = _device(device)
-    h = _Holder(dev)
+    h = _Holder(dev, pack=True)
     a = L.PbTransportArgs()
     a.rng = _RNG[rng]
     a.precision = _PREC[precision]
@@ -338,28 +359,14 @@ def simulate_trajectories(E0_keV, Ne, thickness_ang=None, element=None, n_atoms_
     cap = int(cap) if cap is not None else 512
     n = int(Ne)
     m = n * cap
-    rows = dict(
-        r_mid=h.empty((m, 3), torch.float64), v_hat=h.empty((m, 3), torch.float64),
-        L_ang=h.empty(m, torch.float64), E_keV=h.empty(m, torch.float64),
-        E_end_keV=h.empty(m, torch.float64), t_ang=h.empty(m, torch.float64),
-        t_end_ang=h.empty(m, torch.float64), elec_id=h.empty(m, torch.int64),
-        layer=h.empty(m, torch.int16), flight_id=h.empty(m, torch.int64),
-        event_kind=h.empty(m, torch.int8),
-    )
     a.cap = cap
-    r = L.PbRows()
-    r.r_mid, r.v_hat, r.L = _ptr(rows["r_mid"]), _ptr(rows["v_hat"]), _ptr(rows["L_ang"])
-    r.E_start, r.E_end = _ptr(rows["E_keV"]), _ptr(rows["E_end_keV"])
-    r.t_start, r.t_end = _ptr(rows["t_ang"]), _ptr(rows["t_end_ang"])
-    r.elec_id, r.layer = _ptr(rows["elec_id"]), _ptr(rows["layer"])
-    r.flight, r.event = _ptr(rows["flight_id"]), _ptr(rows["event_kind"])
+    r, _block, _parts = _row_block(h, m)
     a.rows = r
     seg_count = h.zeros(n, torch.int64)
     exit_code = h.zeros(n, torch.int8)
     final_E = h.zeros(n, torch.float64)
     a.seg_count, a.exit_code, a.final_E = _ptr(seg_count), _ptr(exit_code), _ptr(final_E)
-    wc = h.zeros(1, torch.int64)
-    status = h.zeros(1, torch.int32)
+    wc, status = h.flag(torch.int64), h.flag(torch.int32)
     a.work_counter, a.status = _ptr(wc), _ptr(status)
     tal_t = None
     if tallies is not None:
@@ -372,6 +379,7 @@ def simulate_trajectories(E0_keV, Ne, thickness_ang=None, element=None, n_atoms_
         tal.n_theta, tal.theta_lo, tal.theta_hi = n_tth, 0.0, float(np.pi)
         tal.deposit = _ptr(tal_t["deposit"])
         a.tallies = tal
+    h.commit()
     L.check(lib.pb_transport(C.byref(a), _stream_ptr(stream)), "pb_transport")
     torch.cuda.synchronize(dev)
     st = int(status.item())
@@ -384,9 +392,17 @@ def simulate_trajectories(E0_keV, Ne, thickness_ang=None, element=None, n_atoms_
             tilt_azim_rad, transverse_distribution, lut=lut, rng=rng, precision=precision,
             entry=entry, cap=int(counts.max()), device=device, stream=stream,
             block_threads=block_threads, tallies=tallies, straggling=straggling)
-    mask = (np.arange(cap)[None, :] < counts[:, None]).reshape(-1)
-    idx = torch.from_numpy(np.flatnonzero(mask)).to(dev)
-    out = {k: v.index_select(0, idx).cpu().numpy() for k, v in rows.items()}
+    # The rows, packed history after history on the device, in one copy.
+    total = int(counts.sum())
+    packed, block, parts = _row_block(h, total)
+    if total:
+        offset = torch.from_numpy(np.cumsum(counts) - counts).to(dev)
+        L.check(lib.pb_rows_compact(C.byref(r), n, cap, _ptr(seg_count), _ptr(offset), C.byref(packed),
+                                    _stream_ptr(stream)), "pb_rows_compact")
+        torch.cuda.synchronize(dev)
+    host = block.cpu().numpy()
+    out = {key: host[o:o + nb].view(str(dtype).removeprefix("torch.")).reshape(shape)
+           for key, o, nb, dtype, shape in parts}
     out["E_repr_keV"] = 0.5 * (out["E_keV"] + out["E_end_keV"])
     out["E_start_keV"] = out["E_keV"]
     codes = exit_code.cpu().numpy()

@@ -386,6 +386,52 @@ __global__ void __launch_bounds__(256) copy_segments_kernel(int n, const int64_t
 }
 }  // namespace
 
+namespace {
+// A warp per history: its rows are short runs (a dozen to a few hundred), each
+// field a coalesced copy.
+__global__ void __launch_bounds__(256) rows_compact_kernel(pb_rows src, int64_t n, int64_t cap,
+                                                           const int64_t *seg_count, const int64_t *offset,
+                                                           pb_rows dst) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
+        const int64_t count = seg_count[i] < cap ? seg_count[i] : cap, from = i * cap, to = offset[i];
+        for (int64_t s = lane; s < 3 * count; s += 32) {
+            dst.r_mid[3 * to + s] = src.r_mid[3 * from + s];
+            dst.v_hat[3 * to + s] = src.v_hat[3 * from + s];
+        }
+        for (int64_t s = lane; s < count; s += 32) {
+            dst.L[to + s] = src.L[from + s];
+            dst.E_start[to + s] = src.E_start[from + s];
+            dst.E_end[to + s] = src.E_end[from + s];
+            dst.t_start[to + s] = src.t_start[from + s];
+            dst.t_end[to + s] = src.t_end[from + s];
+            dst.elec_id[to + s] = src.elec_id[from + s];
+            dst.flight[to + s] = src.flight[from + s];
+            dst.layer[to + s] = src.layer[from + s];
+            dst.event[to + s] = src.event[from + s];
+        }
+    }
+}
+}  // namespace
+
+int pb_rows_compact(const pb_rows *src, int64_t n, int64_t cap, const int64_t *seg_count, const int64_t *offset,
+                    const pb_rows *dst, void *stream) {
+    if (!src || !dst || n < 0 || cap < 0) return fail(PB_ERR_INVALID, "pb_rows_compact: need src, dst, n >= 0, cap >= 0");
+    if (n == 0 || cap == 0) return PB_OK;
+    for (const pb_rows *r : {src, dst})
+        if (!r->r_mid || !r->v_hat || !r->L || !r->E_start || !r->E_end || !r->t_start || !r->t_end || !r->elec_id ||
+            !r->layer || !r->flight || !r->event)
+            return fail(PB_ERR_INVALID, "pb_rows_compact: every field of src and dst must be set");
+    if (!seg_count || !offset) return fail(PB_ERR_INVALID, "pb_rows_compact: seg_count and offset must be set");
+    const int64_t blocks = (n + 7) / 8;
+    const int64_t grid = blocks < 16 * (int64_t)device_sms() ? blocks : 16 * (int64_t)device_sms();
+    rows_compact_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(*src, n, cap, seg_count, offset, *dst);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "pb_rows_compact: launch");
+    return PB_OK;
+}
+
 int pb_copy_segments(int32_t n, const int64_t *desc, void *stream) {
     if (n < 0 || (n > 0 && !desc)) return fail(PB_ERR_INVALID, "pb_copy_segments: need n >= 0 and desc");
     if (n == 0) return PB_OK;

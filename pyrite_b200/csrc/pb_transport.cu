@@ -1020,10 +1020,12 @@ static cudaError_t launch_transport_t(const pb_transport_args &a, cudaStream_t s
     if (err != cudaSuccess) return err;
     if (per_sm < 1) per_sm = 1;
     // Histories per warp: the fewest that put the launch on the GPU's resident
-    // warps in one wave, all 32 lanes from there on.
+    // warps in one wave, all 32 lanes from there on. Up to 32 histories stay in one
+    // warp: its appends come in event order, so that a segment buffer too small
+    // for them keeps the same segments on every run.
     const int64_t warps = (int64_t)sms * per_sm * std::max(threads / 32, 1);
     int lanes = 32;
-    if (threads % 32 == 0) lanes = (int)std::min<int64_t>(32, std::max<int64_t>(1, (a.n + warps - 1) / warps));
+    if (threads % 32 == 0 && a.n > 32) lanes = (int)std::min<int64_t>(32, std::max<int64_t>(1, (a.n + warps - 1) / warps));
     if (lanes <= kStageLanes && a.seg.L != nullptr) dyn += (size_t)(threads / 32) * sizeof(SegStage);
     const int64_t per_block = (int64_t)lanes * (threads / 32 > 0 ? threads / 32 : 1);
     int64_t want = threads % 32 == 0 ? (a.n + per_block - 1) / per_block : (a.n + threads - 1) / threads;

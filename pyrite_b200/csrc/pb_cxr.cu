@@ -39,11 +39,15 @@
 namespace pb {
 
 constexpr int kSegTile = 16;
-constexpr int kCxrThreads = 256;  // two resident blocks per SM (128 registers each)
-// Reflection rows per pass: 120 on the float path (a pass's prefilter
-// survivors then fill the block's threads about twice, with a smaller idle
-// tail than at 64 rows, measured 10 % faster on the control variate's
-// sub-sample), 48 on the FP64 path, whose staged tables need the room.
+constexpr int kCxrThreads = 256;
+// Two blocks an SM (128 registers). Three of the float instances fit 80 registers
+// and 75 KB, but the kernel is bound by issue, not latency: 8192 histories of the
+// 50 MeV Si scene took 95.9 ms with three and 82.7 with two, whose passes are
+// larger.
+constexpr int kCxrBlocks = 2;
+// Reflection rows per pass: 120 on the float path (a pass's prefilter survivors
+// then fill the block's threads about one and a half times), 48 on the FP64 path,
+// whose queues and tables take twice the room.
 template <class Real>
 constexpr int row_chunk() { return sizeof(Real) == 4 ? 120 : 48; }
 template <class Real>
@@ -63,6 +67,11 @@ enum WinClass { kWin4 = 0, kWin8, kWin16, kWin32, kWinStrip, kWinAxis, kWinClass
 constexpr int kStripSpan = 124;
 // Strip lines wait for one another over several window phases.
 constexpr int kStripRun = kCxrThreads / 2;
+// The list's lines by class: two classes share an index array, one from each end
+// (a line is in one class, so the ends cannot meet).
+__device__ __forceinline__ int win_slot(int cls, int k) {
+    return (cls >> 1) * kWideCap + ((cls & 1) ? kWideCap - 1 - k : k);
+}
 constexpr int kMaxTab = 4096;   // E_tab / delta staged in shared memory up to this size
 
 // Math of the line chain. FP64 uses IEEE operations throughout (parity with
@@ -219,13 +228,13 @@ __device__ __forceinline__ void locate(Cell<Real> &c, const Real *grid, int n, R
     }
 }
 
+// The value at a bracket; off the table's ends the bracket is the end cell, whose
+// outer value is held.
 template <class Real, class T>
-__device__ __forceinline__ Real gather(const T *f, int n, int idx, Real frac, bool below, bool above) {
-    const Real f0 = (Real)f[idx - 1];
-    Real y = f0 + frac * ((Real)f[idx] - f0);
-    if (below) y = (Real)f[0];
-    if (above) y = (Real)f[n - 1];
-    return y;
+__device__ __forceinline__ Real gather(const T *f, int idx, Real frac, bool below, bool above) {
+    const Real f0 = (Real)f[idx - 1], f1 = (Real)f[idx];
+    const Real y = f0 + frac * (f1 - f0);
+    return below ? f0 : above ? f1 : y;
 }
 
 // cxr/_recoil.py:35-76
@@ -365,10 +374,12 @@ __device__ __forceinline__ bool pair_may_keep(const SegPre<Real> &sp, const RowP
     if (dtail == nullptr) return true;
     const Real E_low = (Real)kHbarcEvAng * rdiv(num, denom_vac) * (Real)(1.0 / 1.5);
     if (E_low < (Real)t.hi_keep) return true;
-    int ix;
-    Real fr;
-    bool bl, ab;
-    bracket<Real>(E_tab, n_tab, E_low, ix, fr, bl, ab, ti);
+    int ix = n_tab - 1;  // the tabulation usually ends at the window: the last cell
+    if (!(E_low >= E_tab[n_tab - 1])) {
+        Real fr;
+        bool bl, ab;
+        bracket<Real>(E_tab, n_tab, E_low, ix, fr, bl, ab, ti);
+    }
     return !(dtail[ix - 1] * r_sqrt(sp.grad2) <= (Real)0.5 * denom_vac);
 }
 
@@ -419,7 +430,7 @@ __device__ __forceinline__ Resonance<Real> pair_resonance(const SegPre<Real> &sp
     for (int pass = 0; pass < 3; ++pass) {
         const Real Er = hbarc * rdiv(v_dot_g_exact, denom);
         locate<Real>(cell, E_tab, n_tab, Er, ti);
-        delta = gather<Real>(delta_tab, n_tab, cell.idx, cell.frac, cell.below, cell.above);
+        delta = gather<Real>(delta_tab, cell.idx, cell.frac, cell.below, cell.above);
         previous = denom;
         denom = denom_vac - delta * sp.v_dot_grad;
     }
@@ -490,18 +501,15 @@ __device__ __forceinline__ PairAmps<Real> pair_amps_from(const SegPre<Real> &sp,
     }
     // cxr/_kernels.py:482-506 couplings, 369-388 attenuation
     const int64_t base = (int64_t)rw.row * n_tab;
-    const Real chi_re = gather<Real>(t.chi_re + base, n_tab, ix, fr, bl, ab);
-    const Real chi_im = gather<Real>(t.chi_im + base, n_tab, ix, fr, bl, ab);
-    const Real u_re = gather<Real>(t.u_re + base, n_tab, ix, fr, bl, ab);
-    const Real u_im = gather<Real>(t.u_im + base, n_tab, ix, fr, bl, ab);
+    const Real chi_re = gather<Real>(t.chi_re + base, ix, fr, bl, ab);
+    const Real chi_im = gather<Real>(t.chi_im + base, ix, fr, bl, ab);
+    const Real u_re = gather<Real>(t.u_re + base, ix, fr, bl, ab);
+    const Real u_im = gather<Real>(t.u_im + base, ix, fr, bl, ab);
     Real mu = 0;
     for (int el = 0; el < (kLayered ? 0 : n_mu); ++el) {
         const Real *lm = log_mu + (int64_t)el * n_tab;
-        const Real f0 = lm[ix - 1];
-        Real v = r_exp(f0 + lfr * (lm[ix] - f0));
-        if (bl) v = r_exp(lm[0]);
-        if (ab) v = r_exp(lm[n_tab - 1]);
-        mu += v;
+        const Real f0 = lm[ix - 1], f1 = lm[ix];
+        mu += r_exp(bl ? f0 : ab ? f1 : f0 + lfr * (f1 - f0));
     }
     o.mu = mu;
     // cxr/_batched.py:789-826, cxr/_line_amplitude.py:14-37
@@ -969,9 +977,6 @@ struct alignas(16) WinLine {
     int pad;
 };
 
-__device__ __forceinline__ void smem_add(float *p, float v) {
-    asm volatile("red.shared.add.f32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "f"(v) : "memory");
-}
 __device__ __forceinline__ void smem_add(double *p, double v) {
     asm volatile("red.shared.add.f64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "d"(v) : "memory");
 }
@@ -1008,7 +1013,7 @@ __device__ __forceinline__ void line_moments(double E_r, double inv_a, double w,
 // B is bound by FP32/FP64 issue and the SFU (one reciprocal, one sine, one
 // cosine per edge).
 template <class Real, bool kLayered>
-__global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a, int K_far, int far_pad) {
+__global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_cxr_args a, int K_far, int far_pad) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr bool kMixed = sizeof(Real) == 4;
     const int n_g = a.tables.n_g;
@@ -1036,7 +1041,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     cur = (unsigned char *)(((uintptr_t)(qW + kLineQueue) + 15) & ~(uintptr_t)15);
     WinLine<Real> *wLine = reinterpret_cast<WinLine<Real> *>(cur);  // window list
     uint16_t *wIdx = reinterpret_cast<uint16_t *>(wLine + kWideCap);  // its lines by class
-    int *scratch = reinterpret_cast<int *>(wIdx + kWinClasses * kWideCap);  // counters
+    int *scratch = reinterpret_cast<int *>(wIdx + kWinClasses / 2 * kWideCap);  // counters
     uint16_t *pq = reinterpret_cast<uint16_t *>(scratch + 64);  // surviving pair ids
     cur = reinterpret_cast<unsigned char *>(pq + kQueue);
     cur = (unsigned char *)(((uintptr_t)cur + 15) & ~(uintptr_t)15);
@@ -1050,8 +1055,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     cur = (unsigned char *)(((uintptr_t)cur + 15) & ~(uintptr_t)15);
     double *spec_s = reinterpret_cast<double *>(cur);
     const int n_mom = n_E + 2 * far_pad;
-    float *spec_f = reinterpret_cast<float *>(spec_s + (binmean ? n_E : 0));  // mixed path: float partials
-    float *edges_f = spec_f + (binmean && kMixed ? n_E : 0);                    // and float bin edges
+    float *edges_f = reinterpret_cast<float *>(spec_s + (binmean ? n_E : 0));  // mixed path: float bin edges
     // Layered absorber: per-segment escape pieces, layer thicknesses and bounds.
     unsigned char *esc_raw = reinterpret_cast<unsigned char *>(edges_f + (binmean && kMixed ? n_E + 1 : 0));
     esc_raw = (unsigned char *)(((uintptr_t)esc_raw + 15) & ~(uintptr_t)15);
@@ -1080,10 +1084,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     if (binmean) {
         for (int j = tid; j < n_E; j += blockDim.x) spec_s[j] = 0.0;
         if (kMixed)
-            for (int j = tid; j <= n_E; j += blockDim.x) {
-                if (j < n_E) spec_f[j] = 0.0f;
-                edges_f[j] = (float)a.edges[j];
-            }
+            for (int j = tid; j <= n_E; j += blockDim.x) edges_f[j] = (float)a.edges[j];
     }
     if (tid == 0) { q_count = 0; p_count = 0; w_count = 0; strip_next = 0; }
     if (tid < kWinClasses) w_class[tid] = 0;
@@ -1146,13 +1147,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
         if constexpr (kMixed) return edges_f[j];
         else return ax.edges[j];
     };
-    // B adds into float partials on the mixed path, else into the spectrum.
-    auto *const spec_part = [&] {
-        if constexpr (kMixed) return spec_f;
-        else return spec_s;
-    }();
     int d_cur = -1;
-    int rounds = 0;  // rounds since the float partials were last folded
 
     // B1: the line in queue slot j, if any, by this thread.
     auto near_round = [&](int j, int d) {
@@ -1197,7 +1192,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
                     Real mass = f_hi - f_lo + ((x_lo < (Real)0 && x_hi >= (Real)0) ? (Real)kPi : (Real)0);
                     const Real xc = (Real)0.5 * (x_lo + x_hi);
                     if (sx <= s_narrow && fabs(xc) >= (Real)2) mass = (Real)kPi * sw * midpoint_mean(xc, sw);
-                    if (bin >= 0 && bin < n_E) smem_add(&spec_part[bin], out * mass);
+                    if (bin >= 0 && bin < n_E) smem_add(&spec_s[bin], (double)(out * mass));
                     x_lo = x_hi;
                     f_lo = f_hi;
                 }
@@ -1212,7 +1207,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
         if (cls < kWinClasses) {
             const int k = base + __popc(mask & ((1u << lane) - 1u));
             wLine[k] = wl;
-            wIdx[cls * kWideCap + atomicAdd(&w_class[cls], 1)] = (uint16_t)k;
+            wIdx[win_slot(cls, atomicAdd(&w_class[cls], 1))] = (uint16_t)k;
         }
     };
 
@@ -1237,8 +1232,8 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
         const Real f2 = __shfl_down_sync(0xffffffffu, f0, 1);
         const Real out = sgn * l.scale * inv_w_r;
         const int next = left ? bin - 1 : bin + 1;
-        if (live && Dh <= l.D1 && bin >= 0 && bin < n_E) smem_add(&spec_part[bin], out * (f1 - f0));
-        if (live && h < G / 2 - 1 && Dh < l.D1 && next >= 0 && next < n_E) smem_add(&spec_part[next], out * (f2 - f1));
+        if (live && Dh <= l.D1 && bin >= 0 && bin < n_E) smem_add(&spec_s[bin], (double)(out * (f1 - f0)));
+        if (live && h < G / 2 - 1 && Dh < l.D1 && next >= 0 && next < n_E) smem_add(&spec_s[next], (double)(out * (f2 - f1)));
     };
 
     auto window_phase = [&]() {
@@ -1246,12 +1241,12 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
             const int G = 4 << cls, per = 32 / G, n = w_class[cls];
             for (int i = warp * per; i < n; i += n_warps * per) {
                 const int k = i + (int)lane / G;
-                const WinLine<Real> &l = wLine[wIdx[cls * kWideCap + min(k, n - 1)]];
+                const WinLine<Real> &l = wLine[wIdx[win_slot(cls, min(k, n - 1))]];
                 visit(l, l.D0, G, k < n);
             }
         }
         for (int i = warp; i < w_class[kWin32]; i += n_warps) {
-            const WinLine<Real> &l = wLine[wIdx[kWin32 * kWideCap + i]];
+            const WinLine<Real> &l = wLine[wIdx[win_slot(kWin32, i)]];
             for (int D = l.D0; D <= l.D1; D += 31) visit(l, D, 32, true);
         }
     };
@@ -1265,23 +1260,31 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
             const int bin = first + (int)lane;
             const Real e = edge_at(bin);
             Real acc = 0;
-            for (int k = 0; k < nw; ++k) {
-                const WinLine<Real> &l = wLine[wIdx[kWinStrip * kWideCap + k]];
-                if (first > l.c + l.D1 || last < l.c - l.D1) continue;
-                const Real sw = l.s * w_r, D = (Real)(bin - l.c), Dm = D - (Real)0.5;
-                const bool on = fabs(D) >= (Real)l.D0 && fabs(D) <= (Real)l.D1;
-                const Real x = l.s * (e - l.E_r);
-                Real mass;
-                if (l.s > s_narrow) {
-                    const Real f = edge_window_bins<Real>(x, Dm, l.d, sw);
-                    mass = __shfl_down_sync(0xffffffffu, f, 1) - f;
-                } else {
-                    const Real f = fabs(x) < (Real)2.2 ? edge_window_near<Real>(x, Dm, l.d, sw) : (Real)0;
-                    mass = __shfl_down_sync(0xffffffffu, f, 1) - f;
-                    const Real xc = fma((Real)0.5, sw, x);
-                    if (fabs(xc) >= (Real)2) mass = window_midpoint<Real>(xc, Dm, l.d, sw);
+            for (int k0 = 0; k0 < nw; k0 += 32) {
+                int idx = 0;
+                bool hit = false;
+                if (k0 + (int)lane < nw) {
+                    idx = wIdx[win_slot(kWinStrip, k0 + (int)lane)];
+                    const int c = wLine[idx].c, D1 = wLine[idx].D1;
+                    hit = first <= c + D1 && last >= c - D1;
                 }
-                if (on) acc = fma(l.scale, mass, acc);
+                for (unsigned todo = __ballot_sync(0xffffffffu, hit); todo; todo &= todo - 1) {
+                    const WinLine<Real> &l = wLine[__shfl_sync(0xffffffffu, idx, __ffs(todo) - 1)];
+                    const Real sw = l.s * w_r, D = (Real)(bin - l.c), Dm = D - (Real)0.5;
+                    const bool on = fabs(D) >= (Real)l.D0 && fabs(D) <= (Real)l.D1;
+                    const Real x = l.s * (e - l.E_r);
+                    Real mass;
+                    if (l.s > s_narrow) {
+                        const Real f = edge_window_bins<Real>(x, Dm, l.d, sw);
+                        mass = __shfl_down_sync(0xffffffffu, f, 1) - f;
+                    } else {
+                        const Real f = fabs(x) < (Real)2.2 ? edge_window_near<Real>(x, Dm, l.d, sw) : (Real)0;
+                        mass = __shfl_down_sync(0xffffffffu, f, 1) - f;
+                        const Real xc = fma((Real)0.5, sw, x);
+                        if (fabs(xc) >= (Real)2) mass = window_midpoint<Real>(xc, Dm, l.d, sw);
+                    }
+                    if (on) acc = fma(l.scale, mass, acc);
+                }
             }
             if (lane < kStripBins && bin < n_E) spec_s[bin] += (double)acc * ax.inv_w;
         }
@@ -1302,7 +1305,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
             const Real e = (Real)e_lo;
             Real acc = 0;
             for (int k = 0; k < nw; ++k) {
-                const WinLine<Real> &l = wLine[wIdx[kWinAxis * kWideCap + k]];
+                const WinLine<Real> &l = wLine[wIdx[win_slot(kWinAxis, k)]];
                 const Real x = l.s * (e - l.E_r);
                 const Real x_hi = __shfl_down_sync(0xffffffffu, x, 1);
                 const Real sw = x_hi - x, xc = (Real)0.5 * (x + x_hi);
@@ -1341,7 +1344,7 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
                 window_phase();
                 const int n_strip = w_class[kWinStrip], n_axis = w_class[kWinAxis];
                 const bool strips = n_strip > kStripRun || (leave && n_strip > 0);
-                // FP64: the window's adds and the strips' sums share spec_s
+                // the window's adds and the strips' sums share spec_s
                 __syncthreads();
                 if (strips) strip_phase();
                 if (n_axis > 0) {
@@ -1351,26 +1354,14 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
                 // strip lines that wait move to the front of the list
                 WinLine<Real> wl;
                 const bool keep = !strips && tid < n_strip;
-                if (keep) wl = wLine[wIdx[kWinStrip * kWideCap + tid]];
+                if (keep) wl = wLine[wIdx[win_slot(kWinStrip, tid)]];
                 __syncthreads();
                 if (keep) {
                     wLine[tid] = wl;
-                    wIdx[kWinStrip * kWideCap + tid] = (uint16_t)tid;
+                    wIdx[win_slot(kWinStrip, tid)] = (uint16_t)tid;
                 }
                 if (tid < kWinClasses) w_class[tid] = tid == kWinStrip && !strips ? n_strip : 0;
                 if (tid == 0) { w_count = strips ? 0 : n_strip; strip_next = 0; }
-            }
-            if constexpr (kMixed) {
-                // Fold the float partials into the FP64 spectrum every four
-                // rounds: about a thousand lines' adds keep float well inside
-                // the path's tolerance.
-                if (K_far > 0 && ++rounds == 4) {
-                    for (int j = tid; j < n_E; j += blockDim.x) {
-                        const float v = spec_f[j];
-                        if (v != 0.0f) { spec_s[j] += (double)v; spec_f[j] = 0.0f; }
-                    }
-                    rounds = 0;
-                }
             }
             more = flush ? nq > 0 : nq >= kCxrThreads;
             __syncthreads();
@@ -1381,10 +1372,6 @@ __global__ void __launch_bounds__(kCxrThreads, 2) cxr_kernel(const pb_cxr_args a
     auto publish = [&](int d) {
         // Publish (and clear) the block's spectrum of direction d.
         __syncthreads();
-        if constexpr (kMixed) {
-            for (int j = tid; j < n_E; j += blockDim.x) { spec_s[j] += (double)spec_f[j]; spec_f[j] = 0.0f; }
-        }
-        rounds = 0;
         double *gspec = a.spec + (int64_t)d * n_E;
         for (int j = tid; j < n_E; j += blockDim.x) {
             if (spec_s[j] != 0.0) atomicAdd(&gspec[j], spec_s[j]);
@@ -1757,12 +1744,12 @@ static size_t cxr_smem_bytes(const pb_cxr_args &a, int far_pad, bool with_moment
     constexpr int kQueue = pair_queue<Real>();
     size_t b = sizeof(RowPre<Real>) * kRowChunk + sizeof(SegPre<Real>) * kSegTile + 16;
     b += sizeof(Real) * 3 * line_queue<Real>() + 16 +
-         (sizeof(WinLine<Real>) + sizeof(uint16_t) * kWinClasses) * kWideCap + sizeof(int) * 64 +
+         (sizeof(WinLine<Real>) + sizeof(uint16_t) * (kWinClasses / 2)) * kWideCap + sizeof(int) * 64 +
          sizeof(uint16_t) * kQueue + 16;
     if (a.tables.n_tab <= kMaxTab) b += sizeof(Real) * (size_t)a.tables.n_tab * (3 + a.tables.n_mu);
     b += 16;
     if (a.quadrature == PB_QUAD_BINMEAN)
-        b += sizeof(double) * (size_t)a.n_E + (sizeof(Real) == 4 ? sizeof(float) * (2 * (size_t)a.n_E + 1) : 0);
+        b += sizeof(double) * (size_t)a.n_E + (sizeof(Real) == 4 ? sizeof(float) * ((size_t)a.n_E + 1) : 0);
     if (a.n_layer > 0)
         b += 16 + sizeof(EscSeg<Real>) * kSegTile + sizeof(double) * 2 * kMaxEscLayers + sizeof(Real) * kMaxEscLayers;
     return b;

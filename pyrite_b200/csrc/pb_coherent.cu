@@ -6,7 +6,7 @@
 // chunk (cxr/_batched_finalize.py:209-243); its CUDA form gives one block per
 // energy and strides the lines over threads (coherent_jit_kernel.py:118-240).
 // Here the work is a line-chunk x energy-tile grid: a CTA stages up to
-// kStage line records into shared memory (96 bytes each, read back as
+// kStage line records into shared memory (144 bytes each, read back as
 // broadcasts), every thread owns kEPT energies and sums the four field
 // components of both polarisations in registers, and writes them once per
 // work item (row, chunk of lines). A second kernel adds a row's chunks in
@@ -37,24 +37,53 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kEPT = 4;                        // energies per thread
+constexpr int kPairs = kEPT / 2;               // as packed pairs
 constexpr int kETile = kThreads * kEPT;        // energies per CTA
 constexpr int kStage = 128;                    // lines per shared-memory stage
 constexpr int64_t kMinChunk = 256;             // lines per work item, lower bound
 constexpr int64_t kTargetItemsTimesTiles = 148 * 3 * 4;  // ~4 waves of 3 CTAs per SM
 constexpr float kSeriesW2 = 1.0e-6f;           // _formation.py:55 FORMATION_SERIES_W2
 
+// Two floats in one register pair, and the packed FP32 arithmetic of sm_100 (one
+// instruction for both halves).
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void f2_get(F2 x, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x.v));
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return d;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+    return d;
+}
+
 // One line record as the field loop reads it, phases in turns. ``fast``
 // lines hold the offset forms Gx = 1.5 * 2^29 - g_phase / 2 pi and
 // Vx = 1.5 * 2^29 - a_vac E_vac / 2 pi; the others hold g_phase / 2 pi and
-// E_vac.
+// E_vac. The float operands of the fast lines are there in both halves of a pair
+// (the others read one half).
 struct alignas(16) CohLine {
     double ps_t, L_t, a_t, h_t;  // phase_slope, L_esc, a_vac, half_dL over 2 pi
     double Gx, Vx;
-    float apb, bma, q, qapb, qbma, csr, csi, cpr, cpi;
+    F2 q2, apb, bma, qapb, qbma;  // q^2, and half of apb, bma, q apb, q bma
+    F2 csr, csi, cpr, cpi;
+    float q;
     int fast;
-    float pad[2];
+    float elec;  // grouped: an electron starts here
+    float pad;
 };
-static_assert(sizeof(CohLine) == 96, "CohLine packs into six 16-byte words");
+static_assert(sizeof(CohLine) == 144, "CohLine packs into nine 16-byte words");
 
 constexpr double kInv2Pi = 0.15915494309189535;
 constexpr double kRound64 = 6755399441055744.0;  // 1.5 * 2^52: x + c - c rounds |x| < 2^51 to an integer
@@ -62,14 +91,11 @@ constexpr float kTwoPiF = 6.2831853071795865f;
 constexpr double kTurnBase = 805306368.0;        // 1.5 * 2^29
 constexpr double kFastLimit = 134217728.0;       // 2^27 turns: offset sums stay in [2^29, 2^30)
 
-// (sin, cos) of 2 pi f, f the fraction of x - kTurnBase, for x in [2^29, 2^30).
-__device__ __forceinline__ void sincos_turns_offset(double x, float &s, float &c) {
+// -(sin, cos) of 2 pi f, f the fraction of x - kTurnBase, for x in [2^29, 2^30):
+// sin(2 pi f) = -sin(2 pi (f - 1/2)), f - 1/2 in [-1/2, 1/2) exactly.
+__device__ __forceinline__ void neg_sincos_turns_offset(double x, float &s, float &c) {
     const unsigned lo = (unsigned)__double2loint(x);
-    const float g = __uint_as_float((lo & 0x7FFFFFu) | 0x3F800000u) - 1.5f;  // f - 1/2 in [-1/2, 1/2)
-    float sg, cg;
-    __sincosf(g * kTwoPiF, &sg, &cg);
-    s = -sg;  // sin(2 pi f) = -sin(2 pi (f - 1/2))
-    c = -cg;
+    __sincosf((__uint_as_float((lo & 0x7FFFFFu) | 0x3F800000u) - 1.5f) * kTwoPiF, &s, &c);
 }
 
 // (sin, cos) of 2 pi t for any FP64 t with |t| < 2^51.
@@ -153,40 +179,48 @@ __device__ __forceinline__ void sincos_taylor(float v, float &sv, float &cv) {
     cv = fmaf(z, pc, 1.f);
 }
 
-// acc += (c_sigma, c_pi) F(v) exp(i phi): the formation factor of the
-// absorbed piece (_formation.py:84-110, series below |w|^2 < 1e-6) rotated by
-// the propagation phase (_batched_finalize.py:213-218).
-__device__ __forceinline__ void add_line_field(const CohLine &l, float vf, float sv, float cv, float sp, float cp,
-                                               float acc[4]) {
-    const float w2 = fmaf(l.q, l.q, vf * vf);
-    float fr, fi;
-    if (w2 < kSeriesW2) {
-        const float half = 0.5f * l.apb;
-        fr = half * (1.f - l.q * l.q * (1.f / 3.f) - vf * vf * (1.f / 6.f));
-        fi = -half * l.q * vf * (1.f / 3.f);
-    } else {
-        const float inv = __fdividef(0.5f, w2);
-        fr = fmaf(vf * l.apb, sv, -l.qbma * cv) * inv;
-        fi = -fmaf(vf * l.bma, cv, l.qapb * sv) * inv;
+// The term (c_sigma, c_pi) F(v) exp(i phi) of one line at two energies, added to
+// acc: the formation factor of the absorbed piece (_formation.py:84-110, series
+// below |w|^2 < 1e-6) rotated by the propagation phase
+// (_batched_finalize.py:213-218). Fast lines come with the signs of both sine and
+// cosine pairs turned, which cancels in the product. nf = -Im F, npi = -Im (F exp(i phi)).
+__device__ __forceinline__ void line_term(const CohLine &l, F2 v, F2 sv, F2 cv, F2 sp, F2 cp, F2 acc[4]) {
+    const F2 minus = f2(-1.f, -1.f);
+    const F2 w2 = f2_fma(v, v, l.q2);
+    float w0, w1;
+    f2_get(w2, w0, w1);
+    const F2 inv = f2(__fdividef(1.f, w0), __fdividef(1.f, w1));
+    F2 fr = f2_mul(f2_fma(f2_mul(v, l.apb), sv, f2_mul(f2_mul(l.qbma, cv), minus)), inv);
+    F2 nf = f2_mul(f2_fma(f2_mul(v, l.bma), cv, f2_mul(l.qapb, sv)), inv);
+    if (fminf(w0, w1) < kSeriesW2) {
+        float vh[2], a[2], r[2], i[2];
+        f2_get(v, vh[0], vh[1]);
+        f2_get(l.apb, a[0], a[1]);
+        f2_get(fr, r[0], r[1]);
+        f2_get(nf, i[0], i[1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if ((k ? w1 : w0) < kSeriesW2) {  // a = apb / 2, with the sign of the line's sin v, cos v
+                if (l.fast) a[k] = -a[k];
+                r[k] = a[k] * (1.f - l.q * l.q * (1.f / 3.f) - vh[k] * vh[k] * (1.f / 6.f));
+                i[k] = a[k] * l.q * vh[k] * (1.f / 3.f);
+            }
+        }
+        fr = f2(r[0], r[1]);
+        nf = f2(i[0], i[1]);
     }
-    const float pr = fmaf(fr, cp, -fi * sp);
-    const float pi = fmaf(fr, sp, fi * cp);
-    acc[0] = fmaf(l.csr, pr, fmaf(-l.csi, pi, acc[0]));
-    acc[1] = fmaf(l.csr, pi, fmaf(l.csi, pr, acc[1]));
-    acc[2] = fmaf(l.cpr, pr, fmaf(-l.cpi, pi, acc[2]));
-    acc[3] = fmaf(l.cpr, pi, fmaf(l.cpi, pr, acc[3]));
+    const F2 pr = f2_fma(nf, sp, f2_mul(fr, cp));
+    const F2 npi = f2_fma(nf, cp, f2_mul(f2_mul(fr, minus), sp));
+    const F2 pi = f2_mul(npi, minus);
+    acc[0] = f2_fma(l.csr, pr, f2_fma(l.csi, npi, acc[0]));
+    acc[1] = f2_fma(l.csr, pi, f2_fma(l.csi, pr, acc[1]));
+    acc[2] = f2_fma(l.cpr, pr, f2_fma(l.cpi, npi, acc[2]));
+    acc[3] = f2_fma(l.cpr, pi, f2_fma(l.cpi, pr, acc[3]));
 }
 
-// The same term added to the row's field and to the current electron's.
-__device__ __forceinline__ void add_line_field2(const CohLine &l, float vf, float sv, float cv, float sp, float cp,
-                                                float acc[4], float acc_e[4]) {
-    float t[4] = {0.f, 0.f, 0.f, 0.f};
-    add_line_field(l, vf, sv, cv, sp, cp, t);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        acc[c] += t[c];
-        acc_e[c] += t[c];
-    }
+// |field|^2 of both polarisations at two energies.
+__device__ __forceinline__ F2 field_square(const F2 f[4]) {
+    return f2_fma(f[0], f[0], f2_fma(f[1], f[1], f2_fma(f[2], f[2], f2_mul(f[3], f[3]))));
 }
 
 struct CohArgs {
@@ -242,13 +276,14 @@ __global__ void __launch_bounds__(kThreads, kGrouped ? 2 : 3) coh_field_kernel(c
         E[m] = e < a.n_E ? a.E[e] : 0.0;
         D[m] = e < a.n_E ? a.dom[e] : 0.0;
     }
-    float acc[kEPT][4];
-#pragma unroll
-    for (int m = 0; m < kEPT; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
+    const F2 zero = f2(0.f, 0.f);
+    F2 acc[kPairs][4];
     // kGrouped: the current electron's field and the item's sum of squares
-    float acc_e[kGrouped ? kEPT : 1][4], pw[kGrouped ? kEPT : 1];
+    F2 acc_e[kGrouped ? kPairs : 1][4], pw[kGrouped ? kPairs : 1];
 #pragma unroll
-    for (int m = 0; m < (kGrouped ? kEPT : 1); ++m) acc_e[m][0] = acc_e[m][1] = acc_e[m][2] = acc_e[m][3] = pw[m] = 0.f;
+    for (int m = 0; m < kPairs; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = zero;
+#pragma unroll
+    for (int m = 0; m < (kGrouped ? kPairs : 1); ++m) acc_e[m][0] = acc_e[m][1] = acc_e[m][2] = acc_e[m][3] = pw[m] = zero;
 
     // largest |E| and |delta_omega| of this CTA's energies (for the fast-path check)
     __shared__ double red[2][kThreads / 32];
@@ -291,20 +326,23 @@ __global__ void __launch_bounds__(kThreads, kGrouped ? 2 : 3) coh_field_kernel(c
             l.fast = phase_span < kFastLimit && v_span < kFastLimit;  // false for NaN too
             l.Gx = l.fast ? kTurnBase - gt : gt;
             l.Vx = l.fast ? kTurnBase - l.a_t * Ev : Ev;
-            l.apb = (float)a.apb[j];
-            l.bma = (float)a.bma[j];
+            const auto both = [](float x) { return f2(x, x); };
+            const float apb = (float)a.apb[j], bma = (float)a.bma[j];
             l.q = (float)a.q[j];
-            l.qapb = l.q * l.apb;
-            l.qbma = l.q * l.bma;
-            l.csr = (float)a.csr[j];
-            l.csi = (float)a.csi[j];
-            l.cpr = (float)a.cpr[j];
-            l.cpi = (float)a.cpi[j];
-            l.pad[0] = l.pad[1] = 0.f;
+            l.q2 = both(l.q * l.q);
+            l.apb = both(0.5f * apb);
+            l.bma = both(0.5f * bma);
+            l.qapb = both(0.5f * (l.q * apb));
+            l.qbma = both(0.5f * (l.q * bma));
+            l.csr = both((float)a.csr[j]);
+            l.csi = both((float)a.csi[j]);
+            l.cpr = both((float)a.cpr[j]);
+            l.cpi = both((float)a.cpi[j]);
+            l.elec = l.pad = 0.f;
             if constexpr (kGrouped) {
                 if (j > j0) {
                     const int64_t ep = a.elec[j - 1], ej = a.elec[j];
-                    l.pad[0] = ej != ep ? 1.f : 0.f;  // an electron starts here
+                    l.elec = ej != ep ? 1.f : 0.f;  // an electron starts here
                     if (ej < ep && a.status) atomicOr(a.status, PB_DEV_BAD_INPUT);
                 }
             }
@@ -312,55 +350,80 @@ __global__ void __launch_bounds__(kThreads, kGrouped ? 2 : 3) coh_field_kernel(c
         }
         __syncthreads();
         for (int i = 0; i < n; ++i) {
-            const CohLine l = sm[i];
+            const CohLine &l = sm[i];
             if constexpr (kGrouped) {
-                if (l.pad[0] != 0.f) {  // uniform: close the previous electron
+                if (l.elec != 0.f) {  // uniform: close the previous electron
 #pragma unroll
-                    for (int m = 0; m < kEPT; ++m) {
-                        pw[m] += acc_e[m][0] * acc_e[m][0] + acc_e[m][1] * acc_e[m][1] +
-                                 acc_e[m][2] * acc_e[m][2] + acc_e[m][3] * acc_e[m][3];
-                        acc_e[m][0] = acc_e[m][1] = acc_e[m][2] = acc_e[m][3] = 0.f;
+                    for (int m = 0; m < kPairs; ++m) {
+                        pw[m] = f2_fma(f2(1.f, 1.f), field_square(acc_e[m]), pw[m]);
+                        acc_e[m][0] = acc_e[m][1] = acc_e[m][2] = acc_e[m][3] = zero;
                     }
                 }
             }
-            if (l.fast) {  // uniform over the block: one line at a time
+            const bool fast = l.fast;  // uniform over the block: one line at a time
 #pragma unroll
-                for (int m = 0; m < kEPT; ++m) {
-                    const double vx = fma(l.a_t, E[m], fma(-l.h_t, D[m], l.Vx));
-                    const float vf = (float)(vx - kTurnBase) * kTwoPiF;
-                    if (a.cutoff > 0.f && fabsf(vf) > a.cutoff) continue;
-                    float sv, cv, sp, cp;
-                    if (fabsf(vf) <= 1.f) sincos_taylor(vf, sv, cv);
-                    else sincos_turns_offset(vx, sv, cv);
-                    sincos_turns_offset(fma(l.ps_t, E[m], fma(-l.L_t, D[m], l.Gx)), sp, cp);
-                    if constexpr (kGrouped) add_line_field2(l, vf, sv, cv, sp, cp, acc[m], acc_e[m]);
-                    else add_line_field(l, vf, sv, cv, sp, cp, acc[m]);
+            for (int m = 0; m < kPairs; ++m) {
+                float vf[2], sv[2], cv[2], sp[2], cp[2];
+                bool cut[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const double Ek = E[2 * m + k], Dk = D[2 * m + k];
+                    double vt, pt;
+                    if (fast) {
+                        vt = fma(l.a_t, Ek, fma(-l.h_t, Dk, l.Vx));
+                        vf[k] = (float)(vt - kTurnBase) * kTwoPiF;
+                        neg_sincos_turns_offset(vt, sv[k], cv[k]);
+                        pt = fma(l.ps_t, Ek, fma(-l.L_t, Dk, l.Gx));
+                        neg_sincos_turns_offset(pt, sp[k], cp[k]);
+                    } else {
+                        vt = fma(l.a_t, Ek - l.Vx, -l.h_t * Dk);
+                        vf[k] = (float)vt * kTwoPiF;
+                        sincos_turns(vt, sv[k], cv[k]);
+                        pt = fma(l.ps_t, Ek, -fma(l.L_t, Dk, l.Gx));
+                        sincos_turns(pt, sp[k], cp[k]);
+                    }
+                    cut[k] = a.cutoff > 0.f && fabsf(vf[k]) > a.cutoff;
+                    if (fabsf(vf[k]) <= 1.f) {
+                        sincos_taylor(vf[k], sv[k], cv[k]);
+                        if (fast) {  // the sign of the two fast pairs cancels in the product
+                            sv[k] = -sv[k];
+                            cv[k] = -cv[k];
+                        }
+                    }
+                    if (cut[k]) sp[k] = cp[k] = 0.f;  // outside the window: no term
                 }
-            } else {
+                const F2 v2 = f2(vf[0], vf[1]), s2 = f2(sv[0], sv[1]), c2 = f2(cv[0], cv[1]);
+                const F2 sp2 = f2(sp[0], sp[1]), cp2 = f2(cp[0], cp[1]);
+                if constexpr (kGrouped) {
+                    F2 t[4] = {zero, zero, zero, zero};
+                    line_term(l, v2, s2, c2, sp2, cp2, t);
+                    const F2 one = f2(1.f, 1.f);
 #pragma unroll
-                for (int m = 0; m < kEPT; ++m) {
-                    const double vt = fma(l.a_t, E[m] - l.Vx, -l.h_t * D[m]);
-                    const float vf = (float)vt * kTwoPiF;
-                    if (a.cutoff > 0.f && fabsf(vf) > a.cutoff) continue;
-                    float sv, cv, sp, cp;
-                    if (fabsf(vf) <= 1.f) sincos_taylor(vf, sv, cv);
-                    else sincos_turns(vt, sv, cv);
-                    sincos_turns(fma(l.ps_t, E[m], -fma(l.L_t, D[m], l.Gx)), sp, cp);
-                    if constexpr (kGrouped) add_line_field2(l, vf, sv, cv, sp, cp, acc[m], acc_e[m]);
-                    else add_line_field(l, vf, sv, cv, sp, cp, acc[m]);
+                    for (int c = 0; c < 4; ++c) {
+                        acc[m][c] = f2_fma(one, t[c], acc[m][c]);
+                        acc_e[m][c] = f2_fma(one, t[c], acc_e[m][c]);
+                    }
+                } else {
+                    line_term(l, v2, s2, c2, sp2, cp2, acc[m]);
                 }
             }
         }
     }
 #pragma unroll
-    for (int m = 0; m < kEPT; ++m) {
-        const int e = e_base + m * kThreads;
-        if (e < a.n_E) {
+    for (int m = 0; m < kPairs; ++m) {
+        float out[5][2];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) a.partial[((size_t)item * 4 + c) * a.n_E + e] = acc[m][c];
-            if constexpr (kGrouped)
-                a.power[(size_t)item * a.n_E + e] = pw[m] + acc_e[m][0] * acc_e[m][0] + acc_e[m][1] * acc_e[m][1] +
-                                                    acc_e[m][2] * acc_e[m][2] + acc_e[m][3] * acc_e[m][3];
+        for (int c = 0; c < 4; ++c) f2_get(acc[m][c], out[c][0], out[c][1]);
+        if constexpr (kGrouped)
+            f2_get(f2_fma(f2(1.f, 1.f), field_square(acc_e[m]), pw[m]), out[4][0], out[4][1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int e = e_base + (2 * m + k) * kThreads;
+            if (e < a.n_E) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) a.partial[((size_t)item * 4 + c) * a.n_E + e] = out[c][k];
+                if constexpr (kGrouped) a.power[(size_t)item * a.n_E + e] = out[4][k];
+            }
         }
     }
 }

@@ -765,7 +765,7 @@ __device__ __forceinline__ float q_osc(float x, float iu) {
 // Bin-mean deposit of a line: exact bin integrals within the line's window
 // (``exact_widths`` first-zero widths, at least K_far bins); beyond it the far
 // envelope w/(2 a^2) / ((E_lo - E_r)(E_hi - E_r)) is carried by three moments
-// about the centre bin and spread by far_field_kernel onto every bin more
+// about the centre bin and spread by far_field_conv_kernel onto every bin more
 // than K_far bins away. A line whose window is wider than K_far removes the
 // envelope again from its extra exact bins, so each bin takes exactly one of
 // the two forms. Lines centred off a non-uniform axis, or too wide for a
@@ -1549,102 +1549,100 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
     }
 }
 
-// Far-field finalize: spec[d][b] += sum_c M[d][c] . envelope(b, c) over the
-// (padded, uniform) centre bins c farther than K_far bins from b.
-__global__ void far_field_kernel(const double *edges, int n_E, int pad, const double *mom,
-                                 double *spec, int K_far) {
-    const int d = blockIdx.y;
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= n_E) return;
-    const int n_mom = n_E + 2 * pad;
-    const double *m = mom + (int64_t)d * n_mom * 3;
-    const double lo = edges[0];
-    const double w = (edges[n_E] - edges[0]) / n_E;
-    const double E_lo = edges[b], E_hi = edges[b + 1];
-    double acc = 0.0;
-    for (int slot = 0; slot < n_mom; ++slot) {
-        const int c = slot - pad;
-        if (c >= b - K_far && c <= b + K_far) continue;
-        const double m0 = m[3 * slot];
-        if (m0 == 0.0) continue;
-        const double E_c = lo + ((double)c + 0.5) * w;
-        const double A = E_lo - E_c, B = E_hi - E_c;
-        const double AB = A * B;
-        const double f0 = 1.0 / AB;
-        const double f1 = (A + B) / (AB * AB);
-        const double f2 = (A * A + AB + B * B) / (AB * AB * AB);
-        acc += m0 * f0 + m[3 * slot + 1] * f1 + m[3 * slot + 2] * f2;
-    }
-    spec[(int64_t)d * n_E + b] += acc;
-}
-
-// The same far field as a convolution on the uniform axis: with the centre
-// bin c and the output bin b a distance D = b - c apart, A = (D - 1/2) w and
-// B = (D + 1/2) w, so the three expansion coefficients are
+// Far field: spec[d][b] += sum_c M[d][c] . envelope(b, c) over the (padded)
+// centre bins c farther than K_far bins from b. The moments sit on a uniform
+// axis, so this is a convolution: with the bins a distance D = b - c apart,
+// A = (D - 1/2) w and B = (D + 1/2) w, and the three expansion coefficients are
 //   f0 = r / w^2, f1 = 2 D r^2 / w^3, f2 = (3 D^2 + 1/4) r^3 / w^4,
 //   r = 1 / (D^2 - 1/4),
-// and r depends on the integer D alone: one table of r per block replaces a
-// division per (bin, centre) pair. A block takes 32 output bins of one
-// direction; its 8 warps split the centre bins into 8 contiguous slices (a
-// warp's lanes read the same centre bin: broadcast loads) and the slices'
-// sums are added in slice order, so the result does not depend on the launch.
-constexpr int kFarBins = 32;
-constexpr int kFarSlices = 8;
+// r a function of the integer D alone. 3 D^2 + 1/4 = 3 / r + 1, so a pair is
+//   w^2 f = r (m0 + r (2 D m1 / w + (3 + r) m2 / w^2)):
+// four FMAs, one step of D and two shared loads (the moment of the centre,
+// broadcast to the warp, serves kFarPer bins; r is consecutive over the lanes
+// and zero within K_far). The first form took the moments from L2 in FP64, a
+// conversion and nine products a pair (2,048 bins x 2,872 centres, mixed: 4
+// directions 90 -> 15 us, 16 directions 153 -> 42 us).
+// A block takes kFarBins bins of one direction and walks the centres in chunks
+// staged with the chunk's r; its 16 warps split each chunk. Sums leave Acc for
+// FP64 after each chunk, and the warps' sums are added in warp order, so the
+// result does not depend on the launch.
+constexpr int kFarPer = 2;             // output bins per thread, 32 apart
+constexpr int kFarBins = 32 * kFarPer;
+constexpr int kFarSlices = 16;
+constexpr int kFarChunk = 512;         // most centres staged at a time
 
-// Acc is the accumulation type: double on the FP64 path, float on the mixed
-// one (a bin's far field is a sum of positive envelope terms and two small
-// corrections, well inside float over 2,100 centres; the slices' partial sums
-// and the spectrum stay FP64).
 template <class Acc>
-__global__ void __launch_bounds__(kFarBins * kFarSlices) far_field_conv_kernel(const double *edges, int n_E, int pad,
-                                                                               const double *mom, double *spec,
-                                                                               int K_far) {
-    extern __shared__ __align__(16) unsigned char far_smem[];
-    Acc *sR = reinterpret_cast<Acc *>(far_smem);  // r(D) for D = -n_mom .. n_mom
-    __shared__ double part[3][kFarSlices][kFarBins];
+struct __align__(16) FarMoment {
+    Acc m0, m1, m2, m2x3;
+};
+
+// Acc is the type of a chunk's products and sums: double on the FP64 path,
+// float on the mixed one (a bin's far field is a sum of positive envelope terms
+// and two small corrections; a chunk's share of a thread is at most 32 terms).
+template <class Acc>
+__global__ void __launch_bounds__(32 * kFarSlices) far_field_conv_kernel(const double *edges, int n_E, int pad,
+                                                                         const double *mom, double *spec, int K_far) {
+    __shared__ FarMoment<Acc> sM[kFarChunk];
+    __shared__ Acc sR[kFarChunk + kFarBins];  // r(D) at D - D_lo
+    __shared__ double part[kFarSlices][kFarBins];
     const int d = blockIdx.y;
     const int n_mom = n_E + 2 * pad;
-    const double w = (edges[n_E] - edges[0]) / n_E;
-    for (int i = threadIdx.x; i <= 2 * n_mom; i += blockDim.x) {
-        const double D = (double)(i - n_mom);
-        sR[i] = (Acc)(1.0 / (D * D - 0.25));
-    }
-    __syncthreads();
-    const int lane = threadIdx.x % kFarBins, slice = threadIdx.x / kFarBins;
-    const int b = blockIdx.x * kFarBins + lane;
+    const int n_chunk = (n_mom + kFarChunk - 1) / kFarChunk;
+    // equal chunks, whole rounds of the warps
+    const int per = ((n_mom + n_chunk - 1) / n_chunk + kFarSlices - 1) / kFarSlices;
+    const int len = per * kFarSlices;
+    const double iw = 1.0 / ((edges[n_E] - edges[0]) / n_E);
+    const double iw2 = iw * iw;
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int b0 = blockIdx.x * kFarBins;
     const double *m = mom + (int64_t)d * n_mom * 3;
-    const int per = (n_mom + kFarSlices - 1) / kFarSlices;
-    const int s0 = slice * per, s1 = min(s0 + per, n_mom);
-    Acc acc0 = 0, acc1 = 0, acc2 = 0;
-    if (b < n_E) {
-        for (int slot = s0; slot < s1; ++slot) {
-            const int c = slot - pad;
-            if (c >= b - K_far && c <= b + K_far) continue;
-            const double m0 = m[3 * slot];
-            if (m0 == 0.0) continue;
-            const int D = b - c;
-            const Acc r = sR[D + n_mom];
-            const Acc Dd = (Acc)D;
-            acc0 = fma((Acc)m0, r, acc0);
-            acc1 = fma((Acc)m[3 * slot + 1], (Acc)2 * Dd * r * r, acc1);
-            acc2 = fma((Acc)m[3 * slot + 2], ((Acc)3 * Dd * Dd + (Acc)0.25) * r * r * r, acc2);
-        }
-    }
-    part[0][slice][lane] = (double)acc0;
-    part[1][slice][lane] = (double)acc1;
-    part[2][slice][lane] = (double)acc2;
-    __syncthreads();
-    if (slice == 0 && b < n_E) {
-        double t0 = 0.0, t1 = 0.0, t2 = 0.0;
+    double sum[kFarPer];
 #pragma unroll
-        for (int k = 0; k < kFarSlices; ++k) {
-            t0 += part[0][k][lane];
-            t1 += part[1][k][lane];
-            t2 += part[2][k][lane];
+    for (int j = 0; j < kFarPer; ++j) sum[j] = 0.0;
+    for (int c0 = 0; c0 < n_mom; c0 += len) {
+        const int n = min(len, n_mom - c0);
+        // r at the distances b0 + t - (c0 - pad + i), t < kFarBins, i < n
+        const int D_lo = b0 - (c0 - pad + n - 1);
+        __syncthreads();  // the last chunk has been read
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const double *mi = m + 3 * (int64_t)(c0 + i);
+            const double m0 = mi[0], m1 = m0 != 0.0 ? mi[1] * iw : 0.0, m2 = m0 != 0.0 ? mi[2] * iw2 : 0.0;
+            sM[i] = {(Acc)m0, (Acc)(2.0 * m1), (Acc)m2, (Acc)(3.0 * m2)};
         }
-        const double iw = 1.0 / w;
-        const double iw2 = iw * iw, iw3 = iw2 * iw, iw4 = iw2 * iw2;
-        spec[(int64_t)d * n_E + b] += t0 * iw2 + t1 * iw3 + t2 * iw4;
+        for (int i = threadIdx.x; i < n + kFarBins - 1; i += blockDim.x) {
+            const int D = D_lo + i;
+            sR[i] = D >= -K_far && D <= K_far ? (Acc)0 : (Acc)(1.0 / ((double)D * (double)D - 0.25));
+        }
+        __syncthreads();
+        const int i0 = min(slice * per, n), i1 = min(i0 + per, n);
+        const Acc *r_at = sR + lane + (n - 1);  // r of bin b0 + lane + 32 j and centre i: r_at[32 j - i]
+        Acc D = (Acc)(b0 + lane - (c0 - pad + i0));
+        Acc acc[kFarPer];
+#pragma unroll
+        for (int j = 0; j < kFarPer; ++j) acc[j] = 0;
+#pragma unroll 4
+        for (int i = i0; i < i1; ++i) {
+            const FarMoment<Acc> q = sM[i];
+#pragma unroll
+            for (int j = 0; j < kFarPer; ++j) {
+                const Acc r = r_at[32 * j - i];
+                const Acc u = fma(D + (Acc)(32 * j), q.m1, fma(q.m2, r, q.m2x3));
+                acc[j] = fma(fma(u, r, q.m0), r, acc[j]);
+            }
+            D -= (Acc)1;
+        }
+#pragma unroll
+        for (int j = 0; j < kFarPer; ++j) sum[j] += (double)acc[j];
+    }
+#pragma unroll
+    for (int j = 0; j < kFarPer; ++j) part[slice][lane + 32 * j] = sum[j];
+    __syncthreads();
+    const int b = b0 + threadIdx.x;
+    if (threadIdx.x < kFarBins && b < n_E) {
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < kFarSlices; ++k) t += part[k][threadIdx.x];
+        spec[(int64_t)d * n_E + b] += t * iw2;
     }
 }
 
@@ -1794,18 +1792,9 @@ static cudaError_t launch_cxr_t(const pb_cxr_args &a, cudaStream_t s, int sms, i
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (K_far > 0) {
-        dim3 fg((unsigned)((a.n_E + 127) / 128), (unsigned)a.n_dir);
-        const size_t tab = sizeof(Real) * (2 * ((size_t)a.n_E + 2 * (size_t)far_pad) + 1);
-        if (tab <= 200 * 1024) {
-            // the moments sit on a uniform axis (far moments are enabled on uniform edges only)
-            auto conv = far_field_conv_kernel<Real>;
-            err = cudaFuncSetAttribute(conv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab);
-            if (err != cudaSuccess) return err;
-            dim3 cg((unsigned)((a.n_E + kFarBins - 1) / kFarBins), (unsigned)a.n_dir);
-            conv<<<cg, kFarBins * kFarSlices, tab, s>>>(a.edges, a.n_E, far_pad, a.far_moments, a.spec, K_far);
-        } else {
-            far_field_kernel<<<fg, 128, 0, s>>>(a.edges, a.n_E, far_pad, a.far_moments, a.spec, K_far);
-        }
+        // far moments are enabled on uniform edges only
+        dim3 cg((unsigned)((a.n_E + kFarBins - 1) / kFarBins), (unsigned)a.n_dir);
+        far_field_conv_kernel<Real><<<cg, 32 * kFarSlices, 0, s>>>(a.edges, a.n_E, far_pad, a.far_moments, a.spec, K_far);
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;
     }

@@ -150,3 +150,25 @@ def test_tiles_without_radiating_segments(n_seg, precision, cuda_device):
     ref = mc_cxr_spectrum(alone, E_grid, "silicon", None, **kw)
     assert np.max(ref) > 0.0
     assert np.max(np.abs(got - ref)) <= (1e-12 if precision == "fp64" else 1e-6) * np.max(ref)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n_E", [2, 45, 63, 64, 65, 364, 366, 1463, 9301])
+def test_far_field_at_the_edges_of_its_chunks(n_E, precision, cuda_device):
+    """Two-width windows leave nearly every bin to the far field, whose blocks
+    take 64 bins and stage the n_E + 2 pad centres in chunks of at most 512
+    (pad = 0.2 n_E + 2: 364 bins fill one chunk, 366 take two)."""
+    from pyrite_b200 import mc_cxr_spectrum
+
+    E_grid = np.linspace(1000.0, 60000.0, n_E)
+    seg, rows, tables, n_hat = _scene(8, 40, E_grid, 1.5e5, 40 + n_E)
+    E, a, w = _lines(seg, rows, tables, n_hat, E_grid)
+    assert E.size > 40
+    ref = _deposit(E, a, w, oracle.energy_bin_edges(E_grid), 2.0) / seg["Ne"]
+    got = mc_cxr_spectrum(seg, E_grid, "silicon", None, tables=tables, n_hat=n_hat, rows=rows,
+                          line_quadrature="bin-mean", precision=precision, exact_widths=2.0, device=cuda_device)
+    if precision == "fp64":
+        assert np.max(np.abs(got - ref)) <= 5e-9 * np.max(np.abs(ref))
+    else:
+        # 320 lines at most: between the single line's 3e-2 and the 2e-3 of many
+        assert np.sum(np.abs(got - ref)) <= 3e-2 * np.sum(np.abs(ref))

@@ -35,6 +35,12 @@
 // no longer depends on the number of energies, and the 16 detector tiles need
 // no direction moments. Segments outside the window (and all of them when a
 // check fails) go through a list to the per-pair kernels.
+//
+// Where the electrons slow down through many energies, one window would leave
+// most of them out: the list is then ordered by quarter octaves of T (T_hi /
+// T_lo <= 1.25, T_lo >= 2.5 k_max) and each has its own polynomials and
+// moments, which the contraction sums; a quarter octave whose polynomials miss
+// the 1e-7 goes to the per-pair kernels alone.
 #include <cstdint>
 
 #include "pb_brem_node.cuh"
@@ -46,7 +52,8 @@ namespace {
 
 constexpr double kNodeMc2 = 510.99895;
 constexpr int kNodeThreads = 256;
-constexpr int kContractThreads = 128;
+constexpr int kContractThreads = 256;
+constexpr int kNodeWinTile = 512;  // the same where the list has windows: enough tiles for every block
 constexpr int kNodeTile = 2048;  // segments a block orders by depth cell at a time (1024: 7 % slower, 4096: 3 %)
 
 __device__ __forceinline__ bool node_radiates(const pb_brem_args &a, int64_t s) {
@@ -59,20 +66,20 @@ __device__ __forceinline__ int64_t node_live(const pb_brem_args &a) {
     return live;
 }
 
-// J_el(T, k) in FP64 (the per-pair FP64 form without w_el and c0 / k; the
-// born logarithm from (p_i + p_f)^2 / (p_i^2 - p_f^2), p_i^2 - p_f^2 =
-// k (T + T_f + 2 m c^2) / (m c^2)^2, without cancellation).
+// J_el(T, k) in FP64 (the per-pair FP64 form without w_el and c0 / k), in units
+// of m c^2: x = T, y = T - k, gamma = 1 + x, p = sqrt(x (x + 2)), beta = p / gamma,
+//   J = ln((p_i + p_f)^2 / (p_i^2 - p_f^2)) (gamma_f / p_f) / (p_i gamma_i (1 - exp(-2 pi alpha Z gamma_f / p_f))),
+// the logarithm's p_i^2 - p_f^2 = k (x + y + 2) without cancellation.
 __device__ double node_J(double T, double k, double Z) {
     const double Tf = T - k;
     if (!(Tf > 0.0) || !(k > 0.0)) return 0.0;
-    const double p_i = sqrt(T * (T + 2.0 * kNodeMc2)) / kNodeMc2;
-    const double b_i = p_i / (1.0 + T / kNodeMc2);
-    const double p_f = sqrt(Tf * (Tf + 2.0 * kNodeMc2)) / kNodeMc2;
-    const double b_f = p_f / (1.0 + Tf / kNodeMc2);
-    const double dpp = k * (T + Tf + 2.0 * kNodeMc2) / (kNodeMc2 * kNodeMc2);
+    constexpr double kInv = 1.0 / kNodeMc2;
+    const double x = T * kInv, y = Tf * kInv;
+    const double p_i = sqrt(x * (x + 2.0)), p_f = sqrt(y * (y + 2.0));
     const double s = p_i + p_f;
-    const double bl = log(s * s / dpp);
-    return b_i / (p_i * p_i) * bl / b_f / (1.0 - exp(-2.0 * kPi * kAlphaFs * Z / b_f));
+    const double bl = log(s * s / (k * kInv * (x + y + 2.0)));
+    const double inv_bf = (1.0 + y) / p_f;
+    return bl * inv_bf / (p_i * (1.0 + x) * (1.0 - exp(-2.0 * kPi * kAlphaFs * Z * inv_bf)));
 }
 
 // Cell of depth z (boundaries zb, n cells): the closed form of the grid, then
@@ -88,18 +95,45 @@ __device__ __forceinline__ int node_cell(const double *zb, int n, double h_min, 
 }
 
 // Extent of the launch: the largest and smallest electron energy of the
-// radiating segments.
-__global__ void __launch_bounds__(kNodeThreads) brem_node_range_kernel(const pb_brem_args a, BremNodeHdr *h) {
+// radiating segments and, for a list with windows, their count and their
+// histogram over quarter octaves. One atomic a block for each extreme: a
+// warp's atomic each on the two addresses took most of this kernel (200,000
+// segments, with the histogram: 8.1 -> 5.2 us).
+__global__ void __launch_bounds__(kNodeThreads) brem_node_range_kernel(const pb_brem_args a, BremNodeHdr *h,
+                                                                       bool count) {
+    __shared__ unsigned int hist[kNodeBins];
+    __shared__ unsigned long long red[2][kNodeThreads / 32];
+    __shared__ unsigned int n_rad;
+    const int tid = threadIdx.x;
+    if (tid < kNodeBins) hist[tid] = 0u;
+    if (tid == 0) n_rad = 0u;
+    __syncthreads();
     const int64_t live = node_live(a);
     unsigned long long mx = 0ULL, mnc = 0ULL;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < live;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        if (!node_radiates(a, s)) continue;
-        const double T = a.E_keV[s];
-        if (!(T > 0.0 && T < 1e300)) continue;
-        const unsigned long long b = (unsigned long long)__double_as_longlong(T);
-        mx = b > mx ? b : mx;
-        mnc = ~b > mnc ? ~b : mnc;
+    unsigned int rads = 0u;
+    const int64_t rounds = (live + blockDim.x * (int64_t)gridDim.x - 1) / (blockDim.x * (int64_t)gridDim.x);
+    for (int64_t r = 0; r < rounds; ++r) {
+        const int64_t s = (r * gridDim.x + blockIdx.x) * (int64_t)blockDim.x + tid;
+        const bool rad = s < live && node_radiates(a, s);
+        rads += rad ? 1u : 0u;
+        const double T = rad ? a.E_keV[s] : 0.0;
+        const bool valid = T > 0.0 && T < 1e300;
+        if (valid) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(T);
+            mx = b > mx ? b : mx;
+            mnc = ~b > mnc ? ~b : mnc;
+        }
+        if (count) {
+            // neighbours mostly share a bin: one add a warp then
+            const int q = valid ? node_bin(T) : -1;
+            int same = 0;
+            __match_all_sync(0xffffffffu, q, &same);
+            if (same) {
+                if ((tid & 31) == 0 && q >= 0 && q < kNodeBins) atomicAdd(&hist[q], 32u);
+            } else if (q >= 0 && q < kNodeBins) {
+                atomicAdd(&hist[q], 1u);
+            }
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -108,146 +142,294 @@ __global__ void __launch_bounds__(kNodeThreads) brem_node_range_kernel(const pb_
         mx = x > mx ? x : mx;
         mnc = y > mnc ? y : mnc;
     }
-    if ((threadIdx.x & 31) == 0 && mx != 0ULL) {
-        atomicMax(&h->t_max_bits, mx);
-        atomicMax(&h->t_minc_bits, mnc);
+    rads = __reduce_add_sync(0xffffffffu, rads);
+    if ((tid & 31) == 0) {
+        red[0][tid >> 5] = mx;
+        red[1][tid >> 5] = mnc;
+        if (rads) atomicAdd(&n_rad, rads);
     }
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kNodeThreads / 32; ++w) {
+            mx = red[0][w] > mx ? red[0][w] : mx;
+            mnc = red[1][w] > mnc ? red[1][w] : mnc;
+        }
+        if (mx != 0ULL) {
+            atomicMax(&h->t_max_bits, mx);
+            atomicMax(&h->t_minc_bits, mnc);
+        }
+        if (n_rad) atomicAdd(&h->n_rad, (unsigned long long)n_rad);
+    }
+    if (count && tid < kNodeBins && hist[tid]) atomicAdd(&h->hist[tid], hist[tid]);
 }
 
-// The window, the depth grid, its nodes and the Lagrange basis (one block).
-__global__ void __launch_bounds__(kNodeThreads) brem_node_setup_kernel(const pb_brem_args a, BremNodeHdr *h) {
-    __shared__ double red[2][kNodeThreads / 32];
-    const int tid = threadIdx.x;
-    double kmax = 0.0, mumax = 0.0;
-    bool finite = true;
+// T_m(t) of the Lagrange basis in monomials: T_{m+1} = 2 t T_m - T_{m-1}.
+struct ChebMonomials {
+    double c[kNodePts][kNodePts];
+};
+constexpr ChebMonomials cheb_monomials() {
+    ChebMonomials t{};
+    t.c[0][0] = 1.0;
+    t.c[1][1] = 1.0;
+    for (int m = 1; m + 1 < kNodePts; ++m)
+        for (int k = 0; k < kNodePts; ++k) t.c[m + 1][k] = (k > 0 ? 2.0 * t.c[m][k - 1] : 0.0) - t.c[m - 1][k];
+    return t;
+}
+__constant__ const ChebMonomials kCheb = cheb_monomials();
+
+// The window or windows, the depth grid, its nodes and the Lagrange basis (one
+// block). Directions, cell boundaries and histogram bins go one to a thread:
+// a single thread's loops of divisions and powers took 23 us (now 10).
+//
+// Windows: the one window holds the electrons of a beam that hardly slows
+// down. Where the energies spread, the segments certainly below it decide, each
+// priced at n_E evaluations of the per-pair form and as much again for its
+// place in the list: above kNodePairWork the quarter octaves clear of the
+// spectrum's tip become one window each. 200,000 electrons of 8 keV to 10 MeV
+// on 2,048 energies, 59 % of them in 24 windows: per-pair form 958 -> 490 us;
+// fit, list, moments and contraction of the windows 143 us, against 141 us for
+// a list of nearly every segment that the one window then gave up. At 300
+// energies a list of 40,000 takes 324 us through the entry point, 436 before;
+// below the line the two are within 10 us.
+constexpr double kNodePairWork = 16777216.0;
+
+__global__ void __launch_bounds__(kNodeThreads) brem_node_setup_kernel(const pb_brem_args a, BremNodeHdr *h,
+                                                                       int max_win) {
+    constexpr int kWarps = kNodeThreads / 32;
+    __shared__ double red[3][kWarps];
+    __shared__ int n_s, go_s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double kmax = 0.0, mumax = 0.0, f_max = 0.0;
+    bool finite = true, up = false, down = false;
     for (int e = tid; e < a.n_E; e += blockDim.x) {
         kmax = fmax(kmax, a.E_grid[e] / 1e3);
         const double m = a.mu[e];
         finite = finite && m >= 0.0 && m < 1e300;
         mumax = fmax(mumax, m);
     }
+    for (int d = tid; d < a.n_dir; d += blockDim.x) {
+        const double nz = a.n_hat[3 * d + 2];
+        f_max = fmax(f_max, 1.0 / fmax(fabs(nz), 1.0e-12));
+        if (nz < 0.0) up = true;
+        else down = true;
+    }
     const bool all_finite = __syncthreads_and(finite);
+    const unsigned int faces = (__syncthreads_or(up) ? 1u : 0u) | (__syncthreads_or(down) ? 2u : 0u);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         kmax = fmax(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
         mumax = fmax(mumax, __shfl_xor_sync(0xffffffffu, mumax, o));
+        f_max = fmax(f_max, __shfl_xor_sync(0xffffffffu, f_max, o));
     }
-    if ((tid & 31) == 0) {
-        red[0][tid >> 5] = kmax;
-        red[1][tid >> 5] = mumax;
+    if (lane == 0) {
+        red[0][warp] = kmax;
+        red[1][warp] = mumax;
+        red[2][warp] = f_max;
+    }
+    if (tid == 0) n_s = kNodeMaxCells + 1;
+    __syncthreads();
+    for (int w = 0; w < kWarps; ++w) {
+        kmax = fmax(kmax, red[0][w]);
+        mumax = fmax(mumax, red[1][w]);
+        f_max = fmax(f_max, red[2][w]);
+    }
+    const double T_hi = __longlong_as_double((long long)h->t_max_bits);
+    const double T_min = __longlong_as_double((long long)~h->t_minc_bits);
+    const double T_lo = fmax(T_min, fmax(T_hi / kNodeWindow, kNodeTip * kmax));
+    const double T_slab = a.thickness;
+    bool ok = h->t_max_bits != 0ULL && all_finite && T_slab > 0.0;
+    // the depth grid: boundary n on thread n, the first at or below the slab's far face ends it
+    const double lam = mumax * f_max;
+    const double h_min = lam > 0.0 ? fmin(1.0 / lam, T_slab) : T_slab;
+    const double z_g = kNodeUniform * h_min;
+    double zb = 0.0;
+    if (tid <= kNodeMaxCells) {
+        zb = tid <= kNodeUniform ? tid * h_min : z_g * pow(kNodeGrowth, (double)(tid - kNodeUniform));
+        if (tid > 0 && !(zb < T_slab)) atomicMin(&n_s, tid);
     }
     __syncthreads();
-    __shared__ int n_s, ok_s;
-    if (tid == 0) {
-        for (int w = 0; w < kNodeThreads / 32; ++w) {
-            kmax = fmax(kmax, red[0][w]);
-            mumax = fmax(mumax, red[1][w]);
-        }
-        double f_max = 0.0;
-        unsigned int faces = 0u;
-        for (int d = 0; d < a.n_dir; ++d) {
-            const double nz = a.n_hat[3 * d + 2];
-            f_max = fmax(f_max, 1.0 / fmax(fabs(nz), 1.0e-12));
-            faces |= nz < 0.0 ? 1u : 2u;
-        }
-        bool ok = h->t_max_bits != 0ULL && all_finite;
-        const double T_hi = __longlong_as_double((long long)h->t_max_bits);
-        const double T_min = __longlong_as_double((long long)~h->t_minc_bits);
-        const double T_lo = fmax(T_min, fmax(T_hi / kNodeWindow, kNodeTip * kmax));
-        ok = ok && T_lo <= T_hi;
-        const double T_slab = a.thickness;
-        ok = ok && T_slab > 0.0;
-        const double lam = mumax * f_max;
-        const double h_min = lam > 0.0 ? fmin(1.0 / lam, T_slab) : T_slab;
-        const double z_g = kNodeUniform * h_min;
-        int n = 0;
-        h->zb[0] = 0.0;
-        while (ok && h->zb[n] < T_slab) {
-            if (n == kNodeMaxCells) {
-                ok = false;
-                break;
-            }
-            ++n;
-            h->zb[n] = n <= kNodeUniform ? n * h_min : z_g * pow(kNodeGrowth, (double)(n - kNodeUniform));
-        }
-        if (ok) h->zb[n] = T_slab;
-        h->n_cells = ok ? n : 0;
-        h->faces = faces;
-        h->T_lo = T_lo;
-        h->T_hi = T_hi;
-        h->Tc = 0.5 * (T_lo + T_hi);
-        h->Th = 0.5 * (T_hi - T_lo);
-        h->h_min = h_min;
-        h->z_g = z_g;
-        n_s = ok ? n : 0;
-        ok_s = ok ? 1 : 0;
-    }
-    __syncthreads();
-    if (!ok_s) return;  // h->ok stays 0 (the workspace was zeroed)
     const int n = n_s;
+    ok = ok && n <= kNodeMaxCells;
+    if (ok && tid <= n) h->zb[tid] = tid < n ? zb : T_slab;
+    int n_win = 0;
+    if (warp == 0) {
+        // two bins a lane, upwards in energy
+        unsigned int below = 0u, in_bins = 0u;
+        unsigned int c[2];
+        unsigned int use[2];
+        for (int k = 0; k < 2; ++k) {
+            const int q = lane + 32 * k;
+            c[k] = h->hist[q];
+            in_bins += c[k];
+            if (node_bin_lo(q + 1) <= T_lo) below += c[k];
+            use[k] = __ballot_sync(0xffffffffu, c[k] > 0u && node_bin_lo(q) >= kNodeTip * kmax);
+        }
+        below = __reduce_add_sync(0xffffffffu, below);
+        in_bins = __reduce_add_sync(0xffffffffu, in_bins);
+        // (bins only count where the list has windows)
+        const unsigned long long left = in_bins ? h->n_rad - in_bins + below : 0ULL;
+        if (ok && max_win > 1 && (double)left * (a.n_E + 1024.0) > kNodePairWork) n_win = min(__popc(use[0]) + __popc(use[1]), max_win);
+        for (int k = 0; k < 2; ++k) {
+            const int q = lane + 32 * k;
+            const int w = __popc(use[k] & ((1u << lane) - 1u)) + (k ? __popc(use[0]) : 0);
+            const bool on = ((use[k] >> lane) & 1u) && w < n_win;
+            h->win_of[q] = on ? w : -1;
+            if (on) {
+                const double lo = node_bin_lo(q), hi = node_bin_lo(q + 1);
+                h->win_Tc[w] = 0.5 * (lo + hi);
+                h->win_Th[w] = 0.5 * (hi - lo);
+                h->win_n[w] = c[k];
+            }
+        }
+        if (lane == 0) {
+            ok = ok && (n_win > 0 || T_lo <= T_hi);
+            h->n_cells = ok ? n : 0;
+            h->faces = faces;
+            h->n_win = n_win;
+            h->T_lo = T_lo;
+            h->T_hi = T_hi;
+            h->Tc = 0.5 * (T_lo + T_hi);
+            h->Th = 0.5 * (T_hi - T_lo);
+            h->h_min = h_min;
+            h->z_g = z_g;
+            if (n_win == 0) {
+                h->win_Tc[0] = 0.5 * (T_lo + T_hi);
+                h->win_Th[0] = 0.5 * (T_hi - T_lo);
+            }
+            go_s = ok ? 1 : 0;
+        }
+    }
+    __syncthreads();
+    if (!go_s) return;  // h->ok stays 0 (the workspace was zeroed)
     // the cells' Chebyshev nodes
     for (int q = tid; q < n * kNodePts; q += blockDim.x) {
         const int c = q / kNodePts, i = q - c * kNodePts;
         const double mid = 0.5 * (h->zb[c] + h->zb[c + 1]), hw = 0.5 * (h->zb[c + 1] - h->zb[c]);
-        h->node[q] = mid + hw * cos((2 * i + 1) * kPi / (2 * kNodePts));
+        h->node[q] = mid + hw * cospi((2 * i + 1) * (1.0 / (2 * kNodePts)));
     }
-    // Lagrange basis of the Chebyshev nodes x_i: l_i(t) = (1/n) [1 + 2 sum_m T_m(x_i) T_m(t)],
-    // with T_m in monomials from T_{m+1} = 2 t T_m - T_{m-1}.
+    // Lagrange basis of the Chebyshev nodes x_i: l_i(t) = (1/n) [1 + 2 sum_m T_m(x_i) T_m(t)]
     if (tid < kNodePts * kNodePts) {
         const int i = tid / kNodePts, j = tid - i * kNodePts;
-        double Tc[kNodePts][kNodePts] = {};
-        Tc[0][0] = 1.0;
-        Tc[1][1] = 1.0;
-        for (int m = 1; m + 1 < kNodePts; ++m)
-            for (int k = 0; k < kNodePts; ++k) Tc[m + 1][k] = (k > 0 ? 2.0 * Tc[m][k - 1] : 0.0) - Tc[m - 1][k];
         double v = 0.0;
         for (int m = 0; m < kNodePts; ++m)
-            v += (m == 0 ? 1.0 : 2.0) / kNodePts * cos(m * (2 * i + 1) * kPi / (2 * kNodePts)) * Tc[m][j];
+            v += (m == 0 ? 1.0 : 2.0) / kNodePts * cospi(m * (2 * i + 1) * (1.0 / (2 * kNodePts))) * kCheb.c[m][j];
         h->Lm[tid] = v;
     }
     __syncthreads();
     if (tid == 0) h->ok = 1u;
 }
 
-// J_el over the window as a degree-5 polynomial in u, per (energy, element):
+// J_el over a window as a degree-5 polynomial in u, per (energy, element):
 // Chebyshev coefficients from six nodes, then monomials; checked against J
-// at u = -1, -1/2, 0, 1/2, 1 to 1e-7 (a miss turns the node form off).
-__global__ void brem_node_fit_kernel(const pb_brem_args a, BremNodeHdr *h, double *A) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.n_E * a.n_el || !h->ok) return;
-    const int e = q / a.n_el, el = q - e * a.n_el;
-    const double k = a.E_grid[e] / 1e3, Z = a.Z[el];
-    const double Tc = h->Tc, Th = h->Th;
-    double *out = A + (int64_t)q * kNodeTDeg;
-    if (!(k > 0.0)) {
-        for (int p = 0; p < kNodeTDeg; ++p) out[p] = 0.0;
-        return;
-    }
-    double f[kNodeTDeg];
-    for (int m = 0; m < kNodeTDeg; ++m) f[m] = node_J(Tc + Th * cos((2 * m + 1) * kPi / (2 * kNodeTDeg)), k, Z);
-    double c[kNodeTDeg];
-    for (int p = 0; p < kNodeTDeg; ++p) {
-        double v = 0.0;
-        for (int m = 0; m < kNodeTDeg; ++m) v += f[m] * cos(p * (2 * m + 1) * kPi / (2 * kNodeTDeg));
-        c[p] = v * (p == 0 ? 1.0 : 2.0) / kNodeTDeg;
-    }
+// at u = -1, -1/2, 0, 1/2, 1 to 1e-7 (a miss turns the node form off, or the
+// window where there are several). 16 lanes take one polynomial, one
+// evaluation of J a lane (one thread for all eleven: 23 us for 2,048 energies,
+// now 5).
+constexpr int kFitLanes = 16;
+__global__ void __launch_bounds__(128) brem_node_fit_kernel(const pb_brem_args a, BremNodeHdr *h, double *A) {
+    const int w = blockIdx.y;
+    if (!__syncthreads_and(h->ok != 0u && w < max(h->n_win, 1))) return;
+    const int q = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kFitLanes);
+    const int lane = threadIdx.x % kFitLanes;
+    const bool on = q < a.n_E * a.n_el;
+    const int e = on ? q / a.n_el : 0, el = on ? q - e * a.n_el : 0;
+    const double k = a.E_grid[e] / 1e3;
+    // lanes 0..5: the nodes; 6..10: the points of the check
+    const double cos_l = cospi((threadIdx.x & 31) * (1.0 / (2 * kNodeTDeg)));  // of the warp's lane: cos(l pi / 12)
+    const double x_l = __shfl_sync(0xffffffffu, cos_l, 2 * lane + 1);
+    const double u = lane < kNodeTDeg ? x_l : -1.0 + 0.5 * (lane - kNodeTDeg);
+    const bool eval = on && lane < kNodeTDeg + 5 && k > 0.0;
+    const double J = eval ? node_J(h->win_Tc[w] + h->win_Th[w] * u, k, a.Z[el]) : 0.0;
+    double c = 0.0;  // lane p < 6: the coefficient of T_p
+    for (int m = 0; m < kNodeTDeg; ++m)
+        c += __shfl_sync(0xffffffffu, J, m, kFitLanes) *
+             __shfl_sync(0xffffffffu, cos_l, lane * (2 * m + 1) % (4 * kNodeTDeg));
+    c *= (lane == 0 ? 1.0 : 2.0) / kNodeTDeg;
+    double cp[kNodeTDeg];
+    for (int p = 0; p < kNodeTDeg; ++p) cp[p] = __shfl_sync(0xffffffffu, c, p, kFitLanes);
     // T_0..T_5 in monomials
-    const double A0 = c[0] - c[2] + c[4], A1 = c[1] - 3.0 * c[3] + 5.0 * c[5], A2 = 2.0 * c[2] - 8.0 * c[4];
-    const double A3 = 4.0 * c[3] - 20.0 * c[5], A4 = 8.0 * c[4], A5 = 16.0 * c[5];
-    out[0] = A0;
-    out[1] = A1;
-    out[2] = A2;
-    out[3] = A3;
-    out[4] = A4;
-    out[5] = A5;
-    bool good = true;
-    for (int t = 0; t < 5; ++t) {
-        const double u = -1.0 + 0.5 * t;
-        const double ex = node_J(Tc + Th * u, k, Z);
-        const double pv = ((((A5 * u + A4) * u + A3) * u + A2) * u + A1) * u + A0;
-        good = good && fabs(pv - ex) <= 1e-7 * fabs(ex);
+    const double P[kNodeTDeg] = {cp[0] - cp[2] + cp[4],      cp[1] - 3.0 * cp[3] + 5.0 * cp[5],
+                                 2.0 * cp[2] - 8.0 * cp[4],  4.0 * cp[3] - 20.0 * cp[5],
+                                 8.0 * cp[4],                16.0 * cp[5]};
+    const double pv = ((((P[5] * u + P[4]) * u + P[3]) * u + P[2]) * u + P[1]) * u + P[0];
+    if (on && lane == 0) {
+        double *out = A + ((int64_t)w * a.n_E * a.n_el + q) * kNodeTDeg;
+#pragma unroll
+        for (int p = 0; p < kNodeTDeg; ++p) out[p] = P[p];
     }
-    if (!good) atomicExch(&h->ok, 0u);
+    if (eval && lane >= kNodeTDeg && !(fabs(pv - J) <= 1e-7 * fabs(J))) {
+        atomicExch(&h->win_bad[w], 1u);
+        if (h->n_win == 0) atomicExch(&h->ok, 0u);
+    }
+}
+
+// Where the windows' segments go in the list: the left-out ones first, then
+// window by window (a window whose fit missed has no part). Whole warps.
+__device__ __forceinline__ void node_window_offsets(const BremNodeHdr *h, int n_win, int lane, int64_t &off,
+                                                    unsigned int &n) {
+    n = lane < n_win && !h->win_bad[lane] ? h->win_n[lane] : 0u;
+    unsigned long long incl = n;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const unsigned long long all = __shfl_sync(0xffffffffu, incl, 31);
+    off = (int64_t)(h->n_rad - all + incl - n);
+}
+
+// Segment list by window: each block counts a tile's segments per window in
+// shared memory, reserves their places with one atomic a window and writes them.
+constexpr int kListPer = 4;  // segments per thread and tile
+__global__ void __launch_bounds__(kNodeThreads) brem_node_list_kernel(const pb_brem_args a, BremNodeHdr *h,
+                                                                      int64_t *idx, int64_t cap) {
+    __shared__ unsigned int cnt[kNodeMaxWin + 1];
+    __shared__ unsigned long long base[kNodeMaxWin + 1];
+    __shared__ int64_t off_s[kNodeMaxWin + 1];
+    __shared__ int win_s[kNodeBins];
+    const int tid = threadIdx.x;
+    const int n_win = h->n_win;
+    if (!h->ok || n_win == 0) return;
+    if (tid < 32) {
+        int64_t off;
+        unsigned int n;
+        node_window_offsets(h, n_win, tid, off, n);
+        off_s[tid + 1] = off;
+        if (tid == 0) off_s[0] = 0;
+    }
+    if (tid < kNodeBins) {
+        const int w = h->win_of[tid];
+        win_s[tid] = w >= 0 && !h->win_bad[w] ? w : -1;
+    }
+    const int64_t live = node_live(a);
+    constexpr int kTile = kNodeThreads * kListPer;
+    for (int64_t t0 = blockIdx.x * (int64_t)kTile; t0 < live; t0 += gridDim.x * (int64_t)kTile) {
+        if (tid <= kNodeMaxWin) cnt[tid] = 0u;
+        __syncthreads();
+        int slot[kListPer];  // 0: left out, w + 1: window w, -1: no part
+        unsigned int rank[kListPer];
+#pragma unroll
+        for (int k = 0; k < kListPer; ++k) {
+            const int64_t s = t0 + k * kNodeThreads + tid;
+            slot[k] = -1;
+            if (s < live && node_radiates(a, s)) {
+                const double T = a.E_keV[s];
+                const int q = T > 0.0 && T < 1e300 ? node_bin(T) : -1;
+                slot[k] = q >= 0 && q < kNodeBins ? win_s[q] + 1 : 0;
+                rank[k] = atomicAdd(&cnt[slot[k]], 1u);
+            }
+        }
+        __syncthreads();
+        if (tid <= kNodeMaxWin && cnt[tid])
+            base[tid] = tid == 0 ? atomicAdd(&h->n_out, (unsigned long long)cnt[0])
+                                 : (unsigned long long)atomicAdd(&h->win_fill[tid - 1], cnt[tid]);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kListPer; ++k) {
+            if (slot[k] < 0) continue;
+            const int64_t at = off_s[slot[k]] + (int64_t)base[slot[k]] + rank[k];
+            if (at < cap) idx[at] = t0 + k * kNodeThreads + tid;
+        }
+    }
 }
 
 // D += A B on the FP64 tensor cores, one m8n8k4 tile: lane l holds
@@ -298,24 +480,41 @@ __global__ void __launch_bounds__(kNodeThreads, 2) brem_node_accum_kernel(const 
     __shared__ unsigned char key_s[kNodeTile];    // start cell per segment (kNodeMaxCells: not in the window)
     __shared__ int cnt_s[kNodeMaxCells + 1];
     __shared__ int n_in_s;
-    __shared__ double prm[6];
-    __shared__ int go_s, nc_s;
+    __shared__ int64_t off_s[kNodeMaxWin];   // windows: start in the list, segments, first tile
+    __shared__ unsigned int win_n_s[kNodeMaxWin];
+    __shared__ int win_t_s[kNodeMaxWin + 1];
+    __shared__ double prm[4];
+    __shared__ int go_s, nc_s, n_win_s;
     __shared__ unsigned int faces_s;
     const int tid = threadIdx.x;
     if (tid == 0) {
         go_s = h->ok ? 1 : 0;
         nc_s = h->n_cells;
+        n_win_s = h->n_win;
         faces_s = h->faces;
         prm[0] = h->T_lo;
         prm[1] = h->T_hi;
-        prm[2] = h->Tc;
-        prm[3] = h->Th > 0.0 ? 1.0 / h->Th : 0.0;
-        prm[4] = h->h_min;
-        prm[5] = h->z_g;
+        prm[2] = h->h_min;
+        prm[3] = h->z_g;
     }
     __syncthreads();
     if (!go_s) return;
-    const int nc = nc_s;
+    const int nc = nc_s, n_win = n_win_s;
+    if (n_win > 0 && tid < 32) {
+        int64_t off;
+        unsigned int n;
+        node_window_offsets(h, n_win, tid, off, n);
+        off_s[tid] = off;
+        win_n_s[tid] = n;
+        int incl = (int)((n + kNodeWinTile - 1) / kNodeWinTile);
+        const int own = incl;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (tid >= o) incl += v;
+        }
+        win_t_s[tid] = incl - own;
+        if (tid == 31) win_t_s[32] = incl;
+    }
     const unsigned int faces = faces_s;
     for (int c = tid; c <= nc; c += blockDim.x) zb_s[c] = h->zb[c];
     for (int c = tid; c < nc; c += blockDim.x) {
@@ -324,7 +523,8 @@ __global__ void __launch_bounds__(kNodeThreads, 2) brem_node_accum_kernel(const 
     }
     for (int q = tid; q < NEL * 2 * kNodeMaxCells * kNodePJ; q += blockDim.x) Ss[q] = 0.0f;
     __syncthreads();
-    const double T_lo = prm[0], T_hi = prm[1], Tc = prm[2], inv_Th = prm[3], h_min = prm[4], z_g = prm[5];
+    const double T_lo = prm[0], T_hi = prm[1], h_min = prm[2], z_g = prm[3];
+    double Tc = h->win_Tc[0], inv_Th = h->win_Th[0] > 0.0 ? 1.0 / h->win_Th[0] : 0.0;
     const double T_slab = a.thickness;
     const double za = 2.0 * kPi * kAlphaFs;
     const int64_t live = node_live(a);
@@ -337,19 +537,62 @@ __global__ void __launch_bounds__(kNodeThreads, 2) brem_node_accum_kernel(const 
     // memory), so that the 32 segments a warp takes share their cells and a
     // round of pieces needs one or two tensor-core products.
     const int f0 = (faces & 1u) ? 0 : 1;
-    const int64_t n_tiles = (live + kNodeTile - 1) / kNodeTile;
-    for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const int64_t t0 = tile * kNodeTile;
+    // The block's sums of window w into the FP64 moments.
+    const auto fold = [&](int w, bool clear) {
+        const int per = nc * kNodePJ;
+        for (int q = tid; q < NEL * 2 * per; q += blockDim.x) {
+            const int ef = q / per, r = q - ef * per;
+            if (!((faces >> (ef & 1)) & 1u)) continue;
+            const int off = ef * kNodeMaxCells * kNodePJ + r;
+            const float v = Ss[off];
+            if (v != 0.0f) atomicAdd(&S[(int64_t)w * NEL * 2 * kNodeMaxCells * kNodePJ + off], (double)v);
+            if (clear) Ss[off] = 0.0f;
+        }
+    };
+    // One window: the blocks stride over the tiles of the segment list. Several:
+    // each takes a contiguous run of the windows' tiles, so that its sums change
+    // window seldom.
+    const int64_t n_tiles = n_win > 0 ? win_t_s[32] : (live + kNodeTile - 1) / kNodeTile;
+    const int64_t tile_0 = n_win > 0 ? n_tiles * blockIdx.x / gridDim.x : blockIdx.x;
+    const int64_t tile_1 = n_win > 0 ? n_tiles * (blockIdx.x + 1) / gridDim.x : n_tiles;
+    int win = 0;
+    bool any = false;
+    for (int64_t tile = tile_0; tile < tile_1; tile += n_win > 0 ? 1 : gridDim.x) {
+        int64_t t0 = tile * kNodeTile;       // first segment, or first entry of the list
+        int64_t t_end = live;
+        int rounds = kNodeTile / kNodeThreads;
+        if (n_win > 0) {
+            int w = win;
+            while (w + 1 < n_win && tile >= win_t_s[w + 1]) ++w;
+            if (w != win || !any) {
+                if (any) {
+                    fold(win, true);
+                    __syncthreads();
+                }
+                win = w;
+                Tc = h->win_Tc[w];
+                inv_Th = 1.0 / h->win_Th[w];
+            }
+            t0 = off_s[w] + (tile - win_t_s[w]) * kNodeWinTile;
+            t_end = off_s[w] + win_n_s[w];
+            rounds = kNodeWinTile / kNodeThreads;
+        }
+        any = true;
         for (int q = tid; q <= kNodeMaxCells; q += blockDim.x) cnt_s[q] = 0;
         __syncthreads();
 #pragma unroll 1
-        for (int k = 0; k < kNodeTile / kNodeThreads; ++k) {
+        for (int k = 0; k < rounds; ++k) {
             const int li = k * kNodeThreads + tid;
-            const int64_t s = t0 + li;
-            const bool rad = s < live && node_radiates(a, s);
-            const double T = rad ? a.E_keV[s] : 0.0;
-            const bool in_win = rad && T >= T_lo && T <= T_hi;
-            const bool left = rad && !in_win;
+            int64_t s = t0 + li;
+            bool in_win = s < t_end, left = false;
+            if (n_win > 0) {
+                if (in_win) s = idx[s];
+            } else {
+                const bool rad = in_win && node_radiates(a, s);
+                const double T = rad ? a.E_keV[s] : 0.0;
+                in_win = rad && T >= T_lo && T <= T_hi;
+                left = rad && !in_win;
+            }
             const unsigned int lm = __ballot_sync(0xffffffffu, left);
             if (lm) {
                 const int ld = __ffs(lm) - 1;
@@ -386,7 +629,7 @@ __global__ void __launch_bounds__(kNodeThreads, 2) brem_node_accum_kernel(const 
         }
         __syncthreads();
 #pragma unroll 1
-        for (int k = 0; k < kNodeTile / kNodeThreads; ++k) {
+        for (int k = 0; k < rounds; ++k) {
             const int li = k * kNodeThreads + tid;
             const int pos = atomicAdd(&cnt_s[key_s[li]], 1);
             ord_s[pos] = (unsigned short)li;
@@ -396,7 +639,8 @@ __global__ void __launch_bounds__(kNodeThreads, 2) brem_node_accum_kernel(const 
         for (int g = warp; g * 32 < n_in; g += kWarps) {
             const int pos = g * 32 + (int)lane;
             const bool in_win = pos < n_in;
-            const int64_t s = in_win ? t0 + ord_s[pos] : 0;
+            int64_t s = in_win ? t0 + ord_s[pos] : 0;
+            if (n_win > 0 && in_win) s = idx[s];
             const double T = in_win ? a.E_keV[s] : 0.0;
             double lo = 0.0, hi = 0.0;
             if (in_win) {
@@ -499,84 +743,118 @@ __global__ void __launch_bounds__(kNodeThreads, 2) brem_node_accum_kernel(const 
         __syncthreads();  // the next tile reuses the order
     }
     __syncthreads();
-    const int per = nc * kNodePJ;
-    for (int q = tid; q < NEL * 2 * per; q += blockDim.x) {
-        const int ef = q / per, r = q - ef * per;
-        if (!((faces >> (ef & 1)) & 1u)) continue;
-        const int off = ef * kNodeMaxCells * kNodePJ + r;
-        const float v = Ss[off];
-        if (v != 0.0f) atomicAdd(&S[off], (double)v);
-    }
+    if (any) fold(win, false);
 }
 
-// One block per photon energy: W_ci from the moments, then every direction's
-// sum over the cells' nodes.
+// kE photon energies a block: the moments of the windows summed over
+// the energy polynomial, W_ci from them, then every direction's sum over the
+// cells' nodes, a warp per (direction, energy) with its lanes over the nodes of
+// all cells. The moments are read once for the block's energies (windows: up
+// to 0.8 MB of them), else the exponentials bound it (one window, 16 directions
+// x 2,048 energies, lanes over cells before: 59 -> 34-40 us).
+constexpr int kE = 4;             // photon energies a block (8: 34 -> 59 us, too few blocks)
+constexpr int kContractWin = 16;  // windows whose coefficients are staged at a time
+
 template <int NEL>
 __global__ void __launch_bounds__(kContractThreads) brem_node_contract_kernel(const pb_brem_args a,
                                                                               const BremNodeHdr *h, const double *A,
                                                                               const double *S) {
-    __shared__ double W[2][kNodeMaxCells][kNodePts];
-    __shared__ double nd_s[kNodeMaxCells * kNodePts];
-    __shared__ double Lm_s[kNodePts * kNodePts];
-    __shared__ double A_s[NEL][kNodeTDeg];
-    __shared__ int go_s, nc_s;
-    __shared__ unsigned int faces_s;
+    __shared__ double Zs[kE][kNodeMaxCells * kNodePts];  // then W
+    __shared__ double Lm_s[kNodePts][kNodePts + 1];
+    __shared__ double A_s[kContractWin][NEL * kNodeTDeg][kE];
     const int tid = threadIdx.x;
-    const int e = blockIdx.x;
-    if (tid == 0) {
-        go_s = (h->ok && a.E_grid[e] > 0.0) ? 1 : 0;
-        nc_s = h->n_cells;
-        faces_s = h->faces;
-    }
-    __syncthreads();
-    if (!go_s) return;
-    const int nc = nc_s;
-    const unsigned int faces = faces_s;
-    for (int q = tid; q < nc * kNodePts; q += blockDim.x) nd_s[q] = h->node[q];
-    for (int q = tid; q < kNodePts * kNodePts; q += blockDim.x) Lm_s[q] = h->Lm[q];
-    for (int q = tid; q < NEL * kNodeTDeg; q += blockDim.x)
-        A_s[q / kNodeTDeg][q % kNodeTDeg] = A[(int64_t)e * NEL * kNodeTDeg + q];
-    __syncthreads();
-    for (int q = tid; q < 2 * nc; q += blockDim.x) {
-        const int f = q / nc, c = q - f * nc;
+    const int e0 = blockIdx.x * kE;
+    if (!h->ok) return;
+    const int nc = h->n_cells;
+    const int n_win = h->n_win > 0 ? h->n_win : 1;
+    const unsigned int faces = h->faces;
+    for (int q = tid; q < kNodePts * kNodePts; q += blockDim.x) Lm_s[q / kNodePts][q % kNodePts] = h->Lm[q];
+    constexpr int kPer = (kNodeMaxCells * kNodePts + kContractThreads - 1) / kContractThreads;
+    for (int f = 0; f < 2; ++f) {
         if (!((faces >> f) & 1u)) continue;
-        double Zj[kNodePts];
+        // Z_cj = sum over windows, elements and powers of A S, a (cell, power of t) a thread
+        double Z[kPer][kE];
 #pragma unroll
-        for (int j = 0; j < kNodePts; ++j) Zj[j] = 0.0;
+        for (int r = 0; r < kPer; ++r)
 #pragma unroll
-        for (int el = 0; el < NEL; ++el) {
-            const double *row = S + ((el * 2 + f) * kNodeMaxCells + c) * kNodePJ;
+            for (int x = 0; x < kE; ++x) Z[r][x] = 0.0;
+        for (int w0 = 0; w0 < n_win; w0 += kContractWin) {
+            const int nw = min(kContractWin, n_win - w0);
+            __syncthreads();
+            // (a window whose fit missed has no moments)
+            for (int q = tid; q < nw * NEL * kNodeTDeg * kE; q += blockDim.x) {
+                const int ep = q % (NEL * kNodeTDeg), r = q / (NEL * kNodeTDeg);
+                const int x = r % kE, w = r / kE;
+                const int e = e0 + x;
+                A_s[w][ep][x] = e < a.n_E && a.E_grid[e] > 0.0 && !h->win_bad[w0 + w]
+                                    ? A[((int64_t)(w0 + w) * a.n_E + e) * NEL * kNodeTDeg + ep] : 0.0;
+            }
+            __syncthreads();
+#pragma unroll 2
+            for (int w = 0; w < nw; ++w) {
 #pragma unroll
-            for (int p = 0; p < kNodeTDeg; ++p) {
-                const double ap = A_s[el][p];
+                for (int el = 0; el < NEL; ++el) {
+                    const double *Sw = S + (((int64_t)(w0 + w) * NEL + el) * 2 + f) * kNodeMaxCells * kNodePJ;
 #pragma unroll
-                for (int j = 0; j < kNodePts; ++j) Zj[j] = fma(ap, row[p * kNodePts + j], Zj[j]);
+                    for (int r = 0; r < kPer; ++r) {
+                        const int q = r * kContractThreads + tid;
+                        if (q >= nc * kNodePts) break;
+                        const double *row = Sw + (q / kNodePts) * kNodePJ + q % kNodePts;
+#pragma unroll
+                        for (int p = 0; p < kNodeTDeg; ++p) {
+                            const double v = row[p * kNodePts];
+#pragma unroll
+                            for (int x = 0; x < kE; ++x) Z[r][x] = fma(A_s[w][el * kNodeTDeg + p][x], v, Z[r][x]);
+                        }
+                    }
+                }
             }
         }
+        __syncthreads();  // the other face's W has been read
 #pragma unroll
-        for (int i = 0; i < kNodePts; ++i) {
-            double v = 0.0;
+        for (int r = 0; r < kPer; ++r) {
+            const int q = r * kContractThreads + tid;
+            if (q >= nc * kNodePts) break;
 #pragma unroll
-            for (int j = 0; j < kNodePts; ++j) v = fma(Lm_s[i * kNodePts + j], Zj[j], v);
-            W[f][c][i] = v;
+            for (int x = 0; x < kE; ++x) Zs[x][q] = Z[r][x];
         }
-    }
-    __syncthreads();
-    const double mu = a.mu[e];
-    const double scale = 16.0 / 3.0 * kAlphaFs * kReCm2 / a.E_grid[e];
-    const int warp = tid >> 5, lane = tid & 31;
-    for (int d = warp; d < a.n_dir; d += kContractThreads / 32) {
-        const double nz = a.n_hat[3 * d + 2];
-        const int f = nz < 0.0 ? 0 : 1;
-        const double lam = mu / fmax(fabs(nz), 1.0e-12);
-        double acc = 0.0;
-        for (int c = lane; c < nc; c += 32) {
+        __syncthreads();
+        // W_ci = sum_j Lm[i][j] Z_cj, the cell's eight in place
 #pragma unroll
-            for (int i = 0; i < kNodePts; ++i) acc = fma(exp(-lam * nd_s[c * kNodePts + i]), W[f][c][i], acc);
+        for (int r = 0; r < kPer; ++r) {
+            const int q = r * kContractThreads + tid;
+            const int c8 = q / kNodePts * kNodePts, i = q % kNodePts;
+            if (q >= nc * kNodePts) break;
+#pragma unroll
+            for (int x = 0; x < kE; ++x) {
+                double v = 0.0;
+#pragma unroll
+                for (int j = 0; j < kNodePts; ++j) v = fma(Lm_s[i][j], Zs[x][c8 + j], v);
+                Z[r][x] = v;
+            }
         }
+        __syncthreads();
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0 && acc != 0.0) atomicAdd(&a.spec[(int64_t)d * a.n_E + e], scale * acc);
+        for (int r = 0; r < kPer; ++r) {
+            const int q = r * kContractThreads + tid;
+            if (q >= nc * kNodePts) break;
+#pragma unroll
+            for (int x = 0; x < kE; ++x) Zs[x][q] = Z[r][x];
+        }
+        __syncthreads();
+        const int warp = tid >> 5, lane = tid & 31;
+        for (int t = warp; t < a.n_dir * kE; t += kContractThreads / 32) {
+            const int d = t / kE, x = t - d * kE, e = e0 + x;
+            const double nz = a.n_hat[3 * d + 2];
+            if (e >= a.n_E || !(a.E_grid[e] > 0.0) || (nz < 0.0 ? 0 : 1) != f) continue;
+            const double lam = a.mu[e] / fmax(fabs(nz), 1.0e-12);
+            double acc = 0.0;
+            for (int q = lane; q < nc * kNodePts; q += 32) acc = fma(exp(-lam * h->node[q]), Zs[x][q], acc);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            const double scale = 16.0 / 3.0 * kAlphaFs * kReCm2 / a.E_grid[e];
+            if (lane == 0 && acc != 0.0) atomicAdd(&a.spec[(int64_t)d * a.n_E + e], scale * acc);
+        }
     }
 }
 
@@ -596,10 +874,12 @@ cudaError_t launch_brem_node(const pb_brem_args &a, cudaStream_t s, int sms, con
     int64_t *ix = reinterpret_cast<int64_t *>(w + l.idx);
     cudaError_t err = cudaMemsetAsync(w, 0, l.zero_bytes, s);
     if (err != cudaSuccess) return err;
-    brem_node_range_kernel<<<sms * 4, kNodeThreads, 0, s>>>(a, h);
-    brem_node_setup_kernel<<<1, kNodeThreads, 0, s>>>(a, h);
+    brem_node_range_kernel<<<sms * 4, kNodeThreads, 0, s>>>(a, h, l.n_win > 1);
+    brem_node_setup_kernel<<<1, kNodeThreads, 0, s>>>(a, h, l.n_win);
+    constexpr int kFitPer = 128 / kFitLanes;
     const int nq = a.n_E * a.n_el;
-    brem_node_fit_kernel<<<(nq + 127) / 128, 128, 0, s>>>(a, h, A);
+    brem_node_fit_kernel<<<dim3((nq + kFitPer - 1) / kFitPer, l.n_win), 128, 0, s>>>(a, h, A);
+    if (l.n_win > 1) brem_node_list_kernel<<<sms * 4, kNodeThreads, 0, s>>>(a, h, ix, l.cap);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     using Accum = void (*)(const pb_brem_args, BremNodeHdr *, double *, int64_t *, int64_t);
@@ -616,7 +896,7 @@ cudaError_t launch_brem_node(const pb_brem_args &a, cudaStream_t s, int sms, con
     if (err != cudaSuccess) return err;
     if (per_sm < 1) per_sm = 1;
     acc<<<sms * per_sm, kNodeThreads, smem, s>>>(a, h, S, ix, l.cap);
-    con<<<a.n_E, kContractThreads, 0, s>>>(a, h, A, S);
+    con<<<(a.n_E + kE - 1) / kE, kContractThreads, 0, s>>>(a, h, A, S);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     *hdr = h;

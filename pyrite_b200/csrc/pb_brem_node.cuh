@@ -15,6 +15,9 @@ constexpr int kNodeTDeg = 6;        // coefficients of the electron-energy polyn
 constexpr int kNodePJ = kNodeTDeg * kNodePts;  // moments per (element, face, cell)
 constexpr int kNodeMaxEl = 2;       // elements the shared accumulator holds
 constexpr double kNodeWindow = 1.1; // T_hi / T_lo of the energy window at most
+constexpr int kNodeMaxWin = 32;     // energy windows of a launch whose electrons slow down (a quarter octave each)
+constexpr int kNodeBins = 64;       // quarter octaves of the electron energy counted: 16 keV to 1 GeV
+constexpr int64_t kNodeWinSeg = (int64_t)1 << 22;  // longest segment list with windows (its index list: 32 MB)
 constexpr double kNodeTip = 2.5;    // T_lo >= 2.5 k_max: the window stays clear of the spectrum's tip
 constexpr int kNodeUniform = 5;     // cells of width h_min before the geometric growth
 constexpr double kNodeGrowth = 1.2;  // deeper cells: width a fifth of their start depth
@@ -27,30 +30,50 @@ struct BremNodeHdr {
     unsigned int ok;                 // the node form scores this launch
     unsigned int faces;              // bit 0: a direction leaves through the top face, bit 1: the bottom
     int n_cells;
-    int pad_;
+    int n_win;                       // windows of the launch (0: one window below the highest energy)
     double T_lo, T_hi, Tc, Th;       // electron-energy window [T_lo, T_hi], centre and half-width
     double h_min, z_g;               // uniform cell width and the depth where the growth starts
     double zb[kNodeMaxCells + 1];    // cell boundaries, depth below the exit face
     double node[kNodeMaxCells * kNodePts];
     double Lm[kNodePts * kNodePts];  // Lagrange basis of the cell nodes in monomials of t: [i][j]
+    unsigned long long n_rad;        // radiating segments
+    unsigned int hist[kNodeBins];    // radiating segments by quarter octave of T
+    int win_of[kNodeBins];           // window of a quarter octave, -1: none
+    double win_Tc[kNodeMaxWin], win_Th[kNodeMaxWin];  // a window's centre and half-width
+    unsigned int win_n[kNodeMaxWin];     // its segments
+    unsigned int win_fill[kNodeMaxWin];  // those listed so far
+    unsigned int win_bad[kNodeMaxWin];   // its fit missed: the per-pair form takes its segments
 };
+
+// Quarter octave of T (> 0) counted from 16 keV: the exponent and the two
+// leading bits of the fraction.
+__device__ __forceinline__ int node_bin(double T) {
+    return (int)((__double_as_longlong(T) >> 50) - (long long)(((1023 + 4) << 2)));
+}
+__device__ __forceinline__ double node_bin_lo(int q) {
+    return __longlong_as_double((long long)(((1023 + 4) << 2) + q) << 50);
+}
 
 // Byte offsets of the workspace parts.
 struct BremNodeLayout {
     size_t hdr, A, S, idx, total, zero_bytes;
-    int64_t cap;  // capacity of the left-out segment list
+    int64_t cap;  // capacity of the segment list
+    int n_win;    // windows the workspace holds
 };
 
 __host__ __device__ inline BremNodeLayout brem_node_layout(const pb_brem_args &a) {
     BremNodeLayout l;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    // With windows the list holds every segment (left out, then window by window).
+    const bool win = a.n_seg <= kNodeWinSeg;
+    l.n_win = win ? kNodeMaxWin : 1;
     l.hdr = 0;
-    l.A = up(sizeof(BremNodeHdr));
-    l.S = up(l.A + sizeof(double) * (size_t)a.n_E * (size_t)a.n_el * kNodeTDeg);
-    l.idx = up(l.S + sizeof(double) * (size_t)a.n_el * 2 * kNodeMaxCells * kNodePJ);
-    l.cap = a.n_seg / 8 + 4096;
+    l.S = up(sizeof(BremNodeHdr));
+    l.A = up(l.S + sizeof(double) * (size_t)l.n_win * (size_t)a.n_el * 2 * kNodeMaxCells * kNodePJ);
+    l.idx = up(l.A + sizeof(double) * (size_t)l.n_win * (size_t)a.n_E * (size_t)a.n_el * kNodeTDeg);
+    l.cap = win ? (a.n_seg > 4096 ? a.n_seg : 4096) : a.n_seg / 8 + 4096;
     l.total = l.idx + sizeof(int64_t) * (size_t)l.cap;
-    l.zero_bytes = l.idx;  // header, coefficients and moments
+    l.zero_bytes = l.A;  // header and moments
     return l;
 }
 

@@ -399,7 +399,13 @@ __global__ void __launch_bounds__(kBremPackedThreads, 3)
     const float T_slab = (float)a.thickness;
     const float mc2 = 510.99895f, inv_mc2 = 1.0f / 510.99895f;
     const float za = (float)(2.0 * kPi * kAlphaFs);
-    const int e0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    // The energy tile turns with the slice: blocks that share an SM (a grid of
+    // one wave deals them an SM count apart) take different tiles, whose work
+    // differs where the electrons lie among the photon energies. (Groups of 64
+    // energies dealt over the blocks even the blocks out, but their warps then
+    // wait for one another at each chunk: 340 -> 366 us.)
+    const int xt = (blockIdx.x + blockIdx.y / ((gridDim.y + gridDim.x - 1) / gridDim.x)) % gridDim.x;
+    const int e0 = 2 * (xt * blockDim.x + threadIdx.x);
     const bool on_a = e0 < a.n_E, on_b = e0 + 1 < a.n_E;
     // per-energy constants, packed (energy e0 low, e0 + 1 high)
     double kd[2], mud[2];
@@ -451,12 +457,19 @@ __global__ void __launch_bounds__(kBremPackedThreads, 3)
         live = (int64_t)nh->n_out;
         sidx = nidx;
     }
+    // A contiguous slice of the segments per block. A list ordered by energy is
+    // dealt out in chunks instead: the electrons below a photon energy cost
+    // nothing, and each block should have its share of them.
+    const bool dealt = sidx != nullptr && nh->n_win > 0;
     const int64_t per = (live + gridDim.y - 1) / gridDim.y;
-    const int64_t s_begin = per * blockIdx.y;
-    int64_t s_end = s_begin + per < live ? s_begin + per : live;
+    const int64_t rounds = (per + kBremChunk - 1) / kBremChunk;
+    const int64_t chunk = dealt ? (per + rounds - 1) / (rounds > 0 ? rounds : 1) : kBremChunk;
+    const int64_t s_begin = (dealt ? chunk : per) * blockIdx.y;
+    const int64_t s_step = dealt ? chunk * gridDim.y : chunk;
+    int64_t s_end = dealt || s_begin + per > live ? live : s_begin + per;
     if (s_end < s_begin) s_end = s_begin;
-    for (int64_t c0s = s_begin; c0s < s_end; c0s += kBremChunk) {
-        const int nc = (int)((s_end - c0s) < kBremChunk ? (s_end - c0s) : kBremChunk);
+    for (int64_t c0s = s_begin; c0s < s_end; c0s += s_step) {
+        const int nc = (int)((s_end - c0s) < chunk ? (s_end - c0s) : chunk);
         __syncthreads();
         float tlo = 3.4e38f, thi = -3.4e38f, nmax = 0.0f;
         for (int j = threadIdx.x; j < nc; j += blockDim.x) {
@@ -504,6 +517,8 @@ __global__ void __launch_bounds__(kBremPackedThreads, 3)
         }
         __syncthreads();
         if (!on_a) continue;
+        // every electron below both photon energies
+        if (!(act_a && thi - f2lo(k2) > 1e-6f) && !(act_b && thi - f2hi(k2) > 1e-6f)) continue;
         // The chunk's electrons span [tlo, thi]. Where that range is narrow
         // (at most 10 % of tlo) and clear of the spectrum's tip, J_el(T) of
         // this thread's two energies is the cubic through four Chebyshev

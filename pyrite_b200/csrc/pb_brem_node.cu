@@ -96,7 +96,7 @@ __device__ __forceinline__ int node_cell(const double *zb, int n, double h_min, 
 
 // Extent of the launch: the largest and smallest electron energy of the
 // radiating segments and, for a list with windows, their count and their
-// histogram over quarter octaves. One atomic a block for each extreme: a
+// histogram over sixteenths of an octave. One atomic a block for each extreme: a
 // warp's atomic each on the two addresses took most of this kernel (200,000
 // segments, with the histogram: 8.1 -> 5.2 us).
 __global__ void __launch_bounds__(kNodeThreads) brem_node_range_kernel(const pb_brem_args a, BremNodeHdr *h,
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kNodeThreads) brem_node_range_kernel(const pb_
     __shared__ unsigned long long red[2][kNodeThreads / 32];
     __shared__ unsigned int n_rad;
     const int tid = threadIdx.x;
-    if (tid < kNodeBins) hist[tid] = 0u;
+    for (int q = tid; q < kNodeBins; q += blockDim.x) hist[q] = 0u;
     if (tid == 0) n_rad = 0u;
     __syncthreads();
     const int64_t live = node_live(a);
@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(kNodeThreads) brem_node_range_kernel(const pb_
         }
         if (n_rad) atomicAdd(&h->n_rad, (unsigned long long)n_rad);
     }
-    if (count && tid < kNodeBins && hist[tid]) atomicAdd(&h->hist[tid], hist[tid]);
+    for (int q = tid; count && q < kNodeBins; q += blockDim.x)
+        if (hist[q]) atomicAdd(&h->hist[q], hist[q]);
 }
 
 // T_m(t) of the Lagrange basis in monomials: T_{m+1} = 2 t T_m - T_{m-1}.
@@ -186,8 +187,9 @@ __constant__ const ChebMonomials kCheb = cheb_monomials();
 // priced at n_E evaluations of the per-pair form and as much again for its
 // place in the list: above kNodePairWork the quarter octaves clear of the
 // spectrum's tip become one window each. 200,000 electrons of 8 keV to 10 MeV
-// on 2,048 energies, 59 % of them in 24 windows: per-pair form 958 -> 490 us;
-// fit, list, moments and contraction of the windows 143 us, against 141 us for
+// on 2,048 energies, 59 % of them in 24 windows: per-pair form 958 -> 490 us
+// (340 on the ordered list); fit, list, moments and contraction of the windows
+// 145 us, against 141 us for
 // a list of nearly every segment that the one window then gave up. At 300
 // energies a list of 40,000 takes 324 us through the entry point, 436 before;
 // below the line the two are within 10 us.
@@ -253,16 +255,19 @@ __global__ void __launch_bounds__(kNodeThreads) brem_node_setup_kernel(const pb_
     if (ok && tid <= n) h->zb[tid] = tid < n ? zb : T_slab;
     int n_win = 0;
     if (warp == 0) {
-        // two bins a lane, upwards in energy
+        // two quarter octaves a lane, upwards in energy
         unsigned int below = 0u, in_bins = 0u;
         unsigned int c[2];
         unsigned int use[2];
         for (int k = 0; k < 2; ++k) {
             const int q = lane + 32 * k;
-            c[k] = h->hist[q];
+            c[k] = 0u;
+            for (int t = 4 * q; t < 4 * q + 4; ++t) {
+                c[k] += h->hist[t];
+                if (node_bin_lo(t + 1) <= T_lo) below += h->hist[t];
+            }
             in_bins += c[k];
-            if (node_bin_lo(q + 1) <= T_lo) below += c[k];
-            use[k] = __ballot_sync(0xffffffffu, c[k] > 0u && node_bin_lo(q) >= kNodeTip * kmax);
+            use[k] = __ballot_sync(0xffffffffu, c[k] > 0u && node_bin_lo(4 * q) >= kNodeTip * kmax);
         }
         below = __reduce_add_sync(0xffffffffu, below);
         in_bins = __reduce_add_sync(0xffffffffu, in_bins);
@@ -275,7 +280,7 @@ __global__ void __launch_bounds__(kNodeThreads) brem_node_setup_kernel(const pb_
             const bool on = ((use[k] >> lane) & 1u) && w < n_win;
             h->win_of[q] = on ? w : -1;
             if (on) {
-                const double lo = node_bin_lo(q), hi = node_bin_lo(q + 1);
+                const double lo = node_bin_lo(4 * q), hi = node_bin_lo(4 * q + 4);
                 h->win_Tc[w] = 0.5 * (lo + hi);
                 h->win_Th[w] = 0.5 * (hi - lo);
                 h->win_n[w] = c[k];
@@ -377,56 +382,79 @@ __device__ __forceinline__ void node_window_offsets(const BremNodeHdr *h, int n_
     off = (int64_t)(h->n_rad - all + incl - n);
 }
 
-// Segment list by window: each block counts a tile's segments per window in
-// shared memory, reserves their places with one atomic a window and writes them.
+// Segment list by window, the left-out part by sixteenths of an octave (its
+// chunks then span little energy, which the per-pair kernel's cubic and its
+// test against the photon energy need: 490 -> 340 us for 82,000 electrons of 8 to
+// 160 keV on 2,048 energies to 60 keV): each block counts a tile's segments per
+// place in shared memory, reserves them with one atomic a place and writes them.
 constexpr int kListPer = 4;  // segments per thread and tile
+constexpr int kListPlaces = kNodeBins + 1 + kNodeMaxWin;  // bins, outside of them, windows
 __global__ void __launch_bounds__(kNodeThreads) brem_node_list_kernel(const pb_brem_args a, BremNodeHdr *h,
                                                                       int64_t *idx, int64_t cap) {
-    __shared__ unsigned int cnt[kNodeMaxWin + 1];
-    __shared__ unsigned long long base[kNodeMaxWin + 1];
-    __shared__ int64_t off_s[kNodeMaxWin + 1];
-    __shared__ int win_s[kNodeBins];
-    const int tid = threadIdx.x;
+    static_assert(kNodeThreads == kNodeBins, "a bin a thread in the scan");
+    __shared__ unsigned int cnt[kListPlaces];
+    __shared__ int64_t base[kListPlaces];
+    __shared__ int64_t off_s[kListPlaces];
+    __shared__ int win_s[kNodeQuarters];
+    __shared__ unsigned int sum_s[kNodeThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n_win = h->n_win;
     if (!h->ok || n_win == 0) return;
-    if (tid < 32) {
-        int64_t off;
-        unsigned int n;
-        node_window_offsets(h, n_win, tid, off, n);
-        off_s[tid + 1] = off;
-        if (tid == 0) off_s[0] = 0;
-    }
-    if (tid < kNodeBins) {
+    if (tid < kNodeQuarters) {
         const int w = h->win_of[tid];
         win_s[tid] = w >= 0 && !h->win_bad[w] ? w : -1;
+    }
+    __syncthreads();
+    {
+        const unsigned int n = win_s[tid >> 2] < 0 ? h->hist[tid] : 0u;
+        unsigned int incl = n;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) sum_s[warp] = incl;
+        __syncthreads();
+        for (int w = 0; w < warp; ++w) incl += sum_s[w];
+        off_s[tid] = incl - n;
+        // outside the bins: after them; the windows follow
+        if (tid == kNodeThreads - 1) off_s[kNodeBins] = incl;
+    }
+    if (warp == 0) {
+        int64_t off;
+        unsigned int n;
+        node_window_offsets(h, n_win, lane, off, n);
+        off_s[kNodeBins + 1 + lane] = off;
+        if (blockIdx.x == 0 && lane == 0) h->n_out = (unsigned long long)off;  // window 0 starts behind the left-out ones
     }
     const int64_t live = node_live(a);
     constexpr int kTile = kNodeThreads * kListPer;
     for (int64_t t0 = blockIdx.x * (int64_t)kTile; t0 < live; t0 += gridDim.x * (int64_t)kTile) {
-        if (tid <= kNodeMaxWin) cnt[tid] = 0u;
+        for (int q = tid; q < kListPlaces; q += blockDim.x) cnt[q] = 0u;
         __syncthreads();
-        int slot[kListPer];  // 0: left out, w + 1: window w, -1: no part
+        int place[kListPer];
         unsigned int rank[kListPer];
 #pragma unroll
         for (int k = 0; k < kListPer; ++k) {
             const int64_t s = t0 + k * kNodeThreads + tid;
-            slot[k] = -1;
+            place[k] = -1;
+            rank[k] = 0u;
             if (s < live && node_radiates(a, s)) {
                 const double T = a.E_keV[s];
                 const int q = T > 0.0 && T < 1e300 ? node_bin(T) : -1;
-                slot[k] = q >= 0 && q < kNodeBins ? win_s[q] + 1 : 0;
-                rank[k] = atomicAdd(&cnt[slot[k]], 1u);
+                place[k] = kNodeBins;
+                if (q >= 0 && q < kNodeBins) place[k] = win_s[q >> 2] >= 0 ? kNodeBins + 1 + win_s[q >> 2] : q;
+                rank[k] = atomicAdd(&cnt[place[k]], 1u);
             }
         }
         __syncthreads();
-        if (tid <= kNodeMaxWin && cnt[tid])
-            base[tid] = tid == 0 ? atomicAdd(&h->n_out, (unsigned long long)cnt[0])
-                                 : (unsigned long long)atomicAdd(&h->win_fill[tid - 1], cnt[tid]);
+        for (int q = tid; q < kListPlaces; q += blockDim.x)
+            if (cnt[q])
+                base[q] = off_s[q] + atomicAdd(q <= kNodeBins ? &h->fill[q] : &h->win_fill[q - kNodeBins - 1], cnt[q]);
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < kListPer; ++k) {
-            if (slot[k] < 0) continue;
-            const int64_t at = off_s[slot[k]] + (int64_t)base[slot[k]] + rank[k];
+            if (place[k] < 0) continue;
+            const int64_t at = base[place[k]] + rank[k];
             if (at < cap) idx[at] = t0 + k * kNodeThreads + tid;
         }
     }

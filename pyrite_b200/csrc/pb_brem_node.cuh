@@ -16,7 +16,8 @@ constexpr int kNodePJ = kNodeTDeg * kNodePts;  // moments per (element, face, ce
 constexpr int kNodeMaxEl = 2;       // elements the shared accumulator holds
 constexpr double kNodeWindow = 1.1; // T_hi / T_lo of the energy window at most
 constexpr int kNodeMaxWin = 32;     // energy windows of a launch whose electrons slow down (a quarter octave each)
-constexpr int kNodeBins = 64;       // quarter octaves of the electron energy counted: 16 keV to 1 GeV
+constexpr int kNodeBins = 256;      // sixteenths of an octave of the electron energy counted: 4 keV to 262 MeV
+constexpr int kNodeQuarters = kNodeBins / 4;
 constexpr int64_t kNodeWinSeg = (int64_t)1 << 22;  // longest segment list with windows (its index list: 32 MB)
 constexpr double kNodeTip = 2.5;    // T_lo >= 2.5 k_max: the window stays clear of the spectrum's tip
 constexpr int kNodeUniform = 5;     // cells of width h_min before the geometric growth
@@ -37,21 +38,22 @@ struct BremNodeHdr {
     double node[kNodeMaxCells * kNodePts];
     double Lm[kNodePts * kNodePts];  // Lagrange basis of the cell nodes in monomials of t: [i][j]
     unsigned long long n_rad;        // radiating segments
-    unsigned int hist[kNodeBins];    // radiating segments by quarter octave of T
-    int win_of[kNodeBins];           // window of a quarter octave, -1: none
+    unsigned int hist[kNodeBins];    // radiating segments by sixteenth of an octave of T
+    unsigned int fill[kNodeBins + 1];    // those listed so far where the bin has no window (the last: outside the bins)
+    int win_of[kNodeQuarters];       // window of a quarter octave, -1: none
     double win_Tc[kNodeMaxWin], win_Th[kNodeMaxWin];  // a window's centre and half-width
     unsigned int win_n[kNodeMaxWin];     // its segments
     unsigned int win_fill[kNodeMaxWin];  // those listed so far
     unsigned int win_bad[kNodeMaxWin];   // its fit missed: the per-pair form takes its segments
 };
 
-// Quarter octave of T (> 0) counted from 16 keV: the exponent and the two
-// leading bits of the fraction.
+// Sixteenth of an octave of T (> 0) counted from 4 keV: the exponent and the
+// four leading bits of the fraction.
 __device__ __forceinline__ int node_bin(double T) {
-    return (int)((__double_as_longlong(T) >> 50) - (long long)(((1023 + 4) << 2)));
+    return (int)((__double_as_longlong(T) >> 48) - (long long)((1023 + 2) << 4));
 }
 __device__ __forceinline__ double node_bin_lo(int q) {
-    return __longlong_as_double((long long)(((1023 + 4) << 2) + q) << 50);
+    return __longlong_as_double((long long)(((1023 + 2) << 4) + q) << 48);
 }
 
 // Byte offsets of the workspace parts.

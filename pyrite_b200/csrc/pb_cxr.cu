@@ -14,16 +14,16 @@
 //    bins within ``exact_widths`` sinc widths of its centre (FP64 sine
 //    integral), and its far field -- the cycle-averaged envelope
 //    1/(2 a^2 (E_lo - E_r)(E_hi - E_r)) -- is carried by three moments per
-//    centre bin in shared memory and spread onto the grid by one finalize
-//    pass (cxr/_bin_quadrature.py:280-560 for the exact and far forms).
+//    centre bin in global memory and spread onto the grid by one convolution
+//    (cxr/_bin_quadrature.py:280-560 for the exact and far forms).
 //    Lines never leave the SM: warp work -> shared-memory spectrum -> one
 //    global atomic per bin per block.
 //  * node sampling: kept lines are appended to a line buffer and reduced
 //    against the grid nodes by a separate kernel (cxr/_cpu_reduce.py:26-50).
 //
-// PB_FP64 evaluates the chain in double; PB_MIXED in float, with the line
-// phase a (E - E_r) formed and range-reduced in double and every
-// accumulation in double.
+// PB_FP64 evaluates the chain and the bins in double; PB_MIXED in float, with
+// the node phase a (E - E_r) formed and range-reduced in double and every
+// spectrum sum in double.
 #include <algorithm>
 #include <climits>
 #include <type_traits>
@@ -52,9 +52,12 @@ template <class Real>
 constexpr int row_chunk() { return sizeof(Real) == 4 ? 120 : 48; }
 template <class Real>
 constexpr int pair_queue() { return kSegTile * row_chunk<Real>(); }  // every pair of a pass may keep a line
-// Kept lines wait here until a whole round of kCxrThreads is there.
+// The prefilter's survivors and the kept lines wait until a whole round of
+// kCxrThreads is there.
 template <class Real>
-constexpr int line_queue() { return pair_queue<Real>() + kCxrThreads; }
+constexpr int surv_queue() { return pair_queue<Real>() + kCxrThreads; }
+template <class Real>
+constexpr int line_queue() { return surv_queue<Real>() + kCxrThreads; }
 constexpr int kStripBins = 31;  // bins a warp owns in the whole-axis phase (32 edges)
 // Window lines collected before the window phase runs; one more round of
 // kCxrThreads lines always fits.
@@ -994,14 +997,17 @@ __device__ __forceinline__ void line_moments(double E_r, double inv_a, double w,
     atomicAdd(&mom[3 * slot + 2], m * dd * dd);
 }
 
-// Persistent blocks over the flattened (direction, segment tile) work, in
-// contiguous ranges, so the grid is an exact multiple of the SM count; a
+// Persistent blocks over the flattened (direction, row chunk, segment tile) work,
+// in contiguous ranges, so the grid is an exact multiple of the SM count; a
 // block flushes its on-chip spectrum whenever its direction changes.
 // Per pass (a segment tile x a chunk of reflection rows):
 //   A0  a cheap prefilter drops pairs whose resonance cannot reach the keep
-//       window and compacts the survivors into a shared queue (warp ballot);
-//   A1  the full chain runs densely over the survivors and pushes kept lines
-//       onto a second shared queue;
+//       window and compacts the survivors into a shared queue (warp ballots);
+//   A1  the full chain runs over the survivors in whole rounds of one per thread
+//       (the rest waits for the next tile's; its own tile stays staged until
+//       then) and pushes kept lines onto a second shared queue. (Rounds of each
+//       tile alone: 2.27 -> 2.14 ms for 14,500 segments, 16 directions, 238 rows
+//       with two-width windows, 78.2 -> 75.9 for 8,192 histories with 64.)
 //   B1  lines leave the queue in whole rounds of one per thread (the rest
 //       waits for the next pass): the owner thread adds the line's far-field
 //       moments and the bins within K_far of its centre, and passes lines
@@ -1025,14 +1031,15 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
     if (a.n_seg_device) n_seg = (int64_t)*a.n_seg_device;
     if (n_seg > a.n_seg && a.n_seg > 0) n_seg = a.n_seg;
 
-    // Shared layout: [rows][segs][queues][tables][spec][moments][float spec]
+    // Shared layout: [rows][segs][queues][tables][spec][float edges][escape pieces]
     unsigned char *cur = smem_raw;
     RowPre<Real> *rows = reinterpret_cast<RowPre<Real> *>(cur);
     constexpr int kRowChunk = row_chunk<Real>();
-    constexpr int kQueue = pair_queue<Real>();
+    constexpr int kQueue = surv_queue<Real>();
+    constexpr int kPairs = pair_queue<Real>();
     cur += sizeof(RowPre<Real>) * kRowChunk;
     SegPre<Real> *segs = reinterpret_cast<SegPre<Real> *>(cur);
-    cur += sizeof(SegPre<Real>) * kSegTile;
+    cur += sizeof(SegPre<Real>) * 2 * kSegTile;  // this tile and the last one
     cur = (unsigned char *)(((uintptr_t)cur + 15) & ~(uintptr_t)15);
     constexpr int kLineQueue = line_queue<Real>();
     Real *qE = reinterpret_cast<Real *>(cur);
@@ -1060,7 +1067,7 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
     unsigned char *esc_raw = reinterpret_cast<unsigned char *>(edges_f + (binmean && kMixed ? n_E + 1 : 0));
     esc_raw = (unsigned char *)(((uintptr_t)esc_raw + 15) & ~(uintptr_t)15);
     EscSeg<Real> *esc = reinterpret_cast<EscSeg<Real> *>(esc_raw);
-    double *lay_zt = reinterpret_cast<double *>(esc + (kLayered ? kSegTile : 0));
+    double *lay_zt = reinterpret_cast<double *>(esc + (kLayered ? 2 * kSegTile : 0));
     double *lay_zb = lay_zt + (kLayered ? kMaxEscLayers : 0);
     Real *lay_t = reinterpret_cast<Real *>(lay_zb + (kLayered ? kMaxEscLayers : 0));
     int &q_count = scratch[40];
@@ -1387,6 +1394,62 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
     // segment list still reaches every SM (a tile below four segments leaves
     // most threads of a pass idle).
     int64_t d_ch = -1, win = -1;
+    // The staged chunk's rows, the two staged tiles (tile ``par`` is the newer), and
+    // the survivors that wait for the next tile's.
+    int ng = 1, par = 0, n_wait = 0, g0 = 0, n_pairs = 0;
+    unsigned ng_magic = 0;
+    int64_t s0_of[2] = {0, 0};
+    // q / ng for the pass's pair ids q < kSegTile * ng by a multiply-high:
+    // magic = floor((2^32 - 1) / ng) + 1 is at least 2^32 / ng and
+    // exceeds it by under one, so q magic / 2^32 lies in
+    // [q / ng, q / ng + q / 2^32) and its floor is exact for q < 2^32 / ng
+    // (one row: magic does not fit 32 bits, and the quotient is q).
+    const auto seg_of = [&](int q) { return ng == 1 ? q : (int)__umulhi((unsigned)q, ng_magic); };
+    // A1: the full chain of pair ``id`` (tile parity x kPairs + pair of the tile;
+    // -1: none), by this thread. All threads call it.
+    const auto chain = [&](int id, int d) {
+        Line<Real> ln;
+        ln.good = false;
+        if (id >= 0) {
+            const int t = id >= kPairs ? 1 : 0;
+            const int q = id - t * kPairs;
+            const int si = seg_of(q);
+            const int gi = q - si * ng;
+            ln = pair_line<Real, kLayered>(segs[t * kSegTile + si], rows[gi], E_tab, delta_tab, log_mu, n_tab, n_mu,
+                                           a.tables, ti, esc + t * kSegTile + si, a, lay_t);
+            if (pairs_out) {
+                const int64_t o = ((int64_t)d * n_seg + s0_of[t] + si) * n_g + g0 + gi * n_chunks;
+                a.pair_E[o] = (double)ln.E_res;
+                a.pair_a[o] = (double)ln.a_width;
+                a.pair_w[o] = (double)ln.weight;
+                a.pair_good[o] = ln.good ? 1 : 0;
+            }
+            if (ln.good && lines_out) {
+                const unsigned long long slot = atomicAdd(a.line_count, 1ULL);
+                if (slot < (unsigned long long)a.line_capacity) {
+                    a.line_E[slot] = (double)ln.E_res;
+                    a.line_a[slot] = (double)ln.a_width;
+                    a.line_w[slot] = (double)ln.weight;
+                    a.line_dir[slot] = d;
+                    if (a.line_seg) a.line_seg[slot] = s0_of[t] + si;
+                } else {
+                    set_status(a.status, PB_DEV_QUEUE_OVERFLOW);
+                }
+            }
+        }
+        if (binmean) {
+            const unsigned mask = __ballot_sync(0xffffffffu, ln.good);
+            int base = 0;
+            if (lane == 0 && mask) base = atomicAdd(&q_count, __popc(mask));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (ln.good) {
+                const int kk = base + __popc(mask & ((1u << lane) - 1u));
+                qE[kk] = ln.E_res;
+                qA[kk] = ln.a_width;
+                qW[kk] = ln.weight;
+            }
+        }
+    };
     // Tiles without a radiating segment are passed over a window of kCxrThreads
     // segments at a time: one flag word per warp, a tile is 4, 8 or 16 of its bits.
     unsigned *const rad_words = reinterpret_cast<unsigned *>(scratch);
@@ -1417,7 +1480,24 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
         // the direction changes or the block ends.
         const bool leave = end || d != d_cur;
         __syncthreads();
-        if (tid == 0) p_count = 0;
+        // A1 over whole rounds of the last tile's survivors (every pair without the
+        // prefilter), oldest first. The rest waits for the next tile's, but not beyond
+        // it (its segments are staged until then), and not for other rows.
+        {
+            const int n_surv = dtail != nullptr ? p_count : n_pairs;
+            const bool all = dtail == nullptr || end || dc != d_ch;
+            int done = 0;
+            while (n_surv - done >= kCxrThreads || (done < n_surv && (all || (done == 0 && n_wait > 0)))) {
+                const int k = done + tid;
+                chain(k < n_surv ? (dtail != nullptr ? (int)pq[k] : par * kPairs + k) : -1, d_cur);
+                done = min(done + kCxrThreads, n_surv);
+            }
+            n_wait = n_surv - done;
+            const uint16_t w = tid < n_wait ? pq[done + tid] : (uint16_t)0;
+            __syncthreads();
+            if (tid < n_wait) pq[tid] = w;
+            if (tid == 0) p_count = n_wait;
+        }
         if (binmean && d_cur >= 0) {
             deposit(leave);
             if (leave) publish(d_cur);
@@ -1427,21 +1507,20 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
         const double *nh = a.n_hat + 3 * d;
         const int64_t s0 = tile * seg_tile;
         const int nst = (int)((n_seg - s0) < seg_tile ? (n_seg - s0) : seg_tile);
+        par ^= 1;
+        s0_of[par] = s0;
         __syncthreads();  // before the staged rows and segments are replaced
-        if (tid < nst) seg_precompute<Real>(segs[tid], a, s0 + tid, nh);
+        SegPre<Real> *const seg_t = segs + par * kSegTile;
+        if (tid < nst) seg_precompute<Real>(seg_t[tid], a, s0 + tid, nh);
         if constexpr (kLayered) {
-            if (tid < nst) esc_precompute<Real>(esc[tid], a, s0 + tid, nh, lay_zt, lay_zb);
+            if (tid < nst) esc_precompute<Real>(esc[par * kSegTile + tid], a, s0 + tid, nh, lay_zt, lay_zb);
         }
         {
-            const int g0 = (int)dc - d * n_chunks;
-            const int ng = (n_g - g0 + n_chunks - 1) / n_chunks;
-            // q / ng for the pass's pair ids q < kSegTile * ng by a multiply-high:
-            // magic = floor((2^32 - 1) / ng) + 1 is at least 2^32 / ng and
-            // exceeds it by under one, so q magic / 2^32 lies in
-            // [q / ng, q / ng + q / 2^32) and its floor is exact for q < 2^32 / ng
-            // (one row: magic does not fit 32 bits, and the quotient is q).
-            const unsigned ng_magic = (unsigned)(0xFFFFFFFFull / (unsigned)ng) + 1u;
-            const auto seg_of = [&](int q) { return ng == 1 ? q : (int)__umulhi((unsigned)q, ng_magic); };
+            if (dc != d_ch) {
+                g0 = (int)dc - d * n_chunks;
+                ng = (n_g - g0 + n_chunks - 1) / n_chunks;
+                ng_magic = (unsigned)(0xFFFFFFFFull / (unsigned)ng) + 1u;
+            }
             for (int j = tid; j < (dc != d_ch ? ng : 0); j += blockDim.x) {
                 const int g = g0 + j * n_chunks;
                 RowPre<Real> &r = rows[j];
@@ -1463,87 +1542,36 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
             d_ch = dc;
             __syncthreads();
             // ---- A0: prefilter and compact the surviving pairs ----
-            const int n_pairs = nst * ng;
-            int n_surv;
-            if (dtail != nullptr) {
-                // Lane ``it`` keeps the survivors' mask of the warp's iteration
-                // ``it`` (at most pair_queue / kCxrThreads = 8 of them): one
-                // shared counter update a warp and pass.
-                const int n_it0 = (n_pairs + (int)blockDim.x - 1) / (int)blockDim.x;
-                unsigned mine = 0;
-                for (int it = 0; it < n_it0; ++it) {
-                    const int q = it * blockDim.x + tid;
-                    bool ok = false;
-                    if (q < n_pairs) {
-                        const int si = seg_of(q);
-                        ok = pair_may_keep<Real>(segs[si], rows[q - si * ng], E_tab, dtail, n_tab, a.tables, ti);
-                    }
-                    const unsigned mask = __ballot_sync(0xffffffffu, ok);
-                    if ((int)lane == it) mine = mask;
-                }
-                int incl = __popc(mine);
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if ((int)lane >= o) incl += v;
-                }
-                int base = 0;
-                if (lane == 31 && incl) base = atomicAdd(&p_count, incl);
-                base = __shfl_sync(0xffffffffu, base, 31) + incl - __popc(mine);  // of iteration ``lane``
-                for (int it = 0; it < n_it0; ++it) {
-                    const unsigned mask = __shfl_sync(0xffffffffu, mine, it);
-                    const int at = __shfl_sync(0xffffffffu, base, it);
-                    if ((mask >> lane) & 1u)
-                        pq[at + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)(it * blockDim.x + tid);
-                }
-                __syncthreads();
-                n_surv = p_count;
-            } else {
-                n_surv = n_pairs;
-            }
-            // ---- A1: the full chain over the survivors ----
-            const int n_it1 = (n_surv + (int)blockDim.x - 1) / (int)blockDim.x;
-            for (int it = 0; it < n_it1; ++it) {
-                const int k = it * blockDim.x + tid;
-                Line<Real> ln;
-                ln.good = false;
-                if (k < n_surv) {
-                    const int q = dtail != nullptr ? (int)pq[k] : k;
+            n_pairs = nst * ng;
+            if (dtail == nullptr) continue;
+            // Lane ``it`` keeps the survivors' mask of the warp's iteration
+            // ``it`` (at most pair_queue / kCxrThreads = 8 of them): one
+            // shared counter update a warp and pass.
+            const int n_it0 = (n_pairs + (int)blockDim.x - 1) / (int)blockDim.x;
+            unsigned mine = 0;
+            for (int it = 0; it < n_it0; ++it) {
+                const int q = it * blockDim.x + tid;
+                bool ok = false;
+                if (q < n_pairs) {
                     const int si = seg_of(q);
-                    const int gi = q - si * ng;
-                    ln = pair_line<Real, kLayered>(segs[si], rows[gi], E_tab, delta_tab, log_mu, n_tab, n_mu,
-                                                   a.tables, ti, esc + si, a, lay_t);
-                    if (pairs_out) {
-                        const int64_t o = ((int64_t)d * n_seg + s0 + si) * n_g + g0 + gi * n_chunks;
-                        a.pair_E[o] = (double)ln.E_res;
-                        a.pair_a[o] = (double)ln.a_width;
-                        a.pair_w[o] = (double)ln.weight;
-                        a.pair_good[o] = ln.good ? 1 : 0;
-                    }
-                    if (ln.good && lines_out) {
-                        const unsigned long long slot = atomicAdd(a.line_count, 1ULL);
-                        if (slot < (unsigned long long)a.line_capacity) {
-                            a.line_E[slot] = (double)ln.E_res;
-                            a.line_a[slot] = (double)ln.a_width;
-                            a.line_w[slot] = (double)ln.weight;
-                            a.line_dir[slot] = d;
-                            if (a.line_seg) a.line_seg[slot] = s0 + si;
-                        } else {
-                            set_status(a.status, PB_DEV_QUEUE_OVERFLOW);
-                        }
-                    }
+                    ok = pair_may_keep<Real>(seg_t[si], rows[q - si * ng], E_tab, dtail, n_tab, a.tables, ti);
                 }
-                if (binmean) {
-                    const unsigned mask = __ballot_sync(0xffffffffu, ln.good);
-                    int base = 0;
-                    if (lane == 0 && mask) base = atomicAdd(&q_count, __popc(mask));
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    if (ln.good) {
-                        const int kk = base + __popc(mask & ((1u << lane) - 1u));
-                        qE[kk] = ln.E_res;
-                        qA[kk] = ln.a_width;
-                        qW[kk] = ln.weight;
-                    }
-                }
+                const unsigned mask = __ballot_sync(0xffffffffu, ok);
+                if ((int)lane == it) mine = mask;
+            }
+            int incl = __popc(mine);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)lane >= o) incl += v;
+            }
+            int base = 0;
+            if (lane == 31 && incl) base = atomicAdd(&p_count, incl);
+            base = __shfl_sync(0xffffffffu, base, 31) + incl - __popc(mine);  // of iteration ``lane``
+            for (int it = 0; it < n_it0; ++it) {
+                const unsigned mask = __shfl_sync(0xffffffffu, mine, it);
+                const int at = __shfl_sync(0xffffffffu, base, it);
+                if ((mask >> lane) & 1u)
+                    pq[at + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)(par * kPairs + it * blockDim.x + tid);
             }
         }
     }
@@ -1739,8 +1767,8 @@ __global__ void __launch_bounds__(kNodeTile) node_reduce_kernel(const double *E_
 template <class Real>
 static size_t cxr_smem_bytes(const pb_cxr_args &a, int far_pad, bool with_moments) {
     constexpr int kRowChunk = row_chunk<Real>();
-    constexpr int kQueue = pair_queue<Real>();
-    size_t b = sizeof(RowPre<Real>) * kRowChunk + sizeof(SegPre<Real>) * kSegTile + 16;
+    constexpr int kQueue = surv_queue<Real>();
+    size_t b = sizeof(RowPre<Real>) * kRowChunk + sizeof(SegPre<Real>) * 2 * kSegTile + 16;
     b += sizeof(Real) * 3 * line_queue<Real>() + 16 +
          (sizeof(WinLine<Real>) + sizeof(uint16_t) * (kWinClasses / 2)) * kWideCap + sizeof(int) * 64 +
          sizeof(uint16_t) * kQueue + 16;
@@ -1749,7 +1777,7 @@ static size_t cxr_smem_bytes(const pb_cxr_args &a, int far_pad, bool with_moment
     if (a.quadrature == PB_QUAD_BINMEAN)
         b += sizeof(double) * (size_t)a.n_E + (sizeof(Real) == 4 ? sizeof(float) * ((size_t)a.n_E + 1) : 0);
     if (a.n_layer > 0)
-        b += 16 + sizeof(EscSeg<Real>) * kSegTile + sizeof(double) * 2 * kMaxEscLayers + sizeof(Real) * kMaxEscLayers;
+        b += 16 + sizeof(EscSeg<Real>) * 2 * kSegTile + sizeof(double) * 2 * kMaxEscLayers + sizeof(Real) * kMaxEscLayers;
     return b;
 }
 

@@ -172,3 +172,39 @@ def test_far_field_at_the_edges_of_its_chunks(n_E, precision, cuda_device):
     else:
         # 320 lines at most: between the single line's 3e-2 and the 2e-3 of many
         assert np.sum(np.abs(got - ref)) <= 3e-2 * np.sum(np.abs(ref))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n_seg,n_g", [(16, 119), (17, 48), (100, 121), (33, 145), (900, 60)])
+def test_waiting_survivors_over_tiles_rows_and_directions(n_seg, n_g, precision, cuda_device):
+    """Pairs that pass the prefilter wait for a whole round over tiles, but not
+    over a change of rows or direction: three directions in one call are the
+    three single calls, and those the sums over single segments (FP64 sums in
+    another order; float partial sums within 1e-6 of the peak)."""
+    from pyrite_b200 import mc_cxr_spectrum
+    from pyrite_b200.tables import SILICON, diamond_hkls, reflection_rows
+
+    E_grid = np.linspace(1000.0, 60000.0, 200)
+    seg, _, tables, n_hat = _scene(n_seg, n_g, E_grid, 1.5e5, n_seg + n_g)
+    n_hats = np.stack([n_hat, n_hat + [0.02, 0.0, 0.0], n_hat + [0.0, 0.03, 0.0]])
+    n_hats /= np.linalg.norm(n_hats, axis=1, keepdims=True)
+    hkl = [h for h in diamond_hkls(9.0) if np.dot(h, (1, 1, 0)) > 0]
+    hkl = hkl[:: max(1, len(hkl) // n_g)][:n_g]  # those of the scene
+    rows = reflection_rows(SILICON, hkl, n_hats, surface_hkl=(2, 2, 0))
+    kw = dict(tables=tables, line_quadrature="bin-mean", precision=precision, exact_widths=8.0, device=cuda_device)
+    tol = 1e-12 if precision == "fp64" else 1e-6
+    got = mc_cxr_spectrum(seg, E_grid, "silicon", None, n_hat=n_hats, rows=rows, **kw)
+    for d in range(3):
+        one_rows = reflection_rows(SILICON, hkl, n_hats[d:d + 1], surface_hkl=(2, 2, 0))
+        one = mc_cxr_spectrum(seg, E_grid, "silicon", None, n_hat=n_hats[d], rows=one_rows, **kw)
+        assert np.max(one) > 0.0
+        assert np.max(np.abs(got[d] - one)) <= tol * np.max(one)
+    if n_seg <= 17:
+        parts = 0.0
+        for i in range(n_seg):
+            s = {k: (v[i:i + 1] if isinstance(v, np.ndarray) else v) for k, v in seg.items()}
+            s["elec_id"] = np.zeros(1, dtype=np.int64)
+            s["Ne"] = 1
+            parts = parts + mc_cxr_spectrum(s, E_grid, "silicon", None, n_hat=n_hats, rows=rows, **kw)
+        parts = parts / seg["Ne"]
+        assert np.max(np.abs(got - parts)) <= tol * np.max(got)

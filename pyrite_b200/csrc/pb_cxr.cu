@@ -1019,7 +1019,8 @@ __device__ __forceinline__ void line_moments(double E_r, double inv_a, double w,
 // B is bound by FP32/FP64 issue and the SFU (one reciprocal, one sine, one
 // cosine per edge).
 template <class Real, bool kLayered>
-__global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_cxr_args a, int K_far, int far_pad) {
+__global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_cxr_args a, int K_far, int far_pad,
+                                                                         bool tab_smem) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr bool kMixed = sizeof(Real) == 4;
     const int n_g = a.tables.n_g;
@@ -1052,7 +1053,6 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
     uint16_t *pq = reinterpret_cast<uint16_t *>(scratch + 64);  // surviving pair ids
     cur = reinterpret_cast<unsigned char *>(pq + kQueue);
     cur = (unsigned char *)(((uintptr_t)cur + 15) & ~(uintptr_t)15);
-    const bool tab_smem = n_tab <= kMaxTab;
     Real *E_tab_s = reinterpret_cast<Real *>(cur);
     Real *delta_s = E_tab_s + (tab_smem ? n_tab : 0);
     Real *logmu_s = delta_s + (tab_smem ? n_tab : 0);
@@ -1765,14 +1765,14 @@ __global__ void __launch_bounds__(kNodeTile) node_reduce_kernel(const double *E_
 }
 
 template <class Real>
-static size_t cxr_smem_bytes(const pb_cxr_args &a, int far_pad, bool with_moments) {
+static size_t cxr_smem_bytes(const pb_cxr_args &a, bool tab_smem) {
     constexpr int kRowChunk = row_chunk<Real>();
     constexpr int kQueue = surv_queue<Real>();
     size_t b = sizeof(RowPre<Real>) * kRowChunk + sizeof(SegPre<Real>) * 2 * kSegTile + 16;
     b += sizeof(Real) * 3 * line_queue<Real>() + 16 +
          (sizeof(WinLine<Real>) + sizeof(uint16_t) * (kWinClasses / 2)) * kWideCap + sizeof(int) * 64 +
          sizeof(uint16_t) * kQueue + 16;
-    if (a.tables.n_tab <= kMaxTab) b += sizeof(Real) * (size_t)a.tables.n_tab * (3 + a.tables.n_mu);
+    if (tab_smem) b += sizeof(Real) * (size_t)a.tables.n_tab * (3 + a.tables.n_mu);
     b += 16;
     if (a.quadrature == PB_QUAD_BINMEAN)
         b += sizeof(double) * (size_t)a.n_E + (sizeof(Real) == 4 ? sizeof(float) * ((size_t)a.n_E + 1) : 0);
@@ -1791,8 +1791,16 @@ static cudaError_t launch_cxr_t(const pb_cxr_args &a, cudaStream_t s, int sms, i
     if (a.n_layer < 0 || a.n_layer > kMaxEscLayers) return cudaErrorInvalidValue;
     if (a.n_layer > 0 && (!a.z_top || !a.z_bot || !a.mu_off || !a.mu_knot || !a.mu_value || !a.mu_slope))
         return cudaErrorInvalidValue;
-    size_t smem = cxr_smem_bytes<Real>(a, far_pad, K_far > 0);
-    if (smem > 220 * 1024 || (binmean && a.n_E > 65535)) return cudaErrorInvalidValue;
+    // FP64 tables that do not fit beside the queues and the spectrum are read from
+    // global memory (without the prefilter, as tables beyond kMaxTab are).
+    constexpr size_t kMaxSmem = 220 * 1024;
+    bool tab_smem = a.tables.n_tab <= kMaxTab;
+    size_t smem = cxr_smem_bytes<Real>(a, tab_smem);
+    if (sizeof(Real) == 8 && tab_smem && smem > kMaxSmem) {
+        tab_smem = false;
+        smem = cxr_smem_bytes<Real>(a, false);
+    }
+    if (smem > kMaxSmem || (binmean && a.n_E > 65535)) return cudaErrorInvalidValue;
     // The float path reads its tables from the shared-memory staging only.
     if (sizeof(Real) == 4 && a.tables.n_tab > kMaxTab) return cudaErrorInvalidValue;
     auto kern = a.n_layer > 0 ? cxr_kernel<Real, true> : cxr_kernel<Real, false>;
@@ -1816,7 +1824,7 @@ static cudaError_t launch_cxr_t(const pb_cxr_args &a, cudaStream_t s, int sms, i
     int64_t gx = (int64_t)sms * per_sm;
     if (gx > work) gx = work;
     if (gx < 1) gx = 1;
-    kern<<<(unsigned)gx, kCxrThreads, smem, s>>>(a, K_far, far_pad);
+    kern<<<(unsigned)gx, kCxrThreads, smem, s>>>(a, K_far, far_pad, tab_smem);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (K_far > 0) {

@@ -208,3 +208,30 @@ def test_waiting_survivors_over_tiles_rows_and_directions(n_seg, n_g, precision,
             parts = parts + mc_cxr_spectrum(s, E_grid, "silicon", None, n_hat=n_hats, rows=rows, **kw)
         parts = parts / seg["Ne"]
         assert np.max(np.abs(got - parts)) <= tol * np.max(got)
+
+
+@pytest.mark.parametrize("quadrature", ["node", "bin-mean"])
+@pytest.mark.parametrize("n_mu", [1, 2, 4])
+def test_largest_tables_with_several_absorbers(n_mu, quadrature, cuda_device):
+    """The FP64 tables of 4,096 energies fit shared memory for one absorber;
+    with more they are read from global memory. The attenuation split evenly
+    over the absorbers is the same attenuation (1e-12 of the peak)."""
+    import dataclasses
+
+    from pyrite_b200 import mc_cxr_spectrum
+    from pyrite_b200 import placeholder_data as P
+    from pyrite_b200.tables import SILICON, diamond_hkls
+
+    E_grid = np.linspace(1000.0, 60000.0, 150)
+    seg, rows, _, n_hat = _scene(40, 30, E_grid, 1.5e5, 8)
+    hkl = [h for h in diamond_hkls(9.0) if np.dot(h, (1, 1, 0)) > 0]
+    hkl = hkl[:: max(1, len(hkl) // 30)][:30]
+    tables = P.line_tables(SILICON, hkl, E_grid, n_tab=4096)
+    assert np.asarray(tables.E_tab).size == 4096
+    lm = np.atleast_2d(np.asarray(tables.log_mu))
+    split = dataclasses.replace(tables, log_mu=np.repeat(lm - np.log(n_mu), n_mu, axis=0))
+    kw = dict(n_hat=n_hat, rows=rows, line_quadrature=quadrature, precision="fp64", device=cuda_device)
+    ref = mc_cxr_spectrum(seg, E_grid, "silicon", None, tables=tables, **kw)
+    got = mc_cxr_spectrum(seg, E_grid, "silicon", None, tables=split, **kw)
+    assert np.max(ref) > 0.0
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(ref)

@@ -61,6 +61,14 @@ MEASURED_BF16_SUSTAINED = float(json.loads((ROOT / "MEASURED_PEAKS.json").read_t
     if (ROOT / "MEASURED_PEAKS.json").exists() else 1400.0
 MEASURED_HBM_GBS = float(json.loads((ROOT / "MEASURED_PEAKS.json").read_text())["hbm_gbs"]) \
     if (ROOT / "MEASURED_PEAKS.json").exists() else 6650.0
+
+
+def _peak_source(name: str) -> str:
+    if (ROOT / "MEASURED_PEAKS.json").exists():
+        return f"MEASURED_PEAKS.json {name} (of measured)"
+    return f"{name} of an earlier measurement on this GPU type (of fallback)"
+
+
 # cxr_kernel<float> on the control variate's sub-sample (4 exact widths, ~14,560 segments, L2-resident):
 # DRAM bytes (read + write) per sampled segment from the one-pass ncu capture of the bench's own
 # sub-sample launches (profiles/cxr_kernel_subsample_si50_65536hist.md): 2.80-2.98 MB per launch.
@@ -852,9 +860,9 @@ def main():
         gbs = NODE_BYTES_PER_SEGMENT * n_seg / (r_head["t_brem"] / 1e3) / 1e9
         rooflines["brem_kernel"] = {
             "bound": "hbm", "kernel": "brem_node_* (depth-node form: energy window and depth grid, moment pass "
-                                      "on the FP64 tensor cores, one contraction block per photon energy)",
+                                      "on the FP64 tensor cores, one contraction block per four photon energies)",
             "achieved": gbs, "peak": MEASURED_HBM_GBS, "unit": "GB/s", "frac": gbs / MEASURED_HBM_GBS,
-            "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
+            "peak_source": _peak_source("hbm_gbs"),
             "census": "%g B per segment (energy, length, z, v_z, electron id); the five launches and the "
                       "left-out segments' per-pair launches all inside the timed brem span" % NODE_BYTES_PER_SEGMENT,
             "node": node_state[0], "segments": n_seg,
@@ -887,7 +895,7 @@ def main():
                       % ("segment; tile heads at readout" if tiles_form else "segment x tile"),
             "achieved": inf_tflops, "peak": MEASURED_BF16_SUSTAINED, "unit": "TFLOP/s",
             "frac": inf_tflops / MEASURED_BF16_SUSTAINED,
-            "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained (of measured)",
+            "peak_source": _peak_source("bf16_tflops_sustained"),
             "traffic": None if tiles_form else DRAM_BYTES_PER_HISTORY["mlp_infer_kernel"] * H}
         # The exact control variate as it runs in the step: every exact_stride-th
         # segment through cxr_kernel<float> with the narrow exact window, plus

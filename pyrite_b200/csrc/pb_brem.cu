@@ -904,20 +904,27 @@ constexpr int kBremChunkLayered = 64;
 // Blocks gather the emitting layer's segments of their slice into a list and
 // stage whole chunks of it: a layer's set of a stack radiates from its own
 // segments alone, most of which sit in other layers' sets. Directions of one
-// detector (one face, narrow spread) go through the moments (kMoments); the
-// others are scored one by one, two exponentials each. The three layers of the
+// detector (one face, narrow spread) go through the moments (kLayMoments); on the
+// mixed path directions that fall into at most four such groups (a detector
+// along the surface: its rows of tiles, on both faces) through four sets of them
+// (kLayGroups); the others are scored one by one, two exponentials each. The three layers of the
 // 10 MeV stack (160,000 segments, 4096 energies, 64 directions, mixed): 478 ms
-// per (segment, energy, direction), 55 with 12 of them in the moments; both
-// bound by issue and the SFU.
-template <class Real, bool kMoments>
+// per (segment, energy, direction), 55 with three detectors in the moments (12 of
+// them), 21 with the fourth, at 90 degrees, in four groups (43 -> 8.8); bound by
+// issue and the SFU.
+enum LayeredForm { kLayDirect = 0, kLayMoments, kLayGroups };
+template <class Real, int kForm>
 __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_brem_args a, int64_t n_seg, int d0) {
     constexpr int kChunk = kBremChunkLayered;
     __shared__ BremSeg<Real> segs[kChunk];
     __shared__ BremPieces<Real> pcs[kChunk];
     __shared__ int list[kChunk + kBremThreads];  // emitting segments of the slice, offsets from s_begin
     __shared__ int n_list;
+    constexpr bool kMoments = kForm == kLayMoments;
     constexpr int kOrder = sizeof(Real) == 8 ? 9 : 3;  // highest moment
+    static_assert(kForm != kLayGroups || (kOrder + 1) * kMaxGroups <= kBremMaxDir, "the groups' moments share the sums");
     __shared__ double acc[kMoments ? kOrder + 1 : kBremMaxDir][kBremThreads];
+    __shared__ DirGroups grp;
     __shared__ Real Zs[kBremMaxEl];
     __shared__ float zl[kBremMaxEl];  // 2 pi alpha Z log2(e)
     __shared__ Real inv_nz[kBremMaxDir];
@@ -926,8 +933,13 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     __shared__ int bad;
     const int nd = (a.n_dir - d0) < kBremMaxDir ? (a.n_dir - d0) : kBremMaxDir;
     double f_c, dl;
-    // both instances make the same test: one of them scores the launch
+    // the instances make the same tests: one of them scores the launch
     if (one_face(a.n_hat, d0, nd, moment_limit<Real>(), f_c, dl) != kMoments) return;
+    if constexpr (sizeof(Real) == 4 && !kMoments) {
+        if (threadIdx.x < 32) direction_groups(a.n_hat, d0, nd, moment_limit<Real>(), grp);
+        __syncthreads();
+        if ((grp.n <= kMaxGroups) != (kForm == kLayGroups)) return;
+    }
     const int n_el = a.n_el;
     const int nl = a.n_layer;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1002,6 +1014,18 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     int64_t s_end = s_begin + per < n_seg ? s_begin + per : n_seg;
     if (s_end < s_begin) s_end = s_begin;
     const Real T_stack = (Real)zb_s[nl - 1];
+    Real g_fc[kMaxGroups] = {}, g_dl[kMaxGroups] = {};
+    bool g_up[kMaxGroups] = {};
+    const int n_grp = kForm == kLayGroups ? grp.n : 0;
+    if constexpr (kForm == kLayGroups) {
+#pragma unroll
+        for (int g = 0; g < kMaxGroups; ++g)
+            if (g < n_grp) {
+                g_fc[g] = (Real)grp.f_c[g];
+                g_dl[g] = (Real)grp.dl[g];
+                g_up[g] = grp.up[g] != 0;
+            }
+    }
     const bool up_all = a.n_hat[3 * d0 + 2] < 0.0;
     if (threadIdx.x == 0) n_list = 0;
     int64_t next = s_begin;  // first segment not looked at yet
@@ -1062,6 +1086,24 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
                                            : esc_pick<Real>(c_dn, m) + mum * (esc_pick<Real>(t_l, m) - fmax(P.u0[p], P.u1[p]));
                     add_moments<kOrder>(nsig * P.f[p], lo, mum * fabs(P.u1[p] - P.u0[p]), (Real)f_c, (Real)dl, part);
                 }
+            } else if constexpr (kForm == kLayGroups) {
+                for (int p = 0; p < P.np; ++p) {
+                    const int m = P.m[p];
+                    const Real mum = esc_pick<Real>(mu_l, m);
+                    const Real lo_up = esc_pick<Real>(c_up, m) + mum * fmin(P.u0[p], P.u1[p]);
+                    const Real lo_dn = esc_pick<Real>(c_dn, m) + mum * (esc_pick<Real>(t_l, m) - fmax(P.u0[p], P.u1[p]));
+                    const Real w = nsig * P.f[p], dep = mum * fabs(P.u1[p] - P.u0[p]);
+#pragma unroll
+                    for (int g = 0; g < kMaxGroups; ++g) {
+                        if (g >= n_grp) break;
+                        Real Q[kOrder + 1];
+#pragma unroll
+                        for (int n = 0; n <= kOrder; ++n) Q[n] = part[g * (kOrder + 1) + n];
+                        add_moments<kOrder>(w, g_up[g] ? lo_up : lo_dn, dep, g_fc[g], g_dl[g], Q);
+#pragma unroll
+                        for (int n = 0; n <= kOrder; ++n) part[g * (kOrder + 1) + n] = Q[n];
+                    }
+                }
             } else for (int p = 0; p < P.np; ++p) {
                 const int m = P.m[p];
                 const Real mum = esc_pick<Real>(mu_l, m), tm = esc_pick<Real>(t_l, m);
@@ -1090,6 +1132,15 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
                 const double v = moments_at(kOrder, f, f_c, dl, [&](int n) { return acc[n][threadIdx.x]; });
                 if (v != 0.0) atomicAdd(&a.spec[(int64_t)(d0 + dd) * a.n_E + e], v);
             }
+    } else if constexpr (kForm == kLayGroups) {
+        if (on)
+            for (int dd = 0; dd < nd; ++dd) {
+                const int g = grp.of[dd];
+                const double f = 1.0 / fmax(fabs(a.n_hat[3 * (d0 + dd) + 2]), 1.0e-12);
+                const double v = moments_at(kOrder, f, grp.f_c[g], grp.dl[g],
+                                            [&](int n) { return acc[g * (kOrder + 1) + n][threadIdx.x]; });
+                if (v != 0.0) atomicAdd(&a.spec[(int64_t)(d0 + dd) * a.n_E + e], v);
+            }
     } else if (on) {
 #pragma unroll
         for (int dd = 0; dd < kBremMaxDir; ++dd)
@@ -1104,11 +1155,13 @@ cudaError_t launch_brem(const pb_brem_args &a, cudaStream_t s, int sms) {
         if (a.n_layer > kMaxEscLayers) return cudaErrorInvalidValue;
         const unsigned gx = (unsigned)((a.n_E + kBremThreads - 1) / kBremThreads);
         using LKern = void (*)(const pb_brem_args, int64_t, int);
-        const LKern kerns[2] = {a.precision == PB_MIXED ? (LKern)brem_layered_kernel<float, true>
-                                                        : (LKern)brem_layered_kernel<double, true>,
-                                a.precision == PB_MIXED ? (LKern)brem_layered_kernel<float, false>
-                                                        : (LKern)brem_layered_kernel<double, false>};
-        for (int k = 0; k < 2; ++k) {
+        const bool mixed = a.precision == PB_MIXED;
+        const LKern kerns[3] = {mixed ? (LKern)brem_layered_kernel<float, kLayMoments>
+                                      : (LKern)brem_layered_kernel<double, kLayMoments>,
+                                mixed ? (LKern)brem_layered_kernel<float, kLayDirect>
+                                      : (LKern)brem_layered_kernel<double, kLayDirect>,
+                                (LKern)brem_layered_kernel<float, kLayGroups>};
+        for (int k = 0; k < (mixed ? 3 : 2); ++k) {
             int per_sm = 0;
             const cudaError_t oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[k], kBremThreads, 0);
             if (oe != cudaSuccess) return oe;

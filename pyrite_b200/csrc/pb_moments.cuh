@@ -44,6 +44,45 @@ __device__ __forceinline__ bool one_face(const double *n_hat, int d0, int nd, do
     return (n_up == nd || n_up == 0) && dl <= limit * f_lo;
 }
 
+// The directions d0 .. d0 + nd - 1 (nd <= 32) as at most kMaxGroups groups of one
+// face and path factors in f_c +- dl, dl <= limit f_min, by one warp: each group
+// is the first direction left and those within 0.98 limit of its path factor.
+// ``of`` gets each direction's group; returns kMaxGroups + 1 where more are needed.
+constexpr int kMaxGroups = 4;
+struct DirGroups {
+    double f_c[kMaxGroups], dl[kMaxGroups];
+    int up[kMaxGroups], of[32];
+    int n;
+};
+__device__ __forceinline__ void direction_groups(const double *n_hat, int d0, int nd, double limit, DirGroups &g) {
+    const int lane = threadIdx.x & 31;
+    const double nz = lane < nd ? n_hat[3 * (d0 + lane) + 2] : 0.0;
+    const double f = 1.0 / fmax(fabs(nz), 1.0e-12);
+    const int up = nz < 0.0 ? 1 : 0;
+    unsigned left = __ballot_sync(0xffffffffu, lane < nd);
+    int n = 0;
+    while (left && n < kMaxGroups) {
+        const int lead = __ffs(left) - 1;
+        const double f0 = __shfl_sync(0xffffffffu, f, lead);
+        const int up0 = __shfl_sync(0xffffffffu, up, lead);
+        const bool in = ((left >> lane) & 1u) && up == up0 && fabs(f - f0) <= 0.98 * limit * fmin(f, f0);
+        double lo = in ? f : f0, hi = lo;
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (in) g.of[lane] = n;
+        if (lane == lead) {
+            g.f_c[n] = 0.5 * (lo + hi);
+            g.dl[n] = 0.5 * (hi - lo);
+            g.up[n] = up;
+        }
+        left &= ~(__ballot_sync(0xffffffffu, in) | (1u << lead));
+        ++n;
+    }
+    if (lane == 0) g.n = left ? kMaxGroups + 1 : n;
+}
+
 // Direction moments of the segment-mean escape, for the FP64 bremsstrahlung, the
 // layered absorber and the characteristic lines (the mixed single-slab kernels
 // carry packed forms of the same recurrence). The truncation after order N is below

@@ -644,7 +644,7 @@ class ScoringCase:
     def kernel_launches_per_batch(self) -> int:
         """This library's kernels launched per batch (transport 1, CXR 2 with
         the far-field convolution; brem: single-slab FP64 one per 16 directions,
-        mixed or layered two, plus the depth-node form's five where it has a
+        mixed or FP64 layered two, mixed layered three, plus the depth-node form's five where it has a
         workspace, six where its segment list may have energy windows)."""
         if getattr(self, "surrogates", None):
             n = 1 + len(self.surrogates) * (2 if self.sur_stride > 0 else 1)
@@ -656,7 +656,8 @@ class ScoringCase:
         else:
             n = 1 + sum(1 + (1 if ca.exact_widths > 0 else 0) for ca in self.cargs_all)
         for b in self.bargs_all:
-            n += (2 if self.precision == L.PB_MIXED or b.n_layer > 0 else 1) * ((self.n_dir + 15) // 16)
+            per_group = 1 + (1 if self.precision == L.PB_MIXED else 0) + (1 if b.n_layer > 0 else 0)
+            n += per_group * ((self.n_dir + 15) // 16)
             if b.work:
                 n += 6 if b.n_seg <= 1 << 22 else 5
         n += len(self.chargs_all)

@@ -90,3 +90,33 @@ def test_stack(n_dir, rho, face, precision, tol, cuda_device):
             ref = oracle.brem_spectrum_layered(_oseg(seg, on), [Z[e] for e, _ in comp], [n for _, n in comp],
                                                oracle.LayerEscape(top, bot), nh, E, mu, seg["Ne"])
             assert np.max(np.abs(g - ref)) <= tol * np.max(ref)
+
+
+@pytest.mark.parametrize("f", [[1.0, 1.3], [1.0, 1.0097, 1.0099, 1.02], [-1.0, 1.0, -1.3, 1.3], [133.0, -133.0, 400.0, -400.0],
+                               [1.0, 1.1, 1.2, 1.3, 1.4], [1.0, -1.0, 1.2, -1.2, 1.5]])
+def test_mixed_stack_direction_groups(f, cuda_device):
+    """Directions in two to four narrow groups (path factors over that of the
+    first, the sign the face) share the exponentials of each group; five groups,
+    or more than 16 directions in a launch, are the per-direction form's. Four
+    directions a group within 0.4 % of it."""
+    from pyrite_b200 import mc_brem_spectrum
+    from pyrite_b200 import placeholder_data as P
+
+    seg = _segments(600, 9)
+    E = np.linspace(1000.0, 60000.0, 129)
+    fs = np.concatenate([np.asarray(f) * (1.0 + s) for s in (0.0, 0.001, -0.002, 0.002)][: 16 // len(f)])
+    nz = np.sign(fs) * 0.9 / np.maximum(np.abs(fs), 1.0)
+    n_hat = np.stack([np.sqrt(1.0 - nz**2), np.zeros(fs.size), nz], 1)
+    mu = np.stack([P.mu_total(c, E) for _, _, c in LAYERS])
+    top, bot = np.array([l[0] for l in LAYERS]), np.array([l[1] for l in LAYERS])
+    seg["layer"] = np.searchsorted(top[1:], seg["r_mid"][:, 2], side="right").astype(np.int32)
+    for k, (_a, _b, comp) in enumerate(LAYERS):
+        got = mc_brem_spectrum(seg, E, composition=comp, n_hat=n_hat, layers=LAYERS, mu_layer=mu, emit_layer=k,
+                               precision="mixed", device=cuda_device)
+        on = seg["layer"] == k
+        for g, nh in zip(got, n_hat):
+            ref = oracle.brem_spectrum_layered(_oseg(seg, on), [Z[e] for e, _ in comp], [n for _, n in comp],
+                                               oracle.LayerEscape(top, bot), nh, E, mu, seg["Ne"])
+            # along the surface all light is attenuated, and a float e^-x carries x ulps
+            tol = 2e-6 * max(1.0, abs(1.0 / nh[2]) / 10.0)
+            assert np.max(np.abs(g - ref)) <= tol * np.max(ref)

@@ -21,6 +21,7 @@
 #include "pb_internal.h"
 #include "pb_layers.cuh"
 #include "pb_moments.cuh"
+#include "pb_slices.h"
 
 namespace pb {
 
@@ -439,15 +440,9 @@ __global__ void __launch_bounds__(kBremPackedThreads, 3)
     // dealt out in chunks instead: the electrons below a photon energy cost
     // nothing, and each block should have its share of them.
     const bool dealt = sidx != nullptr && nh->n_win > 0;
-    const int64_t per = (live + gridDim.y - 1) / gridDim.y;
-    const int64_t rounds = (per + kBremChunk - 1) / kBremChunk;
-    const int64_t chunk = dealt ? (per + rounds - 1) / (rounds > 0 ? rounds : 1) : kBremChunk;
-    const int64_t s_begin = (dealt ? chunk : per) * blockIdx.y;
-    const int64_t s_step = dealt ? chunk * gridDim.y : chunk;
-    int64_t s_end = dealt || s_begin + per > live ? live : s_begin + per;
-    if (s_end < s_begin) s_end = s_begin;
-    for (int64_t c0s = s_begin; c0s < s_end; c0s += s_step) {
-        const int nc = (int)((s_end - c0s) < chunk ? (s_end - c0s) : chunk);
+    const SegSlice sl = seg_slice(live, blockIdx.y, gridDim.y, kBremChunk, dealt);
+    for (int64_t c0s = sl.begin; c0s < sl.end; c0s += sl.step) {
+        const int nc = (int)((sl.end - c0s) < sl.chunk ? (sl.end - c0s) : sl.chunk);
         __syncthreads();
         float tlo = 3.4e38f, thi = -3.4e38f, nmax = 0.0f;
         for (int j = threadIdx.x; j < nc; j += blockDim.x) {
@@ -740,10 +735,8 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
     }
     // Slices of the live segments (the count read on the device), so every
     // block of the wave has work.
-    const int64_t per = (n_seg + gridDim.y - 1) / gridDim.y;
-    const int64_t s_begin = per * blockIdx.y;
-    int64_t s_end = s_begin + per < n_seg ? s_begin + per : n_seg;
-    if (s_end < s_begin) s_end = s_begin;
+    const SegSlice sl = seg_slice(n_seg, blockIdx.y, gridDim.y, kChunk, false);
+    const int64_t s_begin = sl.begin, s_end = sl.end;
     for (int64_t c0s = s_begin; c0s < s_end; c0s += kChunk) {
         const int nc = (int)((s_end - c0s) < kChunk ? (s_end - c0s) : kChunk);
         __syncthreads();
@@ -1009,10 +1002,8 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     }
     // Slices of the live segments (the count read on the device), so every
     // block of the wave has work.
-    const int64_t per = (n_seg + gridDim.y - 1) / gridDim.y;
-    const int64_t s_begin = per * blockIdx.y;
-    int64_t s_end = s_begin + per < n_seg ? s_begin + per : n_seg;
-    if (s_end < s_begin) s_end = s_begin;
+    const SegSlice sl = seg_slice(n_seg, blockIdx.y, gridDim.y, kChunk, false);
+    const int64_t s_begin = sl.begin, s_end = sl.end;
     const Real T_stack = (Real)zb_s[nl - 1];
     Real g_fc[kMaxGroups] = {}, g_dl[kMaxGroups] = {};
     bool g_up[kMaxGroups] = {};

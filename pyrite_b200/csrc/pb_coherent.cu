@@ -390,8 +390,15 @@ __global__ void __launch_bounds__(kThreads, kGrouped ? 2 : 3) coh_field_kernel(c
                             cv[k] = -cv[k];
                         }
                     }
-                    if (cut[k]) sp[k] = cp[k] = 0.f;  // outside the window: no term
                 }
+                // Outside the window a line adds nothing, whatever its amplitude.
+                if (cut[0] && cut[1]) continue;
+                const auto inside = [&](F2 with, F2 without) {  // halves with a term, halves without
+                    float a0, a1, b0, b1;
+                    f2_get(with, a0, a1);
+                    f2_get(without, b0, b1);
+                    return f2(cut[0] ? b0 : a0, cut[1] ? b1 : a1);
+                };
                 const F2 v2 = f2(vf[0], vf[1]), s2 = f2(sv[0], sv[1]), c2 = f2(cv[0], cv[1]);
                 const F2 sp2 = f2(sp[0], sp[1]), cp2 = f2(cp[0], cp[1]);
                 if constexpr (kGrouped) {
@@ -400,11 +407,17 @@ __global__ void __launch_bounds__(kThreads, kGrouped ? 2 : 3) coh_field_kernel(c
                     const F2 one = f2(1.f, 1.f);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
+                        if (cut[0] || cut[1]) t[c] = inside(t[c], zero);
                         acc[m][c] = f2_fma(one, t[c], acc[m][c]);
                         acc_e[m][c] = f2_fma(one, t[c], acc_e[m][c]);
                     }
                 } else {
-                    line_term(l, v2, s2, c2, sp2, cp2, acc[m]);
+                    F2 t[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) t[c] = acc[m][c];
+                    line_term(l, v2, s2, c2, sp2, cp2, t);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[m][c] = cut[0] || cut[1] ? inside(t[c], acc[m][c]) : t[c];
                 }
             }
         }

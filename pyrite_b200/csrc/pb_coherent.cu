@@ -245,7 +245,9 @@ struct CohArgs {
 // items move a shared bound alike, so the items still partition the row),
 // and besides the row's field the kernel sums every electron's own field,
 // squares it where the electron ends and adds the squares up per item.
-template <bool kGrouped>
+// kWindow: lines count within the cutoff only (an instance of its own, so that the
+// one without a window carries none of it).
+template <bool kGrouped, bool kWindow>
 __global__ void __launch_bounds__(kThreads, kGrouped ? 2 : 3) coh_field_kernel(const CohArgs a) {
     __shared__ CohLine sm[kStage];
     const int64_t item = blockIdx.x;
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(kThreads, kGrouped ? 2 : 3) coh_field_kernel(c
                         pt = fma(l.ps_t, Ek, -fma(l.L_t, Dk, l.Gx));
                         sincos_turns(pt, sp[k], cp[k]);
                     }
-                    cut[k] = a.cutoff > 0.f && fabsf(vf[k]) > a.cutoff;
+                    cut[k] = kWindow && fabsf(vf[k]) > a.cutoff;
                     if (fabsf(vf[k]) <= 1.f) {
                         sincos_taylor(vf[k], sv[k], cv[k]);
                         if (fast) {  // the sign of the two fast pairs cancels in the product
@@ -669,20 +671,22 @@ cudaError_t launch_coherent_impl(const pb_coherent_args &p, const int64_t *elec,
     a.status = p.status;
     dim3 grid((unsigned)n_item_max, (unsigned)n_etiles(p.n_E));
     const unsigned fin_blocks = (unsigned)((p.n_E + kFinE - 1) / kFinE);
+    const bool window = a.cutoff > 0.f;
+    const auto field = elec ? (window ? coh_field_kernel<true, true> : coh_field_kernel<true, false>)
+                            : (window ? coh_field_kernel<false, true> : coh_field_kernel<false, false>);
     if (fields) {  // streamed: fold into the persistent planes, no squaring yet
-        if (elec) coh_field_kernel<true><<<grid, kThreads, 0, s>>>(a);
-        else coh_field_kernel<false><<<grid, kThreads, 0, s>>>(a);
+        field<<<grid, kThreads, 0, s>>>(a);
         dim3 fgrid((unsigned)((p.n_E + kFinalizeThreads - 1) / kFinalizeThreads),
                    (unsigned)(p.n_row < 65535 ? p.n_row : 65535));
         coh_fold_kernel<<<fgrid, kFinalizeThreads, 0, s>>>(p.n_row, p.n_E, item_off, partial, elec ? a.power : nullptr,
                                                            fields, pw_planes);
     } else if (elec) {
-        coh_field_kernel<true><<<grid, kThreads, 0, s>>>(a);
+        field<<<grid, kThreads, 0, s>>>(a);
         coh_finalize_kernel<true><<<fin_blocks, kFinE * kFinT, 0, s>>>(p.n_row, p.n_E, item_off, p.row_weight, F_row,
                                                                        partial, a.power, finalize_parts(p.n_row),
                                                                        p.scale, p.spec);
     } else {
-        coh_field_kernel<false><<<grid, kThreads, 0, s>>>(a);
+        field<<<grid, kThreads, 0, s>>>(a);
         coh_finalize_kernel<false><<<fin_blocks, kFinE * kFinT, 0, s>>>(p.n_row, p.n_E, item_off, p.row_weight,
                                                                         nullptr, partial, nullptr,
                                                                         finalize_parts(p.n_row), p.scale, p.spec);

@@ -28,9 +28,6 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relax
 # reference's event decisions; the scorers may contract.
 PER_FILE = {
     "pb_transport.cu": ["-fmad=false"],
-    # Fields of normal floats: the SFU forms without their subnormal branches (the
-    # CXR scorer keeps them, its line weights reach into the subnormal range).
-    "pb_coherent.cu": ["-ftz=true"],
 }
 SOURCES = ["pb_capi.cu", "pb_transport.cu", "pb_cxr.cu", "pb_brem.cu", "pb_brem_node.cu", "pb_char.cu", "pb_mlp.cu", "pb_coherent.cu"]
 

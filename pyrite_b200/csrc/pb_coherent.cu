@@ -92,10 +92,21 @@ constexpr double kTurnBase = 805306368.0;        // 1.5 * 2^29
 constexpr double kFastLimit = 134217728.0;       // 2^27 turns: offset sums stay in [2^29, 2^30)
 
 // -(sin, cos) of 2 pi f, f the fraction of x - kTurnBase, for x in [2^29, 2^30):
-// sin(2 pi f) = -sin(2 pi (f - 1/2)), f - 1/2 in [-1/2, 1/2) exactly.
+// sin(2 pi f) = -sin(2 pi (f - 1/2)), f - 1/2 in [-1/2, 1/2) exactly. f - 1/2 is
+// a multiple of 2^-23, never a subnormal number, so the SFU forms that flush
+// those give the same values without the branches for them.
 __device__ __forceinline__ void neg_sincos_turns_offset(double x, float &s, float &c) {
     const unsigned lo = (unsigned)__double2loint(x);
-    __sincosf((__uint_as_float((lo & 0x7FFFFFu) | 0x3F800000u) - 1.5f) * kTwoPiF, &s, &c);
+    const float a = (__uint_as_float((lo & 0x7FFFFFu) | 0x3F800000u) - 1.5f) * kTwoPiF;
+    asm("sin.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(a));
+    asm("cos.approx.ftz.f32 %0, %1;" : "=f"(c) : "f"(a));
+}
+
+// 1 / x on the SFU; x is |w|^2 of a line, at least kSeriesW2 where the result counts.
+__device__ __forceinline__ float rcp_w2(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
 // (sin, cos) of 2 pi t for any FP64 t with |t| < 2^51.
@@ -189,7 +200,7 @@ __device__ __forceinline__ void line_term(const CohLine &l, F2 v, F2 sv, F2 cv, 
     const F2 w2 = f2_fma(v, v, l.q2);
     float w0, w1;
     f2_get(w2, w0, w1);
-    const F2 inv = f2(__fdividef(1.f, w0), __fdividef(1.f, w1));
+    const F2 inv = f2(rcp_w2(w0), rcp_w2(w1));
     F2 fr = f2_mul(f2_fma(f2_mul(v, l.apb), sv, f2_mul(f2_mul(l.qbma, cv), minus)), inv);
     F2 nf = f2_mul(f2_fma(f2_mul(v, l.bma), cv, f2_mul(l.qapb, sv)), inv);
     if (fminf(w0, w1) < kSeriesW2) {

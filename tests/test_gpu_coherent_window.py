@@ -54,3 +54,21 @@ def test_amplitudes_outside_the_window_do_not_count(n_E, blend, phase, cuda_devi
     assert inside.sum() > 50 and outside.sum() > 200 and np.isfinite(ref).all()
     assert np.array_equal(got[outside], ref[outside])
     assert not np.isfinite(got[inside]).any()
+
+
+def test_amplitudes_below_the_smallest_normal_float(cuda_device):
+    """Records whose amplitudes are subnormal floats keep their fields: the
+    spectrum is that of amplitudes 2^133 as large times 2^-266. 300 lines round
+    some ten times each to multiples of 1.4e-45, which for amplitudes of about
+    1e-40 and fields of 1e-39 comes to 2e-5 of the field if every rounding is its
+    own; 2e-4 of the spectrum."""
+    from pyrite_b200.coherent import coherent_reduce
+
+    E = np.linspace(5000.0, 15000.0, 500)
+    rec = _records(300, E, 1e5, 3)
+    tiny = dict(rec, **{k: rec[k] * 2.0**-133 for k in ("cs_re", "cs_im", "cp_re", "cp_im")})
+    dom = np.zeros(E.size)
+    ref = coherent_reduce(rec, [300], [1.0], E, dom, device=cuda_device).cpu().numpy() * 2.0**-266
+    got = coherent_reduce(tiny, [300], [1.0], E, dom, device=cuda_device).cpu().numpy()
+    assert np.linalg.norm(ref) > 0.0
+    assert np.linalg.norm(got / 2.0**-266 - ref / 2.0**-266) <= 2e-4 * np.linalg.norm(ref / 2.0**-266)

@@ -472,7 +472,9 @@ int pb_brem_score(const pb_brem_args *args, void *stream);
 
 /* Workspace bytes the depth-node form of pb_brem_score needs for these
  * arguments (precision, n_el, n_E, n_seg, n_layer): 0 where the form does
- * not apply (FP64, layered absorbers, more than two elements). */
+ * not apply (FP64, layered absorbers, more than two elements). The size never
+ * falls as n_seg, n_E or n_el grow: one workspace for the longest list does
+ * for all. */
 int pb_brem_work_size(const pb_brem_args *args, int64_t *bytes);
 
 /* Characteristic line yields of a segment list (accumulated). */

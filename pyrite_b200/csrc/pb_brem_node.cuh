@@ -63,19 +63,31 @@ struct BremNodeLayout {
     int n_win;    // windows the workspace holds
 };
 
-__host__ __device__ inline BremNodeLayout brem_node_layout(const pb_brem_args &a) {
+__host__ __device__ inline BremNodeLayout brem_node_parts(const pb_brem_args &a, int64_t n_seg) {
     BremNodeLayout l;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     // With windows the list holds every segment (left out, then window by window).
-    const bool win = a.n_seg <= kNodeWinSeg;
+    const bool win = n_seg <= kNodeWinSeg;
     l.n_win = win ? kNodeMaxWin : 1;
     l.hdr = 0;
     l.S = up(sizeof(BremNodeHdr));
     l.A = up(l.S + sizeof(double) * (size_t)l.n_win * (size_t)a.n_el * 2 * kNodeMaxCells * kNodePJ);
     l.idx = up(l.A + sizeof(double) * (size_t)l.n_win * (size_t)a.n_E * (size_t)a.n_el * kNodeTDeg);
-    l.cap = win ? (a.n_seg > 4096 ? a.n_seg : 4096) : a.n_seg / 8 + 4096;
+    l.cap = win ? (n_seg > 4096 ? n_seg : 4096) : n_seg / 8 + 4096;
     l.total = l.idx + sizeof(int64_t) * (size_t)l.cap;
     l.zero_bytes = l.A;  // header and moments
+    return l;
+}
+
+// A workspace sized for a list holds every shorter one: past the longest list
+// with windows, whose parts alone need less, the size stays at that list's
+// (38 MB for 2,048 energies and one element) until the longer list needs more.
+__host__ __device__ inline BremNodeLayout brem_node_layout(const pb_brem_args &a) {
+    BremNodeLayout l = brem_node_parts(a, a.n_seg);
+    if (a.n_seg > kNodeWinSeg) {
+        const size_t least = brem_node_parts(a, kNodeWinSeg).total;
+        if (l.total < least) l.total = least;
+    }
     return l;
 }
 

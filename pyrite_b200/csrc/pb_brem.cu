@@ -120,6 +120,8 @@ __device__ __forceinline__ void brem_stage(BremSeg<Real> &b, const pb_brem_args 
         b.inv_e2 = 1.0f / b.e2;
     }
     const bool rad = a.elec_id[s] < a.Ne && (a.seg_layer == nullptr || a.seg_layer[s] == a.emit_layer);
+    // (FP64: below every photon energy, so that its depth moves no reference)
+    if (sizeof(Real) == 8 && !rad) b.T = (Real)0;
     const Real path_cm = (Real)a.L[s] * (Real)1e-8;
     for (int el = 0; el < a.n_el; ++el) {
         b.nL[el] = rad ? (Real)(a.n_ang3[el] * 1e24) * (Real)1 * path_cm : (Real)0;
@@ -711,6 +713,7 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
             order = dl == 0.0 ? 0 : (rho <= 0.002 ? 5 : 9);
         }
     }
+    double z_ref = a.thickness;  // FP64 moments: depth below the exit face that they count from
     const double k_kev_d = on ? a.E_grid[e] / 1e3 : 1.0;
     const Real k = (Real)k_kev_d;
     const Real mu = on ? (Real)a.mu[e] : (Real)0;
@@ -777,8 +780,9 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
         if constexpr (sizeof(Real) == 8) {
             // acc[n] holds the thread's summed moment n until the end. (Two
             // exponentials a pair instead of two a direction, FP64 pipe bound: 20,000
-            // segments, 2,048 energies, 16 directions 5.4 -> 1.0 ms a call.)
+            // segments, 2,048 energies, 16 directions 5.17 -> 0.80 ms.)
             const bool up_all = side_all > 0;
+            const double above = -moment_above<double>() / f_c;
             const auto moments = [&](auto tag) {
                 constexpr int N = decltype(tag)::value;
                 double Q[N + 1] = {};
@@ -788,7 +792,18 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
                     if (!(T_f > 1e-6 && k > 0.0)) continue;
                     const double nsig = brem_nsig<double, NEL>(b, k, T_f, Zs, n_el, k_ev, c0, za, mc2, kk, zl);
                     const double lo = up_all ? fmin(b.e0, b.e1) : T_slab - fmax(b.e0, b.e1);
-                    add_moments<N>(nsig, mu * lo, mu * fabs(b.e1 - b.e0), f_c, dl, Q);
+                    double a_lo = mu * (lo - z_ref);
+                    if (a_lo < above) {
+#pragma unroll
+                        for (int n = 0; n <= N; ++n) {
+                            acc[n][threadIdx.x] += Q[n];
+                            Q[n] = 0.0;
+                        }
+                        rebase_moments(N, mu * (z_ref - lo), f_c, dl, [&](int n) -> double & { return acc[n][threadIdx.x]; });
+                        z_ref = lo;
+                        a_lo = 0.0;
+                    }
+                    add_moments<N>(nsig, a_lo, mu * fabs(b.e1 - b.e0), f_c, 0.0, dl, Q);
                 }
 #pragma unroll
                 for (int n = 0; n <= N; ++n) acc[n][threadIdx.x] += Q[n];
@@ -866,7 +881,8 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
             if (on)
                 for (int dd = 0; dd < nd; ++dd) {
                     const double f = 1.0 / fmax(fabs(a.n_hat[3 * (d0 + dd) + 2]), 1.0e-12);
-                    const double v = moments_at(order, f, f_c, dl, [&](int n) { return acc[n][threadIdx.x]; });
+                    const double v = exp(-mu * z_ref * f) *
+                                     moments_at(order, f, f_c, dl, [&](int n) { return acc[n][threadIdx.x]; });
                     if (v != 0.0) atomicAdd(&a.spec[(int64_t)(d0 + dd) * a.n_E + e], v);
                 }
             return;
@@ -885,11 +901,14 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
 // whole-layer optical depths above and below each layer, so a piece's end
 // depths cost one FMA each and its transmission the reference's closed form
 // (brem.py:1195-1200, segment_escape.py:276-289), weighted by its fraction.
-template <class Real>
+template <class Real, bool kMom>
 struct BremPieces {
     int np;
     int m[kMaxEscLayers];
-    Real f[kMaxEscLayers], u0[kMaxEscLayers], u1[kMaxEscLayers];
+    // The ends' depths below the layer's top; moments: u0 and u1 are the depths of the
+    // end nearer the upper and of that nearer the lower face from the layer's own face
+    // there (one exit face: u0 is that face's), d the depth difference of the ends.
+    Real f[kMaxEscLayers], u0[kMaxEscLayers], u1[kMaxEscLayers], d[kMom ? kMaxEscLayers : 1];
 };
 
 constexpr int kBremChunkLayered = 64;
@@ -900,17 +919,19 @@ constexpr int kBremChunkLayered = 64;
 // detector (one face, narrow spread) go through the moments (kLayMoments); on the
 // mixed path directions that fall into at most four such groups (a detector
 // along the surface: its rows of tiles, on both faces) through four sets of them
-// (kLayGroups); the others are scored one by one, two exponentials each. The three layers of the
-// 10 MeV stack (160,000 segments, 4096 energies, 64 directions, mixed): 478 ms
-// per (segment, energy, direction), 55 with three detectors in the moments (12 of
-// them), 21 with the fourth, at 90 degrees, in four groups (43 -> 8.8); bound by
-// issue and the SFU.
+// (kLayGroups); the others are scored one by one, two exponentials each. The three
+// layers of the 10 MeV stack (160,000 segments, 4096 energies, 64 directions, mixed):
+// 478 ms per (segment, energy, direction), 28 with three detectors in the moments
+// (15 of them) and the fourth, at 90 degrees, in four groups (13); bound by issue and
+// the SFU. (22 without a reference that moves with the shallowest piece and with
+// coarser exponentials: light from below an absorber was then off by up to 5e-3 of
+// itself, now 4e-6.)
 enum LayeredForm { kLayDirect = 0, kLayMoments, kLayGroups };
 template <class Real, int kForm>
 __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_brem_args a, int64_t n_seg, int d0) {
     constexpr int kChunk = kBremChunkLayered;
     __shared__ BremSeg<Real> segs[kChunk];
-    __shared__ BremPieces<Real> pcs[kChunk];
+    __shared__ BremPieces<Real, kForm != kLayDirect> pcs[kChunk];
     __shared__ int list[kChunk + kBremThreads];  // emitting segments of the slice, offsets from s_begin
     __shared__ int n_list;
     constexpr bool kMoments = kForm == kLayMoments;
@@ -1005,19 +1026,50 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     const SegSlice sl = seg_slice(n_seg, blockIdx.y, gridDim.y, kChunk, false);
     const int64_t s_begin = sl.begin, s_end = sl.end;
     const Real T_stack = (Real)zb_s[nl - 1];
-    Real g_fc[kMaxGroups] = {}, g_dl[kMaxGroups] = {};
+    Real g_fc[kMaxGroups] = {}, g_c2[kMaxGroups] = {}, g_dl[kMaxGroups] = {};
+    const Real c2 = (Real)(f_c * 1.4426950408889634);
     bool g_up[kMaxGroups] = {};
+    Real f_up = 0, f_dn = 0;  // largest path factor of a group on each face
     const int n_grp = kForm == kLayGroups ? grp.n : 0;
     if constexpr (kForm == kLayGroups) {
 #pragma unroll
         for (int g = 0; g < kMaxGroups; ++g)
             if (g < n_grp) {
                 g_fc[g] = (Real)grp.f_c[g];
+                g_c2[g] = (Real)(grp.f_c[g] * 1.4426950408889634);
                 g_dl[g] = (Real)grp.dl[g];
                 g_up[g] = grp.up[g] != 0;
+                (g_up[g] ? f_up : f_dn) = fmax(g_up[g] ? f_up : f_dn, g_fc[g]);
             }
     }
+    const Real above_up = -moment_above<Real>() / (kMoments ? (Real)f_c : f_up), above_dn = -moment_above<Real>() / f_dn;
     const bool up_all = a.n_hat[3 * d0 + 2] < 0.0;
+    // Moments: the optical depths below the upper and the lower face that they count
+    // from, the whole stack's at first; c_up and c_dn count from there too (one exit
+    // face: c_up and ref_up are that face's).
+    double ref_up = 0.0, ref_dn = 0.0;
+    const auto count_from = [&](bool upper, double to, Real (&c)[kMaxEscLayers]) {
+        double run = -to;
+        if (upper) {
+#pragma unroll
+            for (int k = 0; k < kMaxEscLayers; ++k) {
+                c[k] = (Real)run;
+                run += (double)mu_l[k] * (double)t_l[k];
+            }
+        } else {
+#pragma unroll
+            for (int k = kMaxEscLayers - 1; k >= 0; --k) {
+                c[k] = (Real)run;
+                run += (double)mu_l[k] * (double)t_l[k];
+            }
+        }
+        return run;
+    };
+    if constexpr (kForm != kLayDirect) {
+        ref_up = ref_dn = count_from(true, 0.0, c_up);
+        count_from(!kMoments || up_all, ref_up, c_up);
+        if (!kMoments) count_from(false, ref_dn, c_dn);
+    }
     if (threadIdx.x == 0) n_list = 0;
     int64_t next = s_begin;  // first segment not looked at yet
     while (true) {
@@ -1046,13 +1098,21 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
             const double z = a.r_mid[3 * s + 2], vz = a.v_hat[3 * s + 2];
             EscPiece pp[kMaxEscLayers];
             const int np = esc_pieces(z - half * vz, z + half * vz, nl, zt_s, zb_s, pp);
-            BremPieces<Real> &P = pcs[j];
+            auto &P = pcs[j];
             P.np = np;
             for (int p = 0; p < np; ++p) {
                 P.m[p] = pp[p].m;
                 P.f[p] = (Real)pp[p].f;
-                P.u0[p] = (Real)pp[p].u0;
-                P.u1[p] = (Real)pp[p].u1;
+                if constexpr (kForm == kLayDirect) {
+                    P.u0[p] = (Real)pp[p].u0;
+                    P.u1[p] = (Real)pp[p].u1;
+                } else {
+                    const double near_up = fmin(pp[p].u0, pp[p].u1);
+                    const double near_dn = zb_s[pp[p].m] - zt_s[pp[p].m] - fmax(pp[p].u0, pp[p].u1);
+                    P.u0[p] = (Real)(kMoments && !up_all ? near_dn : near_up);
+                    P.u1[p] = (Real)near_dn;
+                    P.d[p] = (Real)fabs(pp[p].u1 - pp[p].u0);
+                }
             }
         }
         __syncthreads();
@@ -1067,32 +1127,51 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
             const Real T_f = b.T - k;
             if (!(T_f > (Real)1e-6 && k > (Real)0)) continue;
             const Real nsig = brem_nsig<Real>(b, k, T_f, Zs, n_el, k_ev, c0, za, mc2, kk, zl);
-            const BremPieces<Real> &P = pcs[j];
-            if constexpr (kMoments) {
+            const auto &P = pcs[j];
+            if constexpr (kForm != kLayDirect) {
+                // The sums of a face move to a reference -a nearer to it.
+                const auto rebase = [&](bool upper, Real a) {
+#pragma unroll
+                    for (int dd = 0; dd < kPart; ++dd) {
+                        acc[dd][threadIdx.x] += (double)part[dd];
+                        part[dd] = 0;
+                    }
+                    for (int g = 0; g < (kMoments ? 1 : n_grp); ++g) {
+                        if (!kMoments && (grp.up[g] != 0) != upper) continue;
+                        rebase_moments(kOrder, -(double)a, kMoments ? f_c : grp.f_c[g], kMoments ? dl : grp.dl[g],
+                                       [&](int n) -> double & { return acc[g * (kOrder + 1) + n][threadIdx.x]; });
+                    }
+                    if (kMoments || upper) count_from(!kMoments || up_all, ref_up += (double)a, c_up);
+                    else count_from(false, ref_dn += (double)a, c_dn);
+                };
                 for (int p = 0; p < P.np; ++p) {
                     const int m = P.m[p];
                     const Real mum = esc_pick<Real>(mu_l, m);
+                    const Real w = nsig * P.f[p], dep = mum * P.d[p];
                     // the piece end nearer the exit face
-                    const Real lo = up_all ? esc_pick<Real>(c_up, m) + mum * fmin(P.u0[p], P.u1[p])
-                                           : esc_pick<Real>(c_dn, m) + mum * (esc_pick<Real>(t_l, m) - fmax(P.u0[p], P.u1[p]));
-                    add_moments<kOrder>(nsig * P.f[p], lo, mum * fabs(P.u1[p] - P.u0[p]), (Real)f_c, (Real)dl, part);
-                }
-            } else if constexpr (kForm == kLayGroups) {
-                for (int p = 0; p < P.np; ++p) {
-                    const int m = P.m[p];
-                    const Real mum = esc_pick<Real>(mu_l, m);
-                    const Real lo_up = esc_pick<Real>(c_up, m) + mum * fmin(P.u0[p], P.u1[p]);
-                    const Real lo_dn = esc_pick<Real>(c_dn, m) + mum * (esc_pick<Real>(t_l, m) - fmax(P.u0[p], P.u1[p]));
-                    const Real w = nsig * P.f[p], dep = mum * fabs(P.u1[p] - P.u0[p]);
+                    Real a_up = esc_pick<Real>(c_up, m) + mum * P.u0[p];
+                    if (a_up < above_up) {
+                        rebase(true, a_up);
+                        a_up = esc_pick<Real>(c_up, m) + mum * P.u0[p];
+                    }
+                    if constexpr (kMoments) {
+                        add_moments<kOrder>(w, a_up, dep, (Real)f_c, c2, (Real)dl, part);
+                    } else {
+                        Real a_dn = esc_pick<Real>(c_dn, m) + mum * P.u1[p];
+                        if (a_dn < above_dn) {
+                            rebase(false, a_dn);
+                            a_dn = esc_pick<Real>(c_dn, m) + mum * P.u1[p];
+                        }
 #pragma unroll
-                    for (int g = 0; g < kMaxGroups; ++g) {
-                        if (g >= n_grp) break;
-                        Real Q[kOrder + 1];
+                        for (int g = 0; g < kMaxGroups; ++g) {
+                            if (g >= n_grp) break;
+                            Real Q[kOrder + 1];
 #pragma unroll
-                        for (int n = 0; n <= kOrder; ++n) Q[n] = part[g * (kOrder + 1) + n];
-                        add_moments<kOrder>(w, g_up[g] ? lo_up : lo_dn, dep, g_fc[g], g_dl[g], Q);
+                            for (int n = 0; n <= kOrder; ++n) Q[n] = part[g * (kOrder + 1) + n];
+                            add_moments<kOrder>(w, g_up[g] ? a_up : a_dn, dep, g_fc[g], g_c2[g], g_dl[g], Q);
 #pragma unroll
-                        for (int n = 0; n <= kOrder; ++n) part[g * (kOrder + 1) + n] = Q[n];
+                            for (int n = 0; n <= kOrder; ++n) part[g * (kOrder + 1) + n] = Q[n];
+                        }
                     }
                 }
             } else for (int p = 0; p < P.np; ++p) {
@@ -1120,7 +1199,8 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
         if (on)
             for (int dd = 0; dd < nd; ++dd) {
                 const double f = 1.0 / fmax(fabs(a.n_hat[3 * (d0 + dd) + 2]), 1.0e-12);
-                const double v = moments_at(kOrder, f, f_c, dl, [&](int n) { return acc[n][threadIdx.x]; });
+                const double v = exp(-ref_up * f) *
+                                 moments_at(kOrder, f, f_c, dl, [&](int n) { return acc[n][threadIdx.x]; });
                 if (v != 0.0) atomicAdd(&a.spec[(int64_t)(d0 + dd) * a.n_E + e], v);
             }
     } else if constexpr (kForm == kLayGroups) {
@@ -1128,7 +1208,8 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
             for (int dd = 0; dd < nd; ++dd) {
                 const int g = grp.of[dd];
                 const double f = 1.0 / fmax(fabs(a.n_hat[3 * (d0 + dd) + 2]), 1.0e-12);
-                const double v = moments_at(kOrder, f, grp.f_c[g], grp.dl[g],
+                const double v = exp(-(grp.up[g] ? ref_up : ref_dn) * f) *
+                                 moments_at(kOrder, f, grp.f_c[g], grp.dl[g],
                                             [&](int n) { return acc[g * (kOrder + 1) + n][threadIdx.x]; });
                 if (v != 0.0) atomicAdd(&a.spec[(int64_t)(d0 + dd) * a.n_E + e], v);
             }

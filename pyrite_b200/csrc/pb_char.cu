@@ -18,7 +18,8 @@
 // take two each. Only the shells that feed the line are interpolated. The first
 // form kept every direction and line of a segment in one thread, each with its
 // own exponentials, shell sum and warp reduction: 918 us for 200,000 segments, 7
-// lines, 16 directions in a three-layer stack, 158 us now; bound by FP64 issue.
+// lines, 16 directions in a three-layer stack, 184 us now (158 with depths counted
+// from the face, which light from below an absorber does not bear); bound by FP64 issue.
 #include <algorithm>
 #include <cstdint>
 #include <type_traits>
@@ -104,6 +105,29 @@ __global__ void __launch_bounds__(kCharThreads, 2) char_yield_kernel(const pb_ch
     double acc[kCharDirs];
 #pragma unroll
     for (int i = 0; i < kCharDirs; ++i) acc[i] = 0.0;
+    // Optical depth below the exit face that the moments count from, the whole
+    // absorber's at first.
+    double ref = 0.0;
+    for (int k = 0; k < n_k; ++k) ref += mu[k] * (z_bot[k] - z_top[k]);
+    const double above = -(double)moment_above<Real>() / f_c;
+    const auto rebase = [&](double to) {
+        if (acc[0] == 0.0) {  // nothing summed yet
+            ref = to;
+            return;
+        }
+        const double c = -(ref - to) * dl, sc = exp(-(ref - to) * f_c);
+#pragma unroll
+        for (int n = kOrder; n >= 0; --n) {
+            double v = acc[n], t = 1.0;
+#pragma unroll
+            for (int j = n - 1; j >= 0; --j) {
+                t *= c * ((double)(j + 1) / (double)(n - j));
+                v = fma(t, acc[j], v);
+            }
+            acc[n] = sc * v;
+        }
+        ref = to;
+    };
 
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + tid; s < n_seg; s += (int64_t)gridDim.x * blockDim.x) {
         if (!(a.elec_id[s] < a.Ne && (a.seg_layer == nullptr || a.seg_layer[s] == a.emit_layer))) continue;
@@ -161,8 +185,11 @@ __global__ void __launch_bounds__(kCharThreads, 2) char_yield_kernel(const pb_ch
             double t0, t1;
             if (moments) {
                 depths(up[0], t0, t1);
+                const double lo = fmin(t0, t1);
+                if (lo - ref < above) rebase(lo);
                 Real Q[kOrder + 1] = {};
-                add_moments<kOrder>((Real)1, (Real)fmin(t0, t1), (Real)fabs(t1 - t0), (Real)f_c, (Real)dl, Q);
+                add_moments<kOrder>((Real)1, (Real)(lo - ref), (Real)fabs(t1 - t0), (Real)f_c,
+                                    (Real)(f_c * 1.4426950408889634), (Real)dl, Q);
 #pragma unroll
                 for (int n = 0; n <= kOrder; ++n) acc[n] = fma(wp, (double)Q[n], acc[n]);
             } else {
@@ -176,6 +203,15 @@ __global__ void __launch_bounds__(kCharThreads, 2) char_yield_kernel(const pb_ch
                                                                    (up[d] ? u1 : t1) * inv_nz[d]);
             }
         }
+    }
+    if (moments) {  // one reference for the block: its nearest
+        double r = ref;
+        for (int o = 16; o > 0; o >>= 1) r = fmin(r, __shfl_xor_sync(0xffffffffu, r, o));
+        if (lane == 0) red[tid >> 5] = r;
+        __syncthreads();
+        for (int k = 0; k < kCharThreads / 32; ++k) r = fmin(r, red[k]);
+        if (r < ref) rebase(r);
+        __syncthreads();
     }
     // Block sums in thread order, one global add per direction.
     double sum[kCharDirs];
@@ -200,7 +236,7 @@ __global__ void __launch_bounds__(kCharThreads, 2) char_yield_kernel(const pb_ch
                 v = sum[kOrder];
 #pragma unroll
                 for (int n = kOrder; n > 0; --n) v = fma(v, h / (double)n, sum[n - 1]);
-                v /= f;
+                v *= exp(-ref * f) / f;
             }
             if (v != 0.0) atomicAdd(&a.line_yield[(int64_t)(d0 + d) * n_line + line], v);
         }

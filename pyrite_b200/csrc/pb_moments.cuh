@@ -86,18 +86,45 @@ __device__ __forceinline__ void direction_groups(const double *n_hat, int d0, in
 // Direction moments of the segment-mean escape, for the FP64 bremsstrahlung, the
 // layered absorber and the characteristic lines (the mixed single-slab kernels
 // carry packed forms of the same recurrence). The truncation after order N is below
-// rho^(N+1) / sqrt(2 pi (N+1)) of the unattenuated term: FP64 takes N = 5 for
+// rho^(N+1) / sqrt(2 pi (N+1)) of the term without attenuation: FP64 takes N = 5 for
 // rho <= 0.002 and N = 9 for rho <= 0.02 (both below 2e-17), the mixed layered
-// path N = 3 for rho <= 0.01 (2e-9).
+// path N = 3 for rho <= 0.01 (2e-9). Where all light comes from below an absorber
+// that would be much of what is left of it, so depths count from a reference near
+// the shallowest piece (moved by rebase_moments when a piece lies more than
+// kAbove / f_c above it) and each direction is attenuated to there by an
+// exponential of its own. A piece kAbove / f_c above the reference is off by
+// (kAbove rho)^(N+1) / (N+1)! of itself: FP64 2e-16, mixed 7e-9.
 template <class Real>
 constexpr double moment_limit() { return sizeof(Real) == 8 ? 0.02 : 0.01; }
+template <class Real>
+constexpr Real moment_above() { return sizeof(Real) == 8 ? (Real)6 : (Real)2; }
+
+// The moments Q(0) .. Q(N) of depths from a reference ``delta`` (optical depth per
+// unit path factor) nearer the exit face: the sums times exp(-delta f), a factor
+// exp(-delta f_c) and a binomial convolution with the powers of -delta dl.
+template <class F>
+__device__ __forceinline__ void rebase_moments(int N, double delta, double f_c, double dl, F Q) {
+    if (Q(0) == 0.0) return;  // nothing summed yet
+    const double c = -delta * dl, s = exp(-delta * f_c);
+#pragma unroll 1
+    for (int n = N; n >= 0; --n) {
+        double v = Q(n), t = 1.0;
+#pragma unroll 1
+        for (int j = n - 1; j >= 0; --j) {
+            t *= c * (double)(j + 1) / (double)(n - j);
+            v = fma(t, Q(j), v);
+        }
+        Q(n) = s * v;
+    }
+}
 
 // Q_n += w P_n of one affine piece: a = optical depth of its shallower end along
 // the face normal, b = the depth difference of its ends, both per unit path
 // factor. Two exponentials serve every direction of the group, where each
 // direction took two of its own.
 template <int N>
-__device__ __forceinline__ void add_moments(double w, double a, double b, double f_c, double dl, double (&Q)[N + 1]) {
+__device__ __forceinline__ void add_moments(double w, double a, double b, double f_c, double, double dl,
+                                            double (&Q)[N + 1]) {
     const double x = b * f_c;
     const double Ea = exp(-a * f_c), em = -expm1(-x);
     double P = w * Ea * f_c * (x > 1.0e-5 ? em / x : 1.0 - 0.5 * x + x * x / 6.0);
@@ -113,23 +140,34 @@ __device__ __forceinline__ void add_moments(double w, double a, double b, double
         }
     }
 }
+// In float the exponentials are the SFU's, of products with c2 = f_c log2(e) rounded
+// once (the rounding of an optical depth dominates their own 2 ulp), and 1 - e^-x is a series to x = 1,
+// where the difference has lost less than one bit: phi(x) = (1 - e^-x) / x =
+// phi(h) (1 - h phi(h) / 2), h = x / 2, phi(h) to h^8 (truncation 3e-10).
 template <int N>
-__device__ __forceinline__ void add_moments(float w, float a, float b, float f_c, float dl, float (&Q)[N + 1]) {
-    constexpr float kLog2e = 1.44269504f;
+__device__ __forceinline__ void add_moments(float w, float a, float b, float f_c, float c2, float dl,
+                                            float (&Q)[N + 1]) {
     const float x = b * f_c;
-    const float Ea = ex2_approx(-kLog2e * a * f_c);
-    float P, Ec;
-    if (x > 0.35f) {
-        Ec = ex2_approx(-kLog2e * (a + b) * f_c);
-        P = w * (Ea - Ec) * (f_c * rcp_approx(x));
+    const float Ea = ex2_approx(-(a * c2));
+    float em, phi;
+    if (x > 1.0f) {
+        em = 1.0f - ex2_approx(-(b * c2));
+        phi = em * rcp_approx(x);
     } else {
-        // phi(x) = (1 - e^-x) / x to x^7: truncation below 1e-9
-        const float phi = fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, -1.0f / 40320.0f, 1.0f / 5040.0f),
-                                                                              -1.0f / 720.0f), 1.0f / 120.0f),
-                                                       -1.0f / 24.0f), 1.0f / 6.0f), -0.5f), 1.0f);
-        P = w * Ea * f_c * phi;
-        Ec = Ea - Ea * (x * phi);
+        const float h = 0.5f * x;
+        float p = fmaf(h, 1.0f / 362880.0f, -1.0f / 40320.0f);
+        p = fmaf(h, p, 1.0f / 5040.0f);
+        p = fmaf(h, p, -1.0f / 720.0f);
+        p = fmaf(h, p, 1.0f / 120.0f);
+        p = fmaf(h, p, -1.0f / 24.0f);
+        p = fmaf(h, p, 1.0f / 6.0f);
+        p = fmaf(h, p, -0.5f);
+        p = fmaf(h, p, 1.0f);
+        phi = fmaf(-0.5f * h * p, p, p);
+        em = x * phi;
     }
+    const float Ec = Ea - Ea * em;
+    float P = w * Ea * (f_c * phi);
     Q[0] += P;
     if constexpr (N > 0) {
         const float ah = -dl * a, ch = -dl * (a + b);

@@ -1321,12 +1321,15 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
             const int bin = strip * kStripBins + (int)lane;
             const double e_lo = a.edges[min(bin, n_E)];
             const Real e = (Real)e_lo;
+            // from the FP64 edges: float edges, and phases all the more, lose the width
+            // of a narrow bin (6e-8 of the energy, and of the distance from the line)
+            const Real width = (Real)(a.edges[min(bin + 1, n_E)] - e_lo);
             Real acc = 0;
             for (int k = 0; k < nw; ++k) {
                 const WinLine<Real> &l = wLine[wIdx[win_slot(kWinAxis, k)]];
                 const Real x = l.s * (e - l.E_r);
                 const Real x_hi = __shfl_down_sync(0xffffffffu, x, 1);
-                const Real sw = x_hi - x, xc = (Real)0.5 * (x + x_hi);
+                const Real sw = l.s * width, xc = (Real)0.5 * (x + x_hi);
                 // (lane 31 holds the strip's last edge and no bin)
                 const bool narrow = sw <= (Real)0.1 && fabs(xc) >= (Real)2 && lane < kStripBins;
                 const unsigned wide_bins = __ballot_sync(0xffffffffu, !narrow && lane < kStripBins);

@@ -137,8 +137,8 @@ __device__ __forceinline__ void brem_stage(BremSeg<Real> &b, const pb_brem_args 
 struct BremKConst {
     float kc;     // k / (m c^2)^2  [1/keV]
     float c2mk;   // 2 m c^2 - k    [keV]
-    float c0k;    // c0 ln 2 / k_ev
-    double c0k64; // c0 / k_ev (FP64 path)
+    float c0k;    // c0 ln 2 / k, k in eV
+    double c0k64; // c0 / k, k in eV (FP64 path)
 };
 
 // sum_el n_el L dsigma/dk(Z_el, T, k) of one staged segment (brem.py:396-479).
@@ -151,7 +151,7 @@ struct BremKConst {
 // ex2 + rcp per element of the Elwert factor).
 template <class Real, int NEL = 0>
 __device__ __forceinline__ Real brem_nsig(const BremSeg<Real> &b, Real k, Real T_f, const Real *Zs, int n_el_rt,
-                                          Real k_ev, Real c0, Real za, Real mc2, const BremKConst &kk,
+                                          Real za, Real mc2, const BremKConst &kk,
                                           const float *zl) {
     // NEL > 0: the element count known at compile time (loops unrolled).
     const int n_el = NEL > 0 ? NEL : n_el_rt;
@@ -227,14 +227,14 @@ struct BremMomentConst {
 
 template <int N, int NEL>
 __device__ __forceinline__ void brem_moment_chunk(const BremSeg<float> *segs, int nc, bool up, float k,
-                                                  const float *Zs, int n_el, float k_ev, float c0, float za,
+                                                  const float *Zs, int n_el, float za,
                                                   float mc2, const BremKConst &kk, const float *zl,
                                                   const BremMomentConst &m, float (&Q)[N + 1]) {
     for (int j = 0; j < nc; ++j) {
         const BremSeg<float> &b = segs[j];
         const float T_f = b.T - k;
         if (!(T_f > 1e-6f && k > 0.0f)) continue;
-        const float nsig = brem_nsig<float, NEL>(b, k, T_f, Zs, n_el, k_ev, c0, za, mc2, kk, zl);
+        const float nsig = brem_nsig<float, NEL>(b, k, T_f, Zs, n_el, za, mc2, kk, zl);
         const float es = up ? b.e0 : b.e1;
         const float ef = es + b.e2;
         const float Ea = ex2_approx(-m.mu_l2fc * es);
@@ -717,8 +717,6 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
     const double k_kev_d = on ? a.E_grid[e] / 1e3 : 1.0;
     const Real k = (Real)k_kev_d;
     const Real mu = on ? (Real)a.mu[e] : (Real)0;
-    const Real k_ev = fmax((Real)(k_kev_d * 1e3), (Real)1e-30);
-    const Real c0 = (Real)(16.0 / 3.0 * kAlphaFs * kReCm2);
     BremKConst kk;
     kk.kc = (float)(k_kev_d / (510.99895 * 510.99895));
     kk.c2mk = (float)(2.0 * 510.99895 - k_kev_d);
@@ -760,17 +758,17 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
                 const bool up_all = side_all > 0;
                 if (order == 0) {
                     float Q[1] = {0.0f};
-                    brem_moment_chunk<0, NEL>(segs, nc, up_all, k, Zs, n_el, k_ev, c0, za, mc2, kk, zl, m, Q);
+                    brem_moment_chunk<0, NEL>(segs, nc, up_all, k, Zs, n_el, za, mc2, kk, zl, m, Q);
                     for (int dd = 0; dd < nd; ++dd)
                         acc[dd][threadIdx.x] += (double)Q[0] * (double)mom_invf[dd];
                 } else if (order == 3) {
                     float Q[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                    brem_moment_chunk<3, NEL>(segs, nc, up_all, k, Zs, n_el, k_ev, c0, za, mc2, kk, zl, m, Q);
+                    brem_moment_chunk<3, NEL>(segs, nc, up_all, k, Zs, n_el, za, mc2, kk, zl, m, Q);
                     for (int dd = 0; dd < nd; ++dd)
                         acc[dd][threadIdx.x] += (double)brem_moment_eval<3>(Q, mom_h[dd]) * (double)mom_invf[dd];
                 } else {
                     float Q[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-                    brem_moment_chunk<5, NEL>(segs, nc, up_all, k, Zs, n_el, k_ev, c0, za, mc2, kk, zl, m, Q);
+                    brem_moment_chunk<5, NEL>(segs, nc, up_all, k, Zs, n_el, za, mc2, kk, zl, m, Q);
                     for (int dd = 0; dd < nd; ++dd)
                         acc[dd][threadIdx.x] += (double)brem_moment_eval<5>(Q, mom_h[dd]) * (double)mom_invf[dd];
                 }
@@ -790,7 +788,7 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
                     const BremSeg<double> &b = segs[j];
                     const double T_f = b.T - k;
                     if (!(T_f > 1e-6 && k > 0.0)) continue;
-                    const double nsig = brem_nsig<double, NEL>(b, k, T_f, Zs, n_el, k_ev, c0, za, mc2, kk, zl);
+                    const double nsig = brem_nsig<double, NEL>(b, k, T_f, Zs, n_el, za, mc2, kk, zl);
                     const double lo = up_all ? fmin(b.e0, b.e1) : T_slab - fmax(b.e0, b.e1);
                     double a_lo = mu * (lo - z_ref);
                     if (a_lo < above) {
@@ -824,7 +822,7 @@ __global__ void __launch_bounds__(kBremThreads, sizeof(Real) == 4 ? 4 : 2)
             const BremSeg<Real> &b = segs[j];
             const Real T_f = b.T - k;
             if (!(T_f > (Real)1e-6 && k > (Real)0)) continue;
-            const Real nsig = brem_nsig<Real, NEL>(b, k, T_f, Zs, n_el, k_ev, c0, za, mc2, kk, zl);
+            const Real nsig = brem_nsig<Real, NEL>(b, k, T_f, Zs, n_el, za, mc2, kk, zl);
             if constexpr (sizeof(Real) == 8) {
 #pragma unroll
                 for (int dd = 0; dd < kBremMaxDir; ++dd) {
@@ -1008,8 +1006,6 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
     }
     const double k_kev_d = on ? a.E_grid[e] / 1e3 : 1.0;
     const Real k = (Real)k_kev_d;
-    const Real k_ev = fmax((Real)(k_kev_d * 1e3), (Real)1e-30);
-    const Real c0 = (Real)(16.0 / 3.0 * kAlphaFs * kReCm2);
     BremKConst kk;
     kk.kc = (float)(k_kev_d / (510.99895 * 510.99895));
     kk.c2mk = (float)(2.0 * 510.99895 - k_kev_d);
@@ -1126,7 +1122,7 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
             const BremSeg<Real> &b = segs[j];
             const Real T_f = b.T - k;
             if (!(T_f > (Real)1e-6 && k > (Real)0)) continue;
-            const Real nsig = brem_nsig<Real>(b, k, T_f, Zs, n_el, k_ev, c0, za, mc2, kk, zl);
+            const Real nsig = brem_nsig<Real>(b, k, T_f, Zs, n_el, za, mc2, kk, zl);
             const auto &P = pcs[j];
             if constexpr (kForm != kLayDirect) {
                 // The sums of a face move to a reference -a nearer to it.

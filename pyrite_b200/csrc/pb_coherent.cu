@@ -30,6 +30,7 @@
 // by v there.
 #include <cstdint>
 
+#include "pb_common.cuh"
 #include "pb_internal.h"
 
 namespace pb {
@@ -44,29 +45,14 @@ constexpr int64_t kMinChunk = 256;             // lines per work item, lower bou
 constexpr int64_t kTargetItemsTimesTiles = 148 * 3 * 4;  // ~4 waves of 3 CTAs per SM
 constexpr float kSeriesW2 = 1.0e-6f;           // _formation.py:55 FORMATION_SERIES_W2
 
-// Two floats in one register pair, and the packed FP32 arithmetic of sm_100 (one
-// instruction for both halves).
+// A packed pair of floats (pb_common.cuh) as a type of its own.
 struct F2 {
     unsigned long long v;
 };
-__device__ __forceinline__ F2 f2(float lo, float hi) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void f2_get(F2 x, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x.v));
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-    F2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return d;
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-    F2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-    return d;
-}
+__device__ __forceinline__ F2 f2(float lo, float hi) { return F2{f2_pack(lo, hi)}; }
+__device__ __forceinline__ void f2_get(F2 x, float &lo, float &hi) { f2_unpack(x.v, lo, hi); }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { return F2{pb::f2_fma(a.v, b.v, c.v)}; }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { return F2{pb::f2_mul(a.v, b.v)}; }
 
 // One line record as the field loop reads it, phases in turns. ``fast``
 // lines hold the offset forms Gx = 1.5 * 2^29 - g_phase / 2 pi and

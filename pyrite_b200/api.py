@@ -273,7 +273,9 @@ def simulate_trajectories(E0_keV, Ne, thickness_ang=None, element=None, n_atoms_
     """Transport ``Ne`` electrons into a slab or layer stack; returns segment rows.
 
     Same contract as the reference's per-electron cores: rows of history i
-    in order, true ``seg_count``, exit counts, entrance snapshot. ``lut`` picks
+    in order, true ``seg_count``, exit counts, entrance snapshot. The row arrays
+    are views of one host block (98 bytes a row): a caller that keeps one of
+    them for long copies it. ``lut`` picks
     the reference's default LUT core or its exact analytic core; ``rng`` the
     reference's SplitMix64 counter stream (draw-for-draw compatible) or
     Philox4x32-10; ``precision`` "fp64" or "mixed". ``entry`` replaces the
@@ -391,7 +393,8 @@ def simulate_trajectories(E0_keV, Ne, thickness_ang=None, element=None, n_atoms_
             beam_dir, composition, layers, beam_fwhm_mm, beam_fwhm_y_mm, tilt_polar_rad,
             tilt_azim_rad, transverse_distribution, lut=lut, rng=rng, precision=precision,
             entry=entry, cap=int(counts.max()), device=device, stream=stream,
-            block_threads=block_threads, tallies=tallies, straggling=straggling)
+            block_threads=block_threads, tallies=tallies, straggling=straggling,
+            elastic_model=elastic_model, elastic_tables=group, stopping_tables=stop)
     # The rows, packed history after history on the device, in one copy.
     total = int(counts.sum())
     packed, block, parts = _row_block(h, total)

@@ -1148,7 +1148,8 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
                     Real a_up = esc_pick<Real>(c_up, m) + mum * P.u0[p];
                     if (a_up < above_up) {
                         rebase(true, a_up);
-                        a_up = esc_pick<Real>(c_up, m) + mum * P.u0[p];
+                        // (the sum's rounding, far above 1 where no light is left at all)
+                        a_up = fmax(esc_pick<Real>(c_up, m) + mum * P.u0[p], above_up);
                     }
                     if constexpr (kMoments) {
                         add_moments<kOrder>(w, a_up, dep, (Real)f_c, c2, (Real)dl, part);
@@ -1156,7 +1157,7 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
                         Real a_dn = esc_pick<Real>(c_dn, m) + mum * P.u1[p];
                         if (a_dn < above_dn) {
                             rebase(false, a_dn);
-                            a_dn = esc_pick<Real>(c_dn, m) + mum * P.u1[p];
+                            a_dn = fmax(esc_pick<Real>(c_dn, m) + mum * P.u1[p], above_dn);
                         }
 #pragma unroll
                         for (int g = 0; g < kMaxGroups; ++g) {

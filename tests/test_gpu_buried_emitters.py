@@ -139,3 +139,22 @@ def test_characteristic_yields(n_dir, rho, face, order, layered, precision, cuda
         assert ref.min() > 0.0
         tau = mu[:, kept].max(0) * SLAB / abs(nh[2])
         assert np.all(np.abs(got - ref) <= (2e-12 if precision == "fp64" else 1e-5 + 2.4e-7 * tau) * ref)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("f", [[1.0], [1.0, 1.005], [1.0, -1.0, 1.3, -1.4]])
+@pytest.mark.parametrize("scale", [1e3, 1e6, 1e9, 1e12])
+def test_no_light_left(scale, f, precision, cuda_device):
+    """Optical depths far beyond what an exponential of it can hold: zero, as the
+    oracle has it, and not a number that float noise of the depth makes."""
+    fs = np.asarray(f)
+    nz = np.sign(fs) * 0.9 / np.abs(fs)
+    n_hat = np.stack([np.sqrt(1.0 - nz**2), np.zeros(fs.size), nz], 1)
+    seg = _segments(300, 0.3, 0.6, "random", True, False, 8)
+    from pyrite_b200 import mc_brem_spectrum
+
+    E = np.linspace(100.0, 2000.0, 40)
+    mu = np.full((3, E.size), scale * 1e3 / SLAB)
+    got = mc_brem_spectrum(seg, E, composition=LAYERS[1][2], n_hat=n_hat, layers=LAYERS, mu_layer=mu, precision=precision,
+                           device=cuda_device)
+    assert np.all(got == 0.0)

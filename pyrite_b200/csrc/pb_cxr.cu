@@ -1321,9 +1321,11 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
             const int bin = strip * kStripBins + (int)lane;
             const double e_lo = a.edges[min(bin, n_E)];
             const Real e = (Real)e_lo;
-            // from the FP64 edges: float edges, and phases all the more, lose the width
-            // of a narrow bin (6e-8 of the energy, and of the distance from the line)
-            const Real width = (Real)(a.edges[min(bin + 1, n_E)] - e_lo);
+            // The width between the edges as they are held here: a bin's mass divided by
+            // it is right to the rounding of the mass, while by the FP64 width it would
+            // carry that of the float edges (5e-4 of 0.8 eV at 8 keV), and a difference
+            // of phases loses a narrow bin's width far from its line.
+            const Real width = __shfl_down_sync(0xffffffffu, e, 1) - e;
             Real acc = 0;
             for (int k = 0; k < nw; ++k) {
                 const WinLine<Real> &l = wLine[wIdx[win_slot(kWinAxis, k)]];
@@ -1342,8 +1344,7 @@ __global__ void __launch_bounds__(kCxrThreads, kCxrBlocks) cxr_kernel(const pb_c
             }
             if (lane < kStripBins && bin < n_E) {
                 // this warp owns the strip's bins until the phase ends
-                const double inv_w = ax.uniform ? ax.inv_w : 1.0 / (a.edges[bin + 1] - e_lo);
-                spec_s[bin] += (double)acc * inv_w;
+                spec_s[bin] += (double)acc / (double)width;
             }
         }
     };

@@ -1125,20 +1125,29 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
             const Real nsig = brem_nsig<Real>(b, k, T_f, Zs, n_el, za, mc2, kk, zl);
             const auto &P = pcs[j];
             if constexpr (kForm != kLayDirect) {
-                // The sums of a face move to a reference -a nearer to it.
-                const auto rebase = [&](bool upper, Real a) {
+                // The sums of a face move to the optical depth at u in layer m as
+                // their reference, formed in FP64 from the face down: a difference of
+                // the float depths would carry the rounding of the last reference's.
+                const auto rebase = [&](bool upper, int m, Real u) {
 #pragma unroll
                     for (int dd = 0; dd < kPart; ++dd) {
                         acc[dd][threadIdx.x] += (double)part[dd];
                         part[dd] = 0;
                     }
+                    const bool from_top = kMoments ? up_all : upper;
+                    double to = (double)esc_pick<Real>(mu_l, m) * (double)u;
+#pragma unroll
+                    for (int k = 0; k < kMaxEscLayers; ++k)
+                        if (from_top ? k < m : k > m) to += (double)mu_l[k] * (double)t_l[k];
+                    double &ref = kMoments || upper ? ref_up : ref_dn;
                     for (int g = 0; g < (kMoments ? 1 : n_grp); ++g) {
                         if (!kMoments && (grp.up[g] != 0) != upper) continue;
-                        rebase_moments(kOrder, -(double)a, kMoments ? f_c : grp.f_c[g], kMoments ? dl : grp.dl[g],
+                        rebase_moments(kOrder, ref - to, kMoments ? f_c : grp.f_c[g], kMoments ? dl : grp.dl[g],
                                        [&](int n) -> double & { return acc[g * (kOrder + 1) + n][threadIdx.x]; });
                     }
-                    if (kMoments || upper) count_from(!kMoments || up_all, ref_up += (double)a, c_up);
-                    else count_from(false, ref_dn += (double)a, c_dn);
+                    ref = to;
+                    if (kMoments || upper) count_from(from_top, to, c_up);
+                    else count_from(false, to, c_dn);
                 };
                 for (int p = 0; p < P.np; ++p) {
                     const int m = P.m[p];
@@ -1147,8 +1156,8 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
                     // the piece end nearer the exit face
                     Real a_up = esc_pick<Real>(c_up, m) + mum * P.u0[p];
                     if (a_up < above_up) {
-                        rebase(true, a_up);
-                        // (the sum's rounding, far above 1 where no light is left at all)
+                        rebase(true, m, P.u0[p]);
+                        // (the rounding of the sum is above 1 only where no light is left)
                         a_up = fmax(esc_pick<Real>(c_up, m) + mum * P.u0[p], above_up);
                     }
                     if constexpr (kMoments) {
@@ -1156,7 +1165,7 @@ __global__ void __launch_bounds__(kBremThreads) brem_layered_kernel(const pb_bre
                     } else {
                         Real a_dn = esc_pick<Real>(c_dn, m) + mum * P.u1[p];
                         if (a_dn < above_dn) {
-                            rebase(false, a_dn);
+                            rebase(false, m, P.u1[p]);
                             a_dn = fmax(esc_pick<Real>(c_dn, m) + mum * P.u1[p], above_dn);
                         }
 #pragma unroll

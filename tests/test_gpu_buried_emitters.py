@@ -158,3 +158,34 @@ def test_no_light_left(scale, f, precision, cuda_device):
     got = mc_brem_spectrum(seg, E, composition=LAYERS[1][2], n_hat=n_hat, layers=LAYERS, mu_layer=mu, precision=precision,
                            device=cuda_device)
     assert np.all(got == 0.0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("f", [[450.0], [450.0, 1300.0], [3.0, -3.0, 450.0, -1300.0]])
+@pytest.mark.parametrize("tau", [1.0, 1e3, 1e5, 1e7])
+def test_segments_through_both_faces_of_an_opaque_stack(tau, f, precision, cuda_device):
+    """Each segment runs from face to face, so a direction sees its end on the
+    exit face whatever the optical depth below: FP64 2e-12 of a value, mixed 4e-6
+    (the float cross section, depth ratio and exponential, a few 1e-7 each)."""
+    from pyrite_b200 import mc_brem_spectrum
+
+    rng = np.random.default_rng(1)
+    fs = np.asarray(f)
+    nz = np.sign(fs) / np.abs(fs)
+    n_hat = np.stack([np.sqrt(1.0 - nz**2), np.zeros(fs.size), nz], 1)
+    n = 40
+    v = np.tile([np.sqrt(0.75), 0.0, 0.5], (n, 1))
+    L = np.full(n, 2.0 * SLAB)
+    r = np.stack([np.zeros(n), np.zeros(n), np.full(n, 0.5 * SLAB)], 1)
+    seg = dict(v_hat=v, E_repr_keV=50.0 + 1000.0 * rng.random(n), L_ang=L, r_mid=r, elec_id=np.arange(n), Ne=n, thickness_ang=SLAB)
+    E = np.linspace(1000.0, 40000.0, 60)
+    comp = LAYERS[2][2]
+    top, bot = np.array([l[0] for l in LAYERS]), np.array([l[1] for l in LAYERS])
+    mu = np.stack([np.geomspace(tau, 0.1 * tau, E.size) / SLAB * k for k in (1.0, 0.7, 1.4)])
+    got = np.atleast_2d(mc_brem_spectrum(seg, E, composition=comp, n_hat=n_hat, layers=LAYERS, mu_layer=mu,
+                                         precision=precision, device=cuda_device))
+    for g, nh in zip(got, n_hat):
+        ref = oracle.brem_spectrum_layered(_oseg(seg), [Z[e] for e, _ in comp], [x for _, x in comp],
+                                           oracle.LayerEscape(top, bot), nh, E, mu, seg["Ne"])
+        assert ref.min() > 0.0
+        assert np.all(np.abs(g - ref) <= (2e-12 if precision == "fp64" else 4e-6) * ref)

@@ -919,8 +919,8 @@ constexpr int kBremChunkLayered = 64;
 // along the surface: its rows of tiles, on both faces) through four sets of them
 // (kLayGroups); the others are scored one by one, two exponentials each. The three
 // layers of the 10 MeV stack (160,000 segments, 4096 energies, 64 directions, mixed):
-// 478 ms per (segment, energy, direction), 28 with three detectors in the moments
-// (15 of them) and the fourth, at 90 degrees, in four groups (13); bound by issue and
+// 478 ms per (segment, energy, direction), 30 with three detectors in the moments
+// (17 of them) and the fourth, at 90 degrees, in four groups (13); bound by issue and
 // the SFU. (22 without a reference that moves with the shallowest piece and with
 // coarser exponentials: light from below an absorber was then off by up to 5e-3 of
 // itself, now 4e-6.)

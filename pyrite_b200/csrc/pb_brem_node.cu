@@ -187,12 +187,13 @@ __constant__ const ChebMonomials kCheb = cheb_monomials();
 // priced at n_E evaluations of the per-pair form and as much again for its
 // place in the list: above kNodePairWork the quarter octaves clear of the
 // spectrum's tip become one window each. 200,000 electrons of 8 keV to 10 MeV
-// on 2,048 energies, 59 % of them in 24 windows: per-pair form 958 -> 490 us
-// (340 on the ordered list); fit, list, moments and contraction of the windows
-// 145 us, against 141 us for
-// a list of nearly every segment that the one window then gave up. At 300
-// energies a list of 40,000 takes 324 us through the entry point, 436 before;
-// below the line the two are within 10 us.
+// on 2,048 energies: 58 % of them lie in 24 windows, of which the three from 2,048,
+// 4,096 and 8,192 keV (1.25 wide, the first quarter of an octave) miss the fit's
+// 1e-7 by up to 2.8 times at 1 keV, so 49 % are scored in 21; per-pair form 958 ->
+// 490 us (340 on the ordered list); fit, list, moments and contraction of the
+// windows 145 us, against 141 us for a list of nearly every segment that the one
+// window then gave up. At 300 energies a list of 40,000 takes 324 us through the
+// entry point, 436 before; below the line the two are within 10 us.
 constexpr double kNodePairWork = 16777216.0;
 
 __global__ void __launch_bounds__(kNodeThreads) brem_node_setup_kernel(const pb_brem_args a, BremNodeHdr *h,
@@ -384,8 +385,8 @@ __device__ __forceinline__ void node_window_offsets(const BremNodeHdr *h, int n_
 
 // Segment list by window, the left-out part by sixteenths of an octave (its
 // chunks then span little energy, which the per-pair kernel's cubic and its
-// test against the photon energy need: 490 -> 340 us for 82,000 electrons of 8 to
-// 160 keV on 2,048 energies to 60 keV): each block counts a tile's segments per
+// test against the photon energy need: 490 -> 340 us for 84,000 electrons of 8 to
+// 160 keV and 18,000 of windows given up, 2,048 energies to 60 keV): each block counts a tile's segments per
 // place in shared memory, reserves them with one atomic a place and writes them.
 constexpr int kListPer = 4;  // segments per thread and tile
 constexpr int kListPlaces = kNodeBins + 1 + kNodeMaxWin;  // bins, outside of them, windows
